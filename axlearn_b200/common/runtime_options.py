@@ -33,7 +33,6 @@ OVERRIDE_ENV = "AXB200_RUNTIME_OPTIONS_OVERRIDE"
 # options.
 KNOBS: dict[str, tuple[str, str]] = {
     "AXB200_GEMM": ("2cta", "2cta: CTA-pair 256x256 tiles where the shape allows; 1cta: single-CTA kernels only."),
-    "AXB_GEMM_SKINNY": ("2", "GEMMs of one row block: 0 general tiles, 1 64-column tiles, 2 64-column tiles and split-K."),
     "AXB_GEMM2_GROUP_M": ("", "Row blocks per raster group of the CTA-pair GEMM (empty: per-mode default)."),
     "AXB200_FLASH_FWD": ("v3", "Flash-attention forward kernel: v3 (scores in registers), v2 or v1."),
     "AXB200_FLASH_BWD": ("fused", "Flash-attention backward: fused (one kernel, 5 GEMMs) or split (dK/dV + dQ kernels)."),

@@ -46,12 +46,6 @@ struct GemmParams {
   int64_t ldc;
   int* status;
   int accumulate;  // C += A*B (read-modify-write in the epilogue)
-  // Split-K (skinny problems): `split_k` CTAs share one output tile, each over a slice of the
-  // k-blocks; fp32 partials go to `ws [split_k, M, N]` and the CTA that arrives last on
-  // `counters[tile]` sums them into C (and leaves the counter at zero for the next launch).
-  int split_k;
-  float* ws;
-  int* counters;
   // Grouped problems (mixture-of-experts), rows sorted by group and every group padded to whole
   // blocks of `group_block_rows` rows (a multiple of 128).  Mode 1: the rows of block b use B
   // matrix number `group_index[b]` (-1 = unused block, skipped); the B tensor map stacks the groups along its outer dim, `b_group_rows`
@@ -92,18 +86,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int n_blocks = (p.N + BN - 1) / BN;
   const int num_tiles = m_blocks * n_blocks;
   const int num_kb = (p.K + kBlockK - 1) / kBlockK;
-  const int split = (!FUSED && p.split_k > 1) ? p.split_k : 1;
   const int gmode = FUSED ? 0 : p.group_mode;
-  // item = (k slice or group, tile); the slices / groups of a tile run as separate items.
-  const int num_items = num_tiles * (gmode == 2 ? p.num_groups : split);
+  // item = (group, tile); the groups of a tile run as separate items.
+  const int num_items = num_tiles * (gmode == 2 ? p.num_groups : 1);
   // k-block range of an item.
   auto kb_range = [&](int ks, int& kb_lo, int& kb_hi) {
     if (gmode == 2) {
       kb_lo = p.group_index[ks] / kBlockK;
       kb_hi = p.group_index[ks + 1] / kBlockK;
     } else {
-      kb_lo = ks * num_kb / split;
-      kb_hi = (ks + 1) * num_kb / split;
+      kb_lo = 0;
+      kb_hi = num_kb;
     }
   };
 
@@ -329,110 +322,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
         crow += static_cast<int64_t>(ks) * p.c_group_stride;
         empty_group = p.group_index[ks] / kBlockK == p.group_index[ks + 1] / kBlockK;
       }
-      if (split > 1) {
-        // Split-K: park the fp32 partial, then the last of the tile's `split` CTAs reduces.
-        // (N is a multiple of 32 here, so a 32-column chunk is entirely inside or outside.)
-        float* wrow = p.ws + (static_cast<int64_t>(ks) * p.M + row) * p.N + n0;
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c, r);
-          tmem_ld_wait();
-          if (c + 32 >= BN) {
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-          }
-          if (row < p.M && n0 + c < p.N) {
-#pragma unroll
-            for (int v = 0; v < 8; ++v)
-              __stcg(reinterpret_cast<uint4*>(wrow + c + 4 * v),
-                     make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]));
-          }
-        }
-        __threadfence();
-        int* last_flag = reinterpret_cast<int*>(bar_base + 512);
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (warp == 2 && lane == 0) {
-          const int prev = atomicAdd(&p.counters[tile], 1);
-          if (prev == split - 1) p.counters[tile] = 0;
-          *last_flag = prev == split - 1;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const bool is_last = *last_flag != 0;
-        if (is_last) {
-          __threadfence();
-          // The 128 epilogue threads sum the tile's partials with coalesced 16-byte accesses,
-          // two vectors per thread and round so that 2 * split loads are in flight at once.
-          const int m0 = m_blk * kBlockM;
-          const int rows_valid = min(kBlockM, p.M - m0);
-          const int vec_per_row = min(BN, p.N - n0) / 4;
-          const int total_vec = rows_valid * vec_per_row;
-          const int et = (warp - 2) * 32 + lane;
-          const int64_t slice = static_cast<int64_t>(p.M) * p.N;
-          for (int idx = et; idx < total_vec; idx += 256) {
-            float4 part[2][8];
-            int64_t off[2];
-            bool on[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int i = idx + u * 128;
-              on[u] = i < total_vec;
-              const int r = on[u] ? i / vec_per_row : 0;
-              const int c4 = on[u] ? i - r * vec_per_row : 0;
-              off[u] = static_cast<int64_t>(m0 + r) * p.N + n0 + c4 * 4;
-#pragma unroll
-              for (int sidx = 0; sidx < 8; ++sidx) {
-                part[u][sidx] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (on[u] && sidx < split)
-                  part[u][sidx] = __ldcg(reinterpret_cast<const float4*>(p.ws + sidx * slice + off[u]));
-              }
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              if (!on[u]) continue;
-              float4 sum = part[u][0];
-#pragma unroll
-              for (int sidx = 1; sidx < 8; ++sidx) {
-                sum.x += part[u][sidx].x;
-                sum.y += part[u][sidx].y;
-                sum.z += part[u][sidx].z;
-                sum.w += part[u][sidx].w;
-              }
-              const int i = idx + u * 128;
-              const int r = i / vec_per_row;
-              const int c4 = i - r * vec_per_row;
-              OutT* dst = C + static_cast<int64_t>(m0 + r) * p.ldc + n0 + c4 * 4;
-              if constexpr (sizeof(OutT) == 2) {
-                if (p.accumulate) {
-                  const uint2 old = *reinterpret_cast<const uint2*>(dst);
-                  sum.x += __uint_as_float(old.x << 16);
-                  sum.y += __uint_as_float(old.x & 0xffff0000u);
-                  sum.z += __uint_as_float(old.y << 16);
-                  sum.w += __uint_as_float(old.y & 0xffff0000u);
-                }
-                *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(sum.x, sum.y), pack_bf16x2(sum.z, sum.w));
-              } else {
-                if (p.accumulate) {
-                  const float4 old = *reinterpret_cast<const float4*>(dst);
-                  sum.x += old.x;
-                  sum.y += old.y;
-                  sum.z += old.z;
-                  sum.w += old.w;
-                }
-                *reinterpret_cast<float4*>(dst) = sum;
-              }
-            }
-          }
-        }
-        // `last_flag` is rewritten by the next item: everyone must have read it first.
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (++acc == 2) {
-          acc = 0;
-          acc_phase ^= 1;
-        }
-        continue;
-      }
       const int n_dst = (FUSED && f.rs_world > 1 && f.rs_mode == 1) ? f.rs_world : 1;
       if (FUSED && f.rs_world > 1 && f.rs_mode == 0 && row < p.M) {
         // Reduce-scatter epilogue: this row goes to its owner's staging slot for this rank
@@ -543,9 +432,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
 template <int BN, int STAGES, bool A_MN, bool B_MN, typename OutT, bool FUSED = false>
 static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda,
                        int64_t ldb, int64_t ldc, int accumulate, int* status, int max_ctas,
-                       cudaStream_t stream, const FusedParams* fused = nullptr, int split_k = 1,
-                       float* ws = nullptr, int* counters = nullptr, int group_mode = 0,
-                       int num_groups = 1, const int* group_index = nullptr,
+                       cudaStream_t stream, const FusedParams* fused = nullptr, int group_mode = 0, int num_groups = 1, const int* group_index = nullptr,
                        int64_t c_group_stride = 0, int group_block_rows = kBlockM) {
   // Grouped mode 1 stacks the groups' B matrices along the outer dim of one tensor map.
   const uint64_t b_stack = group_mode == 1 ? static_cast<uint64_t>(num_groups) : 1;
@@ -615,14 +502,13 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   }
   const int m_blocks = (M + kBlockM - 1) / kBlockM;
   const int n_blocks = (N + BN - 1) / BN;
-  int grid = m_blocks * n_blocks * (group_mode == 2 ? num_groups : (split_k > 1 ? split_k : 1));
+  int grid = m_blocks * n_blocks * (group_mode == 2 ? num_groups : 1);
   int cap = max_ctas > 0 && max_ctas < sm_count() ? max_ctas : sm_count();
   // All CTAs must be co-resident (one per SM): tiles may wait on flags that every CTA's copy
   // warp contributes to.
   if (grid > cap) grid = cap;
   if (grid < 1) return -12;
-  GemmParams p{M, N, K, C, ldc, status, accumulate, split_k, ws, counters,
-               group_mode, num_groups, group_index, B_MN ? K : N, c_group_stride, group_block_rows};
+  GemmParams p{M, N, K, C, ldc, status, accumulate, group_mode, num_groups, group_index, B_MN ? K : N, c_group_stride, group_block_rows};
   kernel<<<grid, FUSED ? kFusedThreads : kNumThreads, kSmem, stream>>>(ta, tb, tl, p, fp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -632,29 +518,14 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   return 0;
 }
 
-// AXB_GEMM_SKINNY selects the treatment of skinny problems (one row block): 0 = the general tiles,
-// 1 = 64-column tiles, 2 (default) = 64-column tiles and split-K.
-static int skinny_mode() {
-  static int mode = -1;
-  if (mode < 0) {
-    const char* e = getenv("AXB_GEMM_SKINNY");
-    mode = (e != nullptr && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 2;
-  }
-  return mode;
-}
-
 template <bool A_MN, bool B_MN, typename OutT>
 static int dispatch_bn(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda,
                        int64_t ldb, int64_t ldc, int accumulate, int* status, int max_ctas,
                        cudaStream_t stream) {
-  // 128x256 tiles when they fill the machine, 128x128 otherwise (more CTAs for small problems),
-  // and 128x64 for skinny decode-time GEMMs (M <= 128), which are weight-streaming problems: the
-  // more CTAs pull weight columns concurrently, the closer they get to the HBM rate.
+  // 128x256 tiles when they fill the machine, 128x128 otherwise (more CTAs for small problems).
+  // Problems of at most 128 rows are weight-streaming problems: gemm_skinny.cu.
   const int m_blocks = (M + kBlockM - 1) / kBlockM;
   const int tiles256 = m_blocks * ((N + 255) / 256);
-  if (m_blocks == 1 && (N + 127) / 128 < sm_count() / 2 && skinny_mode() >= 1)
-    return launch_gemm<64, 8, A_MN, B_MN, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate, status,
-                                                max_ctas, stream);
   if (N >= 256 && tiles256 >= sm_count() / 2)
     return launch_gemm<256, 4, A_MN, B_MN, OutT>(A, B, C, M, N, K, lda, ldb, ldc, accumulate,
                                                   status, max_ctas, stream);
@@ -662,60 +533,7 @@ static int dispatch_bn(const void* A, const void* B, void* C, int M, int N, int 
                                                 max_ctas, stream);
 }
 
-// Split-K plan for a skinny problem (one row block): how many CTAs share an output tile so that
-// the weight stream is pulled by (nearly) every SM.  1 = no split.
-static int splitk_plan(int M, int N, int K) {
-  if (M > kBlockM || (N % 32) != 0 || skinny_mode() < 2) return 1;
-  const int tiles = (N + 63) / 64;
-  const int num_kb = (K + kBlockK - 1) / kBlockK;
-  if ((N + 127) / 128 >= sm_count() / 2) return 1;
-  int split = sm_count() / tiles;
-  if (split > num_kb / 4) split = num_kb / 4;  // at least four k-blocks per slice
-  if (split > 8) split = 8;
-  // The hand-over (fence, counter, reduction by the last CTA) costs about as much as two dozen
-  // k-blocks of streaming: split only when it takes more than that off every CTA's loop.
-  if (split < 2 || num_kb - num_kb / split < 24) return 1;
-  return split;
-}
-
 }  // namespace axb
-
-extern "C" int axb_gemm_splitk_plan(int M, int N, int K) { return axb::splitk_plan(M, N, K); }
-
-// Skinny GEMM (M <= 128, N a multiple of 32) with split-K: `ws` holds split * M * N floats and
-// `counters` ceil(N / 64) ints that are zero on entry (the kernel leaves them zero).  The caller
-// owns both and must not share them between launches that may overlap in time.
-extern "C" int axb_gemm_bf16_splitk(const void* A, const void* B, void* C, int M, int N, int K,
-                                    int64_t lda, int64_t ldb, int64_t ldc, int a_mn_major,
-                                    int b_mn_major, int out_fp32, int accumulate, int split,
-                                    void* ws, void* counters, int* status, int max_ctas,
-                                    cudaStream_t stream) {
-  using namespace axb;
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
-      (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(C) & 15) ||
-      (ldc % (out_fp32 ? 4 : 8)) || (reinterpret_cast<uintptr_t>(ws) & 15))
-    return -10;
-  if (M > kBlockM || (N % 32) || split < 2 || split > (K + kBlockK - 1) / kBlockK || ws == nullptr ||
-      counters == nullptr)
-    return -15;
-#define AXB_SPLITK_CASE(AM, BM)                                                                    \
-  if (a_mn_major == (AM ? 1 : 0) && b_mn_major == (BM ? 1 : 0)) {                                  \
-    if (out_fp32)                                                                                  \
-      return launch_gemm<64, 8, AM, BM, float>(A, B, C, M, N, K, lda, ldb, ldc, accumulate,       \
-                                               status, max_ctas, stream, nullptr, split,          \
-                                               static_cast<float*>(ws), static_cast<int*>(counters)); \
-    return launch_gemm<64, 8, AM, BM, __nv_bfloat16>(A, B, C, M, N, K, lda, ldb, ldc, accumulate,  \
-                                                     status, max_ctas, stream, nullptr, split,     \
-                                                     static_cast<float*>(ws), static_cast<int*>(counters)); \
-  }
-  AXB_SPLITK_CASE(false, false)
-  AXB_SPLITK_CASE(false, true)
-  AXB_SPLITK_CASE(true, false)
-  AXB_SPLITK_CASE(true, true)
-#undef AXB_SPLITK_CASE
-  return -11;
-}
 
 // AXB200_GEMM=1cta keeps every problem on the single-CTA kernels (for comparisons).
 static bool cta_pairs_enabled() {
@@ -768,11 +586,9 @@ extern "C" int axb_gemm_bf16_grouped(const void* A, const void* B, void* C, int 
   if (a_mn_major == (AM ? 1 : 0) && b_mn_major == (BM ? 1 : 0) && out_fp32 == (sizeof(T) == 4)) { \
     if (N >= 256)                                                                                  \
       return launch_gemm<256, 4, AM, BM, T>(A, B, C, M, N, K, lda, ldb, ldc, 0, status, max_ctas,  \
-                                            stream, nullptr, 1, nullptr, nullptr, mode,           \
-                                            num_groups, group_index, c_group_stride, block_rows);  \
+                                            stream, nullptr, mode, num_groups, group_index, c_group_stride, block_rows);  \
     return launch_gemm<128, 6, AM, BM, T>(A, B, C, M, N, K, lda, ldb, ldc, 0, status, max_ctas,    \
-                                          stream, nullptr, 1, nullptr, nullptr, mode, num_groups, \
-                                          group_index, c_group_stride, block_rows);                \
+                                          stream, nullptr, mode, num_groups, group_index, c_group_stride, block_rows);                \
   }
   AXB_GROUPED_CASE(false, false, __nv_bfloat16)
   AXB_GROUPED_CASE(false, true, __nv_bfloat16)

@@ -81,8 +81,8 @@ class _Sigs:
                           c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
     axb_gemm_splitk_plan = [c_int, c_int, c_int]
     axb_multimem_allreduce = [ctypes.c_uint64, c_int64, c_int, c_int, c_void_p]
-    axb_gemm_bf16_splitk = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64,
-                            c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
+    axb_gemm_skinny = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64,
+                       c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     axb_rmsnorm_fwd = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_float, c_void_p]
     axb_rmsnorm_bwd_ctas = [c_int64]
     axb_rmsnorm_fast_supported = [c_int]
@@ -186,31 +186,6 @@ def _operand(t: torch.Tensor, contraction_dim: int) -> tuple[torch.Tensor, int, 
     return t, u[0], u[1]
 
 
-_splitk_plans: dict[tuple, int] = {}
-_splitk_ws: dict[tuple, tuple[torch.Tensor, torch.Tensor]] = {}
-
-
-def _splitk_plan(m: int, n: int, k: int) -> int:
-    key = (m > 0, n, k)
-    if key not in _splitk_plans:
-        _splitk_plans[key] = lib().axb_gemm_splitk_plan(m, n, k)
-    return _splitk_plans[key]
-
-
-def _splitk_workspace(device: torch.device, floats: int) -> tuple[torch.Tensor, torch.Tensor]:
-    """fp32 partials + tile counters of the split-K skinny GEMM, one pair per (device, stream):
-    launches on one stream are ordered, so they can share it.  (Allocated through torch, so a
-    first use during CUDA-graph capture lands in the graph's pool.)"""
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream())
-    have = _splitk_ws.get(key)
-    if have is None or have[0].numel() < floats:
-        ws = torch.empty(max(floats, 1 << 21), dtype=torch.float32, device=device)
-        counters = have[1] if have is not None else torch.zeros(4096, dtype=torch.int32, device=device)
-        have = (ws, counters)
-        _splitk_ws[key] = have
-    return have
-
-
 def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None,
          out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False,
          max_ctas: int = 0) -> torch.Tensor:
@@ -231,15 +206,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None
         return out if accumulate else out.zero_()
     if max_ctas == 0 and COMM_RESERVED_SMS:
         max_ctas = max(8, _sm_count(a.device) - COMM_RESERVED_SMS)
-    if m <= 128 and n % 32 == 0:
-        split = _splitk_plan(m, n, k)
-        if split > 1:
-            ws, counters = _splitk_workspace(a.device, split * m * n)
-            rc = lib().axb_gemm_bf16_splitk(
-                a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, lda, ldb, out.stride(0), a_mn, b_mn,
-                1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0, split, ws.data_ptr(),
-                counters.data_ptr(), status_word(a.device).data_ptr(), max_ctas, _stream())
-            _check(rc, "axb_gemm_bf16_splitk")
+    if m <= 128:
+        # Decoding steps, short prompts: the weight-streaming kernel.  Its CTAs are short and none waits for a
+        # peer, so the cap that keeps persistent CTAs resident beside communication kernels does not concern it.
+        rc = lib().axb_gemm_skinny(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, lda, ldb, out.stride(0),
+                                   a_mn, b_mn, 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0, 0,
+                                   status_word(a.device).data_ptr(), _stream())
+        if rc != -20:
+            _check(rc, "axb_gemm_skinny")
             return out
     if GEMM_VARIANT == "2cta" and m >= 512 and n >= 256 and ((m + 255) // 256) * ((n + 255) // 256) >= 64:
         # Large problems: CTA pairs on 256 x 256 tiles.

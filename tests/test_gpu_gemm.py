@@ -103,6 +103,29 @@ def test_skinny_gemm_split_k(m, n, k, b_t):
         assert cuda_ops.lib().axb_gemm_splitk_plan(m, n, k) > 1
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize("n,k", [(8, 64), (136, 72), (1000, 8), (4096, 640), (18952, 128), (37896, 64)])
+@pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, True)])
+def test_skinny_gemm_edges(m, n, k, a_t, b_t):
+    """Row counts at the edges of the tiles, feature and K remainders, one wave of wide CTAs and one more; every
+    split gives the same sums.  fp32 sums of K bf16 products: the error is a few K * 2^-24 of sum |a b|."""
+    from axlearn_b200.ops import cuda_ops
+
+    torch.manual_seed(3)
+    pad = (m + 7) // 8 * 8
+    a = torch.randn(k, pad, device="cuda").bfloat16()[:, :m].t() if a_t else torch.randn(m, k, device="cuda").bfloat16()
+    b = torch.randn(n, k, device="cuda").bfloat16().t() if b_t else torch.randn(k, n, device="cuda").bfloat16()
+    ref = a.double() @ b.double()
+    bound = 4 * k * 2.0 ** -24 * (a.double().abs() @ b.double().abs()) + 1e-30
+    out = cuda_ops.gemm(a, b, out_dtype=torch.float32)
+    assert ((out.double() - ref).abs() <= bound).all()
+    base = torch.randn(m, n, device="cuda")
+    acc = base.clone()
+    cuda_ops.gemm(a, b, out=acc, accumulate=True)
+    assert ((acc.double() - ref - base.double()).abs() <= bound + 2.0 ** -22 * (ref.abs() + base.abs())).all()
+    cuda_ops.check_status()
+
+
 def _close_elementwise(out, ref, atol, rtol):
     """Per-element ``|out - ref| <= atol + rtol * |ref|`` (an error confined to small outputs or one
     tile edge cannot hide behind the largest value)."""
