@@ -281,4 +281,4 @@ class PaddedEmbedding(Embedding):
 
     def attend(self, x: Tensor) -> Tensor:
         w = self.parameters["weight"]
-        return ops.linear_f32(x, w.to(x.dtype).t())[..., :self._config.num_embeddings]
+        return ops.linear_f32(x, w.to(x.dtype).t(), resident=w.dtype == x.dtype)[..., :self._config.num_embeddings]

@@ -52,7 +52,8 @@ class PaddedLinear(BaseLayer):
             fan_axes=FanAxes(in_axis=-1, out_axis=-2))}
 
     def forward(self, x: Tensor) -> Tensor:
-        return ops.linear(x, self.parameters["weight"].to(x.dtype).t())
+        w = self.parameters["weight"]
+        return ops.linear(x, w.to(x.dtype).t(), resident=w.dtype == x.dtype)
 
 
 _side_streams: dict = {}

@@ -30,6 +30,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "chain.cuh"
+
 namespace axb {
 
 constexpr int kHeadDim = 128;
@@ -64,6 +66,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
 template <int GT>
 __global__ void __launch_bounds__(kDecodeThreads, GT == 1 ? 8 : 1)
 decode_attn_kernel(DecodeParams p) {
+  chain_link();
   const int split = blockIdx.x;
   const int groups_per_kv = (p.num_q_heads / p.num_kv_heads) / GT;
   const int kvh = blockIdx.y / groups_per_kv;
@@ -208,6 +211,7 @@ decode_attn_kernel(DecodeParams p) {
 template <int GT>
 __global__ void __launch_bounds__(kDecodeThreads)
 decode_attn_rows_kernel(DecodeParams p) {
+  chain_link();
   const int split = blockIdx.x;
   const int hg = blockIdx.y;  // group of four KV heads
   const int b = blockIdx.z;
@@ -344,6 +348,7 @@ decode_attn_rows_kernel(DecodeParams p) {
 __global__ void __launch_bounds__(kHeadDim)
 decode_combine_kernel(const float* __restrict__ part_out, const float* __restrict__ part_ml,
                       __nv_bfloat16* __restrict__ out, int splits) {
+  chain_link();
   const int64_t row = blockIdx.x;  // b * Nq + head
   const int d = threadIdx.x;
   float mm = -INFINITY;
@@ -365,6 +370,7 @@ rope_append_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restr
                    __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool,
                    const int* __restrict__ page_table, const int* __restrict__ lengths, int num_q_heads,
                    int num_kv_heads, int page_size, int max_pages, float log2_theta, int apply_rope) {
+  chain_link();
   const int b = blockIdx.y;
   const int head = blockIdx.x;  // 0..Nq+2Nkv-1
   const int i = threadIdx.x;
@@ -446,9 +452,9 @@ extern "C" int axb_decode_attn(const void* q, const void* k_pool, const void* v_
   const bool few_row_ctas = static_cast<int64_t>(B) * (num_kv_heads / 4) <= 8;
   if (rows_ok && num_kv_heads % 4 == 0 && g == 4 && !few_row_ctas) {
     dim3 rgrid(splits, num_kv_heads / 4, B);
-    decode_attn_rows_kernel<4><<<rgrid, kDecodeThreads, 0, stream>>>(p);
+    launch_chained(decode_attn_rows_kernel<4>, rgrid, kDecodeThreads, 0, stream, p);
     if (splits > 1)
-      decode_combine_kernel<<<B * num_q_heads, kHeadDim, 0, stream>>>(p.part_out, p.part_ml, p.out, splits);
+      launch_chained(decode_combine_kernel, B * num_q_heads, kHeadDim, 0, stream, p.part_out, p.part_ml, p.out, splits);
     return cudaGetLastError() == cudaSuccess ? 0 : -4;
   }
   int gt = (g % 4 == 0) ? 4 : (g % 2 == 0) ? 2 : 1;
@@ -456,13 +462,13 @@ extern "C" int axb_decode_attn(const void* q, const void* k_pool, const void* v_
   if (gt > gt_cap) gt = gt_cap;
   dim3 grid(splits, num_kv_heads * (g / gt), B);
   if (gt == 4)
-    decode_attn_kernel<4><<<grid, kDecodeThreads, 0, stream>>>(p);
+    launch_chained(decode_attn_kernel<4>, grid, kDecodeThreads, 0, stream, p);
   else if (gt == 2)
-    decode_attn_kernel<2><<<grid, kDecodeThreads, 0, stream>>>(p);
+    launch_chained(decode_attn_kernel<2>, grid, kDecodeThreads, 0, stream, p);
   else
-    decode_attn_kernel<1><<<grid, kDecodeThreads, 0, stream>>>(p);
+    launch_chained(decode_attn_kernel<1>, grid, kDecodeThreads, 0, stream, p);
   if (splits > 1)
-    decode_combine_kernel<<<B * num_q_heads, kHeadDim, 0, stream>>>(p.part_out, p.part_ml, p.out, splits);
+    launch_chained(decode_combine_kernel, B * num_q_heads, kHeadDim, 0, stream, p.part_out, p.part_ml, p.out, splits);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -474,8 +480,7 @@ extern "C" int axb_rope_append_paged(const void* qkv, void* q_out, void* k_pool,
   if (head_dim != kHeadDim) return -10;
   if (B <= 0) return 0;
   dim3 grid(num_q_heads + 2 * num_kv_heads, B);
-  rope_append_kernel<<<grid, kHeadDim / 2, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out),
+  launch_chained(rope_append_kernel, grid, kHeadDim / 2, 0, stream, static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out),
       static_cast<__nv_bfloat16*>(k_pool), static_cast<__nv_bfloat16*>(v_pool), page_table, lengths,
       num_q_heads, num_kv_heads, page_size, max_pages, log2f(theta), apply_rope);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
@@ -486,6 +491,7 @@ namespace axb {
 // out[r, c] = silu(gu[r, c]) * gu[r, F + c] for gu = [rows, 2F] (gate | up packed by one GEMM).
 __global__ void swiglu_packed_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                      int64_t rows, int F) {
+  chain_link();
   const int64_t total = rows * (F / 2);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -507,7 +513,6 @@ extern "C" int axb_swiglu_packed(const void* gu, void* out, int64_t rows, int F,
   if (total <= 0) return 0;
   int64_t ctas = (total + 255) / 256;
   if (ctas > 148 * 8) ctas = 148 * 8;
-  axb::swiglu_packed_kernel<<<static_cast<int>(ctas), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), rows, F);
+  axb::launch_chained(axb::swiglu_packed_kernel, static_cast<int>(ctas), 256, 0, stream, static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), rows, F);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

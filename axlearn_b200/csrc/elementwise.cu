@@ -7,6 +7,7 @@
 // 374-417 (RMSNorm), axlearn/common/attention.py:1301-1349 (RoPE), :3354-3370 (SwiGLU),
 // axlearn/common/loss.py:234-327 (cross entropy) and axlearn/common/optimizers.py:741-856,
 // 1149-1184 (AdamW chain, global-norm clip).
+#include "chain.cuh"
 #include "no_alloc.h"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -71,6 +72,7 @@ __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __res
                                    const bf16* __restrict__ scale, bf16* __restrict__ y,
                                    bf16* __restrict__ sum_out, float* __restrict__ rstd_out,
                                    int64_t rows, int D, float eps) {
+  chain_link();
   __shared__ float red[32];
   const int nvec = D / 8;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -196,6 +198,7 @@ __global__ void __launch_bounds__(256, 3)
 rmsnorm_fwd_warp_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
                         const bf16* __restrict__ scale, bf16* __restrict__ y, bf16* __restrict__ sum_out,
                         float* __restrict__ rstd_out, int64_t rows, float eps) {
+  chain_link();
   constexpr int P = VPL * 256;
   constexpr int D = P * WPR;
   constexpr int kRowsPerCta = 8 / WPR;
@@ -866,8 +869,7 @@ extern "C" int axb_rmsnorm_fwd(const void* x, const void* residual, const void* 
   if (D % 8) return -10;
   const int threads = D >= 2048 ? 256 : 128;
   const int grid = static_cast<int>(rows < 148 * 8 ? rows : 148 * 8);
-  rmsnorm_fwd_kernel<<<grid, threads, 0, stream>>>(
-      static_cast<const bf16*>(x), static_cast<const bf16*>(residual),
+  launch_chained(rmsnorm_fwd_kernel, grid, threads, 0, stream, static_cast<const bf16*>(x), static_cast<const bf16*>(residual),
       static_cast<const bf16*>(scale), static_cast<bf16*>(y), static_cast<bf16*>(sum_out), rstd,
       rows, D, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
@@ -904,8 +906,7 @@ static int launch_rmsnorm_fwd_warp(const void* x, const void* residual, const vo
                                    float* rstd, int64_t rows, float eps, cudaStream_t stream) {
   const int64_t want = (rows + 8 / WPR - 1) / (8 / WPR);
   const int grid = static_cast<int>(want < 148 * 3 ? want : 148 * 3);
-  rmsnorm_fwd_warp_kernel<VPL, WPR><<<grid, 256, 0, stream>>>(
-      static_cast<const bf16*>(x), static_cast<const bf16*>(residual), static_cast<const bf16*>(scale),
+  launch_chained(rmsnorm_fwd_warp_kernel<VPL, WPR>, grid, 256, 0, stream, static_cast<const bf16*>(x), static_cast<const bf16*>(residual), static_cast<const bf16*>(scale),
       static_cast<bf16*>(y), static_cast<bf16*>(sum_out), rstd, rows, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

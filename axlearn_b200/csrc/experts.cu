@@ -13,6 +13,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "mma_sync.cuh"
 
 namespace axb {
@@ -95,6 +96,7 @@ constexpr int kRsThreads = 512, kRsWarps = kRsThreads / 32;
 
 template <typename T, int EPL>
 __global__ void __launch_bounds__(kRsThreads) route_small_kernel(RouteArgs a) {
+  chain_link();
   __shared__ int s_id[kRtMaxPairs], s_place[kRtMaxPairs], s_base[kRtMaxExperts + 1];
   __shared__ float s_w[kRtMaxPairs];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pairs = a.tokens * a.top;
@@ -242,6 +244,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) expert_combine_kernel(const T* __restrict__ y, const int* __restrict__ place,
                                                              T* __restrict__ out, int64_t y_ld, int64_t out_ld, int top,
                                                              int width) {
+  chain_link();
   const int64_t t = blockIdx.x;
   constexpr int V = sizeof(T) == 2 ? 8 : 4;  // width is a multiple of 8
   for (int c = threadIdx.x * V; c < width; c += 128 * V) {
@@ -275,9 +278,9 @@ template <int EPL>
 int launch_small(const RouteArgs& a, cudaStream_t stream) {
   const int want = (a.tokens * a.top + 1) / 2, grid = want < 148 ? want : 148;
   if (a.act_bf16)
-    route_small_kernel<__nv_bfloat16, EPL><<<grid, kRsThreads, 0, stream>>>(a);
+    launch_chained(route_small_kernel<__nv_bfloat16, EPL>, grid, kRsThreads, 0, stream, a);
   else
-    route_small_kernel<float, EPL><<<grid, kRsThreads, 0, stream>>>(a);
+    launch_chained(route_small_kernel<float, EPL>, grid, kRsThreads, 0, stream, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -321,10 +324,8 @@ extern "C" int axb_expert_combine(const void* y, const int* place, void* out, in
   if (tokens <= 0) return 0;
   if (width <= 0 || (width % 8) || (y_ld % 8) || (out_ld % 8) || top <= 0) return -10;
   if (act_bf16)
-    axb::expert_combine_kernel<__nv_bfloat16><<<static_cast<unsigned>(tokens), 128, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(y), place, static_cast<__nv_bfloat16*>(out), y_ld, out_ld, top, width);
+    axb::launch_chained(axb::expert_combine_kernel<__nv_bfloat16>, static_cast<unsigned>(tokens), 128, 0, stream, static_cast<const __nv_bfloat16*>(y), place, static_cast<__nv_bfloat16*>(out), y_ld, out_ld, top, width);
   else
-    axb::expert_combine_kernel<float><<<static_cast<unsigned>(tokens), 128, 0, stream>>>(
-        static_cast<const float*>(y), place, static_cast<float*>(out), y_ld, out_ld, top, width);
+    axb::launch_chained(axb::expert_combine_kernel<float>, static_cast<unsigned>(tokens), 128, 0, stream, static_cast<const float*>(y), place, static_cast<float*>(out), y_ld, out_ld, top, width);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

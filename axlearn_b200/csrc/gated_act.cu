@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "gate_math.cuh"
 
 namespace axb {
@@ -13,6 +14,7 @@ namespace axb {
 template <typename T, int K>
 __global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, int64_t n, int F, int up_off,
                                  int64_t ld, int64_t out_ld, float limit, float alpha) {
+  chain_link();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t row = i / out_ld;
@@ -24,6 +26,7 @@ __global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, 
 template <int K>
 __global__ void gated_act_vec_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int64_t n8,
                                      int up_off, int64_t ld, int64_t out_ld, float limit, float alpha) {
+  chain_link();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   const int64_t per_row = out_ld / 8, row = i / per_row;
@@ -48,16 +51,14 @@ static int launch_gated_act(const void* gu, void* out, int64_t rows, int F, int 
                             int act_bf16, float limit, float alpha, cudaStream_t stream) {
   if (act_bf16 && F % 8 == 0 && up_off % 8 == 0 && ld % 8 == 0 && out_ld == F) {
     const int64_t n8 = rows * (F / 8);
-    gated_act_vec_kernel<K><<<static_cast<unsigned>((n8 + 255) / 256), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), n8, up_off, ld, out_ld, limit, alpha);
+    launch_chained(gated_act_vec_kernel<K>, static_cast<unsigned>((n8 + 255) / 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), n8, up_off, ld, out_ld, limit, alpha);
   } else {
     const int64_t n = rows * out_ld;
     const unsigned grid = static_cast<unsigned>((n + 255) / 256);
     if (act_bf16)
-      gated_act_kernel<__nv_bfloat16, K><<<grid, 256, 0, stream>>>(
-          static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), n, F, up_off, ld, out_ld, limit, alpha);
+      launch_chained(gated_act_kernel<__nv_bfloat16, K>, grid, 256, 0, stream, static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), n, F, up_off, ld, out_ld, limit, alpha);
     else
-      gated_act_kernel<float, K><<<grid, 256, 0, stream>>>(static_cast<const float*>(gu), static_cast<float*>(out), n, F,
+      launch_chained(gated_act_kernel<float, K>, grid, 256, 0, stream, static_cast<const float*>(gu), static_cast<float*>(out), n, F,
                                                            up_off, ld, out_ld, limit, alpha);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;

@@ -23,6 +23,8 @@
 // What is left at the small sizes is the launch, the first tile's latency and the hand-over (about 5 us together).
 #include <atomic>
 
+#include "chain.cuh"
+#include "cluster.cuh"
 #include "host_utils.cuh"
 #include "sm100.cuh"
 
@@ -61,25 +63,8 @@ struct SkinnyGemmParams {
   int* status;
   int accumulate;
   int split;
+  int w_resident;  // in a chained launch: nothing that runs just before this kernel writes W
 };
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
-__device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, uint32_t rank) {
-  uint32_t a;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
 
 template <typename OutT>
 __device__ __forceinline__ void skinny_store(OutT* dst, float v, int accumulate) {
@@ -131,17 +116,14 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  chain_start_next();
 
   bool ok = true;
   if (warp == 0) {
     if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = kb_lo; kb < kb_hi; ++kb) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, kStatusWaitTimeoutProducer)) break;
+      auto load_w = [&](int stage, int k0) {
         uint8_t* sw = smem + stage * S::kStageBytes;
         mbar_arrive_expect_tx(&full_bar[stage], S::kStageBytes);
-        const int k0 = kb * kSkK;
         if constexpr (!W_MN) {
 #pragma unroll
           for (int t = 0; t < S::kTiles; ++t)
@@ -151,6 +133,21 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 #pragma unroll
           for (int j = 0; j < S::kFeatures / 64; ++j)
             tma_load_2d(sw + j * 8192, &tmap_w, &full_bar[stage], n0 + j * 64, k0);
+        }
+      };
+      // The stages are empty at the start: in a chained launch with resident weights they fill with weights while the
+      // kernels before this one still run, and only X waits for them.
+      const int early = p.w_resident ? (kb_hi - kb_lo < kStages ? kb_hi - kb_lo : kStages) : 0;
+      for (int i = 0; i < early; ++i) load_w(i, (kb_lo + i) * kSkK);
+      chain_wait();
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        uint8_t* sw = smem + stage * S::kStageBytes;
+        const int k0 = kb * kSkK;
+        if (kb - kb_lo >= early) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, kStatusWaitTimeoutProducer)) break;
+          load_w(stage, k0);
         }
         if constexpr (!X_MN) {
           tma_load_2d(sw + S::kWBytes, &tmap_x, &full_bar[stage], k0, 0);
@@ -167,6 +164,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
   } else if (warp == 1) {
     if (elect_one()) {
+      chain_wait();
       constexpr uint32_t idesc = umma_idesc_f16(kSkTile, BN, 1, 1, W_MN ? 1 : 0, X_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
@@ -199,6 +197,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       if (fed) tc_commit(done_bar);
     }
   } else {
+    chain_wait();  // ahead of the first read or write of C
     ok = mbar_wait_warp(done_bar, 0, p.status, kStatusWaitTimeoutEpilogue);
   }
   __syncwarp();
@@ -316,11 +315,11 @@ struct SkinnyKernel {
     cfg.blockDim = dim3(kSkThreads);
     cfg.dynamicSmemBytes = S::kSmem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim = {static_cast<unsigned>(p.split), 1, 1};
     cfg.attrs = attr;
-    cfg.numAttrs = p.split > 1 ? 1 : 0;
+    cfg.numAttrs = static_cast<unsigned>(chain_attribute(attr, p.split > 1 ? 1 : 0));
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tw, tx, p);
     if (e != cudaSuccess) {
       fprintf(stderr, "axb skinny gemm: launch failed: %s\n", cudaGetErrorString(e));
@@ -383,6 +382,13 @@ static int launch_skinny(const void* X, const void* W, int64_t ldx, int64_t ldw,
 
 }  // namespace axb
 
+// Chains the launches of the calling thread (chain.cuh) from here on; returns the previous setting.
+extern "C" int axb_chain_launches(int on) {
+  const int before = axb::chain_launches ? 1 : 0;
+  axb::chain_launches = on != 0;
+  return before;
+}
+
 // K slices that the kernel would choose for a problem with K-major X and N-major W (1 = no split).
 extern "C" int axb_gemm_splitk_plan(int M, int N, int K) {
   using namespace axb;
@@ -400,10 +406,11 @@ extern "C" int axb_gemm_splitk_plan(int M, int N, int K) {
 // C[M, N] (bf16 or fp32, row pitch ldc) = X * W (+ C when accumulate), M <= 128.
 //   x_mn_major = 0: X is [M, K] row-major (pitch ldx);         1: X is stored [K, M] row-major.
 //   w_mn_major = 0: W is stored [N, K] row-major (pitch ldw);  1: W is [K, N] row-major.
+// `w_resident`: W is not written by what runs before it on the stream (weights); counts in chained launches only.
 // `split`: K slices per tile, 0 = the kernel's own choice.  Alignment as for axb_gemm_bf16; -20 = not one of mine.
 extern "C" int axb_gemm_skinny(const void* X, const void* W, void* C, int M, int N, int K, int64_t ldx, int64_t ldw,
                                int64_t ldc, int x_mn_major, int w_mn_major, int out_fp32, int accumulate, int split,
-                               int* status, cudaStream_t stream) {
+                               int w_resident, int* status, cudaStream_t stream) {
   using namespace axb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   // One wave of two-tile CTAs at most: beyond it the persistent 256-column tiles of gemm.cu, which overlap a tile's
@@ -415,7 +422,7 @@ extern "C" int axb_gemm_skinny(const void* X, const void* W, void* C, int M, int
       (reinterpret_cast<uintptr_t>(C) & 15) || (ldc % (out_fp32 ? 4 : 8)))
     return -10;
   if (split < 0 || split > kSkMaxSplit || split > (K + kSkK - 1) / kSkK) return -15;
-  const SkinnyGemmParams p{M, N, K, C, ldc, status, accumulate, split};
+  const SkinnyGemmParams p{M, N, K, C, ldc, status, accumulate, split, w_resident && chain_launches ? 1 : 0};
 #define AXB_SKINNY_BN(BN, XM, WM, T) return launch_skinny<BN, XM, WM, T>(X, W, ldx, ldw, p, stream)
 #define AXB_SKINNY(WM, T)                                  \
   do {                                                     \

@@ -21,6 +21,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "mma_sync.cuh"
 
 namespace axb {
@@ -66,6 +67,7 @@ constexpr int kGdThreads = 256;
 // V = 4: vdim is a multiple of 4 (vector accesses to the state); V = 1: any vdim.
 template <typename T, int V>
 __global__ void __launch_bounds__(kGdThreads) gla_decode_kernel(GlaArgs a) {
+  chain_link();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   T* out = static_cast<T*>(a.out) + static_cast<int64_t>(b) * a.out_ld + h * a.vdim;
@@ -913,7 +915,7 @@ int launch_gla_decode(const GlaArgs& a, cudaStream_t stream) {
       return -3;
     configured = smem;
   }
-  gla_decode_kernel<T, V><<<dim3(a.heads, a.B), kGdThreads, smem, stream>>>(a);
+  launch_chained(gla_decode_kernel<T, V>, dim3(a.heads, a.B), kGdThreads, smem, stream, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chain.cuh"
+
 namespace axb {
 
 struct HyperArgs {
@@ -108,6 +110,7 @@ constexpr int max_threads(int S) { return S >= 1 && S <= 4 ? 512 : 256; }
 
 template <typename TS, typename T, int S, int V>
 __global__ void __launch_bounds__(max_threads(S)) hyper_step_kernel(HyperArgs a) {
+  chain_link();
   extern __shared__ float u_row[];  // [width]
   __shared__ float2 scratch[32];
   __shared__ float s_mix[kMaxStreams * kMaxStreams], s_out[kMaxStreams], s_read[kMaxStreams];
@@ -229,7 +232,7 @@ static int launch_hyper(const HyperArgs& a, cudaStream_t stream) {
   const int want = (a.width / V + 31) / 32 * 32;
   const int cap = a.rows <= 512 ? max_threads(S) : 256;
   const int threads = want < 64 ? 64 : (want > cap ? cap : want);
-  kernel<<<static_cast<unsigned>(a.rows), threads, smem, stream>>>(a);
+  launch_chained(kernel, static_cast<unsigned>(a.rows), threads, smem, stream, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -21,6 +21,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "mma_sync.cuh"
 
 namespace axb {
@@ -63,6 +64,7 @@ constexpr int kLpThreads = 128;
 // blockIdx.z = 0: the latent and the key part; z > 0: queries of `heads_per` heads.
 template <typename T>
 __global__ void __launch_bounds__(kLpThreads) latent_prep_kernel(LatentArgs a, int heads_per) {
+  chain_link();
   extern __shared__ float2 s_turn[];  // (cos, sin) per pair
   __shared__ float red[kLpThreads / 32];
   const int t = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(kLpThreads) latent_prep_kernel(LatentArgs a, i
 constexpr int kLvTokens = 4;
 
 __global__ void __launch_bounds__(64 * kLvTokens) latent_prep_vec_kernel(LatentArgs a) {
+  chain_link();
   using bf16 = __nv_bfloat16;
   extern __shared__ float2 s_turn[];  // [4][rot_dims / 2] (cos, sin)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = a.rot_dims / 2;
@@ -311,6 +314,7 @@ __host__ __device__ inline LdSmem ld_smem(int row_w, int heads) {
 // MT tiles of 16 heads per CTA.
 template <int MT>
 __global__ void __launch_bounds__(kLdThreads, 1) latent_decode_kernel(LatentArgs a) {
+  chain_link();
   using bf16 = __nv_bfloat16;
   constexpr int HB = MT * 16;
   extern __shared__ __align__(16) uint8_t ld_mem[];
@@ -513,6 +517,7 @@ __global__ void __launch_bounds__(kLdThreads, 1) latent_decode_kernel(LatentArgs
 
 // One CTA per (query row, head): parts weighted by their maxima, four columns per thread.
 __global__ void __launch_bounds__(128) latent_merge_kernel(LatentArgs a) {
+  chain_link();
   __shared__ float s_w[kLdMaxSplits];
   const int64_t row = blockIdx.x;
   const int h = blockIdx.y, tid = threadIdx.x;
@@ -576,8 +581,8 @@ int launch_latent_decode(const LatentArgs& a, cudaStream_t stream) {
     configured = smem;
   }
   const dim3 grid(a.B * a.T, a.splits, (a.heads + MT * 16 - 1) / (MT * 16));
-  latent_decode_kernel<MT><<<grid, kLdThreads, smem, stream>>>(a);
-  if (a.splits > 1) latent_merge_kernel<<<dim3(a.B * a.T, a.heads), 128, 0, stream>>>(a);
+  latent_decode_kernel<MT><<<grid, kLdThreads, smem, stream>>>(a);  // one even wave: not chained
+  if (a.splits > 1) launch_chained(latent_merge_kernel, dim3(a.B * a.T, a.heads), 128, 0, stream, a);
   return latent_launched();
 }
 
@@ -593,7 +598,7 @@ extern "C" int axb_latent_prep(const axb::LatentArgs* args, cudaStream_t stream)
   if (a.act_bf16 && a.qbuf == nullptr && a.lat != nullptr && !(aligned & 7)) {
     const int64_t ctas = (static_cast<int64_t>(a.B) * a.T + axb::kLvTokens - 1) / axb::kLvTokens;
     if (smem * axb::kLvTokens <= 48 * 1024) {
-      axb::latent_prep_vec_kernel<<<static_cast<unsigned>(ctas), 64 * axb::kLvTokens, smem * axb::kLvTokens, stream>>>(a);
+      axb::launch_chained(axb::latent_prep_vec_kernel, static_cast<unsigned>(ctas), 64 * axb::kLvTokens, smem * axb::kLvTokens, stream, a);
       return axb::latent_launched();
     }
   }
@@ -601,9 +606,9 @@ extern "C" int axb_latent_prep(const axb::LatentArgs* args, cudaStream_t stream)
   const int heads_per = static_cast<int64_t>(a.B) * a.T <= 1024 ? 4 : 32;
   const dim3 grid(a.T, a.B, 1 + (a.heads + heads_per - 1) / heads_per);
   if (a.act_bf16)
-    axb::latent_prep_kernel<__nv_bfloat16><<<grid, axb::kLpThreads, smem, stream>>>(a, heads_per);
+    axb::launch_chained(axb::latent_prep_kernel<__nv_bfloat16>, grid, axb::kLpThreads, smem, stream, a, heads_per);
   else
-    axb::latent_prep_kernel<float><<<grid, axb::kLpThreads, smem, stream>>>(a, heads_per);
+    axb::launch_chained(axb::latent_prep_kernel<float>, grid, axb::kLpThreads, smem, stream, a, heads_per);
   return axb::latent_launched();
 }
 

@@ -25,6 +25,7 @@
 
 #include <type_traits>
 
+#include "chain.cuh"
 #include "mma_sync.cuh"
 
 namespace axb {
@@ -224,6 +225,7 @@ __global__ void ssd_ring_kernel(SsdArgs a) {
 // a thread holds its NV vectors between the two passes; NV = 0: any width, computed twice.
 template <typename T, int V, int NV>
 __global__ void __launch_bounds__(256) ssd_norm_kernel(SsdArgs a) {
+  chain_link();
   const int inner = a.heads * a.vdim, width = inner / a.norm_groups, c0 = blockIdx.y * width;
   const int64_t row = blockIdx.x;
   const T* y = static_cast<const T*>(a.y) + row * inner + c0;
@@ -292,6 +294,7 @@ constexpr int kSdThreads = 256;
 // V = 4: vdim is a multiple of 4; V = 1: any vdim.
 template <typename T, int V>
 __global__ void __launch_bounds__(kSdThreads, 4) ssd_decode_kernel(SsdArgs a) {
+  chain_link();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int P = a.vdim, N = a.state, inner = a.heads * P, channels = ssd_channels(a);
@@ -930,7 +933,7 @@ int launch_decode(const SsdArgs& a, cudaStream_t stream) {
       return -3;
     configured = smem;
   }
-  ssd_decode_kernel<T, V><<<dim3(a.heads, a.B), kSdThreads, smem, stream>>>(a);
+  ssd_decode_kernel<T, V><<<dim3(a.heads, a.B), kSdThreads, smem, stream>>>(a);  // one even wave: not chained
   return launched();
 }
 
@@ -968,15 +971,15 @@ int norm(const SsdArgs& a, cudaStream_t stream) {
   const int threads = want < 32 ? 32 : (want > 256 ? 256 : want);
   const dim3 grid(static_cast<unsigned>(rows), a.norm_groups);
   if (!vec)
-    ssd_norm_kernel<T, 1, 0><<<grid, threads, 0, stream>>>(a);
+    launch_chained(ssd_norm_kernel<T, 1, 0>, grid, threads, 0, stream, a);
   else if (width <= 8 * 256)
-    ssd_norm_kernel<T, 8, 1><<<grid, threads, 0, stream>>>(a);
+    launch_chained(ssd_norm_kernel<T, 8, 1>, grid, threads, 0, stream, a);
   else if (width <= 16 * 256)
-    ssd_norm_kernel<T, 8, 2><<<grid, threads, 0, stream>>>(a);
+    launch_chained(ssd_norm_kernel<T, 8, 2>, grid, threads, 0, stream, a);
   else if (width <= 32 * 256)
-    ssd_norm_kernel<T, 8, 4><<<grid, threads, 0, stream>>>(a);
+    launch_chained(ssd_norm_kernel<T, 8, 4>, grid, threads, 0, stream, a);
   else
-    ssd_norm_kernel<T, 8, 0><<<grid, threads, 0, stream>>>(a);
+    launch_chained(ssd_norm_kernel<T, 8, 0>, grid, threads, 0, stream, a);
   return launched();
 }
 

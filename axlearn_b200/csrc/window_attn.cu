@@ -23,6 +23,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "chain.cuh"
+
 namespace axb {
 
 struct WindowArgs {
@@ -94,6 +96,7 @@ constexpr int kWdThreads = 256, kWdWarps = kWdThreads / 32, kMaxSplits = 64;
 // head per CTA.
 template <typename T, int GT, int LPK, int NC, int U, bool kAligned>
 __global__ void __launch_bounds__(kWdThreads, 2) window_decode_kernel(WindowArgs a) {
+  chain_link();
   constexpr int VEC = 16 / sizeof(T);
   constexpr int E = NC * VEC;                // elements per lane
   constexpr int KPW = 32 / LPK;              // keys per warp and step
@@ -489,9 +492,9 @@ template <typename T, int GT, int LPK, int NC, int U>
 static int launch_decode(const WindowArgs& a, bool aligned, cudaStream_t stream) {
   const dim3 grid(a.splits, a.heads / GT, a.B);
   if (aligned)
-    window_decode_kernel<T, GT, LPK, NC, U, true><<<grid, kWdThreads, 0, stream>>>(a);
+    launch_chained(window_decode_kernel<T, GT, LPK, NC, U, true>, grid, kWdThreads, 0, stream, a);
   else
-    window_decode_kernel<T, GT, LPK, NC, U, false><<<grid, kWdThreads, 0, stream>>>(a);
+    launch_chained(window_decode_kernel<T, GT, LPK, NC, U, false>, grid, kWdThreads, 0, stream, a);
   return cudaGetLastError() == cudaSuccess ? zero_tail<T>(a, stream) : -4;
 }
 

@@ -177,7 +177,7 @@ class BaseDecodeEngine:
             for t, old in zip(buffers, saved):
                 t.copy_(old)
             self._graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self._graph):
+            with torch.cuda.graph(self._graph), cuda_ops.chained_launches():
                 self._step()
 
     @torch.no_grad()
@@ -312,7 +312,7 @@ class DecodeEngine(BaseDecodeEngine):
 
     def _logits(self, hidden: Tensor) -> Tensor:
         hn = cuda_ops.rms_norm(hidden, self.w["final_norm"], self.dims.norm_eps)
-        return cuda_ops.gemm(hn, self.w["head"].t(), out_dtype=torch.float32)
+        return cuda_ops.gemm(hn, self.w["head"].t(), out_dtype=torch.float32, resident=True)
 
     # ------------------------------------------------------------------ decode
     def _step(self) -> None:
@@ -326,7 +326,7 @@ class DecodeEngine(BaseDecodeEngine):
         x = self.w["emb"][self.tokens]                                        # [B, D]
         for li, lw in enumerate(self.w["layers"]):
             hn = cuda_ops.rms_norm(x, lw.attn_norm, d.norm_eps)
-            qkv = cuda_ops.gemm(hn, lw.wqkv)
+            qkv = cuda_ops.gemm(hn, lw.wqkv, resident=True)
             q = decode_ops.rope_append_paged(
                 qkv, self.k_pools[li], self.v_pools[li], self.page_table, self.lengths,
                 num_q_heads=self.nq_l, theta=d.rope_theta)
@@ -337,13 +337,13 @@ class DecodeEngine(BaseDecodeEngine):
             if self.world > 1:
                 x = self._gemm_reduce(attn2, lw.wo, x, 2 * li)
             else:
-                cuda_ops.gemm(attn2, lw.wo, out=x, accumulate=True)           # x += attn @ Wo
+                cuda_ops.gemm(attn2, lw.wo, out=x, accumulate=True, resident=True)  # x += attn @ Wo
             hn = cuda_ops.rms_norm(x, lw.ffn_norm, d.norm_eps)
-            act = decode_ops.swiglu_packed(cuda_ops.gemm(hn, lw.wgu))
+            act = decode_ops.swiglu_packed(cuda_ops.gemm(hn, lw.wgu, resident=True))
             if self.world > 1:
                 x = self._gemm_reduce(act, lw.wdown, x, 2 * li + 1)
             else:
-                cuda_ops.gemm(act, lw.wdown, out=x, accumulate=True)
+                cuda_ops.gemm(act, lw.wdown, out=x, accumulate=True, resident=True)
         self.logits.copy_(self._logits(x))
         self.tokens.copy_(self.logits.argmax(dim=-1))
         self.launches_per_step = cuda_ops.launch_count - before

@@ -13,6 +13,7 @@ timeout in a per-device status word instead of hanging; ``check_status()`` raise
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 import os
@@ -81,8 +82,9 @@ class _Sigs:
                           c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
     axb_gemm_splitk_plan = [c_int, c_int, c_int]
     axb_multimem_allreduce = [ctypes.c_uint64, c_int64, c_int, c_int, c_void_p]
+    axb_chain_launches = [c_int]
     axb_gemm_skinny = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64,
-                       c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
+                       c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     axb_rmsnorm_fwd = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_float, c_void_p]
     axb_rmsnorm_bwd_ctas = [c_int64]
     axb_rmsnorm_fast_supported = [c_int]
@@ -186,16 +188,31 @@ def _operand(t: torch.Tensor, contraction_dim: int) -> tuple[torch.Tensor, int, 
     return t, u[0], u[1]
 
 
+@contextlib.contextmanager
+def chained_launches():
+    """Chains the kernels that the calling thread launches inside (``csrc/chain.cuh``): for the capture of a
+    decoding step, whose graph runs after everything that wrote its weights."""
+    h = lib()
+    before = h.axb_chain_launches(1)
+    try:
+        yield
+    finally:
+        h.axb_chain_launches(before)
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None,
          out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False,
-         max_ctas: int = 0) -> torch.Tensor:
-    """``a[M, K] @ b[K, N]`` on the tcgen05 kernel; operands may be transposed views."""
+         max_ctas: int = 0, resident: bool = False) -> torch.Tensor:
+    """``a[M, K] @ b[K, N]`` on the tcgen05 kernel; operands may be transposed views.  ``resident``: ``b`` is a
+    weight that nothing in a captured step writes, so that its first tiles may be read ahead of the kernels before
+    (``chained_launches``)."""
     assert a.dim() == 2 and b.dim() == 2 and a.shape[1] == b.shape[0], (a.shape, b.shape)
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
     m, k = a.shape
     n = b.shape[1]
     a, a_mn, lda = _operand(a, 1)
-    b, b_mn, ldb = _operand(b, 0)
+    given, (b, b_mn, ldb) = b, _operand(b, 0)
+    resident = resident and b.data_ptr() == given.data_ptr()  # a copy of a weight is not one
     if out is None:
         out = torch.empty((m, n), dtype=out_dtype, device=a.device)
     else:
@@ -211,7 +228,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None
         # peer, so the cap that keeps persistent CTAs resident beside communication kernels does not concern it.
         rc = lib().axb_gemm_skinny(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, lda, ldb, out.stride(0),
                                    a_mn, b_mn, 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0, 0,
-                                   status_word(a.device).data_ptr(), _stream())
+                                   1 if resident else 0, status_word(a.device).data_ptr(), _stream())
         if rc != -20:
             _check(rc, "axb_gemm_skinny")
             return out
@@ -323,9 +340,12 @@ class _Linear(torch.autograd.Function):
         return dx, dw
 
 
-def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def linear(x: torch.Tensor, w: torch.Tensor, *, resident: bool = False) -> torch.Tensor:
+    """``resident``: as in ``gemm``; without gradients only."""
     if x.shape[-1] % 8 or w.shape[1] % 8:
         return torch.matmul(x, w)
+    if resident and not torch.is_grad_enabled() and _fused_fsdp_info(w) is None:
+        return gemm(x.reshape(-1, x.shape[-1]), w, resident=True).reshape(x.shape[:-1] + (w.shape[1],))
     return _Linear.apply(x, w)
 
 

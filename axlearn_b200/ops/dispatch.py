@@ -112,20 +112,20 @@ class _LinearKept(torch.autograd.Function):
         return dx, dw, None
 
 
-def _linear_impl(x, w):
+def _linear_impl(x, w, resident=False):
     if _cuda(x, w) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
-        return _ops().linear(x, w)
+        return _ops().linear(x, w, resident=resident)
     return torch.matmul(x, w)
 
 
-def linear(x, w):
+def linear(x, w, *, resident: bool = False):
     """``x[..., K] @ w[K, N]`` with fp32 accumulation.  Inside a replayed layer whose remat
     policy keeps this product (``axlearn_b200.common.remat``), the replay reuses the kept result
     instead of running the GEMM again."""
     from axlearn_b200.common import remat
 
     if remat.active() is None:
-        return _linear_impl(x, w)
+        return _linear_impl(x, w, resident)
     on_kernel = _cuda(x, w) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
     # A GEMM that carries a parameter gather for a neighbouring layer has to run even when its
     # own result is known.
@@ -138,11 +138,11 @@ def linear(x, w):
     return _LinearKept.apply(x, w, y)
 
 
-def linear_f32(x, w):
+def linear_f32(x, w, *, resident: bool = False):
     """``x[..., K] @ w[K, N]`` with an fp32 result (the accumulators as they are): output heads."""
     if _cuda(x, w) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and not (
             torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)):
-        y = _ops().gemm(x.reshape(-1, x.shape[-1]), w, out_dtype=torch.float32)
+        y = _ops().gemm(x.reshape(-1, x.shape[-1]), w, out_dtype=torch.float32, resident=resident)
         return y.reshape(x.shape[:-1] + (w.shape[1],))
     return linear(x, w).float()
 

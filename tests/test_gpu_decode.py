@@ -35,6 +35,35 @@ def test_paged_decode_attention_matches_reference(nq, nkv, splits):
     assert err < 2e-2 * max(1.0, ref.abs().max().item()), err
 
 
+def test_chained_step_sees_new_weights_and_matches_separate_launches():
+    """A captured step reads its first weight tiles ahead of the kernels before it: new weights written right before a
+    replay have to show, and the logits are those of separately launched kernels bit for bit."""
+    from axlearn_b200.inference.decode_engine import DecodeEngine, FujiDims, LayerWeights
+
+    d, f, vocab, nq, nkv, b = 256, 512, 1024, 4, 2, 3
+    g = torch.Generator(device="cuda").manual_seed(0)
+
+    def w(*shape):
+        return (torch.randn(*shape, device="cuda", generator=g) * shape[0] ** -0.5).bfloat16()
+
+    layers = [LayerWeights(attn_norm=1 + 0.1 * w(d), wqkv=w(d, (nq + 2 * nkv) * 128), wo=w(nq * 128, d),
+                           ffn_norm=1 + 0.1 * w(d), wgu=w(d, 2 * f), wdown=w(f, d)) for _ in range(3)]
+    weights = {"layers": layers, "emb": w(vocab, d) * 16, "head": w(vocab, d), "final_norm": 1 + 0.1 * w(d)}
+    dims = FujiDims(num_layers=3, hidden_dim=d, num_heads=nq, num_kv_heads=nkv, head_dim=128, ffn_dim=f, vocab_size=vocab)
+    engines = [DecodeEngine(weights, dims, batch=b, max_len=64, use_graph=use) for use in (True, False)]
+    ids = torch.randint(0, vocab, (b, 9), device="cuda", generator=g)
+    for e in engines:
+        e.prefill(ids)
+    tokens = ids[:, 0]
+    for _ in range(6):
+        for lw in layers:
+            for t in (lw.wqkv, lw.wo, lw.wgu, lw.wdown):
+                t.copy_(w(*t.shape))
+        chained, plain = (e.step_logits(tokens).clone() for e in engines)
+        assert torch.equal(chained, plain)
+        tokens = plain.argmax(dim=-1)
+
+
 def test_rope_append_writes_page_slot_and_rotates():
     from axlearn_b200.ops import decode_ops, reference
 
