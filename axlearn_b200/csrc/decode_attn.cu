@@ -1,16 +1,29 @@
 // Decode-time attention over a paged KV cache, and the fused RoPE + cache append that feeds it.
 //
-// One new token per sequence attends to everything cached for that sequence.  The work is a
-// matrix-vector product per (sequence, KV head): every cached K and V byte is read exactly once
-// and nothing is reused, so the kernel is built to keep HBM busy rather than the tensor cores:
+// One new token per sequence attends to everything cached for that sequence; every cached K and V byte is used by the
+// query heads of one KV head only, so the bound is the rate at which the cache comes out of HBM, and, for few or short
+// sequences, the chain length -> page -> K -> softmax -> merge.
 //
-//   grid = (KV splits, KV heads x query-head groups, sequences), 128 threads.
-//   A warp walks the sequence's pages; 8 lanes share one key (16 dims = two 16-byte loads each),
-//   so a warp covers 4 keys per step and one 16-token page in 4 steps, with the loads of the
-//   whole page issued before the first use.  Scores are reduced over the 8 lanes with three
-//   shuffles, the softmax is kept online per lane group, and each lane accumulates its 16 dims
-//   of P*V.  Warps (and lane groups) merge through shared memory; KV splits write partial
-//   (max, sum, out) triples that `decode_combine_kernel` merges.
+// One CTA of four warps takes one (KV split, KV head, up to eight of its query heads), so K and V are read once for a
+// whole group of query heads.  A warp walks every fourth tile of 16 tokens of its split through a ring of two tiles
+// (8 KB of K and V each) that `cp.async` fills ahead of the arithmetic; three CTAs fit an SM.
+//   S = Q K^T: rows 0-7 of the m16n8k16 tile are the query heads, K is the B operand (a lane takes 8 neighbouring dims
+//   of a key; Q uses the same order of dims).
+//   O^T = V^T P^T: 16 dims are the rows, the heads the columns (the scores' accumulators are the B operand as they
+//   lie); a lane packs two keys' V entries into one register of the A operand.  P enters as two bf16 terms, i.e. with
+//   about 16 mantissa bits.
+// The warps meet in shared memory and the KV splits of up to a cluster (8) in distributed shared memory, so there is no
+// second launch; more splits leave partials (max, sum, out) for `decode_combine_kernel`.
+//
+// Measured against the two CUDA-core kernels that this replaces (one query head per 8 lanes, or four query heads on
+// four neighbouring KV heads; us a launch, weights of other layers in between, K and V bytes at 6.65 TB/s in brackets):
+//   batch  1, 16 heads on 16,  300 tokens  14.3 ->  4.8 (0.4)   batch 16, 32 on  8, up to 2048  64.4 ->  27.1 (13)
+//   batch  1, 32 heads on  8, 4000 tokens  20.2 -> 10.0 (2.5)   batch 64, 32 on  8, up to 1000 116.7 ->  42.0 (23)
+//   batch  4, 32 heads on  8, 2000 tokens  31.6 -> 12.4 (4.9)   batch 64, 32 on 32, up to 2000 208.8 -> 187.4 (184)
+//   batch  8, 16 heads on 16, up to 2000   36.9 -> 24.6 (13)    batch 64, 16 on 16, up to 500   46.1 ->  36.9 (23)
+// Three tiles a ring and two CTAs an SM: as fast for few CTAs, 10 % slower for many; registers instead of shared memory
+// for the tiles: 1.3 to 2 times as long.  What is left with ragged lengths is that the longest sequence's CTAs finish
+// last: a split is a share of its own sequence.
 //
 // Cache layout: pool [num_pages, page_size, Nkv, H] for K and for V (H = 128), page table
 // [B, max_pages] of pool page ids, `lengths[b]` = number of valid tokens (the new token
@@ -27,10 +40,10 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
-#include <stdlib.h>
-#include <string.h>
 
 #include "chain.cuh"
+#include "cluster.cuh"
+#include "mma_sync.cuh"
 
 namespace axb {
 
@@ -50,299 +63,266 @@ struct DecodeParams {
   float scale_log2;           // softmax scale * log2(e)
 };
 
-__device__ __forceinline__ void unpack8(const uint4& u, float* f) {
-  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = __bfloat1622float2(p[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
+constexpr int kMmaRows = 8;       // query heads of a CTA
+constexpr int kTileKeys = 16;
+constexpr int kMaxClusterSplits = 8;
+
+constexpr int kTileBytes = 2 * kTileKeys * kHeadDim * 2;  // K and V
+constexpr int kStages = 2;
+constexpr int attn_smem_bytes(int rows) {
+  const int merge = (4 + 1) * rows * (kHeadDim + 2) * 4, tiles = 4 * kStages * kTileBytes;
+  return merge > tiles ? merge : tiles;
 }
 
-// GT query heads of one KV head per CTA (GT = 1, 2 or 4).
-// One query head per CTA (GT == 1) fits 64 registers without spills: eight CTAs per SM instead of
-// six, i.e. 1184 resident CTAs, so that a 32 x 32-head batch is one wave instead of 1.15.
-template <int GT>
-__global__ void __launch_bounds__(kDecodeThreads, GT == 1 ? 8 : 1)
+// head + rest = (x, y) >= 0 to about 16 mantissa bits, the head rounded down.  The rest of a positive number stays
+// positive, so that an infinite V gives an infinity as in one product, not 0 * infinity.
+__device__ __forceinline__ void split_down(float x, float y, uint32_t& head, uint32_t& rest) {
+  const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
+  head = __byte_perm(ux, uy, 0x7632);
+  const float dx = x - __uint_as_float(ux & 0xffff0000u), dy = y - __uint_as_float(uy & 0xffff0000u);
+  const float tiny = 1.17549435e-38f;
+  rest = pack2(x > 0.f ? fmaxf(dx, tiny) : dx, y > 0.f ? fmaxf(dy, tiny) : dy);
+}
+
+// 16 bytes to shared memory, zeros when `ok` is false (`src` is not read then).
+__device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+template <bool kCluster>
+__global__ void __launch_bounds__(kDecodeThreads)
 decode_attn_kernel(DecodeParams p) {
   chain_link();
+  extern __shared__ __align__(16) float s_part[];  // the warps' tiles; then 4 warps and the CTA: [rows][kHeadDim] sums,
+                                                   // [rows] maxima, [rows] weights
   const int split = blockIdx.x;
-  const int groups_per_kv = (p.num_q_heads / p.num_kv_heads) / GT;
-  const int kvh = blockIdx.y / groups_per_kv;
-  const int qh0 = kvh * (p.num_q_heads / p.num_kv_heads) + (blockIdx.y % groups_per_kv) * GT;
+  const int group = p.num_q_heads / p.num_kv_heads;
+  const int parts = (group + kMmaRows - 1) / kMmaRows;
+  const int kvh = blockIdx.y / parts;
+  const int first = blockIdx.y % parts * kMmaRows;
+  const int rows = min(kMmaRows, group - first);
+  const int qh0 = kvh * group + first;
   const int b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kq = lane >> 3;   // key slot within a step (0..3)
-  const int dc = lane & 7;    // dim chunk: dims [16*dc, 16*dc + 16)
+  const int r = lane >> 2, c = lane & 3;
   const int len = p.lengths[b];
-  const int num_pages = (len + p.page_size - 1) / p.page_size;
-  // Pages [pg_lo, pg_hi) belong to this split.
-  const int per_split = (num_pages + p.splits - 1) / p.splits;
-  const int pg_lo = split * per_split;
-  const int pg_hi = min(num_pages, pg_lo + per_split);
+  const int tiles = (len + kTileKeys - 1) / kTileKeys;
+  const int per_split = (tiles + p.splits - 1) / p.splits;
+  const int hi = min(tiles, (split + 1) * per_split);
+  const int* table = p.page_table + static_cast<int64_t>(b) * p.max_pages;
 
-  float q[GT][16];
-#pragma unroll
-  for (int g = 0; g < GT; ++g) {
-    const uint4* qp = reinterpret_cast<const uint4*>(
-        p.q + (static_cast<int64_t>(b) * p.num_q_heads + qh0 + g) * kHeadDim + dc * 16);
-    unpack8(qp[0], q[g]);
-    unpack8(qp[1], q[g] + 8);
-  }
-  float m[GT], l[GT], acc[GT][16];
-#pragma unroll
-  for (int g = 0; g < GT; ++g) {
-    m[g] = -INFINITY;
-    l[g] = 0.f;
-#pragma unroll
-    for (int d = 0; d < 16; ++d) acc[g][d] = 0.f;
-  }
+  // Slot (token row of the pools) of key `lane & 15` of a tile, -1 beyond the sequence.
+  auto slot_of = [&](int tile) {
+    const int t = tile * kTileKeys + (lane & 15);
+    if (tile >= hi || t >= len) return -1;
+    return __ldg(table + t / p.page_size) * p.page_size + t % p.page_size;
+  };
 
-  const int64_t row_stride = static_cast<int64_t>(p.num_kv_heads) * kHeadDim;  // one token
-  const int steps_per_page = p.page_size / 4;
-  for (int pg = pg_lo + warp; pg < pg_hi; pg += kDecodeThreads / 32) {
-    const int page = p.page_table[static_cast<int64_t>(b) * p.max_pages + pg];
-    const int64_t base = (static_cast<int64_t>(page) * p.page_size) * row_stride + kvh * kHeadDim + dc * 16;
-    const int tok0 = pg * p.page_size;
-    for (int st = 0; st < steps_per_page; ++st) {
-      const int t = st * 4 + kq;
-      const bool valid = tok0 + t < len;
-      uint4 k0 = make_uint4(0, 0, 0, 0), k1 = k0, v0 = k0, v1 = k0;
-      if (valid) {
-        const uint4* kp = reinterpret_cast<const uint4*>(p.k_pool + base + t * row_stride);
-        const uint4* vp = reinterpret_cast<const uint4*>(p.v_pool + base + t * row_stride);
-        k0 = __ldg(kp);
-        k1 = __ldg(kp + 1);
-        v0 = __ldg(vp);
-        v1 = __ldg(vp + 1);
+  const int64_t row_stride = static_cast<int64_t>(p.num_kv_heads) * kHeadDim;
+  const int head_off = kvh * kHeadDim + (lane & 15) * 8;
+  uint8_t* ring = reinterpret_cast<uint8_t*>(s_part) + warp * kStages * kTileBytes;
+  const uint32_t ring_addr = sptr(ring);
+  // A row of a tile is 16 chunks of 16 bytes.  Chunks are swapped within their row so that the eight lanes of a
+  // 128-byte phase hit all banks: they read two neighbouring rows of K, and every second row of V.
+  auto k_chunk = [](int row, int chunk) { return row * 256 + ((chunk ^ ((row & 1) << 2)) << 4); };
+  auto v_chunk = [](int row, int chunk) { return row * 256 + ((chunk ^ (row & 6)) << 4); };
+  auto load_tile = [&](int stage, int slot) {  // half a warp per row: two rows of K or V an instruction
+    const uint32_t dst = ring_addr + stage * kTileBytes;
+#pragma unroll
+    for (int i = 0; i < kTileKeys / 2; ++i) {
+      const int row = 2 * i + (lane >> 4);
+      const int at = __shfl_sync(0xffffffffu, slot, row);
+      const int64_t off = (at < 0 ? 0 : at) * row_stride + head_off;
+      cp16_or_zero(dst + k_chunk(row, lane & 15), p.k_pool + off, at >= 0);
+      cp16_or_zero(dst + kTileBytes / 2 + v_chunk(row, lane & 15), p.v_pool + off, at >= 0);
+    }
+  };
+
+  constexpr int kStep = kDecodeThreads / 32;
+  int tile = split * per_split + warp;
+  int slots[kStages];
+#pragma unroll
+  for (int i = 0; i < kStages; ++i) slots[i] = slot_of(tile + i * kStep);
+#pragma unroll
+  for (int i = 0; i < kStages; ++i) {
+    if (tile + i * kStep < hi) load_tile(i, slots[i]);
+    cp_commit();
+  }
+  int slot = slot_of(tile + kStages * kStep);
+  uint4 q[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    q[j] = r < rows ? *reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(b) * p.num_q_heads + qh0 + r) * kHeadDim +
+                                                      j * 32 + c * 8)
+                    : make_uint4(0, 0, 0, 0);
+  float m = -INFINITY, l = 0.f;
+  float acc[8][4];  // [16 dims][heads 2c, 2c + 1]
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+
+  int stage = 0;
+  for (; tile < hi; tile += kStep) {
+    cp_wait_group<kStages - 1>();
+    __syncwarp();
+    const uint8_t* kt = ring + stage * kTileBytes;
+    const uint8_t* vt = kt + kTileBytes / 2;
+    float s[4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint4 k = *reinterpret_cast<const uint4*>(kt + k_chunk(n * 8 + r, j * 4 + c));
+        const uint32_t a0[4] = {q[j].x, 0u, q[j].y, 0u}, a1[4] = {q[j].z, 0u, q[j].w, 0u};
+        mma(d, a0, k.x, k.y);
+        mma(d, a1, k.z, k.w);
       }
-      float kf[16], vf[16];
-      unpack8(k0, kf);
-      unpack8(k1, kf + 8);
-      unpack8(v0, vf);
-      unpack8(v1, vf + 8);
+      const int t = tile * kTileKeys + n * 8 + 2 * c;
+      s[2 * n] = t < len ? d[0] * p.scale_log2 : -INFINITY;
+      s[2 * n + 1] = t + 1 < len ? d[1] * p.scale_log2 : -INFINITY;
+    }
+    float top = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    const float m_new = fmaxf(m, top);
+    if (__any_sync(0xffffffffu, m_new != m)) {
+      const float corr = m_new == -INFINITY ? 1.f : exp2f(m - m_new);
+      l *= corr;
+      const float c0 = __shfl_sync(0xffffffffu, corr, 8 * c), c1 = __shfl_sync(0xffffffffu, corr, 8 * c + 4);
 #pragma unroll
-      for (int g = 0; g < GT; ++g) {
-        float s = 0.f;
+      for (int i = 0; i < 8; ++i) {
+        acc[i][0] *= c0;
+        acc[i][1] *= c1;
+        acc[i][2] *= c0;
+        acc[i][3] *= c1;
+      }
+      m = m_new;
+    }
+    // exp2(-inf - -inf) would be NaN: a row that has seen no finite score keeps zeros.
 #pragma unroll
-        for (int d = 0; d < 16; ++d) s += q[g][d] * kf[d];
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        s = valid ? s * p.scale_log2 : -INFINITY;
-        const float m_new = fmaxf(m[g], s);
-        // exp2(-inf - -inf) would be NaN: a lane group that has seen no valid key keeps zeros.
-        const float corr = (m_new == -INFINITY) ? 1.f : exp2f(m[g] - m_new);
-        const float pr = (m_new == -INFINITY) ? 0.f : exp2f(s - m_new);
-        l[g] = l[g] * corr + pr;
+    for (int i = 0; i < 4; ++i) s[i] = m == -INFINITY ? 0.f : exp2f(s[i] - m);
+    l += (s[0] + s[1]) + (s[2] + s[3]);
+    uint32_t head[2], rest[2];
+    split_down(s[0], s[1], head[0], rest[0]);
+    split_down(s[2], s[3], head[1], rest[1]);
 #pragma unroll
-        for (int d = 0; d < 16; ++d) acc[g][d] = acc[g][d] * corr + pr * vf[d];
-        m[g] = m_new;
+    for (int j = 0; j < 2; ++j) {
+      uint32_t v[4][4];  // keys 2c, 2c + 1, 8 + 2c, 8 + 2c + 1: the columns of P that this lane holds
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(v[i]) =
+            *reinterpret_cast<const uint4*>(vt + v_chunk((i >> 1) * 8 + 2 * c + (i & 1), j * 8 + r));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t a[4] = {__byte_perm(v[0][e], v[1][e], 0x5410), __byte_perm(v[0][e], v[1][e], 0x7632),
+                               __byte_perm(v[2][e], v[3][e], 0x5410), __byte_perm(v[2][e], v[3][e], 0x7632)};
+        mma(acc[j * 4 + e], a, head[0], head[1]);
+        mma(acc[j * 4 + e], a, rest[0], rest[1]);
       }
     }
+    __syncwarp();  // the stage has been read
+    if (tile + kStages * kStep < hi) load_tile(stage, slot);
+    cp_commit();
+    slot = slot_of(tile + (kStages + 1) * kStep);
+    if (++stage == kStages) stage = 0;
   }
+  cp_wait_all();
+  __syncthreads();  // the merge buffers overlay the tiles
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
 
-  // Merge the 4 key slots of each warp (lanes with equal dc), then the 4 warps via shared memory.
-  __shared__ float s_m[4][GT], s_l[4][GT];
-  __shared__ float s_acc[4][GT][kHeadDim];
+  // Rows r and r + 8 of MMA tile (j, e) are dims 64 j + 8 r + 2 e and the next.
+  const int per_warp = rows * kHeadDim;
+  float* s_m = s_part + 5 * per_warp;
+  float* s_l = s_m + 5 * rows;
 #pragma unroll
-  for (int g = 0; g < GT; ++g) {
+  for (int n = 0; n < 2; ++n) {
+    if (2 * c + n >= rows) break;
+    float* dst = s_part + warp * per_warp + (2 * c + n) * kHeadDim + r * 8;
 #pragma unroll
-    for (int off = 8; off <= 16; off <<= 1) {
-      const float m_o = __shfl_xor_sync(0xffffffffu, m[g], off);
-      const float l_o = __shfl_xor_sync(0xffffffffu, l[g], off);
-      const float m_new = fmaxf(m[g], m_o);
-      const float c_self = (m_new == -INFINITY) ? 1.f : exp2f(m[g] - m_new);
-      const float c_oth = (m_new == -INFINITY) ? 1.f : exp2f(m_o - m_new);
-      l[g] = l[g] * c_self + l_o * c_oth;
-#pragma unroll
-      for (int d = 0; d < 16; ++d) {
-        const float a_o = __shfl_xor_sync(0xffffffffu, acc[g][d], off);
-        acc[g][d] = acc[g][d] * c_self + a_o * c_oth;
-      }
-      m[g] = m_new;
-    }
-    if (kq == 0) {
-#pragma unroll
-      for (int d = 0; d < 16; ++d) s_acc[warp][g][dc * 16 + d] = acc[g][d];
-      if (dc == 0) {
-        s_m[warp][g] = m[g];
-        s_l[warp][g] = l[g];
-      }
-    }
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<float2*>(dst + (i >> 2) * 64 + (i & 3) * 2) = make_float2(acc[i][n], acc[i][2 + n]);
+  }
+  if (r < rows && c == 0) {
+    s_m[warp * rows + r] = m;
+    s_l[warp * rows + r] = l;
   }
   __syncthreads();
   // Thread d owns output dim d.
   const int d = threadIdx.x;
-#pragma unroll
-  for (int g = 0; g < GT; ++g) {
+  for (int g = 0; g < rows; ++g) {
     float mm = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) mm = fmaxf(mm, s_m[w][g]);
+    for (int w = 0; w < 4; ++w) mm = fmaxf(mm, s_m[w * rows + g]);
     float ll = 0.f, o = 0.f;
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      const float c = (mm == -INFINITY) ? 0.f : exp2f(s_m[w][g] - mm);
-      ll += s_l[w][g] * c;
-      o += s_acc[w][g][d] * c;
+      const float f = mm == -INFINITY ? 0.f : exp2f(s_m[w * rows + g] - mm);
+      ll += s_l[w * rows + g] * f;
+      o += s_part[w * per_warp + g * kHeadDim + d] * f;
     }
-    const int64_t row = (static_cast<int64_t>(b) * p.num_q_heads + qh0 + g) * p.splits + split;
+    const int64_t row = static_cast<int64_t>(b) * p.num_q_heads + qh0 + g;
     if (p.splits == 1) {
-      p.out[(static_cast<int64_t>(b) * p.num_q_heads + qh0 + g) * kHeadDim + d] =
-          __float2bfloat16(ll > 0.f ? o / ll : 0.f);
-    } else {
-      p.part_out[row * kHeadDim + d] = o;
+      p.out[row * kHeadDim + d] = __float2bfloat16(ll > 0.f ? o / ll : 0.f);
+    } else if (kCluster) {
+      s_part[4 * per_warp + g * kHeadDim + d] = o;
       if (d == 0) {
-        p.part_ml[row * 2] = mm;
-        p.part_ml[row * 2 + 1] = ll;
+        s_m[4 * rows + g] = mm;
+        s_l[4 * rows + g] = ll;
+      }
+    } else {
+      p.part_out[(row * p.splits + split) * kHeadDim + d] = o;
+      if (d == 0) {
+        p.part_ml[(row * p.splits + split) * 2] = mm;
+        p.part_ml[(row * p.splits + split) * 2 + 1] = ll;
       }
     }
+  }
+  if constexpr (kCluster) {
+    cluster_sync_all();
+    for (int g = split; g < rows; g += p.splits) {
+      float mv[kMaxClusterSplits], lv[kMaxClusterSplits], ov[kMaxClusterSplits];
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s) {
+        const bool have = s < p.splits;
+        mv[s] = have ? ld_cluster_f32(sptr(s_m + 4 * rows + g), s) : -INFINITY;
+        lv[s] = have ? ld_cluster_f32(sptr(s_l + 4 * rows + g), s) : 0.f;
+        ov[s] = have ? ld_cluster_f32(sptr(s_part + 4 * per_warp + g * kHeadDim + d), s) : 0.f;
+      }
+      float mm = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s) mm = fmaxf(mm, mv[s]);
+      float ll = 0.f, o = 0.f;
+#pragma unroll
+      for (int s = 0; s < kMaxClusterSplits; ++s) {
+        const float f = mm == -INFINITY ? 0.f : exp2f(mv[s] - mm);
+        ll += lv[s] * f;
+        o += ov[s] * f;
+      }
+      p.out[(static_cast<int64_t>(b) * p.num_q_heads + qh0 + g) * kHeadDim + d] =
+          __float2bfloat16(ll > 0.f ? o / ll : 0.f);
+    }
+    cluster_sync_all();  // a CTA's shared memory outlives its readers
   }
 }
 
-// Row-contiguous variant for caches with a multiple of four KV heads: a warp reads ONE token
-// across FOUR neighbouring KV heads per load (8 lanes x 32 bytes per head = 1 KB contiguous in
-// the pool, where the per-head kernel above reads four 256-byte pieces 1 KB or more apart), so
-// every DRAM burst it opens is used in full.  Lane group `hl` (8 lanes) owns KV head 4 * hg + hl
-// and all GT query heads attending to it; nothing is merged across lane groups, only across the
-// four warps (which split the pages).  GT = query heads per KV head (2 or 4; the launcher keeps
-// GT = 1 on the per-head kernel, which is as fast or faster there).
-template <int GT>
-__global__ void __launch_bounds__(kDecodeThreads)
-decode_attn_rows_kernel(DecodeParams p) {
-  chain_link();
-  const int split = blockIdx.x;
-  const int hg = blockIdx.y;  // group of four KV heads
-  const int b = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int hl = lane >> 3;   // KV head within the group
-  const int dc = lane & 7;    // dim chunk: dims [16*dc, 16*dc + 16)
-  const int kvh = hg * 4 + hl;
-  const int qh0 = kvh * GT;
-  const int len = p.lengths[b];
-  const int num_pages = (len + p.page_size - 1) / p.page_size;
-  const int per_split = (num_pages + p.splits - 1) / p.splits;
-  const int pg_lo = split * per_split;
-  const int pg_hi = min(num_pages, pg_lo + per_split);
-
-  float q[GT][16];
-#pragma unroll
-  for (int g = 0; g < GT; ++g) {
-    const uint4* qp = reinterpret_cast<const uint4*>(
-        p.q + (static_cast<int64_t>(b) * p.num_q_heads + qh0 + g) * kHeadDim + dc * 16);
-    unpack8(qp[0], q[g]);
-    unpack8(qp[1], q[g] + 8);
-  }
-  float m[GT], l[GT], acc[GT][16];
-#pragma unroll
-  for (int g = 0; g < GT; ++g) {
-    m[g] = -INFINITY;
-    l[g] = 0.f;
-#pragma unroll
-    for (int d = 0; d < 16; ++d) acc[g][d] = 0.f;
-  }
-
-  const int64_t row_stride = static_cast<int64_t>(p.num_kv_heads) * kHeadDim;  // one token
-  constexpr int kPageStride = kDecodeThreads / 32;
-  constexpr int kBatch = GT >= 4 ? 2 : 4;  // tokens whose loads are in flight together
-  const int* table_row = p.page_table + static_cast<int64_t>(b) * p.max_pages;
-  int page = (pg_lo + warp < pg_hi) ? __ldg(table_row + pg_lo + warp) : 0;
-  for (int pg = pg_lo + warp; pg < pg_hi; pg += kPageStride) {
-    // The next page's id is requested before this page's rows (it is a dependent load).
-    const int next_page = (pg + kPageStride < pg_hi) ? __ldg(table_row + pg + kPageStride) : 0;
-    const int64_t base = (static_cast<int64_t>(page) * p.page_size) * row_stride + kvh * kHeadDim + dc * 16;
-    const int tok0 = pg * p.page_size;
-    for (int t0 = 0; t0 < p.page_size; t0 += kBatch) {
-      uint4 kk[kBatch][2], vv[kBatch][2];
-      bool ok[kBatch];
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        const int t = t0 + u;
-        ok[u] = t < p.page_size && tok0 + t < len;
-        kk[u][0] = kk[u][1] = vv[u][0] = vv[u][1] = make_uint4(0, 0, 0, 0);
-        if (ok[u]) {
-          const uint4* kp = reinterpret_cast<const uint4*>(p.k_pool + base + t * row_stride);
-          const uint4* vp = reinterpret_cast<const uint4*>(p.v_pool + base + t * row_stride);
-          kk[u][0] = __ldg(kp);
-          kk[u][1] = __ldg(kp + 1);
-          vv[u][0] = __ldg(vp);
-          vv[u][1] = __ldg(vp + 1);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) {
-        if (t0 + u >= p.page_size) break;
-        float kf[16], vf[16];
-        unpack8(kk[u][0], kf);
-        unpack8(kk[u][1], kf + 8);
-        unpack8(vv[u][0], vf);
-        unpack8(vv[u][1], vf + 8);
-#pragma unroll
-        for (int g = 0; g < GT; ++g) {
-          float s = 0.f;
-#pragma unroll
-          for (int d = 0; d < 16; ++d) s += q[g][d] * kf[d];
-          s += __shfl_xor_sync(0xffffffffu, s, 1);
-          s += __shfl_xor_sync(0xffffffffu, s, 2);
-          s += __shfl_xor_sync(0xffffffffu, s, 4);
-          s = ok[u] ? s * p.scale_log2 : -INFINITY;
-          const float m_new = fmaxf(m[g], s);
-          const float corr = (m_new == -INFINITY) ? 1.f : exp2f(m[g] - m_new);
-          const float pr = (m_new == -INFINITY) ? 0.f : exp2f(s - m_new);
-          l[g] = l[g] * corr + pr;
-#pragma unroll
-          for (int d = 0; d < 16; ++d) acc[g][d] = acc[g][d] * corr + pr * vf[d];
-          m[g] = m_new;
-        }
-      }
-    }
-    page = next_page;
-  }
-
-  // Merge the four warps' partial results per (KV head of the group, query head).
-  __shared__ float s_m[4][4][GT], s_l[4][4][GT];
-  __shared__ float s_acc[4][4][GT][kHeadDim];
-#pragma unroll
-  for (int g = 0; g < GT; ++g) {
-#pragma unroll
-    for (int d = 0; d < 16; ++d) s_acc[warp][hl][g][dc * 16 + d] = acc[g][d];
-    if (dc == 0) {
-      s_m[warp][hl][g] = m[g];
-      s_l[warp][hl][g] = l[g];
-    }
-  }
-  __syncthreads();
-  // Thread (warp w, lane) finishes KV head w of the group: lane owns dims [4 * lane, 4 * lane + 4).
-  const int oh = warp;
-#pragma unroll
-  for (int g = 0; g < GT; ++g) {
-    float mm = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) mm = fmaxf(mm, s_m[w][oh][g]);
-    float ll = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float c = (mm == -INFINITY) ? 0.f : exp2f(s_m[w][oh][g] - mm);
-      ll += s_l[w][oh][g] * c;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) o[e] += s_acc[w][oh][g][lane * 4 + e] * c;
-    }
-    const int qh = (hg * 4 + oh) * GT + g;
-    const int64_t row = (static_cast<int64_t>(b) * p.num_q_heads + qh) * p.splits + split;
-    if (p.splits == 1) {
-      __nv_bfloat16* dst = p.out + (static_cast<int64_t>(b) * p.num_q_heads + qh) * kHeadDim + lane * 4;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) dst[e] = __float2bfloat16(ll > 0.f ? o[e] / ll : 0.f);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) p.part_out[row * kHeadDim + lane * 4 + e] = o[e];
-      if (lane == 0) {
-        p.part_ml[row * 2] = mm;
-        p.part_ml[row * 2 + 1] = ll;
-      }
-    }
-  }
+template <bool kCluster>
+static int launch_attn(const DecodeParams& p, dim3 grid, int rows, cudaStream_t stream) {
+  constexpr auto kernel = decode_attn_kernel<kCluster>;
+  static const cudaError_t configured = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                             attn_smem_bytes(kMmaRows));
+  if (configured != cudaSuccess) return -3;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {grid.x, 1, 1};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kDecodeThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(attn_smem_bytes(rows));
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = static_cast<unsigned>(chain_attribute(attr, kCluster ? 1 : 0));
+  return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? 0 : -4;
 }
 
 __global__ void __launch_bounds__(kHeadDim)
@@ -432,42 +412,12 @@ extern "C" int axb_decode_attn(const void* q, const void* k_pool, const void* v_
   p.max_pages = max_pages;
   p.splits = splits;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
-  // AXB_DECODE_ATTN=head keeps the per-head kernel for every shape (for comparisons).
-  // head1 / head2 additionally cap the query heads per CTA at 1 / 2.
-  static int rows_ok = -1, gt_cap = 4;
-  if (rows_ok < 0) {
-    const char* e = getenv("AXB_DECODE_ATTN");
-    if (e != nullptr && strcmp(e, "head1") == 0) gt_cap = 1;
-    if (e != nullptr && strcmp(e, "head2") == 0) gt_cap = 2;
-    rows_ok = (e != nullptr && strncmp(e, "head", 4) == 0) ? 0 : 1;
-  }
-  // Measured (2048 cached tokens, 32 query heads, bytes of K and V counted once):
-  //   * four query heads per KV head, 8 KV heads: the row-contiguous kernel reaches 2250 GB/s at
-  //     batch 64 and 1845 at batch 16 against 2073 / 1579 for one query head per CTA (which re-reads
-  //     K and V through the L2 four times); at batch 4 the latter wins (1057 against 840) because
-  //     the row kernel has too few CTAs to cover the machine;
-  //   * two query heads per KV head (16 KV heads, batch 64): one query head per CTA 3870, row kernel
-  //     3531 -- eight resident CTAs per SM at 64 registers beat two at 221;
-  //   * one query head per KV head: the per-head kernel throughout.
-  const bool few_row_ctas = static_cast<int64_t>(B) * (num_kv_heads / 4) <= 8;
-  if (rows_ok && num_kv_heads % 4 == 0 && g == 4 && !few_row_ctas) {
-    dim3 rgrid(splits, num_kv_heads / 4, B);
-    launch_chained(decode_attn_rows_kernel<4>, rgrid, kDecodeThreads, 0, stream, p);
-    if (splits > 1)
-      launch_chained(decode_combine_kernel, B * num_q_heads, kHeadDim, 0, stream, p.part_out, p.part_ml, p.out, splits);
-    return cudaGetLastError() == cudaSuccess ? 0 : -4;
-  }
-  int gt = (g % 4 == 0) ? 4 : (g % 2 == 0) ? 2 : 1;
-  if (rows_ok && (g == 2 || (g == 4 && num_kv_heads % 4 == 0))) gt = 1;
-  if (gt > gt_cap) gt = gt_cap;
-  dim3 grid(splits, num_kv_heads * (g / gt), B);
-  if (gt == 4)
-    launch_chained(decode_attn_kernel<4>, grid, kDecodeThreads, 0, stream, p);
-  else if (gt == 2)
-    launch_chained(decode_attn_kernel<2>, grid, kDecodeThreads, 0, stream, p);
-  else
-    launch_chained(decode_attn_kernel<1>, grid, kDecodeThreads, 0, stream, p);
-  if (splits > 1)
+  const bool cluster = splits > 1 && splits <= kMaxClusterSplits;
+  const dim3 grid(splits, num_kv_heads * ((g + kMmaRows - 1) / kMmaRows), B);
+  const int rows = g < kMmaRows ? g : kMmaRows;
+  const int rc = cluster ? launch_attn<true>(p, grid, rows, stream) : launch_attn<false>(p, grid, rows, stream);
+  if (rc != 0) return rc;
+  if (splits > kMaxClusterSplits)
     launch_chained(decode_combine_kernel, B * num_q_heads, kHeadDim, 0, stream, p.part_out, p.part_ml, p.out, splits);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -226,7 +226,7 @@ class DecodeEngine(BaseDecodeEngine):
         self.v_pools = [torch.zeros(pool, dtype=torch.bfloat16, device=self.device) for _ in range(d.num_layers)]
         self.page_table = torch.arange(batch * self.max_pages, dtype=torch.int32, device=self.device).reshape(
             batch, self.max_pages)
-        self.splits = decode_ops.default_splits(batch, self.nkv_l, self.nq_l // self.nkv_l, self.max_len, page_size)
+        self.splits = decode_ops.tile_splits(batch, self.nkv_l, self.nq_l // self.nkv_l, self.max_len)
         self._scratch = torch.empty(
             max(1, decode_ops._lib().axb_decode_attn_scratch_floats(batch, self.nq_l, self.splits)),  # pylint: disable=protected-access
             dtype=torch.float32, device=self.device)

@@ -50,8 +50,7 @@ def _lib():
 
 
 def _kernel_shape(batch: int, num_kv_heads: int, group: int) -> tuple[int, int]:
-    """``(CTAs of one split, CTAs that fit one SM)`` of the kernel that the launcher picks (mirrors
-    ``axb_decode_attn``): 128 threads each, residency limited by registers -- 64 with the occupancy
+    """``(CTAs of one split, CTAs that fit one SM)`` that ``default_splits`` reckons with: 128 threads each, residency limited by registers -- 64 with the occupancy
     bound / 125 / 193 for the per-head kernel with 1 / 2 / 4 query heads per CTA, 225 for the
     row-contiguous kernel of four KV heads x four query heads."""
     mode = os.environ.get("AXB_DECODE_ATTN", "")
@@ -66,7 +65,7 @@ def _kernel_shape(batch: int, num_kv_heads: int, group: int) -> tuple[int, int]:
 
 
 def default_splits(batch: int, num_kv_heads: int, group: int, max_len: int, page_size: int, sms: int = 148) -> int:
-    """KV splits: enough CTAs for up to four per SM without splitting below 8 pages; once that grid
+    """KV splits for callers that fix them without ``tile_splits`` (which the engine uses): enough CTAs for up to four per SM without splitting below 8 pages; once that grid
     is more than one wave of resident CTAs, the nearby split count whose last wave is fullest (the
     CTAs of a decode step all run about equally long, so a grid of 1.15 waves takes the time of 2)."""
     ctas, resident = _kernel_shape(batch, num_kv_heads, group)
@@ -84,6 +83,17 @@ def default_splits(batch: int, num_kv_heads: int, group: int, max_len: int, page
     candidates = range(max(1, base - 4), min(smax, base + 7) + 1)
     best = max(fill(s) for s in candidates)
     return next(s for s in candidates if fill(s) >= 0.95 * best)
+
+
+def tile_splits(batch: int, num_kv_heads: int, group: int, max_len: int, sms: int = 148) -> int:
+    """KV splits of a decoding step: one wave of CTAs (three fit an SM; one takes a split, a KV head and eight query
+    heads), since the CTAs of a second wave find no empty SM to start on -- 128 CTAs: 3 splits 27 us, 8 splits 32; 64
+    CTAs: 6 splits 17 us, 8 splits 22 -- and at least half a 16-token tile for each of a CTA's four warps.  Beyond 8, where
+    a second launch merges them, only while 8 would leave most SMs empty (4 CTAs, 3000 tokens: 8.5 us with 16 splits,
+    9.6 with 8 or 32; 16 CTAs: 11 with either)."""
+    ctas = batch * num_kv_heads * ((group + 7) // 8)
+    splits = max(1, min(max_len // 32, 3 * sms // ctas))
+    return min(splits, 8 if 16 * ctas > sms else 16)
 
 
 def paged_decode_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, page_table: torch.Tensor,

@@ -166,7 +166,7 @@ def bench_decode_attn(args) -> dict:
     table = torch.randperm(b * pages, device="cuda").to(torch.int32).reshape(b, pages).contiguous()
     lengths = torch.full((b,), t, dtype=torch.int32, device="cuda")
     q = torch.randn(b, nq, h, device="cuda").bfloat16()
-    splits = args.splits or decode_ops.default_splits(b, nkv, nq // nkv, t, ps)
+    splits = args.splits or decode_ops.tile_splits(b, nkv, nq // nkv, t)
     scratch = torch.empty(decode_ops._lib().axb_decode_attn_scratch_floats(b, nq, splits), device="cuda")  # pylint: disable=protected-access
     out = torch.empty_like(q)
     ours = _time(lambda: decode_ops.paged_decode_attention(q, k, v, table, lengths, splits=splits, out=out,

@@ -35,6 +35,40 @@ def test_paged_decode_attention_matches_reference(nq, nkv, splits):
     assert err < 2e-2 * max(1.0, ref.abs().max().item()), err
 
 
+@pytest.mark.parametrize("nq,nkv", [(3, 3), (12, 4), (16, 2), (12, 1), (20, 2)])
+@pytest.mark.parametrize("page_size,splits", [(4, 1), (12, 2), (16, 5), (16, 8), (20, 9)])
+def test_paged_decode_attention_at_tile_and_split_edges(nq, nkv, page_size, splits):
+    """Lengths around the 16-token tiles and the four warps' stride, rows that leave splits empty, up to eight and more
+    than eight query heads per KV head, cluster merges (2 to 8 splits) and the merge launch (9)."""
+    from axlearn_b200.ops import decode_ops
+
+    lens = [0, 1, 15, 16, 17, 63, 64, 65, 129, 240]
+    b, max_pages, h = len(lens), 240 // page_size, 128
+    k, v, table = _pools(b, max_pages, page_size, nkv, h, seed=splits)
+    lengths = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q = (2 * torch.randn(b, nq, h, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))).bfloat16()
+    out = decode_ops.paged_decode_attention(q, k, v, table, lengths, splits=splits)
+    ref = decode_ops.reference_paged_attention(q[1:], k, v, table[1:], lengths[1:])
+    assert not out[0].any()  # nothing cached
+    # The output's rounding to bf16 (8 significant bits: half a unit is up to 2^-8 of a value), and sums of values of
+    # size max|v| in 32 bits with P to 2^-15.
+    bound = 2.0 ** -8 * ref.abs() + 2.0 ** -14 * v.abs().max().float()
+    assert ((out[1:].float() - ref).abs() <= bound).all()
+
+
+def test_paged_decode_attention_keeps_infinite_values():
+    from axlearn_b200.ops import decode_ops
+
+    k, v, table = _pools(2, 3, 16, 2, 128, seed=3)
+    v[table[0, 1].long(), 5, 1, 7] = float("inf")
+    lengths = torch.tensor([40, 33], dtype=torch.int32, device="cuda")
+    q = torch.randn(2, 4, 128, device="cuda").bfloat16()
+    for splits in (1, 3):
+        out = decode_ops.paged_decode_attention(q, k, v, table, lengths, splits=splits).float()
+        bad = ~torch.isfinite(out)
+        assert (out[0, 2:, 7] == float("inf")).all() and bad.sum() == 2
+
+
 def test_chained_step_sees_new_weights_and_matches_separate_launches():
     """A captured step reads its first weight tiles ahead of the kernels before it: new weights written right before a
     replay have to show, and the logits are those of separately launched kernels bit for bit."""
