@@ -438,6 +438,58 @@ extern "C" int axb_rope_append_paged(const void* qkv, void* q_out, void* k_pool,
 
 namespace axb {
 
+// Whole prompts: qkv [B * T, (Nq + 2 Nkv) * H] of one projection.  Rotates q in place and puts rotated k and plain v into
+// the sequences' runs of the pools (sequence b at token row b * pool_rows), where attention reads them: one pass over
+// the projection, which replaces copies of q, k and v out of it, two rotations and two copies into the pools
+// (a layer's 16384 x 48 heads: 80 us against 445, of 61 at the copy rate; 333 x 24 heads: 3 us against 18).  A thread
+// keeps its (sin, cos) pairs in registers and has four 16-byte loads in flight.
+constexpr int kRopeThreads = 256;
+
+__global__ void __launch_bounds__(kRopeThreads)
+rope_append_prompt_kernel(uint4* __restrict__ qkv, uint4* __restrict__ k_pool, uint4* __restrict__ v_pool,
+                          const float4* __restrict__ table, int64_t rows, int T, int64_t pool_rows, int num_q_heads,
+                          int num_kv_heads) {
+  constexpr int kVecs = kHeadDim / 8, kHeads = kRopeThreads / kVecs, kFlight = 4;
+  const int pv = threadIdx.x % kVecs, h0 = threadIdx.x / kVecs;
+  const int heads = num_q_heads + 2 * num_kv_heads;
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
+    const int64_t b = row / T;
+    const int t = static_cast<int>(row - b * T);
+    const float4* tab = table + static_cast<int64_t>(t) * (kHeadDim / 4) + pv * 2;
+    const float4 sc0 = __ldg(tab), sc1 = __ldg(tab + 1);  // (s0, c0, s1, c1), (s2, c2, s3, c3)
+    const float sn[4] = {sc0.x, sc0.z, sc1.x, sc1.z}, cs[4] = {sc0.y, sc0.w, sc1.y, sc1.w};
+    uint4* src = qkv + row * heads * kVecs + pv;
+    const int64_t slot = (b * pool_rows + t) * num_kv_heads;
+    for (int n0 = h0; n0 < heads; n0 += kHeads * kFlight) {
+      uint4 v[kFlight];
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u)
+        if (n0 + u * kHeads < heads) v[u] = src[(n0 + u * kHeads) * kVecs];
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u) {
+        const int n = n0 + u * kHeads;
+        if (n >= heads) break;
+        if (n >= num_q_heads + num_kv_heads) {
+          v_pool[(slot + n - num_q_heads - num_kv_heads) * kVecs + pv] = v[u];
+          continue;
+        }
+        uint32_t* w = reinterpret_cast<uint32_t*>(&v[u]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = unpack2(w[q]);
+          w[q] = pack2(f.x * cs[q] - f.y * sn[q], f.y * cs[q] + f.x * sn[q]);
+        }
+        if (n < num_q_heads)
+          src[n * kVecs] = v[u];
+        else
+          k_pool[(slot + n - num_q_heads) * kVecs + pv] = v[u];
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ float silu_times(float g, float u) { return g / (1.f + __expf(-g)) * u; }
+
 // out[r, c] = silu(gu[r, c]) * gu[r, F + c] for gu = [rows, 2F] (gate | up packed by one GEMM).
 __global__ void swiglu_packed_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                      int64_t rows, int F) {
@@ -449,20 +501,80 @@ __global__ void swiglu_packed_kernel(const __nv_bfloat16* __restrict__ gu, __nv_
     const int c = static_cast<int>(i % (F / 2)) * 2;
     const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gu + r * 2 * F + c));
     const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gu + r * 2 * F + F + c));
-    const float a = g.x / (1.f + __expf(-g.x)) * u.x;
-    const float b = g.y / (1.f + __expf(-g.y)) * u.y;
-    *reinterpret_cast<__nv_bfloat162*>(out + r * F + c) = __floats2bfloat162_rn(a, b);
+    *reinterpret_cast<__nv_bfloat162*>(out + r * F + c) = __floats2bfloat162_rn(silu_times(g.x, u.x), silu_times(g.y, u.y));
+  }
+}
+
+// The same, 16 bytes a load, for F % 8 == 0 and 16-byte aligned operands: a block takes 256 vectors of one row, so no
+// index is divided, and a thread has four loads in flight.  16384 x 14336: 474 -> 221 us (212 at the copy rate).
+constexpr int kSwigluThreads = 256, kSwigluVecs = 2;
+
+__global__ void __launch_bounds__(kSwigluThreads)
+swiglu_packed_vec_kernel(const uint4* __restrict__ gu, uint4* __restrict__ out, int64_t rows, int vecs) {
+  chain_link();
+  const int c0 = blockIdx.x * (kSwigluThreads * kSwigluVecs) + threadIdx.x;
+  for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
+    uint4 g[kSwigluVecs], u[kSwigluVecs];
+#pragma unroll
+    for (int i = 0; i < kSwigluVecs; ++i) {
+      const int c = c0 + i * kSwigluThreads;
+      if (c < vecs) {
+        g[i] = __ldg(gu + row * 2 * vecs + c);
+        u[i] = __ldg(gu + row * 2 * vecs + vecs + c);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kSwigluVecs; ++i) {
+      const int c = c0 + i * kSwigluThreads;
+      if (c >= vecs) break;
+      uint32_t* gw = reinterpret_cast<uint32_t*>(&g[i]);
+      const uint32_t* uw = reinterpret_cast<const uint32_t*>(&u[i]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 a = unpack2(gw[k]), b = unpack2(uw[k]);
+        gw[k] = pack2(silu_times(a.x, b.x), silu_times(a.y, b.y));
+      }
+      out[row * vecs + c] = g[i];
+    }
   }
 }
 
 }  // namespace axb
 
+// qkv [B * T, (Nq + 2 Nkv) * 128], pools at the first sequence's run, `pool_rows` token rows a sequence (>= T); `table` of
+// axb_rope_table.  Pointers 16-byte aligned.
+extern "C" int axb_rope_append_prompt(void* qkv, void* k_pool, void* v_pool, const float* table, int B, int T,
+                                      int64_t pool_rows, int num_q_heads, int num_kv_heads, int head_dim,
+                                      cudaStream_t stream) {
+  using namespace axb;
+  const uintptr_t align = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_pool) |
+                          reinterpret_cast<uintptr_t>(v_pool) | reinterpret_cast<uintptr_t>(table);
+  if (head_dim != kHeadDim || pool_rows < T || num_q_heads <= 0 || num_kv_heads <= 0 || (align & 15)) return -10;
+  const int64_t rows = static_cast<int64_t>(B) * T;
+  if (rows <= 0) return 0;
+  const int64_t grid = rows < 148 * 16 ? rows : 148 * 16;
+  rope_append_prompt_kernel<<<static_cast<unsigned>(grid), kRopeThreads, 0, stream>>>(
+      static_cast<uint4*>(qkv), static_cast<uint4*>(k_pool), static_cast<uint4*>(v_pool),
+      reinterpret_cast<const float4*>(table), rows, T, pool_rows, num_q_heads, num_kv_heads);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
 extern "C" int axb_swiglu_packed(const void* gu, void* out, int64_t rows, int F, cudaStream_t stream) {
+  using namespace axb;
   if (F % 2) return -10;
   const int64_t total = rows * (F / 2);
   if (total <= 0) return 0;
+  if (F % 8 == 0 && !((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(out)) & 15)) {
+    const int vecs = F / 8;
+    const dim3 grid((vecs + kSwigluThreads * kSwigluVecs - 1) / (kSwigluThreads * kSwigluVecs),
+                    static_cast<unsigned>(rows < 65535 ? rows : 65535));
+    launch_chained(swiglu_packed_vec_kernel, grid, kSwigluThreads, 0, stream, static_cast<const uint4*>(gu),
+                   static_cast<uint4*>(out), rows, vecs);
+    return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  }
   int64_t ctas = (total + 255) / 256;
   if (ctas > 148 * 8) ctas = 148 * 8;
-  axb::launch_chained(axb::swiglu_packed_kernel, static_cast<int>(ctas), 256, 0, stream, static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), rows, F);
+  launch_chained(swiglu_packed_kernel, static_cast<unsigned>(ctas), 256, 0, stream, static_cast<const __nv_bfloat16*>(gu),
+                 static_cast<__nv_bfloat16*>(out), rows, F);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -445,7 +445,7 @@ __global__ void rope_table_kernel(const int64_t* __restrict__ pos, float2* __res
   const int i = idx % hp, t = idx / hp;
   const float inv_freq = exp2f(-(2.f * i / H) * log2_theta);
   float s, c;
-  sincosf(static_cast<float>(pos[t]) * inv_freq, &s, &c);
+  sincosf(static_cast<float>(pos != nullptr ? pos[t] : t) * inv_freq, &s, &c);
   table[idx] = make_float2(s, c);
 }
 
@@ -1022,6 +1022,16 @@ extern "C" int axb_rope(const void* x, void* y, const int64_t* positions, int64_
         static_cast<const bf16*>(x), static_cast<bf16*>(y), positions, B, T, N, H, log2f(theta),
         backward ? -1.f : 1.f);
   }
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+// table [T, H / 2] of (sin, cos) for positions 0 .. T - 1.
+extern "C" int axb_rope_table(float* table, int T, int H, float theta, cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (H <= 0 || H % 2) return -10;
+  const int hp = H / 2;
+  rope_table_kernel<<<(T * hp + 255) / 256, 256, 0, stream>>>(nullptr, reinterpret_cast<float2*>(table), T, hp, H,
+                                                              log2f(theta));
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

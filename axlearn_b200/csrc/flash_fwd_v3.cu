@@ -554,7 +554,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (!kStrided && ok && row < p.T) {
       __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) +
                             ((static_cast<int64_t>(batch) * p.T + row) * p.N + head) * H + half * (H / 2);
-      if (half == 0) {
+      if (half == 0 && p.lse != nullptr) {
         p.lse[(static_cast<int64_t>(batch) * p.N + head) * p.T + row] =
             (l_sum > 0.f) ? (m_ref * 0.6931471805599453f + logf(l_sum)) : -INFINITY;
       }
@@ -681,14 +681,18 @@ __global__ void seg_tile_ranges_kernel(const int* __restrict__ q_seg, const int*
 }
 
 // Heads of `h` columns starting at column 0 of rows `ld` elements apart.
-static int make_packed_map(CUtensorMap* map, const void* base, int B, int L, int N, int h, int64_t ld) {
+static int make_strided_map(CUtensorMap* map, const void* base, int B, int L, int N, int h, int64_t ld, int64_t batch_ld) {
   uint64_t dims[4] = {static_cast<uint64_t>(h), static_cast<uint64_t>(N), static_cast<uint64_t>(L),
                       static_cast<uint64_t>(B)};
   uint64_t strides[3] = {static_cast<uint64_t>(h) * 2, static_cast<uint64_t>(ld) * 2,
-                         static_cast<uint64_t>(L) * ld * 2};
+                         static_cast<uint64_t>(batch_ld) * 2};
   uint32_t box[4] = {64, 1, 128, 1};
   return make_tensor_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box,
                          CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+static int make_packed_map(CUtensorMap* map, const void* base, int B, int L, int N, int h, int64_t ld) {
+  return make_strided_map(map, base, B, L, N, h, ld, L * ld);
 }
 
 template <int H, bool kGeneral, bool kGated, bool kLatent>
@@ -773,6 +777,35 @@ extern "C" int axb_flash_fwd_v3(const void* q, const void* k, const void* v, voi
     return general ? launch_flash_fwd3<128, true>(q, k, v, p, stream) : launch_flash_fwd3<128, false>(q, k, v, p, stream);
   }
   return general ? launch_flash_fwd3<64, true>(q, k, v, p, stream) : launch_flash_fwd3<64, false>(q, k, v, p, stream);
+}
+
+// Causal attention of whole prompts read where they lie: q rows are q_ld apart (sequences q_batch), k and v rows kv_ld
+// (kv_batch), as in a packed projection and a KV cache; head h of a row at column h * H, H of 64 or 128.  Pitches are
+// multiples of 8, pointers 16-byte aligned; out [B, T, N, H] contiguous.
+extern "C" int axb_flash_fwd_strided(const void* q, const void* k, const void* v, void* out, int B, int T, int N, int Nkv,
+                                     int H, int64_t q_ld, int64_t q_batch, int64_t kv_ld, int64_t kv_batch,
+                                     float softmax_scale, int* status, cudaStream_t stream) {
+  using namespace axb;
+  if (B <= 0 || T <= 0 || N <= 0 || Nkv <= 0 || N % Nkv != 0 || (H != 64 && H != 128) ||
+      ((q_ld | q_batch | kv_ld | kv_batch) % 8) || q_ld < static_cast<int64_t>(N) * H ||
+      kv_ld < static_cast<int64_t>(Nkv) * H)
+    return -10;
+  const uintptr_t align = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
+                          reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out);
+  if (align & 15) return -10;
+  FlashFwd3Params p;
+  p.out = out, p.lse = nullptr;
+  p.q_seg = nullptr, p.k_seg = nullptr, p.ranges = nullptr;
+  p.B = B, p.T = T, p.S = T, p.N = N, p.Nkv = Nkv, p.H = H;
+  p.sc = softmax_scale * 1.4426950408889634f, p.cap_in = 0.f, p.cap_out = 0.f;
+  p.causal = 1, p.q_offset = 0, p.window = -1, p.status = status;
+  p.gate = nullptr, p.gate_ld = 0, p.out_ld = 0, p.vdim = H, p.every = 1, p.bias = 0, p.rot_dim = 0, p.coef = 0.f;
+  CUtensorMap tq, tk, tv;
+  if (make_strided_map(&tq, q, B, T, N, H, q_ld, q_batch) || make_strided_map(&tk, k, B, T, Nkv, H, kv_ld, kv_batch) ||
+      make_strided_map(&tv, v, B, T, Nkv, H, kv_ld, kv_batch))
+    return -2;
+  if (H == 128) return run_flash_fwd3<128, false, false, false>(tq, tk, tv, tq, tk, p, stream);
+  return run_flash_fwd3<64, false, false, false>(tq, tk, tv, tq, tk, p, stream);
 }
 
 // Gated sliding-window attention of whole prompts (positions from 0), see window_attn.cu for the formula.

@@ -36,7 +36,7 @@ from typing import Any, Optional
 import torch
 
 from axlearn_b200.common.utils import flatten_items
-from axlearn_b200.ops import attention_ops, cuda_ops, decode_ops
+from axlearn_b200.ops import cuda_ops, decode_ops
 
 Tensor = torch.Tensor
 
@@ -256,6 +256,19 @@ class DecodeEngine(BaseDecodeEngine):
         return self._allreduce.finish(site, residual=residual.reshape(-1)).reshape(residual.shape)
 
     # ------------------------------------------------------------------ prefill
+    def _add_norm(self, x: Tensor, branch: Optional[Tensor], scale: Tensor) -> tuple[Tensor, Tensor]:
+        """``x + branch`` (``x`` without a branch) and its norm, in one pass where the kernel takes the width."""
+        if branch is None:
+            return x, cuda_ops.rms_norm(x, scale, self.dims.norm_eps)
+        return cuda_ops.add_rms_norm(x, branch, scale, self.dims.norm_eps)
+
+    def _sum_ranks(self, x: Tensor) -> Tensor:
+        if self.world > 1:
+            import torch.distributed as dist
+
+            dist.all_reduce(x, group=self.group)
+        return x
+
     @torch.no_grad()
     def prefill(self, prompt_ids: Tensor, lengths: Optional[Tensor] = None) -> Tensor:
         """Runs the prompts ``[batch, T]``, fills the caches and returns the greedy first token of
@@ -267,40 +280,29 @@ class DecodeEngine(BaseDecodeEngine):
         assert b == self.batch and t <= self.max_len
         h = d.head_dim
         per_chunk = max(1, self._prefill_chunk_tokens // t)
-        positions = torch.arange(t, device=self.device)
+        table = decode_ops.rope_table(t, h, d.rope_theta, self.device)
         last_hidden = torch.empty((b, d.hidden_dim), dtype=torch.bfloat16, device=self.device)
         for b0 in range(0, b, per_chunk):
             b1 = min(b, b0 + per_chunk)
             x = self.w["emb"][prompt_ids[b0:b1]]                              # [bs, T, D]
+            branch = None  # what the last product adds to x: summed inside the next norm
             for li, lw in enumerate(self.w["layers"]):
-                hn = cuda_ops.rms_norm(x, lw.attn_norm, d.norm_eps)
-                qkv = cuda_ops.linear(hn, lw.wqkv).reshape(b1 - b0, t, self.nq_l + 2 * self.nkv_l, h)
-                q = cuda_ops.rope(qkv[:, :, :self.nq_l], positions, d.rope_theta)
-                k = cuda_ops.rope(qkv[:, :, self.nq_l:self.nq_l + self.nkv_l], positions, d.rope_theta)
-                v = qkv[:, :, self.nq_l + self.nkv_l:].contiguous()
-                kp = self.k_pools[li].view(b, self.max_len, self.nkv_l, h)
-                vp = self.v_pools[li].view(b, self.max_len, self.nkv_l, h)
-                kp[b0:b1, :t] = k
-                vp[b0:b1, :t] = v
-                attn = attention_ops.flash_attention(q, k, v, causal=True, softmax_scale=self._softmax_scale)
-                o = cuda_ops.linear(attn.reshape(b1 - b0, t, self.nq_l * h), lw.wo)
-                if self.world > 1:
-                    import torch.distributed as dist
-
-                    dist.all_reduce(o, group=self.group)
-                x = x + o
-                hn = cuda_ops.rms_norm(x, lw.ffn_norm, d.norm_eps)
+                x, hn = self._add_norm(x, branch, lw.attn_norm)
+                qkv = cuda_ops.linear(hn, lw.wqkv)
+                attn = decode_ops.prompt_attention(
+                    qkv, self.k_pools[li].view(b, self.max_len, self.nkv_l, h)[b0:b1],
+                    self.v_pools[li].view(b, self.max_len, self.nkv_l, h)[b0:b1], table, num_q_heads=self.nq_l,
+                    softmax_scale=self._softmax_scale)
+                branch = self._sum_ranks(cuda_ops.linear(attn, lw.wo))
+                x, hn = self._add_norm(x, branch, lw.ffn_norm)
                 gu = cuda_ops.linear(hn, lw.wgu)
                 act = decode_ops.swiglu_packed(gu.reshape(-1, gu.shape[-1]))
-                dn = cuda_ops.linear(act, lw.wdown).reshape(x.shape)
-                if self.world > 1:
-                    dist.all_reduce(dn, group=self.group)
-                x = x + dn
+                branch = self._sum_ranks(cuda_ops.linear(act, lw.wdown).reshape(x.shape))
             if lengths is None:
-                last_hidden[b0:b1] = x[:, -1]
+                last = (slice(None), -1)
             else:
-                idx = (lengths[b0:b1].long() - 1).clamp(min=0)
-                last_hidden[b0:b1] = x[torch.arange(b1 - b0, device=self.device), idx]
+                last = (torch.arange(b1 - b0, device=self.device), (lengths[b0:b1].long() - 1).clamp(min=0))
+            last_hidden[b0:b1] = x[last] if branch is None else x[last] + branch[last]
         if lengths is None:
             self.lengths.fill_(t)
         else:

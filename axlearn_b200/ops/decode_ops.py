@@ -37,6 +37,14 @@ def _lib():
         h.axb_rope_append_paged.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                             c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p]
         h.axb_rope_append_paged.restype = c_int
+        h.axb_rope_table.argtypes = [c_void_p, c_int, c_int, c_float, c_void_p]
+        h.axb_rope_table.restype = c_int
+        h.axb_rope_append_prompt.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int64, c_int,
+                                             c_int, c_int, c_void_p]
+        h.axb_rope_append_prompt.restype = c_int
+        h.axb_flash_fwd_strided.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                            c_int64, c_int64, c_int64, c_int64, c_float, c_void_p, c_void_p]
+        h.axb_flash_fwd_strided.restype = c_int
         h.axb_swiglu_packed.argtypes = [c_void_p, c_void_p, c_int64, c_int, c_void_p]
         h.axb_swiglu_packed.restype = c_int
         h.axb_allreduce_push.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
@@ -150,6 +158,35 @@ def rope_append_paged(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Ten
                                       cuda_ops._stream())  # pylint: disable=protected-access
     cuda_ops._check(rc, "axb_rope_append_paged")  # pylint: disable=protected-access
     return q_out
+
+
+def rope_table(length: int, dim: int, theta: float, device) -> torch.Tensor:
+    """fp32 ``[length, dim / 2, 2]``: (sin, cos) of positions ``0 .. length - 1``, for ``prompt_attention``."""
+    table = torch.empty((length, dim // 2, 2), dtype=torch.float32, device=device)
+    rc = _lib().axb_rope_table(table.data_ptr(), length, dim, theta, cuda_ops._stream())  # pylint: disable=protected-access
+    cuda_ops._check(rc, "axb_rope_table")  # pylint: disable=protected-access
+    return table
+
+
+def prompt_attention(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, table: torch.Tensor, *,
+                     num_q_heads: int, softmax_scale: float) -> torch.Tensor:
+    """Whole prompts from position 0: ``qkv [B, T, (Nq + 2 Nkv) * H]`` of one projection (its q columns are rotated
+    in place), pools ``[B, S, Nkv, H]`` with S >= T token rows a sequence, which get rotated k and plain v and are what
+    causal attention reads.  Returns ``[B, T, Nq * H]``."""
+    b, t, width = qkv.shape
+    _, rows, nkv, h = k_pool.shape
+    assert qkv.is_contiguous() and k_pool.is_contiguous() and v_pool.is_contiguous() and k_pool.shape[0] == b
+    assert width == (num_q_heads + 2 * nkv) * h and table.shape[0] >= t and table.is_contiguous()
+    stream = cuda_ops._stream()  # pylint: disable=protected-access
+    rc = _lib().axb_rope_append_prompt(qkv.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), table.data_ptr(), b, t,
+                                       rows, num_q_heads, nkv, h, stream)
+    cuda_ops._check(rc, "axb_rope_append_prompt")  # pylint: disable=protected-access
+    out = torch.empty((b, t, num_q_heads * h), dtype=qkv.dtype, device=qkv.device)
+    rc = _lib().axb_flash_fwd_strided(qkv.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(), b, t,
+                                      num_q_heads, nkv, h, width, t * width, nkv * h, rows * nkv * h, softmax_scale,
+                                      cuda_ops.status_word(qkv.device).data_ptr(), stream)
+    cuda_ops._check(rc, "axb_flash_fwd_strided")  # pylint: disable=protected-access
+    return out
 
 
 def swiglu_packed(gu: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -122,6 +122,37 @@ def test_rope_append_writes_page_slot_and_rotates():
     assert torch.equal(k, k0) and torch.equal(v, v0)
 
 
+@pytest.mark.parametrize("b,t,nq,nkv", [(1, 1, 4, 4), (2, 127, 6, 2), (3, 129, 16, 1), (1, 300, 40, 8)])
+def test_prompt_attention_equals_rotation_copies_and_attention(b, t, nq, nkv):
+    """Bit for bit what separate rotations, copies into the cache and attention on contiguous tensors give; rows of the
+    cache beyond the prompts stay."""
+    from axlearn_b200.ops import attention_ops, cuda_ops, decode_ops
+
+    h, rows = 128, t + 5
+    qkv = torch.randn(b, t, (nq + 2 * nkv) * h, device="cuda").bfloat16()
+    kp, vp = (torch.full((b, rows, nkv, h), 7.0, device="cuda").bfloat16() for _ in range(2))
+    x, pos = qkv.clone().reshape(b, t, nq + 2 * nkv, h), torch.arange(t, device="cuda")
+    q, k = cuda_ops.rope(x[:, :, :nq], pos, 5e5), cuda_ops.rope(x[:, :, nq:nq + nkv], pos, 5e5)
+    v = x[:, :, nq + nkv:].contiguous()
+    want = attention_ops.flash_attention(q, k, v, causal=True, softmax_scale=0.1)
+    got = decode_ops.prompt_attention(qkv, kp, vp, decode_ops.rope_table(t, h, 5e5, "cuda"), num_q_heads=nq,
+                                      softmax_scale=0.1)
+    cuda_ops.check_status()
+    assert torch.equal(kp[:, :t], k) and torch.equal(vp[:, :t], v) and (kp[:, t:] == 7).all() and (vp[:, t:] == 7).all()
+    assert torch.equal(got.reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("rows,f", [(1, 8), (3, 98), (2, 4096), (5, 4104), (70000, 16)])
+def test_swiglu_packed_sizes(rows, f):
+    """Vector and pairwise paths, around a block's 512 vectors, and more rows than a grid is high."""
+    from axlearn_b200.ops import decode_ops
+
+    gu = torch.randn(rows, 2 * f, device="cuda").bfloat16()
+    ref = torch.nn.functional.silu(gu[:, :f].double()) * gu[:, f:].double()
+    # Rounding to bf16, and a 32-bit sigmoid to about 2^-20 of itself.
+    assert ((decode_ops.swiglu_packed(gu).double() - ref).abs() <= (2.0 ** -8 + 2.0 ** -18) * ref.abs() + 1e-30).all()
+
+
 def test_swiglu_packed():
     from axlearn_b200.ops import decode_ops
 
