@@ -36,7 +36,7 @@ from typing import Any, Optional
 import torch
 
 from axlearn_b200.common.utils import flatten_items
-from axlearn_b200.ops import cuda_ops, decode_ops
+from axlearn_b200.ops import cuda_ops, decode_ops, step_ops
 
 Tensor = torch.Tensor
 
@@ -307,14 +307,15 @@ class DecodeEngine(BaseDecodeEngine):
             self.lengths.fill_(t)
         else:
             self.lengths.copy_(lengths.to(self.lengths.dtype))
-        self.logits.copy_(self._logits(last_hidden))
-        self.tokens.copy_(self.logits.argmax(dim=-1))
+        self._logits(last_hidden)
+        step_ops.step_end(self.logits, self.tokens)
         self._check_status()
         return self.tokens.clone()
 
-    def _logits(self, hidden: Tensor) -> Tensor:
+    def _logits(self, hidden: Tensor) -> None:
+        """Output norm and head, into ``self.logits``."""
         hn = cuda_ops.rms_norm(hidden, self.w["final_norm"], self.dims.norm_eps)
-        return cuda_ops.gemm(hn, self.w["head"].t(), out_dtype=torch.float32, resident=True)
+        cuda_ops.gemm(hn, self.w["head"].t(), out=self.logits, resident=True)
 
     # ------------------------------------------------------------------ decode
     def _step(self) -> None:
@@ -322,10 +323,14 @@ class DecodeEngine(BaseDecodeEngine):
         its K/V, and leaves the next token in ``self.tokens``."""
         d = self.dims
         before = cuda_ops.launch_count
-        self.lengths.add_(1).clamp_(max=self.max_len)   # rows that ran out of room rewrite their last slot
         if self._allreduce is not None:
             self._allreduce.begin_step()
-        x = self.w["emb"][self.tokens]                                        # [B, D]
+        # Rows that ran out of room rewrite their last slot.
+        if step_ops.embed_rows_supported(self.w["emb"], self.tokens):
+            x = step_ops.embed_rows(self.w["emb"], self.tokens, wrap=True, lengths=self.lengths, max_len=self.max_len)
+        else:
+            self.lengths.add_(1).clamp_(max=self.max_len)
+            x = self.w["emb"][self.tokens]                                    # [B, D]
         for li, lw in enumerate(self.w["layers"]):
             hn = cuda_ops.rms_norm(x, lw.attn_norm, d.norm_eps)
             qkv = cuda_ops.gemm(hn, lw.wqkv, resident=True)
@@ -346,8 +351,8 @@ class DecodeEngine(BaseDecodeEngine):
                 x = self._gemm_reduce(act, lw.wdown, x, 2 * li + 1)
             else:
                 cuda_ops.gemm(act, lw.wdown, out=x, accumulate=True, resident=True)
-        self.logits.copy_(self._logits(x))
-        self.tokens.copy_(self.logits.argmax(dim=-1))
+        self._logits(x)
+        step_ops.step_end(self.logits, self.tokens)
         self.launches_per_step = cuda_ops.launch_count - before
 
 
@@ -409,8 +414,7 @@ class ModuleDecodeEngine(BaseDecodeEngine):
                 inside = torch.nonzero((at_rows >= b0) & (at_rows < b1))[:, 0]
                 picked.append((inside, hidden[at_rows[inside] - b0, at_pos[inside]]))
         self.lengths.copy_(lengths)
-        self.logits.copy_(self._logits(torch.cat(last)))
-        self.tokens.copy_(self.logits.argmax(dim=-1))
+        step_ops.step_end(self._logits(torch.cat(last)), self.tokens, logits_out=self.logits)
         if logits_at is None:
             self._check_status()
             return self.tokens.clone()
@@ -432,26 +436,29 @@ class ModuleDecodeEngine(BaseDecodeEngine):
         live = live.to(device=self.device, dtype=torch.int32)
         states, out = self._call("extend_step", cached_states=self.states, input_ids=token_ids.to(self.device),
                                  live_step_len=live)
-        self._keep(states)
+        for mine, new in self._changed(states):
+            mine.copy_(new)
         self.lengths.add_(live)
         logits = out["logits"].float()
         self.logits.copy_(logits[torch.arange(b, device=self.device), (live.long() - 1).clamp(min=0)])
         self._check_status()
         return logits
 
-    def _keep(self, states: dict) -> None:
-        for (_, mine), (_, new) in zip(flatten_items(self.states), flatten_items(states)):
-            if mine.data_ptr() != new.data_ptr():
-                mine.copy_(new)
+    def _changed(self, states: dict) -> list:
+        """``(own buffer, new tensor)`` of the states that a call did not change in place."""
+        return [(mine, new) for (_, mine), (_, new) in zip(flatten_items(self.states), flatten_items(states))
+                if mine.data_ptr() != new.data_ptr()]
 
     def _step(self) -> None:
         before = cuda_ops.launch_count
         states, out = self._call("extend_step", cached_states=self.states, input_ids=self.tokens[:, None],
                                  live_step_len=self.active)
-        self._keep(states)
-        self.lengths.add_(self.active)
-        self.logits.copy_(out["logits"][:, -1])
-        self.tokens.copy_(self.logits.argmax(dim=-1))
+        kept = self._changed(states)
+        for mine, new in kept:
+            if mine.shape != (self.batch,):
+                mine.copy_(new)
+        step_ops.step_end(out["logits"][:, -1], self.tokens, logits_out=self.logits, lengths=self.lengths,
+                          active=self.active, kept=[pair for pair in kept if pair[0].shape == (self.batch,)])
         self.launches_per_step = cuda_ops.launch_count - before
 
 

@@ -98,6 +98,45 @@ def test_chained_step_sees_new_weights_and_matches_separate_launches():
         tokens = plain.argmax(dim=-1)
 
 
+@pytest.mark.parametrize("b,v,ld", [(1, 1, 4), (3, 33, 40), (2, 4096, 4096), (5, 32768, 32768), (2, 32772, 32776)])
+def test_step_end_picks_as_torch_and_keeps(b, v, ld):
+    """Vector and element paths around one pass of the block; ties go to the first, NaN above all."""
+    from axlearn_b200.ops import step_ops
+
+    g = torch.Generator(device="cuda").manual_seed(v)
+    logits = torch.randint(-50, 50, (b, ld), device="cuda", generator=g).float()[:, :v]
+    if v > 1:
+        logits[0] = float("-inf")
+    if b > 2:
+        logits[1, [v // 3, v // 2]] = float("nan")
+    tokens = torch.full((b,), -1, dtype=torch.int64, device="cuda")
+    lengths, active = (torch.arange(b, dtype=torch.int32, device="cuda") + i for i in range(2))
+    kept = [(torch.zeros(b, dtype=torch.int32, device="cuda"), lengths + 10 * i) for i in range(3)]
+    copy = torch.empty((b, v), device="cuda")
+    want_lengths = lengths + active
+    step_ops.step_end(logits, tokens, logits_out=copy, lengths=lengths, active=active, kept=kept)
+    # numpy names the first of equals, and the first NaN.
+    assert tokens.tolist() == logits.cpu().numpy().argmax(axis=-1).tolist()
+    assert torch.equal(copy.nan_to_num(99.0), logits.nan_to_num(99.0))
+    assert torch.equal(lengths, want_lengths) and all(torch.equal(x, y) for x, y in kept)
+
+
+@pytest.mark.parametrize("width", [8, 264, 2048, 4104])
+def test_embed_rows_gathers_and_marks_bad_ids(width):
+    from axlearn_b200.ops import cuda_ops, step_ops
+
+    table = torch.randn(7, width, device="cuda").bfloat16()
+    ids = torch.tensor([[6], [0], [-2]], device="cuda")
+    lengths = torch.tensor([3, 8, 9], dtype=torch.int32, device="cuda")
+    out = step_ops.embed_rows(table, ids, wrap=True, lengths=lengths, max_len=9)
+    assert torch.equal(out, table[ids]) and lengths.tolist() == [4, 9, 9]
+    cuda_ops.check_status()
+    out = step_ops.embed_rows(table, ids)
+    assert torch.equal(out[:2], table[ids[:2]]) and out[2].isnan().all()
+    with pytest.raises(RuntimeError, match="status 5"):
+        cuda_ops.check_status()
+
+
 def test_rope_append_writes_page_slot_and_rotates():
     from axlearn_b200.ops import decode_ops, reference
 
