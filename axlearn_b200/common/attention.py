@@ -1288,7 +1288,7 @@ def scaled_hidden_dim(scale: float = 4, *, round_up_to_multiples_of: Optional[in
 def _first_model_axis(linear) -> Any:
     """Output-dim entry of a linear's partition spec (tensor parallel layers route their input
     through a gradient all-reduce, which makes a new tensor per linear)."""
-    spec = getattr(linear.config, "param_partition_spec", None)
+    spec = getattr(linear._config, "param_partition_spec", None)  # pylint: disable=protected-access
     return spec[-1] if spec else None
 
 
@@ -1450,7 +1450,7 @@ class TransformerLayer(BaseTransformerLayer):
                          attention_logit_biases=self_attention_logit_biases, return_aux=return_aux)
         # Pre-norm blocks hand the attention branch to the feed-forward layer unsummed: its
         # normalisation adds it (one pass instead of an add and a norm).
-        defer = (mode == ForwardMode.FORWARD and self.self_attention.config.structure == "prenorm"
+        defer = (mode == ForwardMode.FORWARD and self.self_attention._config.structure == "prenorm"  # pylint: disable=protected-access
                  and getattr(self.feed_forward, "ACCEPTS_PENDING_RESIDUAL", False)
                  and not (cross_attention_data is not None and "cross_attention" in self._children))
         if mode == ForwardMode.FORWARD:

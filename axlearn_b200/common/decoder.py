@@ -238,9 +238,9 @@ class Decoder(BaseLayer):
         with child_context("emb"):
             with child_context("token_emb"):
                 w = emb.token_emb._weight()  # pylint: disable=protected-access
-                if coll.has_axis((emb.token_emb.config.param_partition_spec or (None, None))[1], "model"):
+                if coll.has_axis((emb.token_emb._config.param_partition_spec or (None, None))[1], "model"):
                     w = coll.all_gather(w, "model", dim=1)
-        return w, getattr(emb.config, "soft_cap_logits", None)
+        return w, getattr(emb._config, "soft_cap_logits", None)  # pylint: disable=protected-access
 
     # ------------------------------------------------------------------ decoding
     def init_states(self, *, batch_size: int, max_sequence_length: int, dtype=None, device=None) -> dict:

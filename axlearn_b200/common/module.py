@@ -110,6 +110,18 @@ def propagate_repeated_output_collections(
 # --------------------------------------------------------------------------------------
 
 
+class _ChildKey:
+    """A child's PRNG key that is derived when it is first read: few modules draw random numbers."""
+
+    __slots__ = ("context", "name")
+
+    def __init__(self, context: "InvocationContext", name: str):
+        self.context, self.name = context, name
+
+    def derive(self) -> torch.Tensor:
+        return prng.fold_in(self.context.prng_key, _name_hash(self.name))
+
+
 @dataclasses.dataclass
 class InvocationContext:
     name: str
@@ -150,7 +162,7 @@ class InvocationContext:
             kwargs["state"] = st.get(name, {}) if isinstance(st, dict) else {}
         if "prng_key" not in overrides:
             kwargs["prng_key"] = (
-                None if self.prng_key is None else prng.fold_in(self.prng_key, _name_hash(name))
+                None if self._prng_key is None else _ChildKey(self, name)  # pylint: disable=no-member
             )
         if "output_collection" not in overrides:
             kwargs["output_collection"] = self.output_collection.get_or_add_child(name)
@@ -188,6 +200,20 @@ class InvocationContext:
         return call
 
 
+def _get_prng_key(self: InvocationContext) -> Optional[torch.Tensor]:
+    if isinstance(self._prng_key, _ChildKey):  # pylint: disable=protected-access
+        self._prng_key = self._prng_key.derive()  # pylint: disable=protected-access
+    return self._prng_key  # pylint: disable=protected-access
+
+
+def _set_prng_key(self: InvocationContext, value) -> None:
+    self._prng_key = value  # pylint: disable=protected-access
+
+
+InvocationContext.prng_key = property(_get_prng_key, _set_prng_key)
+
+
+@functools.lru_cache(maxsize=4096)
 def _name_hash(name: str) -> int:
     return int(hashlib.md5(name.encode()).hexdigest(), 16) % (2**31 - 1)
 
@@ -268,8 +294,12 @@ def _wrap_method(fn: Callable) -> Callable:
             finally:
                 torch.cuda.nvtx.range_pop()
         try:
-            with set_current_context(target):
+            stack = _tls.stack
+            stack.append(target)
+            try:
                 out = self._call_in_context(fn, args, kwargs)
+            finally:
+                stack.pop()
             if debug_utils.active_checks():
                 debug_utils.check_outputs(out, where=f"{self.path()} [{type(self).__name__}.{fn.__name__}]")
             return out

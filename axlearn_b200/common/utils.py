@@ -105,6 +105,9 @@ def flatten_items(
     def walk(prefix: str, node: Any):
         if node is None:
             return
+        if isinstance(node, torch.Tensor):
+            out.append((prefix, node))
+            return
         kids = None if (is_leaf is not None and is_leaf(node)) else _children(node)
         if kids is None:
             out.append((prefix, node))

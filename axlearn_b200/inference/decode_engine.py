@@ -260,7 +260,14 @@ class DecodeEngine(BaseDecodeEngine):
         """``x + branch`` (``x`` without a branch) and its norm, in one pass where the kernel takes the width."""
         if branch is None:
             return x, cuda_ops.rms_norm(x, scale, self.dims.norm_eps)
-        return cuda_ops.add_rms_norm(x, branch, scale, self.dims.norm_eps)
+        y, total, _ = cuda_ops._rmsnorm_forward(  # pylint: disable=protected-access
+            x, branch, scale.to(torch.bfloat16).contiguous(), self.dims.norm_eps)
+        return total, y
+
+    @staticmethod
+    def _product(x: Tensor, w: Tensor) -> Tensor:
+        """``x [rows, K] @ w``: the kernel without an autograd node around it where it takes the sizes."""
+        return cuda_ops.linear(x, w) if x.shape[1] % 8 or w.shape[1] % 8 else cuda_ops.gemm(x, w)
 
     def _sum_ranks(self, x: Tensor) -> Tensor:
         if self.world > 1:
@@ -284,25 +291,26 @@ class DecodeEngine(BaseDecodeEngine):
         last_hidden = torch.empty((b, d.hidden_dim), dtype=torch.bfloat16, device=self.device)
         for b0 in range(0, b, per_chunk):
             b1 = min(b, b0 + per_chunk)
-            x = self.w["emb"][prompt_ids[b0:b1]]                              # [bs, T, D]
+            rows = (b1 - b0) * t
+            x = self.w["emb"][prompt_ids[b0:b1].reshape(rows)]                # [bs * T, D]
             branch = None  # what the last product adds to x: summed inside the next norm
             for li, lw in enumerate(self.w["layers"]):
                 x, hn = self._add_norm(x, branch, lw.attn_norm)
-                qkv = cuda_ops.linear(hn, lw.wqkv)
+                qkv = self._product(hn, lw.wqkv).reshape(b1 - b0, t, -1)
                 attn = decode_ops.prompt_attention(
                     qkv, self.k_pools[li].view(b, self.max_len, self.nkv_l, h)[b0:b1],
                     self.v_pools[li].view(b, self.max_len, self.nkv_l, h)[b0:b1], table, num_q_heads=self.nq_l,
                     softmax_scale=self._softmax_scale)
-                branch = self._sum_ranks(cuda_ops.linear(attn, lw.wo))
+                branch = self._sum_ranks(self._product(attn.reshape(rows, self.nq_l * h), lw.wo))
                 x, hn = self._add_norm(x, branch, lw.ffn_norm)
-                gu = cuda_ops.linear(hn, lw.wgu)
-                act = decode_ops.swiglu_packed(gu.reshape(-1, gu.shape[-1]))
-                branch = self._sum_ranks(cuda_ops.linear(act, lw.wdown).reshape(x.shape))
+                act = decode_ops.swiglu_packed(self._product(hn, lw.wgu))
+                branch = self._sum_ranks(self._product(act, lw.wdown))
             if lengths is None:
                 last = (slice(None), -1)
             else:
                 last = (torch.arange(b1 - b0, device=self.device), (lengths[b0:b1].long() - 1).clamp(min=0))
-            last_hidden[b0:b1] = x[last] if branch is None else x[last] + branch[last]
+            x = x.view(b1 - b0, t, -1)
+            last_hidden[b0:b1] = x[last] if branch is None else x[last] + branch.view(x.shape)[last]
         if lengths is None:
             self.lengths.fill_(t)
         else:

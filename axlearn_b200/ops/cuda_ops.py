@@ -105,7 +105,7 @@ class _Sigs:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())  # pylint: disable=protected-access
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -166,26 +166,30 @@ def _sm_count(device: torch.device) -> int:
     return _sm_counts[idx]
 
 
+def _layout(t: torch.Tensor, contraction_dim: int):
+    """``(mn_major flag, leading dim)`` of a 2-D operand that the kernels read as it lies, else None."""
+    inner, outer = t.stride(contraction_dim), t.stride(1 - contraction_dim)
+    # Degenerate dims (size 1) can make both strides look contiguous; prefer K-major.
+    if inner == 1 and outer % 8 == 0 and outer >= t.shape[contraction_dim]:
+        return 0, outer
+    if outer == 1 and inner % 8 == 0 and inner >= t.shape[1 - contraction_dim]:
+        return 1, inner
+    return None
+
+
 def _operand(t: torch.Tensor, contraction_dim: int) -> tuple[torch.Tensor, int, int]:
     """Returns (tensor, mn_major flag, leading dim) for a 2-D bf16 operand whose contraction
     dim is ``contraction_dim``; copies only if the layout is unusable."""
-    other = 1 - contraction_dim
-
-    def usable(x):
-        if x.stride(contraction_dim) == 1 and x.stride(other) % 8 == 0 and x.stride(other) >= x.shape[contraction_dim]:
-            return 0, x.stride(other)
-        if x.stride(other) == 1 and x.stride(contraction_dim) % 8 == 0 and x.stride(contraction_dim) >= x.shape[other]:
-            return 1, x.stride(contraction_dim)
-        return None
-
-    # Degenerate dims (size 1) can make both strides look contiguous; prefer K-major.
-    u = usable(t) if t.data_ptr() % 16 == 0 else None
+    u = _layout(t, contraction_dim) if t.data_ptr() % 16 == 0 else None
     if u is None:
         t = t.contiguous()
-        u = usable(t)
+        u = _layout(t, contraction_dim)
         if u is None:
             raise ValueError(f"GEMM operand of shape {tuple(t.shape)} needs dims that are multiples of 8")
     return t, u[0], u[1]
+
+
+_chain = threading.local()
 
 
 @contextlib.contextmanager
@@ -194,10 +198,12 @@ def chained_launches():
     decoding step, whose graph runs after everything that wrote its weights."""
     h = lib()
     before = h.axb_chain_launches(1)
+    _chain.on = True
     try:
         yield
     finally:
         h.axb_chain_launches(before)
+        _chain.on = bool(before)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None,
@@ -341,10 +347,10 @@ class _Linear(torch.autograd.Function):
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, *, resident: bool = False) -> torch.Tensor:
-    """``resident``: as in ``gemm``; without gradients only."""
+    """``resident``: as in ``gemm``; counts in the capture of a decoding step, which has no gradients."""
     if x.shape[-1] % 8 or w.shape[1] % 8:
         return torch.matmul(x, w)
-    if resident and not torch.is_grad_enabled() and _fused_fsdp_info(w) is None:
+    if resident and getattr(_chain, "on", False) and not torch.is_grad_enabled() and _fused_fsdp_info(w) is None:
         return gemm(x.reshape(-1, x.shape[-1]), w, resident=True).reshape(x.shape[:-1] + (w.shape[1],))
     return _Linear.apply(x, w)
 

@@ -158,6 +158,7 @@ class Mesh:
             raise ValueError(f"duplicate axis names {axis_names}")
         self.ranks = ranks
         self.axis_names = tuple(axis_names)
+        self._shape = dict(zip(self.axis_names, self.ranks.shape))
         if rank is None:
             rank = dist.get_rank() if dist.is_available() and dist.is_initialized() else 0
         self.rank = int(rank)
@@ -174,14 +175,14 @@ class Mesh:
     # ------------------------------------------------------------------ shape queries
     @property
     def shape(self) -> dict[str, int]:
-        return dict(zip(self.axis_names, self.ranks.shape))
+        return dict(self._shape)
 
     @property
     def size(self) -> int:
         return int(self.ranks.size)
 
     def axis_size(self, axes: AxisSpec) -> int:
-        return math.prod(self.shape[a] for a in _axes_tuple(axes)) if _axes_tuple(axes) else 1
+        return math.prod(self._shape[a] for a in _axes_tuple(axes)) if axes else 1
 
     def axis_index(self, axes: AxisSpec) -> int:
         """Linear index of this rank along ``axes`` (first axis is most significant)."""
@@ -192,7 +193,7 @@ class Mesh:
 
     def present_axes(self, axes: AxisSpec) -> tuple[str, ...]:
         """Subset of ``axes`` that exist in this mesh with extent > 1."""
-        return tuple(a for a in _axes_tuple(axes) if a in self.shape and self.shape[a] > 1)
+        return tuple(a for a in _axes_tuple(axes) if self._shape.get(a, 1) > 1)
 
     def ranks_along(self, axes: AxisSpec, *, coords: Optional[dict[str, int]] = None) -> list[int]:
         """Global ranks of the group that varies ``axes`` and fixes all other coordinates
