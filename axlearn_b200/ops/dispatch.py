@@ -112,9 +112,9 @@ class _LinearKept(torch.autograd.Function):
         return dx, dw, None
 
 
-def _linear_impl(x, w, resident=False):
+def _linear_impl(x, w):
     if _cuda(x, w) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
-        return _ops().linear(x, w, resident=resident)
+        return _ops().linear(x, w)
     return torch.matmul(x, w)
 
 
@@ -125,7 +125,9 @@ def linear(x, w, *, resident: bool = False):
     from axlearn_b200.common import remat
 
     if remat.active() is None:
-        return _linear_impl(x, w, resident)
+        if resident and _cuda(x, w) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
+            return _ops().linear(x, w, resident=True)
+        return _linear_impl(x, w)
     on_kernel = _cuda(x, w) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
     # A GEMM that carries a parameter gather for a neighbouring layer has to run even when its
     # own result is known.
