@@ -501,7 +501,7 @@ class Embedding(BaseLayer):
     def forward(self, x: Tensor) -> Tensor:
         cfg = self._config
         w = self._weight()
-        y = F.embedding(x.long(), w)
+        y = ops.embedding(x.long(), w)
         if coll.has_axis(_spec_entry(cfg.param_partition_spec, 1), "model"):
             # Feature dim is split over "model": assemble full rows.
             y = coll.all_gather(y, "model", dim=-1)

@@ -1076,7 +1076,9 @@ extern "C" int axb_ce_fwd_bwd(void* logits, int is_fp32, const int64_t* targets,
 extern "C" int axb_adamw(float* p, const void* g, int g_is_bf16, float* m, float* v, void* shadow,
                          const float* grad_scale, int64_t n, float lr, float wd, float b1, float b2,
                          float eps, float bc1, float bc2, cudaStream_t stream) {
-  const int grid = grid_for((n + 3) / 4, 256, 148 * 8);
+  // 134 M parameters, blocks per SM: 4 638 us, 8 640, 16 613 (574 at the copy rate); two vectors a thread or loads past
+  // the caches gain nothing on top, 32 contiguous bytes a thread take twice as long.
+  const int grid = grid_for((n + 3) / 4, 256, 148 * 16);
   if (g_is_bf16)
     adamw_kernel<bf16><<<grid, 256, 0, stream>>>(p, static_cast<const bf16*>(g), m, v,
                                                  static_cast<bf16*>(shadow), grad_scale, n, lr, wd,

@@ -10,6 +10,7 @@ the first GPU call raises instead of silently falling back.
 from axlearn_b200.ops.dispatch import (  # noqa: F401
     attention,
     cross_entropy,
+    embedding,
     linear,
     linear_f32,
     lm_head_cross_entropy,

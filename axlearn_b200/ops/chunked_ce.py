@@ -60,8 +60,10 @@ class _ChunkedLmHeadCE(torch.autograd.Function):
         need_grad = need_h or need_w
         inv_denom = (1.0 / denom).to(torch.float32)
         w_vd = weight if vocab_major else weight.t()  # [V, D] view
-        dh = torch.empty_like(h2) if need_h else None
-        dw = torch.zeros(w_vd.shape, dtype=torch.float32, device=weight.device) if need_w else None
+        # One chunk's products are the gradients themselves; more are summed (the weight's in 32 bits).
+        one = 0 < n <= chunk_tokens
+        dh = torch.empty_like(h2) if need_h and not one else None
+        dw = torch.zeros(w_vd.shape, dtype=torch.float32, device=weight.device) if need_w and not one else None
         sums = torch.zeros(3, dtype=torch.float32, device=hidden.device)
         for s in range(0, n, chunk_tokens):
             e = min(n, s + chunk_tokens)
@@ -71,6 +73,10 @@ class _ChunkedLmHeadCE(torch.autograd.Function):
                 logits, t1[s:e], l1[s:e], z_loss_scale, inv_denom, need_grad
             )
             sums += torch.stack([ce, z, correct])
+            if one:
+                dh = dispatch.linear(dlogits, w_vd).to(h2.dtype) if need_h else None
+                dw = dispatch.linear(dlogits.t(), hc) if need_w else None
+                continue
             if need_h:
                 dh[s:e] = dispatch.linear(dlogits, w_vd)
             if need_w:
@@ -91,8 +97,8 @@ class _ChunkedLmHeadCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_loss, *_):
         dh, dw = ctx.saved_tensors
-        gh = None if dh is None else (dh * g_loss.to(dh.dtype)).reshape(ctx.hidden_shape)
-        gw = None if dw is None else dw * g_loss.to(dw.dtype)
+        gh = None if dh is None else dispatch.scaled(dh, g_loss).reshape(ctx.hidden_shape)
+        gw = None if dw is None else dispatch.scaled(dw, g_loss)
         return gh, gw, None, None, None, None, None, None
 
 

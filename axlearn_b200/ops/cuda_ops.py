@@ -100,6 +100,8 @@ class _Sigs:
                       c_float, c_int64, c_int, c_int, c_void_p]
     axb_adamw = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_float,
                  c_float, c_float, c_float, c_float, c_float, c_float, c_void_p]
+    axb_embedding_bwd = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
+    axb_scale_bf16 = [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]
     axb_sumsq_ctas = []
     axb_sumsq = [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_float, c_int, c_void_p]
 
@@ -631,6 +633,59 @@ def cross_entropy(logits, targets, *, live_targets=None, z_loss_scale: float = 0
     denom = num_live.clamp_min(1.0) if denominator is None else denominator.to(torch.float32)
     loss, ce, z, acc = _CrossEntropy.apply(logits, targets, live_targets, float(z_loss_scale), denom)
     return loss, {"cross_entropy_loss": ce, "z_loss": z, "accuracy": acc, "num_live": num_live}
+
+
+# ------------------------------------------------------------------------------------------
+# Embedding.
+# ------------------------------------------------------------------------------------------
+
+
+class _Embedding(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, ids, w):
+        ctx.save_for_backward(ids)
+        ctx.rows = w.shape[0]
+        return torch.nn.functional.embedding(ids, w)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (ids,) = ctx.saved_tensors
+        if torch.is_grad_enabled() or dy.dtype != torch.bfloat16:
+            # A gradient that may be differentiated again.
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids, ctx.rows, -1, False)
+        d, n = dy.shape[-1], ids.numel()
+        dy = dy.contiguous()
+        if dy.data_ptr() % 16:
+            dy = dy.clone()
+        ids = ids.contiguous()
+        dw = torch.empty((ctx.rows, d), dtype=dy.dtype, device=dy.device)
+        work = torch.empty(n + 3 * ctx.rows, dtype=torch.int32, device=dy.device)
+        _check(lib().axb_embedding_bwd(dy.data_ptr(), ids.data_ptr(), dw.data_ptr(), work.data_ptr(), n, ctx.rows, d,
+                                       _stream()), "axb_embedding_bwd")
+        return None, dw
+
+
+def embedding(ids: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``w[ids]`` with the table's gradient in one pass over it.  Forward-mode and function transforms, which know the
+    operator but not an autograd node around it, keep the operator."""
+    if not (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.requires_grad and torch.is_grad_enabled()
+            and w.shape[1] % 8 == 0 and w.numel() > 0 and ids.dtype == torch.int64 and ids.numel() < 1 << 30
+            and torch.autograd.forward_ad._current_level < 0  # pylint: disable=protected-access
+            and not torch._C._are_functorch_transforms_active()):  # pylint: disable=protected-access
+        return torch.nn.functional.embedding(ids, w)
+    return _Embedding.apply(ids, w)
+
+
+def scaled(x: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
+    """``x * g.to(x.dtype)`` for a scalar ``g`` on the device."""
+    dense = x if x.is_contiguous() else x.t() if x.dim() == 2 and x.t().is_contiguous() else None
+    if (dense is None or not x.is_cuda or x.dtype != torch.bfloat16 or g.dtype != torch.float32 or g.numel() != 1
+            or x.numel() % 8 or x.data_ptr() % 16 or torch.is_grad_enabled()
+            or torch._C._are_functorch_transforms_active()):  # pylint: disable=protected-access
+        return x * g.to(x.dtype)
+    out = torch.empty_like(dense)
+    _check(lib().axb_scale_bf16(dense.data_ptr(), g.data_ptr(), out.data_ptr(), x.numel(), _stream()), "axb_scale_bf16")
+    return out if dense is x else out.t()
 
 
 # ------------------------------------------------------------------------------------------

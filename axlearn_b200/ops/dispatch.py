@@ -140,6 +140,20 @@ def linear(x, w, *, resident: bool = False):
     return _LinearKept.apply(x, w, y)
 
 
+def scaled(x, g):
+    """``x * g.to(x.dtype)`` for a scalar tensor ``g``."""
+    if _cuda(x, g):
+        return _ops().scaled(x, g)
+    return x * g.to(x.dtype)
+
+
+def embedding(ids, w):
+    """``w[ids]``: rows of an embedding table."""
+    if _cuda(w):
+        return _ops().embedding(ids, w)
+    return torch.nn.functional.embedding(ids, w)
+
+
 def linear_f32(x, w, *, resident: bool = False):
     """``x[..., K] @ w[K, N]`` with an fp32 result (the accumulators as they are): output heads."""
     if _cuda(x, w) and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and not (

@@ -180,3 +180,52 @@ def test_adamw_and_sumsq():
     ref = g.float().pow(2).sum() + 0.5 * p.pow(2).sum()
     assert abs(ss.item() - ref.item()) < 1e-4 * ref.item()
     assert ss.item() == cuda_ops.sum_of_squares([g, p], [1.0, 0.5]).item()
+
+
+@pytest.mark.parametrize("v,d,n", [(1, 8, 1), (7, 264, 5), (5000, 2056, 333), (4100, 512, 20000)])
+def test_embedding_gradient(v, d, n):
+    """Rows nobody uses, short lists, rows above 32 tokens (walked in order), more columns than a block takes at once; the
+    sum is one rounding away from 64 bits and the same in every run."""
+    from axlearn_b200.ops import cuda_ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ids = torch.randint(0, v, (1, n), device="cuda", generator=g)
+    ids[0, :n // 3] = v // 2  # a frequent token
+    w = torch.randn(v, d, device="cuda", generator=g).bfloat16().requires_grad_()
+    dy = torch.randn(1, n, d, device="cuda", generator=g).bfloat16()
+    runs = []
+    for _ in range(2):
+        y = cuda_ops.embedding(ids, w)
+        assert torch.equal(y, w[ids])
+        (dw,) = torch.autograd.grad(y, w, dy)
+        runs.append(dw)
+    assert torch.equal(*runs)
+    want = torch.zeros(v, d, device="cuda", dtype=torch.float64).index_add_(0, ids[0], dy[0].double())
+    size = torch.zeros_like(want).index_add_(0, ids[0], dy[0].double().abs())
+    # Half a unit of bf16 (up to 2^-8 of the sum) and a 32-bit sum of up to n terms in order.
+    assert ((runs[0].double() - want).abs() <= 2.0 ** -8 * want.abs() + n * 2.0 ** -24 * size).all()
+
+
+def test_embedding_gradient_can_be_differentiated_again():
+    from axlearn_b200.ops import cuda_ops
+
+    w = torch.randn(6, 16, device="cuda").bfloat16().requires_grad_()
+    ids = torch.tensor([[1, 1, 4]], device="cuda")
+    dy = torch.randn(1, 3, 16, device="cuda").bfloat16().requires_grad_()
+    (dw,) = torch.autograd.grad(cuda_ops.embedding(ids, w), w, dy, create_graph=True)
+    (back,) = torch.autograd.grad(dw.float().sum(), dy)
+    assert torch.equal(back, torch.ones_like(back))
+
+
+@pytest.mark.parametrize("shape", [(8,), (3, 2056), (70001, 8)])
+def test_scaled_equals_the_product(shape):
+    from axlearn_b200.ops import cuda_ops
+
+    x = torch.randn(*shape, device="cuda").bfloat16()
+    for value in (1.0, 0.37, float("inf")):
+        g = torch.tensor(value, device="cuda")
+        assert torch.equal(cuda_ops.scaled(x, g).nan_to_num(5.0), (x * g.bfloat16()).nan_to_num(5.0))
+        if x.dim() == 2:
+            got = cuda_ops.scaled(x.t(), g)
+            assert got.stride() == x.t().stride() and torch.equal(got.nan_to_num(5.0), (x.t() * g.bfloat16()).nan_to_num(5.0))
+
