@@ -277,7 +277,9 @@ class Decoder(BaseLayer):
         (stacks that support it; None: all)."""
         time_step = cached_states["time_step"]
         steps = input_ids.shape[1]
-        positions = time_step[:, None] + torch.arange(steps, device=input_ids.device)[None]
+        # (One token, the decoding step: a launch less.)
+        positions = (time_step[:, None].long() if steps == 1
+                     else time_step[:, None] + torch.arange(steps, device=input_ids.device)[None])
         states, out = self._forward_for_mode(
             mode=ForwardMode.EXTEND_STEP,
             input_batch={"input_ids": input_ids, "positions": positions},
