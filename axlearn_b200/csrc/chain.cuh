@@ -6,6 +6,11 @@
 // it has finished and is visible.  All threads call it, ahead of any early return: a successor that waits for this
 // kernel thereby waits for all kernels before it, too.  Launched in the ordinary way both instructions do nothing.
 //
+// What earlier kernels write (activations, lengths, partial results, copies of parameters) is read with ordinary loads,
+// through pointers without `__restrict__`, and never with `__ldg`: the read-only path is promised for data that is
+// constant while the kernel is resident, which a chained kernel is before its input is written, and no wait orders it.
+// Only tables of parameters that a step does not write may be `const __restrict__`.
+//
 // Launches are chained only while the calling thread captures a decoding step (`axb_chain_launches`): there, what may
 // be read ahead of the wait is known.  Kernels that stream much memory in one wave or with many small CTAs (expert
 // products, state-space and latent decoding) keep ordinary launches: started early, their CTAs go to the SMs that

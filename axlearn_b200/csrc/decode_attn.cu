@@ -115,7 +115,7 @@ decode_attn_kernel(DecodeParams p) {
   auto slot_of = [&](int tile) {
     const int t = tile * kTileKeys + (lane & 15);
     if (tile >= hi || t >= len) return -1;
-    return __ldg(table + t / p.page_size) * p.page_size + t % p.page_size;
+    return table[t / p.page_size] * p.page_size + t % p.page_size;
   };
 
   const int64_t row_stride = static_cast<int64_t>(p.num_kv_heads) * kHeadDim;
@@ -326,8 +326,7 @@ static int launch_attn(const DecodeParams& p, dim3 grid, int rows, cudaStream_t 
 }
 
 __global__ void __launch_bounds__(kHeadDim)
-decode_combine_kernel(const float* __restrict__ part_out, const float* __restrict__ part_ml,
-                      __nv_bfloat16* __restrict__ out, int splits) {
+decode_combine_kernel(const float* part_out, const float* part_ml, __nv_bfloat16* out, int splits) {
   chain_link();
   const int64_t row = blockIdx.x;  // b * Nq + head
   const int d = threadIdx.x;
@@ -346,10 +345,9 @@ decode_combine_kernel(const float* __restrict__ part_out, const float* __restric
 // qkv: [B, (Nq + 2 Nkv) * H] (q heads, then k heads, then v heads).  One CTA per (b, head);
 // thread i rotates the pair (2i, 2i+1).
 __global__ void __launch_bounds__(kHeadDim / 2)
-rope_append_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ q_out,
-                   __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool,
-                   const int* __restrict__ page_table, const int* __restrict__ lengths, int num_q_heads,
-                   int num_kv_heads, int page_size, int max_pages, float log2_theta, int apply_rope) {
+rope_append_kernel(const __nv_bfloat16* qkv, __nv_bfloat16* q_out, __nv_bfloat16* k_pool, __nv_bfloat16* v_pool,
+                   const int* page_table, const int* lengths, int num_q_heads, int num_kv_heads, int page_size,
+                   int max_pages, float log2_theta, int apply_rope) {
   chain_link();
   const int b = blockIdx.y;
   const int head = blockIdx.x;  // 0..Nq+2Nkv-1
@@ -491,8 +489,7 @@ rope_append_prompt_kernel(uint4* __restrict__ qkv, uint4* __restrict__ k_pool, u
 __device__ __forceinline__ float silu_times(float g, float u) { return g / (1.f + __expf(-g)) * u; }
 
 // out[r, c] = silu(gu[r, c]) * gu[r, F + c] for gu = [rows, 2F] (gate | up packed by one GEMM).
-__global__ void swiglu_packed_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
-                                     int64_t rows, int F) {
+__global__ void swiglu_packed_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out, int64_t rows, int F) {
   chain_link();
   const int64_t total = rows * (F / 2);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -510,7 +507,7 @@ __global__ void swiglu_packed_kernel(const __nv_bfloat16* __restrict__ gu, __nv_
 constexpr int kSwigluThreads = 256, kSwigluVecs = 2;
 
 __global__ void __launch_bounds__(kSwigluThreads)
-swiglu_packed_vec_kernel(const uint4* __restrict__ gu, uint4* __restrict__ out, int64_t rows, int vecs) {
+swiglu_packed_vec_kernel(const uint4* gu, uint4* out, int64_t rows, int vecs) {
   chain_link();
   const int c0 = blockIdx.x * (kSwigluThreads * kSwigluVecs) + threadIdx.x;
   for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
@@ -519,8 +516,8 @@ swiglu_packed_vec_kernel(const uint4* __restrict__ gu, uint4* __restrict__ out, 
     for (int i = 0; i < kSwigluVecs; ++i) {
       const int c = c0 + i * kSwigluThreads;
       if (c < vecs) {
-        g[i] = __ldg(gu + row * 2 * vecs + c);
-        u[i] = __ldg(gu + row * 2 * vecs + vecs + c);
+        g[i] = gu[row * 2 * vecs + c];
+        u[i] = gu[row * 2 * vecs + vecs + c];
       }
     }
 #pragma unroll

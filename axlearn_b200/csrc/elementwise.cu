@@ -68,10 +68,8 @@ __device__ __forceinline__ float block_max(float x, float* red) {
 // One CTA per row (grid-stride). D % 8 == 0. rstd[row] is kept for the backward pass.
 // If `residual` is given, computes s = x + residual first, writes s to `sum_out` and
 // normalises s (the pre-norm residual add of a transformer block fused in).
-__global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
-                                   const bf16* __restrict__ scale, bf16* __restrict__ y,
-                                   bf16* __restrict__ sum_out, float* __restrict__ rstd_out,
-                                   int64_t rows, int D, float eps) {
+__global__ void rmsnorm_fwd_kernel(const bf16* x, const bf16* residual, const bf16* scale, bf16* y, bf16* sum_out,
+                                   float* rstd_out, int64_t rows, int D, float eps) {
   chain_link();
   __shared__ float red[32];
   const int nvec = D / 8;
@@ -195,9 +193,8 @@ __device__ __forceinline__ Bf16x8 ld_again(const Bf16x8* p) {
 // lane holds at most eight vectors and three CTAs fit an SM (more rows, hence bytes, in flight).
 template <int VPL, int WPR>
 __global__ void __launch_bounds__(256, 3)
-rmsnorm_fwd_warp_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
-                        const bf16* __restrict__ scale, bf16* __restrict__ y, bf16* __restrict__ sum_out,
-                        float* __restrict__ rstd_out, int64_t rows, float eps) {
+rmsnorm_fwd_warp_kernel(const bf16* x, const bf16* residual, const bf16* scale, bf16* y, bf16* sum_out, float* rstd_out,
+                        int64_t rows, float eps) {
   chain_link();
   constexpr int P = VPL * 256;
   constexpr int D = P * WPR;

@@ -241,9 +241,8 @@ __global__ void __launch_bounds__(kRtThreads) route_gather_kernel(RouteArgs a) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128) expert_combine_kernel(const T* __restrict__ y, const int* __restrict__ place,
-                                                             T* __restrict__ out, int64_t y_ld, int64_t out_ld, int top,
-                                                             int width) {
+__global__ void __launch_bounds__(128) expert_combine_kernel(const T* y, const int* place, T* out, int64_t y_ld,
+                                                             int64_t out_ld, int top, int width) {
   chain_link();
   const int64_t t = blockIdx.x;
   constexpr int V = sizeof(T) == 2 ? 8 : 4;  // width is a multiple of 8

@@ -12,8 +12,8 @@
 namespace axb {
 
 template <typename T, int K>
-__global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, int64_t n, int F, int up_off,
-                                 int64_t ld, int64_t out_ld, float limit, float alpha) {
+__global__ void gated_act_kernel(const T* gu, T* out, int64_t n, int F, int up_off, int64_t ld, int64_t out_ld,
+                                 float limit, float alpha) {
   chain_link();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -24,8 +24,8 @@ __global__ void gated_act_kernel(const T* __restrict__ gu, T* __restrict__ out, 
 }
 
 template <int K>
-__global__ void gated_act_vec_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int64_t n8,
-                                     int up_off, int64_t ld, int64_t out_ld, float limit, float alpha) {
+__global__ void gated_act_vec_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out, int64_t n8, int up_off, int64_t ld,
+                                     int64_t out_ld, float limit, float alpha) {
   chain_link();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n8) return;

@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(kEndThreads) step_end_kernel(StepEndArgs a) {
 
 // One CTA per token, 16 bytes a thread and pass.  An id outside the table gives NaN and a mark in the status word.
 __global__ void __launch_bounds__(256)
-embed_rows_kernel(const uint4* __restrict__ table, const int64_t* __restrict__ ids, uint4* __restrict__ out,
-                  int* __restrict__ lengths, int max_len, int V, int vecs, int64_t table_ld, int wrap, int* status) {
+embed_rows_kernel(const uint4* __restrict__ table, const int64_t* ids, uint4* out, int* lengths, int max_len, int V,
+                  int vecs, int64_t table_ld, int wrap, int* status) {
   chain_link();
   const int64_t b = blockIdx.x;
   int64_t id = ids[b];

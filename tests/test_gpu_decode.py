@@ -98,6 +98,68 @@ def test_chained_step_sees_new_weights_and_matches_separate_launches():
         tokens = plain.argmax(dim=-1)
 
 
+@pytest.mark.parametrize("d,f,vocab,nq,nkv,b", [(2048, 5632, 4096, 16, 16, 1), (4096, 14336, 8192, 32, 8, 16)])
+def test_chained_steps_at_serving_widths(d, f, vocab, nq, nkv, b):
+    """Kernels that overlap for long: replays of the chained step against separate launches, bit for bit."""
+    from axlearn_b200.inference.decode_engine import DecodeEngine, FujiDims, LayerWeights
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+
+    def w(*shape):
+        return (torch.randn(*shape, device="cuda", generator=g) * shape[0] ** -0.5).bfloat16()
+
+    layers = [LayerWeights(attn_norm=1 + 0.1 * w(d), wqkv=w(d, (nq + 2 * nkv) * 128), wo=w(nq * 128, d),
+                           ffn_norm=1 + 0.1 * w(d), wgu=w(d, 2 * f), wdown=w(f, d)) for _ in range(4)]
+    weights = {"layers": layers, "emb": w(vocab, d) * 16, "head": w(vocab, d), "final_norm": 1 + 0.1 * w(d)}
+    dims = FujiDims(num_layers=4, hidden_dim=d, num_heads=nq, num_kv_heads=nkv, head_dim=128, ffn_dim=f, vocab_size=vocab)
+    engines = [DecodeEngine(weights, dims, batch=b, max_len=512, use_graph=use) for use in (True, False)]
+    ids = torch.randint(0, vocab, (b, 300), device="cuda", generator=g)
+    lengths = torch.randint(1, 301, (b,), device="cuda", generator=g)
+    for e in engines:
+        e.prefill(ids, lengths=lengths)
+    for i in range(24):
+        chained, plain = (e.step_logits(ids[:, i]).clone() for e in engines)
+        assert torch.equal(chained, plain), i
+
+
+@pytest.mark.parametrize("b", [1, 5])
+@pytest.mark.parametrize("family,name", [("sagisun", "wide"), ("sagisun", "mixed"), ("zukitar", "wide"),
+                                         ("zukitar", "small")])
+def test_chained_module_steps_see_new_weights_and_match_separate_launches(family, name, b, tmp_path):
+    """Mixers on a side stream, gates, routing and states inside the chain, with weights changed before each replay."""
+    import importlib
+
+    from axlearn_b200.common.utils import flatten_items
+    from axlearn_b200.inference.decode_engine import ModuleDecodeEngine
+    from axlearn_b200.inference.model_loader import load_model
+
+    ckpt = importlib.import_module(f"tests.{family}_checkpoints")
+    cfg = ckpt.CONFIGS[name]
+    loaded = load_model(ckpt.save(tmp_path, cfg, ckpt.random_tensors(cfg, seed=3)), dtype=torch.bfloat16, device="cuda")
+    params = loaded.parameters["decoder"]
+    engines = [ModuleDecodeEngine(loaded.decoder, params, batch=b, max_len=200, device="cuda", use_graph=use)
+               for use in (True, False)]
+    g = torch.Generator().manual_seed(b)
+    ids = torch.randint(0, cfg["vocab"], (b, 70), generator=g).cuda()
+    lengths = torch.randint(1, 71, (b,), generator=g)
+    for e in engines:
+        e.prefill(ids, lengths=lengths)
+    matrices = [t for _, t in flatten_items(params) if t.dim() >= 2]
+    assert matrices
+    for i in range(20):
+        if i % 4 == 0:
+            for t in matrices:
+                t.mul_(1.0 + 0.25 * (-1) ** (i // 4))
+        active = torch.ones(b, dtype=torch.int32)
+        active[i % b] = int(b == 1 or i % 3 > 0)
+        for e in engines:
+            e.set_active(active)
+        chained, plain = (e.step_logits(ids[:, i]).clone() for e in engines)
+        assert torch.equal(chained, plain), i
+        for (_, x), (_, y) in zip(flatten_items(engines[0].states), flatten_items(engines[1].states)):
+            assert torch.equal(x, y)
+
+
 @pytest.mark.parametrize("b,v,ld", [(1, 1, 4), (3, 33, 40), (2, 4096, 4096), (5, 32768, 32768), (2, 32772, 32776)])
 def test_step_end_picks_as_torch_and_keeps(b, v, ld):
     """Vector and element paths around one pass of the block; ties go to the first, NaN above all."""
