@@ -8,6 +8,7 @@
 // axlearn/common/loss.py:234-327 (cross entropy) and axlearn/common/optimizers.py:741-856,
 // 1149-1184 (AdamW chain, global-norm clip).
 #include "chain.cuh"
+#include "mma_sync.cuh"
 #include "no_alloc.h"
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -65,12 +66,15 @@ __device__ __forceinline__ float block_max(float x, float* red) {
 }
 
 // ------------------------------------------------------------------------------ RMSNorm
+// Every forward kernel exists twice.  Launched in the ordinary way its inputs are constant while it runs, and the read-only
+// path lets the compiler move the loads of the scale past the stores of a row (8192 x 4096: 24 us, with ordinary loads 33).
+// In a chained launch (chain.cuh) it is resident before its inputs are written, so it takes them with ordinary loads.
+
 // One CTA per row (grid-stride). D % 8 == 0. rstd[row] is kept for the backward pass.
 // If `residual` is given, computes s = x + residual first, writes s to `sum_out` and
 // normalises s (the pre-norm residual add of a transformer block fused in).
-__global__ void rmsnorm_fwd_kernel(const bf16* x, const bf16* residual, const bf16* scale, bf16* y, bf16* sum_out,
-                                   float* rstd_out, int64_t rows, int D, float eps) {
-  chain_link();
+__device__ __forceinline__ void rmsnorm_fwd_rows(const bf16* x, const bf16* residual, const bf16* scale, bf16* y,
+                                                 bf16* sum_out, float* rstd_out, int64_t rows, int D, float eps) {
   __shared__ float red[32];
   const int nvec = D / 8;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -112,6 +116,19 @@ __global__ void rmsnorm_fwd_kernel(const bf16* x, const bf16* residual, const bf
       yr[i] = o;
     }
   }
+}
+
+__global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
+                                   const bf16* __restrict__ scale, bf16* __restrict__ y,
+                                   bf16* __restrict__ sum_out, float* __restrict__ rstd_out,
+                                   int64_t rows, int D, float eps) {
+  rmsnorm_fwd_rows(x, residual, scale, y, sum_out, rstd_out, rows, D, eps);
+}
+
+__global__ void rmsnorm_fwd_chained_kernel(const bf16* x, const bf16* residual, const bf16* scale, bf16* y,
+                                           bf16* sum_out, float* rstd_out, int64_t rows, int D, float eps) {
+  chain_link();
+  rmsnorm_fwd_rows(x, residual, scale, y, sum_out, rstd_out, rows, D, eps);
 }
 
 // dx = rstd * (g - xhat * mean(g * xhat)), g = dy * scale, xhat = x * rstd.
@@ -191,19 +208,24 @@ __device__ __forceinline__ Bf16x8 ld_again(const Bf16x8* p) {
 
 // WPR warps share a row (each a contiguous 256 * VPL-element part); wide rows are split so that a
 // lane holds at most eight vectors and three CTAs fit an SM (more rows, hence bytes, in flight).
-template <int VPL, int WPR>
-__global__ void __launch_bounds__(256, 3)
-rmsnorm_fwd_warp_kernel(const bf16* x, const bf16* residual, const bf16* scale, bf16* y, bf16* sum_out, float* rstd_out,
-                        int64_t rows, float eps) {
-  chain_link();
+// kStage: a thread keeps its vectors of the scale in shared memory, where ordinary loads of them would wait for the stores of
+// the row before (few rows: 1 x 2048 1.84 us against 2.17 with the read-only path; 8192 x 4096 25.4 against 24.2).
+template <int VPL, int WPR, bool kStage>
+__device__ __forceinline__ void rmsnorm_fwd_warp_rows(const bf16* x, const bf16* residual, const bf16* scale, bf16* y,
+                                                      bf16* sum_out, float* rstd_out, int64_t rows, float eps) {
   constexpr int P = VPL * 256;
   constexpr int D = P * WPR;
   constexpr int kRowsPerCta = 8 / WPR;
   __shared__ float ss_part[8];
+  __shared__ Bf16x8 s_scale[kStage ? VPL * 256 : 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int part = warp % WPR, slot = warp / WPR;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kRowsPerCta;
   const Bf16x8* sc = reinterpret_cast<const Bf16x8*>(scale + part * P);
+  if constexpr (kStage) {
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) cp16(s_scale + i * 256 + threadIdx.x, sc + i * 32 + lane);
+  }
   for (int64_t row = static_cast<int64_t>(blockIdx.x) * kRowsPerCta + slot; row < rows; row += stride) {
     const Bf16x8* xr = reinterpret_cast<const Bf16x8*>(x + row * D + part * P);
     Bf16x8 a[VPL];
@@ -242,10 +264,15 @@ rmsnorm_fwd_warp_kernel(const bf16* x, const bf16* residual, const bf16* scale, 
     }
     const float rstd = rsqrtf(ss / D + eps);
     if (lane == 0 && part == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
+    if constexpr (kStage) cp_wait_all();  // (at the first row)
     Bf16x8* yr = reinterpret_cast<Bf16x8*>(y + row * D + part * P);
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-      const Bf16x8 s = sc[i * 32 + lane];
+      Bf16x8 s;
+      if constexpr (kStage)
+        s = s_scale[i * 256 + threadIdx.x];
+      else
+        s = sc[i * 32 + lane];
       Bf16x8 o;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -258,6 +285,23 @@ rmsnorm_fwd_warp_kernel(const bf16* x, const bf16* residual, const bf16* scale, 
       yr[i * 32 + lane] = o;
     }
   }
+  if constexpr (kStage) cp_wait_all();  // warps without a row
+}
+
+template <int VPL, int WPR>
+__global__ void __launch_bounds__(256, 3)
+rmsnorm_fwd_warp_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual,
+                        const bf16* __restrict__ scale, bf16* __restrict__ y, bf16* __restrict__ sum_out,
+                        float* __restrict__ rstd_out, int64_t rows, float eps) {
+  rmsnorm_fwd_warp_rows<VPL, WPR, false>(x, residual, scale, y, sum_out, rstd_out, rows, eps);
+}
+
+template <int VPL, int WPR>
+__global__ void __launch_bounds__(256, 3)
+rmsnorm_fwd_warp_chained_kernel(const bf16* x, const bf16* residual, const bf16* scale, bf16* y, bf16* sum_out,
+                                float* rstd_out, int64_t rows, float eps) {
+  chain_link();
+  rmsnorm_fwd_warp_rows<VPL, WPR, true>(x, residual, scale, y, sum_out, rstd_out, rows, eps);
 }
 
 // Backward, WPR warps per row (each owns a contiguous 256 * VPL-element part of it; two warps
@@ -866,9 +910,9 @@ extern "C" int axb_rmsnorm_fwd(const void* x, const void* residual, const void* 
   if (D % 8) return -10;
   const int threads = D >= 2048 ? 256 : 128;
   const int grid = static_cast<int>(rows < 148 * 8 ? rows : 148 * 8);
-  launch_chained(rmsnorm_fwd_kernel, grid, threads, 0, stream, static_cast<const bf16*>(x), static_cast<const bf16*>(residual),
-      static_cast<const bf16*>(scale), static_cast<bf16*>(y), static_cast<bf16*>(sum_out), rstd,
-      rows, D, eps);
+  const auto kernel = chain_launches ? rmsnorm_fwd_chained_kernel : rmsnorm_fwd_kernel;
+  launch_chained(kernel, grid, threads, 0, stream, static_cast<const bf16*>(x), static_cast<const bf16*>(residual),
+                 static_cast<const bf16*>(scale), static_cast<bf16*>(y), static_cast<bf16*>(sum_out), rstd, rows, D, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -903,8 +947,9 @@ static int launch_rmsnorm_fwd_warp(const void* x, const void* residual, const vo
                                    float* rstd, int64_t rows, float eps, cudaStream_t stream) {
   const int64_t want = (rows + 8 / WPR - 1) / (8 / WPR);
   const int grid = static_cast<int>(want < 148 * 3 ? want : 148 * 3);
-  launch_chained(rmsnorm_fwd_warp_kernel<VPL, WPR>, grid, 256, 0, stream, static_cast<const bf16*>(x), static_cast<const bf16*>(residual), static_cast<const bf16*>(scale),
-      static_cast<bf16*>(y), static_cast<bf16*>(sum_out), rstd, rows, eps);
+  const auto kernel = chain_launches ? rmsnorm_fwd_warp_chained_kernel<VPL, WPR> : rmsnorm_fwd_warp_kernel<VPL, WPR>;
+  launch_chained(kernel, grid, 256, 0, stream, static_cast<const bf16*>(x), static_cast<const bf16*>(residual),
+                 static_cast<const bf16*>(scale), static_cast<bf16*>(y), static_cast<bf16*>(sum_out), rstd, rows, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
