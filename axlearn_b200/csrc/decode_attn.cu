@@ -8,10 +8,15 @@
 // whole group of query heads.  A warp walks every fourth tile of 16 tokens of its split through a ring of two tiles
 // (8 KB of K and V each) that `cp.async` fills ahead of the arithmetic; three CTAs fit an SM.
 //   S = Q K^T: rows 0-7 of the m16n8k16 tile are the query heads, K is the B operand (a lane takes 8 neighbouring dims
-//   of a key; Q uses the same order of dims).
+//   of a key; Q uses the same order of dims).  Four chains of two products each, added in 32 bits.
 //   O^T = V^T P^T: 16 dims are the rows, the heads the columns (the scores' accumulators are the B operand as they
-//   lie); a lane packs two keys' V entries into one register of the A operand.  P enters as two bf16 terms, i.e. with
-//   about 16 mantissa bits.
+//   lie); a lane packs two keys' V entries into one register of the A operand.  P enters as three bf16 terms that add
+//   up to its 32 bits.  Up to four (two) heads leave room for two (four) copies of them in the tile: copy i takes term i
+//   of P, so that two (one) products do for three.  A tile's products are added to the sums in 32 bits.
+// Relative error against 64 bits before the output's rounding, the two CUDA-core kernels that this replaces / this (two
+// bf16 terms and one chain: 1.4e-6 throughout): 8 x 16 heads on 16, up to 2000 tokens 2.5e-7 / 2.4e-7; 16 x 32 on 8, up to
+// 2048 2.7e-7 / 2.5e-7; 1 x 32 on 8, up to 4000 3.3e-7 / 2.9e-7.  Time of two terms / three (us a launch, inputs beyond
+// L2): 18.6 / 18.8, 21.4 / 22.4, 10.8 / 11.2; without the copies 20.0, 23.1 and 11.2.
 // The warps meet in shared memory and the KV splits of up to a cluster (8) in distributed shared memory, so there is no
 // second launch; more splits leave partials (max, sum, out) for `decode_combine_kernel`.
 //
@@ -74,14 +79,20 @@ constexpr int attn_smem_bytes(int rows) {
   return merge > tiles ? merge : tiles;
 }
 
-// head + rest = (x, y) >= 0 to about 16 mantissa bits, the head rounded down.  The rest of a positive number stays
-// positive, so that an infinite V gives an infinity as in one product, not 0 * infinity.
-__device__ __forceinline__ void split_down(float x, float y, uint32_t& head, uint32_t& rest) {
-  const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
-  head = __byte_perm(ux, uy, 0x7632);
-  const float dx = x - __uint_as_float(ux & 0xffff0000u), dy = y - __uint_as_float(uy & 0xffff0000u);
+// term[0] + term[1] + term[2] = (x, y) >= 0, exactly: a 24-bit mantissa is three of 8 bits, cut off from the top.  Every
+// term of a positive number is positive (2^-126 stands in for nothing left, as in a fourth term), so that an infinite V
+// gives an infinity as in one product, not 0 * infinity.
+template <int N>
+__device__ __forceinline__ void split_exact(float x, float y, uint32_t (&term)[N]) {
   const float tiny = 1.17549435e-38f;
-  rest = pack2(x > 0.f ? fmaxf(dx, tiny) : dx, y > 0.f ? fmaxf(dy, tiny) : dy);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
+    term[i] = __byte_perm(ux, uy, 0x7632);
+    const float dx = x - __uint_as_float(ux & 0xffff0000u), dy = y - __uint_as_float(uy & 0xffff0000u);
+    x = x > 0.f ? fmaxf(dx, tiny) : dx;
+    y = y > 0.f ? fmaxf(dy, tiny) : dy;
+  }
 }
 
 // 16 bytes to shared memory, zeros when `ok` is false (`src` is not read then).
@@ -89,7 +100,7 @@ __device__ __forceinline__ void cp16_or_zero(uint32_t dst, const void* src, bool
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-template <bool kCluster>
+template <bool kCluster, int kCopies>
 __global__ void __launch_bounds__(kDecodeThreads)
 decode_attn_kernel(DecodeParams p) {
   chain_link();
@@ -105,6 +116,8 @@ decode_attn_kernel(DecodeParams p) {
   const int b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = lane >> 2, c = lane & 3;
+  constexpr int kHeads = kMmaRows / kCopies, kPasses = (3 + kCopies - 1) / kCopies;
+  const int head = r % kHeads, copy = r / kHeads;
   const int len = p.lengths[b];
   const int tiles = (len + kTileKeys - 1) / kTileKeys;
   const int per_split = (tiles + p.splits - 1) / p.splits;
@@ -151,12 +164,12 @@ decode_attn_kernel(DecodeParams p) {
   int slot = slot_of(tile + kStages * kStep);
   uint4 q[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    q[j] = r < rows ? *reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(b) * p.num_q_heads + qh0 + r) * kHeadDim +
-                                                      j * 32 + c * 8)
-                    : make_uint4(0, 0, 0, 0);
+  for (int j = 0; j < 4; ++j) {
+    const int64_t row = static_cast<int64_t>(b) * p.num_q_heads + qh0 + head;
+    q[j] = head < rows ? *reinterpret_cast<const uint4*>(p.q + row * kHeadDim + j * 32 + c * 8) : make_uint4(0, 0, 0, 0);
+  }
   float m = -INFINITY, l = 0.f;
-  float acc[8][4];  // [16 dims][heads 2c, 2c + 1]
+  float acc[8][4];  // [16 dims][columns 2c, 2c + 1]
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 
@@ -169,17 +182,17 @@ decode_attn_kernel(DecodeParams p) {
     float s[4];
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      float part[4][4] = {};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const uint4 k = *reinterpret_cast<const uint4*>(kt + k_chunk(n * 8 + r, j * 4 + c));
         const uint32_t a0[4] = {q[j].x, 0u, q[j].y, 0u}, a1[4] = {q[j].z, 0u, q[j].w, 0u};
-        mma(d, a0, k.x, k.y);
-        mma(d, a1, k.z, k.w);
+        mma(part[(2 * j) % 4], a0, k.x, k.y);
+        mma(part[(2 * j + 1) % 4], a1, k.z, k.w);
       }
       const int t = tile * kTileKeys + n * 8 + 2 * c;
-      s[2 * n] = t < len ? d[0] * p.scale_log2 : -INFINITY;
-      s[2 * n + 1] = t + 1 < len ? d[1] * p.scale_log2 : -INFINITY;
+      s[2 * n] = t < len ? ((part[0][0] + part[2][0]) + (part[1][0] + part[3][0])) * p.scale_log2 : -INFINITY;
+      s[2 * n + 1] = t + 1 < len ? ((part[0][1] + part[2][1]) + (part[1][1] + part[3][1])) * p.scale_log2 : -INFINITY;
     }
     float top = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
@@ -202,9 +215,17 @@ decode_attn_kernel(DecodeParams p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) s[i] = m == -INFINITY ? 0.f : exp2f(s[i] - m);
     l += (s[0] + s[1]) + (s[2] + s[3]);
-    uint32_t head[2], rest[2];
-    split_down(s[0], s[1], head[0], rest[0]);
-    split_down(s[2], s[3], head[1], rest[1]);
+    constexpr int kTerms = kPasses * kCopies;
+    uint32_t t0[kTerms], t1[kTerms], p0[kPasses], p1[kPasses];  // all terms; those of this copy
+    split_exact(s[0], s[1], t0);
+    split_exact(s[2], s[3], t1);
+#pragma unroll
+    for (int i = 0; i < kPasses; ++i) {
+      p0[i] = t0[i * kCopies], p1[i] = t1[i * kCopies];
+#pragma unroll
+      for (int u = 1; u < kCopies; ++u)
+        if (copy == u) p0[i] = t0[i * kCopies + u], p1[i] = t1[i * kCopies + u];
+    }
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       uint32_t v[4][4];  // keys 2c, 2c + 1, 8 + 2c, 8 + 2c + 1: the columns of P that this lane holds
@@ -216,8 +237,11 @@ decode_attn_kernel(DecodeParams p) {
       for (int e = 0; e < 4; ++e) {
         const uint32_t a[4] = {__byte_perm(v[0][e], v[1][e], 0x5410), __byte_perm(v[0][e], v[1][e], 0x7632),
                                __byte_perm(v[2][e], v[3][e], 0x5410), __byte_perm(v[2][e], v[3][e], 0x7632)};
-        mma(acc[j * 4 + e], a, head[0], head[1]);
-        mma(acc[j * 4 + e], a, rest[0], rest[1]);
+        float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = kPasses - 1; i >= 0; --i) mma(o, a, p0[i], p1[i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j * 4 + e][i] += o[i];
       }
     }
     __syncwarp();  // the stage has been read
@@ -230,6 +254,15 @@ decode_attn_kernel(DecodeParams p) {
   __syncthreads();  // the merge buffers overlay the tiles
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
+
+  // The copies' terms of P meet.
+#pragma unroll
+  for (int off = 2; off >= 4 / kCopies; off /= 2) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][e] += __shfl_xor_sync(0xffffffffu, acc[i][e], off);
+  }
 
   // Rows r and r + 8 of MMA tile (j, e) are dims 64 j + 8 r + 2 e and the next.
   const int per_warp = rows * kHeadDim;
@@ -306,9 +339,9 @@ decode_attn_kernel(DecodeParams p) {
   }
 }
 
-template <bool kCluster>
+template <bool kCluster, int kCopies>
 static int launch_attn(const DecodeParams& p, dim3 grid, int rows, cudaStream_t stream) {
-  constexpr auto kernel = decode_attn_kernel<kCluster>;
+  constexpr auto kernel = decode_attn_kernel<kCluster, kCopies>;
   static const cudaError_t configured = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                              attn_smem_bytes(kMmaRows));
   if (configured != cudaSuccess) return -3;
@@ -413,7 +446,10 @@ extern "C" int axb_decode_attn(const void* q, const void* k_pool, const void* v_
   const bool cluster = splits > 1 && splits <= kMaxClusterSplits;
   const dim3 grid(splits, num_kv_heads * ((g + kMmaRows - 1) / kMmaRows), B);
   const int rows = g < kMmaRows ? g : kMmaRows;
-  const int rc = cluster ? launch_attn<true>(p, grid, rows, stream) : launch_attn<false>(p, grid, rows, stream);
+  const auto launch = rows <= 2   ? (cluster ? launch_attn<true, 4> : launch_attn<false, 4>)
+                      : rows <= 4 ? (cluster ? launch_attn<true, 2> : launch_attn<false, 2>)
+                                  : (cluster ? launch_attn<true, 1> : launch_attn<false, 1>);
+  const int rc = launch(p, grid, rows, stream);
   if (rc != 0) return rc;
   if (splits > kMaxClusterSplits)
     launch_chained(decode_combine_kernel, B * num_q_heads, kHeadDim, 0, stream, p.part_out, p.part_ml, p.out, splits);

@@ -56,6 +56,31 @@ def test_paged_decode_attention_at_tile_and_split_edges(nq, nkv, page_size, spli
     assert ((out[1:].float() - ref).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("nq,nkv", [(4, 4), (8, 4), (12, 4), (16, 4), (20, 4), (32, 4), (36, 4)])
+def test_paged_decode_attention_keeps_32_bit_probabilities(nq, nkv):
+    """The splits' 32-bit partials, merged here in 64 bits, for every number of copies of the heads in a tile.  Scores of up
+    to 32 (in powers of two) are rounded by up to 2^-20 in 32 bits, and their probabilities with them; 16-bit terms of P
+    would show as 2^-17 a probability, 1.4e-6 of the result."""
+    from axlearn_b200.ops import decode_ops
+
+    b, t, h, splits = 3, 1500, 128, 9
+    k, v, table = _pools(b, (t + 15) // 16, 16, nkv, h, seed=nq)
+    lengths = torch.tensor([1500, 777, 130], dtype=torch.int32, device="cuda")
+    q = (2 * torch.randn(b, nq, h, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))).bfloat16()
+    scratch = torch.empty(b * nq * splits * (h + 2), device="cuda")
+    decode_ops.paged_decode_attention(q, k, v, table, lengths, splits=splits, scratch=scratch)
+    sums = scratch[:b * nq * splits * h].view(b, nq, splits, h).double()
+    top, total = scratch[b * nq * splits * h:].view(b, nq, splits, 2).double().unbind(-1)
+    weight = torch.exp2(top - top.amax(-1, keepdim=True))
+    got = (sums * weight[..., None]).sum(2) / (total * weight).sum(-1)[..., None]
+    for i in range(b):
+        n = int(lengths[i])
+        kk, vv = (x[table[i].long()].reshape(-1, nkv, h)[:n].double().repeat_interleave(nq // nkv, 1) for x in (k, v))
+        p = (torch.einsum("nh,snh->ns", q[i].double(), kk) * h ** -0.5).softmax(-1)
+        want = torch.einsum("ns,snh->nh", p, vv)
+        assert (got[i] - want).norm() <= 2.0 ** -20 * want.norm()
+
+
 def test_paged_decode_attention_keeps_infinite_values():
     from axlearn_b200.ops import decode_ops
 
