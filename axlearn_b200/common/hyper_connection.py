@@ -23,7 +23,7 @@ from axlearn_b200.common.config import REQUIRED, InstantiableConfig, Required, c
 from axlearn_b200.common.layers import Embedding
 from axlearn_b200.common.module import nowrap
 from axlearn_b200.common.sequence_mixer import PaddedLinear, vector_spec
-from axlearn_b200.ops import hyper_ops, step_ops
+from axlearn_b200.ops import cuda_ops, hyper_ops, step_ops
 from axlearn_b200.ops.hyper_ops import padded
 
 Tensor = torch.Tensor
@@ -277,8 +277,8 @@ class PaddedEmbedding(Embedding):
 
     def forward(self, x: Tensor) -> Tensor:
         w = self.parameters["weight"]
-        if x.shape[-1] == 1 and not torch.is_grad_enabled() and step_ops.embed_rows_supported(w, x):
-            return step_ops.embed_rows(w, x)[..., :self._config.dim]  # a decoding step
+        if cuda_ops.launches_chained() and not torch.is_grad_enabled() and step_ops.embed_rows_supported(w, x):
+            return step_ops.embed_rows(w, x)[..., :self._config.dim]  # a decoding step: its engine has looked at the ids
         rows = torch.nn.functional.embedding(x.long(), self.parameters["weight"])
         return rows[..., :self._config.dim]
 

@@ -116,8 +116,30 @@ embed_rows_kernel(const uint4* __restrict__ table, const int64_t* ids, uint4* ou
   }
 }
 
+// Tokens that a caller hands to a step, one CTA; ids outside [low, high) become 0, and `ok` tells whether there were none.
+__global__ void __launch_bounds__(256)
+take_tokens_kernel(const int64_t* ids, int64_t* tokens, int count, int64_t low, int64_t high, bool* ok) {
+  int good = 1;
+  for (int i = threadIdx.x; i < count; i += 256) {
+    const int64_t id = ids[i];
+    const bool inside = id >= low && id < high;
+    tokens[i] = inside ? id : 0;
+    good &= inside;
+  }
+  good = __syncthreads_and(good);
+  if (threadIdx.x == 0) *ok = good != 0;
+}
+
 }  // namespace
 }  // namespace axb
+
+// tokens [count] = ids [count], see the kernel.
+extern "C" int axb_take_tokens(const int64_t* ids, int64_t* tokens, int count, int64_t low, int64_t high, bool* ok,
+                               cudaStream_t stream) {
+  if (count <= 0) return 0;
+  axb::take_tokens_kernel<<<1, 256, 0, stream>>>(ids, tokens, count, low, high, ok);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
 
 // Returns 0, -10 for unsupported sizes.
 extern "C" int axb_step_end(const axb::StepEndArgs* args, cudaStream_t stream) {

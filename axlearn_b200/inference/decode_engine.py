@@ -131,6 +131,8 @@ class BaseDecodeEngine:
         self.logits = torch.zeros(batch, vocab_size, dtype=torch.float32, device=self.device)
         self._use_graph = use_graph and self.device.type == "cuda"
         self._graph: Optional[torch.cuda.CUDAGraph] = None
+        # Whether the ids that `step_logits` took last lie in the table.
+        self._ids_ok = torch.ones((), dtype=torch.bool, device=self.device)
         self.launches_per_step = 0
 
     def prefill(self, prompt_ids: Tensor, lengths: Optional[Tensor] = None) -> Tensor:
@@ -138,6 +140,10 @@ class BaseDecodeEngine:
 
     def _step(self) -> None:
         raise NotImplementedError(type(self))
+
+    def _id_range(self) -> Optional[tuple]:
+        """``(lowest id, highest id + 1)`` that the embedding takes; None: not known, the embedding itself checks."""
+        return None
 
     def _mutable_buffers(self) -> list:
         """Buffers a step changes and that a warm-up step must leave as they were."""
@@ -178,18 +184,32 @@ class BaseDecodeEngine:
                 t.copy_(old)
             self._graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self._graph), cuda_ops.chained_launches():
+                # The assertion runs beside the step (behind it: 2.5 us more a step).
+                s.wait_stream(torch.cuda.current_stream(self.device))
+                with torch.cuda.stream(s):
+                    step_ops.assert_ids(self._ids_ok)
                 self._step()
+                torch.cuda.current_stream(self.device).wait_stream(s)
 
     @torch.no_grad()
     def step_logits(self, tokens: Tensor) -> Tensor:
         """Feeds one token per sequence (``[batch]``: the token at each sequence's current end),
         appends its K/V and returns the fp32 logits of the next position ``[batch, vocab]`` -- the
-        engine as a ``tokens -> scores`` function for samplers and searches that live outside."""
+        engine as a ``tokens -> scores`` function for samplers and searches that live outside.
+
+        An id outside the embedding table raises ``IndexError`` where it is in host memory; on the GPU it fails an
+        assertion there, which the next synchronisation reports, as in the embedding operator."""
         self._ensure_graph()
-        self.tokens.copy_(tokens.reshape(-1))
+        bounds = self._id_range() if self.device.type == "cuda" else None
+        if bounds is None:
+            self.tokens.copy_(tokens.reshape(-1))
+        else:
+            step_ops.take_tokens(tokens.reshape(-1), self.tokens, *bounds, self._ids_ok)
         if self._graph is not None:
             self._graph.replay()
         else:
+            if bounds is not None:
+                step_ops.assert_ids(self._ids_ok)
             self._step()
         return self.logits
 
@@ -238,6 +258,10 @@ class DecodeEngine(BaseDecodeEngine):
         self._prefill_chunk_tokens = prefill_chunk_tokens
 
     # ------------------------------------------------------------------ shared pieces
+    def _id_range(self) -> Optional[tuple]:
+        rows = self.w["emb"].shape[0]
+        return -rows, rows  # negative ids count from the end
+
     def _gemm_reduce(self, a: Tensor, w: Tensor, residual: Tensor, site: int) -> Tensor:
         """``residual + sum over ranks of (a @ w)``; the finish kernel sums the peers' slots.
 
@@ -389,6 +413,10 @@ class ModuleDecodeEngine(BaseDecodeEngine):
 
     def _mutable_buffers(self) -> list:
         return super()._mutable_buffers() + [t for _, t in flatten_items(self.states)]
+
+    def _id_range(self) -> Optional[tuple]:
+        table = self.params.get("emb", {}).get("token_emb", {}).get("weight")
+        return None if table is None else (0, table.shape[0])
 
     def set_active(self, rows: Tensor) -> None:
         """``rows [batch]``: nonzero = takes part in the following steps."""

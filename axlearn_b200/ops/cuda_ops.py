@@ -208,6 +208,11 @@ def chained_launches():
         _chain.on = bool(before)
 
 
+def launches_chained() -> bool:
+    """Whether the calling thread is inside ``chained_launches``."""
+    return getattr(_chain, "on", False)
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None,
          out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False,
          max_ctas: int = 0, resident: bool = False) -> torch.Tensor:
@@ -352,7 +357,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, *, resident: bool = False) -> torch
     """``resident``: as in ``gemm``; counts in the capture of a decoding step, which has no gradients."""
     if x.shape[-1] % 8 or w.shape[1] % 8:
         return torch.matmul(x, w)
-    if resident and getattr(_chain, "on", False) and not torch.is_grad_enabled() and _fused_fsdp_info(w) is None:
+    if resident and launches_chained() and not torch.is_grad_enabled() and _fused_fsdp_info(w) is None:
         return gemm(x.reshape(-1, x.shape[-1]), w, resident=True).reshape(x.shape[:-1] + (w.shape[1],))
     return _Linear.apply(x, w)
 

@@ -27,7 +27,8 @@ def _lib():
         h.axb_step_end.argtypes = [ctypes.POINTER(_StepEndArgs), c_void_p]
         h.axb_embed_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_int64, c_int,
                                      c_void_p, c_void_p]
-        h.axb_step_end.restype = h.axb_embed_rows.restype = c_int
+        h.axb_take_tokens.argtypes = [c_void_p, c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p]
+        h.axb_step_end.restype = h.axb_embed_rows.restype = h.axb_take_tokens.restype = c_int
         _configured = True
     return h
 
@@ -63,6 +64,30 @@ def step_end(logits: torch.Tensor, tokens: torch.Tensor, *, logits_out: Optional
     args.ld, args.B, args.V, args.kept = logits.stride(0), b, v, len(kept)
     rc = _lib().axb_step_end(ctypes.byref(args), cuda_ops._stream())  # pylint: disable=protected-access
     cuda_ops._check(rc, "axb_step_end")  # pylint: disable=protected-access
+
+
+def assert_ids(ok: torch.Tensor) -> None:
+    """An assertion on the device, as in torch's embedding: the next synchronisation reports it."""
+    torch._assert_async(ok, "token id outside the embedding table")  # pylint: disable=protected-access
+
+
+def take_tokens(ids: torch.Tensor, tokens: torch.Tensor, low: int, high: int, ok: torch.Tensor) -> None:
+    """``tokens.copy_(ids)`` (``tokens``: int64 on the GPU) for ids that have to lie in ``[low, high)``.
+
+    Ids in host memory raise ``IndexError`` before anything is launched.  Of ids on the GPU ``ok`` (a bool) tells whether
+    all do; the others become 0."""
+    if not ids.is_cuda:
+        if ids.numel() and not (low <= int(ids.min()) and int(ids.max()) < high):
+            raise IndexError(f"token id outside the embedding table: ids go from {low} to {high - 1}")
+        tokens.copy_(ids)
+        ok.fill_(True)
+        return
+    if not (ids.dtype == torch.int64 and ids.shape == tokens.shape and ids.is_contiguous() and ids.device == tokens.device):
+        tokens.copy_(ids)
+        ids = tokens
+    rc = _lib().axb_take_tokens(ids.data_ptr(), tokens.data_ptr(), tokens.numel(), low, high, ok.data_ptr(),
+                                cuda_ops._stream())  # pylint: disable=protected-access
+    cuda_ops._check(rc, "axb_take_tokens")  # pylint: disable=protected-access
 
 
 def embed_rows_supported(table: torch.Tensor, ids: torch.Tensor) -> bool:

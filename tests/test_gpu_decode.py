@@ -185,6 +185,82 @@ def test_chained_module_steps_see_new_weights_and_match_separate_launches(family
             assert torch.equal(x, y)
 
 
+def _fuji_engine(use_graph, batch=3):
+    from axlearn_b200.inference.decode_engine import DecodeEngine, FujiDims, LayerWeights
+
+    d, f, vocab, nq, nkv = 256, 512, 1000, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(0)
+
+    def w(*shape):
+        return (torch.randn(*shape, device="cuda", generator=g) * shape[0] ** -0.5).bfloat16()
+
+    layers = [LayerWeights(attn_norm=1 + 0.1 * w(d), wqkv=w(d, (nq + 2 * nkv) * 128), wo=w(nq * 128, d),
+                           ffn_norm=1 + 0.1 * w(d), wgu=w(d, 2 * f), wdown=w(f, d)) for _ in range(2)]
+    weights = {"layers": layers, "emb": w(vocab, d) * 16, "head": w(vocab, d), "final_norm": 1 + 0.1 * w(d)}
+    dims = FujiDims(num_layers=2, hidden_dim=d, num_heads=nq, num_kv_heads=nkv, head_dim=128, ffn_dim=f, vocab_size=vocab)
+    return DecodeEngine(weights, dims, batch=batch, max_len=64, use_graph=use_graph), vocab, -vocab, vocab
+
+
+def _module_engine(use_graph, tmp_path, batch=3):
+    from axlearn_b200.inference.decode_engine import ModuleDecodeEngine
+    from axlearn_b200.inference.model_loader import load_model
+    from tests import sagisun_checkpoints as ckpt
+
+    cfg = ckpt.CONFIGS["odd"]
+    loaded = load_model(ckpt.save(tmp_path, cfg, ckpt.random_tensors(cfg)), dtype=torch.bfloat16, device="cuda")
+    engine = ModuleDecodeEngine(loaded.decoder, loaded.parameters["decoder"], batch=batch, max_len=64, device="cuda",
+                                use_graph=use_graph)
+    return engine, cfg["vocab"], 0, (cfg["vocab"] + 31) // 32 * 32  # rows of the padded table
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("kind", ["fuji", "module"])
+def test_step_logits_refuses_ids_outside_the_table(kind, use_graph, monkeypatch, tmp_path):
+    """On the host before anything runs; on the GPU by the operator's way, an assertion on the device: a stand-in for it
+    records here which flag it is given (in the captured step, or by every separate one)."""
+    from axlearn_b200.ops import cuda_ops
+
+    engine, vocab, low, high = _fuji_engine(use_graph) if kind == "fuji" else _module_engine(use_graph, tmp_path)
+    asserted = []
+    monkeypatch.setattr(torch, "_assert_async", lambda ok, message: asserted.append(ok))
+    ids = torch.randint(0, vocab, (3, 5), device="cuda")
+    engine.prefill(ids)
+    lengths = engine.lengths.clone()
+    for bad in (high, low - 1, 1 << 40, -(1 << 40)):
+        with pytest.raises(IndexError, match="outside"):
+            engine.step_logits(torch.tensor([0, bad, 1]))
+        assert torch.equal(engine.lengths, lengths)
+        logits = engine.step_logits(torch.tensor([0, bad, 1], device="cuda"))
+        assert not engine._ids_ok  # pylint: disable=protected-access
+        assert logits.isfinite().all()  # the step itself has not seen the id
+        engine.prefill(ids)
+    cuda_ops.check_status()
+    given = torch.tensor([low, high - 1, 0], device="cuda")
+    for feed in (given, given.cpu(), given.int(), given[:, None]):
+        engine.prefill(ids)
+        got = engine.step_logits(feed).clone()
+        engine.prefill(ids)
+        assert engine._ids_ok  # pylint: disable=protected-access
+        assert torch.equal(got, engine.step_logits(given)) and got.isfinite().all()
+    assert len(asserted) == (1 if use_graph else 12)
+    assert all(ok is engine._ids_ok for ok in asserted)  # pylint: disable=protected-access
+
+
+def test_a_layer_call_with_one_token_keeps_the_embedding_operator(monkeypatch, tmp_path):
+    """The gather that only marks bad ids is for captured steps, whose engine has looked at them."""
+    from axlearn_b200.ops import step_ops
+
+    engine = _module_engine(False, tmp_path)[0]
+    engine.prefill(torch.randint(0, 60, (3, 4), device="cuda"))
+
+    def refuse(*_, **__):
+        raise AssertionError("the marking gather outside of a captured step")
+
+    monkeypatch.setattr(step_ops, "embed_rows", refuse)
+    engine.extend(torch.randint(0, 60, (3, 1), device="cuda"))
+    engine.step_logits(torch.randint(0, 60, (3,), device="cuda"))
+
+
 @pytest.mark.parametrize("b,v,ld", [(1, 1, 4), (3, 33, 40), (2, 4096, 4096), (5, 32768, 32768), (2, 32772, 32776)])
 def test_step_end_picks_as_torch_and_keeps(b, v, ld):
     """Vector and element paths around one pass of the block; ties go to the first, NaN above all."""
