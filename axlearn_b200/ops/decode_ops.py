@@ -19,7 +19,7 @@ from typing import Optional
 
 import torch
 
-from axlearn_b200.ops import cuda_ops
+from axlearn_b200.ops import cuda_ops, flash_sm100
 
 c_void_p, c_int, c_int64, c_float = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_float
 _configured = False
@@ -172,7 +172,8 @@ def prompt_attention(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tens
                      num_q_heads: int, softmax_scale: float) -> torch.Tensor:
     """Whole prompts from position 0: ``qkv [B, T, (Nq + 2 Nkv) * H]`` of one projection (its q columns are rotated
     in place), pools ``[B, S, Nkv, H]`` with S >= T token rows a sequence, which get rotated k and plain v and are what
-    causal attention reads.  Returns ``[B, T, Nq * H]``."""
+    causal attention reads.  Returns ``[B, T, Nq * H]``.  The forward kernels that ``AXB200_FLASH_FWD`` names beside v3
+    read contiguous operands, copied here."""
     b, t, width = qkv.shape
     _, rows, nkv, h = k_pool.shape
     assert qkv.is_contiguous() and k_pool.is_contiguous() and v_pool.is_contiguous() and k_pool.shape[0] == b
@@ -181,6 +182,11 @@ def prompt_attention(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tens
     rc = _lib().axb_rope_append_prompt(qkv.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), table.data_ptr(), b, t,
                                        rows, num_q_heads, nkv, h, stream)
     cuda_ops._check(rc, "axb_rope_append_prompt")  # pylint: disable=protected-access
+    if flash_sm100.FORWARD_VARIANT != "v3":
+        q = qkv[..., :num_q_heads * h].reshape(b, t, num_q_heads, h).contiguous()
+        out, _ = flash_sm100.forward(q, k_pool[:, :t].contiguous(), v_pool[:, :t].contiguous(), causal=True,
+                                     scale=softmax_scale)
+        return out.reshape(b, t, num_q_heads * h)
     out = torch.empty((b, t, num_q_heads * h), dtype=qkv.dtype, device=qkv.device)
     rc = _lib().axb_flash_fwd_strided(qkv.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(), b, t,
                                       num_q_heads, nkv, h, width, t * width, nkv * h, rows * nkv * h, softmax_scale,

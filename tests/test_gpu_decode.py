@@ -344,6 +344,28 @@ def test_prompt_attention_equals_rotation_copies_and_attention(b, t, nq, nkv):
     assert torch.equal(got.reshape(want.shape), want)
 
 
+@pytest.mark.parametrize("variant", ["v1", "v2"])
+def test_prompt_attention_follows_the_chosen_forward_kernel(variant, monkeypatch):
+    """Bit for bit that kernel on separate tensors, where it was always v3."""
+    from axlearn_b200.ops import cuda_ops, decode_ops, flash_sm100
+
+    b, t, nq, nkv, h = 2, 150, 6, 2, 128
+    qkv = torch.randn(b, t, (nq + 2 * nkv) * h, device="cuda").bfloat16()
+    kp, vp = (torch.zeros((b, t + 5, nkv, h), device="cuda").bfloat16() for _ in range(2))
+    table = decode_ops.rope_table(t, h, 5e5, "cuda")
+    v3 = decode_ops.prompt_attention(qkv.clone(), kp, vp, table, num_q_heads=nq, softmax_scale=0.1)
+    q = cuda_ops.rope(qkv.reshape(b, t, nq + 2 * nkv, h)[:, :, :nq], torch.arange(t, device="cuda"), 5e5)
+    monkeypatch.setattr(flash_sm100, "FORWARD_VARIANT", variant)
+    want, _ = flash_sm100.forward(q.contiguous(), kp[:, :t].contiguous(), vp[:, :t].contiguous(), causal=True, scale=0.1)
+    calls, forward = [], flash_sm100.forward
+    monkeypatch.setattr(flash_sm100, "forward", lambda *a, **k: calls.append(1) or forward(*a, **k))
+    got = decode_ops.prompt_attention(qkv, kp, vp, table, num_q_heads=nq, softmax_scale=0.1)
+    cuda_ops.check_status()
+    assert calls and torch.equal(got.reshape(want.shape), want)
+    # Each is within bf16 roundings of P and the output (2^-8 each) of the same sums of values of size max|v|.
+    assert ((got.float() - v3.float()).abs() <= 2.0 ** -6 * vp.abs().max().float()).all()
+
+
 @pytest.mark.parametrize("rows,f", [(1, 8), (3, 98), (2, 4096), (5, 4104), (70000, 16)])
 def test_swiglu_packed_sizes(rows, f):
     """Vector and pairwise paths, around a block's 512 vectors, and more rows than a grid is high."""
