@@ -71,6 +71,8 @@ def lib() -> ctypes.CDLL:
                     fn = getattr(h, name)
                     fn.argtypes = getattr(_Sigs, name)
                     fn.restype = c_int
+            if hasattr(h, "axb_embedding_bwd_bytes"):
+                h.axb_embedding_bwd_bytes.restype = c_int64
             _lib_handle = h
     return _lib_handle
 
@@ -101,6 +103,7 @@ class _Sigs:
     axb_adamw = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_float,
                  c_float, c_float, c_float, c_float, c_float, c_float, c_void_p]
     axb_embedding_bwd = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
+    axb_embedding_bwd_bytes = [c_int, c_int, c_int]
     axb_scale_bf16 = [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]
     axb_sumsq_ctas = []
     axb_sumsq = [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_float, c_int, c_void_p]
@@ -664,7 +667,7 @@ class _Embedding(torch.autograd.Function):
             dy = dy.clone()
         ids = ids.contiguous()
         dw = torch.empty((ctx.rows, d), dtype=dy.dtype, device=dy.device)
-        work = torch.empty(n + 3 * ctx.rows, dtype=torch.int32, device=dy.device)
+        work = torch.empty(lib().axb_embedding_bwd_bytes(n, ctx.rows, d), dtype=torch.uint8, device=dy.device)
         _check(lib().axb_embedding_bwd(dy.data_ptr(), ids.data_ptr(), dw.data_ptr(), work.data_ptr(), n, ctx.rows, d,
                                        _stream()), "axb_embedding_bwd")
         return None, dw
@@ -675,6 +678,7 @@ def embedding(ids: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     operator but not an autograd node around it, keep the operator."""
     if not (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.requires_grad and torch.is_grad_enabled()
             and w.shape[1] % 8 == 0 and w.numel() > 0 and ids.dtype == torch.int64 and ids.numel() < 1 << 30
+            and type(w) in (torch.Tensor, torch.nn.Parameter)  # (not a traced or wrapped table)
             and torch.autograd.forward_ad._current_level < 0  # pylint: disable=protected-access
             and not torch._C._are_functorch_transforms_active()):  # pylint: disable=protected-access
         return torch.nn.functional.embedding(ids, w)

@@ -206,6 +206,64 @@ def test_embedding_gradient(v, d, n):
     assert ((runs[0].double() - want).abs() <= 2.0 ** -8 * want.abs() + n * 2.0 ** -24 * size).all()
 
 
+def _skewed_ids(kind, v, n, g):
+    if kind == "one":
+        return torch.full((n,), v // 2, device="cuda")
+    if kind == "half":
+        ids = torch.randint(0, v, (n,), device="cuda", generator=g)
+        ids[torch.rand(n, device="cuda", generator=g) < 0.5] = 0
+        return ids
+    if kind == "runs":  # lists of 65 tokens: segments begin and end inside rows
+        return (torch.cumsum(torch.ones(n, dtype=torch.int64, device="cuda"), 0) // 65) % v
+    rank = torch.arange(1, v + 1, device="cuda", dtype=torch.float32)  # text-like: frequency 1 / rank
+    return torch.multinomial(1 / rank, n, replacement=True, generator=g)
+
+
+@pytest.mark.parametrize("kind", ["one", "half", "runs", "zipf"])
+@pytest.mark.parametrize("v,d,n", [(3, 8, 33), (300, 264, 64), (40, 2056, 65), (300, 512, 129), (1000, 2056, 8192),
+                                   (130, 64, 140000), (50, 16, 600000)])
+def test_embedding_gradient_of_frequent_ids(kind, v, d, n):
+    """Rows that are ordered in a bitmap (above 32 tokens; more tokens than its window), summed by segment (of 64 to
+    512 tokens) and merged, for every way a row can lie over the segments."""
+    from axlearn_b200.ops import cuda_ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ids = _skewed_ids(kind, v, n, g)
+    w = torch.zeros(v, d, device="cuda").bfloat16().requires_grad_()
+    dy = torch.randn(n, d, device="cuda", generator=g).bfloat16()
+    runs = [torch.autograd.grad(cuda_ops.embedding(ids, w), w, dy)[0] for _ in range(2)]
+    assert torch.equal(*runs)
+    want = torch.zeros(v, d, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
+    size = torch.zeros_like(want).index_add_(0, ids, dy.double().abs())
+    # Half a unit of bf16 (up to 2^-8 of the sum), and a 32-bit sum of up to 512 terms and of up to n / 512 + 1 such sums.
+    terms = min(n, 512) + n // 512 + 1
+    assert ((runs[0].double() - want).abs() <= 2.0 ** -8 * want.abs() + terms * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("kind", ["half", "one"])
+def test_frequent_ids_cost_no_more_than_the_operator(kind):
+    from axlearn_b200.ops import cuda_ops
+
+    v, d, n = 32768, 4096, 8192
+    g = torch.Generator(device="cuda").manual_seed(0)
+    ids = _skewed_ids(kind, v, n, g)
+    w = torch.zeros(v, d, device="cuda").bfloat16().requires_grad_()
+    dy = torch.randn(n, d, device="cuda", generator=g).bfloat16()
+
+    def best(embedding):
+        y, times = embedding(ids, w), []
+        for _ in range(8):
+            a, z = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            torch.autograd.grad(y, w, dy, retain_graph=True)
+            z.record()
+            z.synchronize()
+            times.append(a.elapsed_time(z))
+        return min(times)
+
+    assert best(cuda_ops.embedding) < best(torch.nn.functional.embedding)
+
+
 def test_embedding_gradient_can_be_differentiated_again():
     from axlearn_b200.ops import cuda_ops
 
