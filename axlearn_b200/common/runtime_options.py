@@ -37,7 +37,8 @@ KNOBS: dict[str, tuple[str, str]] = {
     "AXB200_FLASH_FWD": ("v3", "Flash-attention forward kernel: v3 (scores in registers), v2 or v1."),
     "AXB200_FLASH_BWD": ("fused", "Flash-attention backward: fused (one kernel, 5 GEMMs) or split (dK/dV + dQ kernels)."),
     "AXB200_RMSNORM": ("warp", "RMSNorm kernels: warp (rows held in registers, where the width allows) or plain."),
-    "AXB_DECODE_ATTN": ("", "head / head1 / head2: `default_splits` reckons with 4 / 1 / 2 query heads per CTA (the decoding engine does not use it)."),
+    "AXB_DECODE_ATTN": ("", "head / head1 / head2: `default_splits` reckons with 4 / 1 / 2 query heads per CTA; the decoding "
+                            "engine does not use it."),
     "AXB200_MOE_GROUP_BLOCK": ("256", "Rows to which each expert's token run is padded (256: CTA-pair grouped GEMM; 128: single CTA)."),
     "AXB_MOE_PEER_EXCHANGE": ("1", "0: NCCL all-to-all for expert parallelism; 1: peer-memory exchange kernels; force: also when sizes are small."),
     "AXB200_FUSED_FSDP": ("1", "0: NCCL all-gather / reduce-scatter for FSDP instead of the GEMM-fused peer-memory paths."),

@@ -323,8 +323,11 @@ extern "C" int axb_expert_combine(const void* y, const int* place, void* out, in
   if (tokens <= 0) return 0;
   if (width <= 0 || (width % 8) || (y_ld % 8) || (out_ld % 8) || top <= 0) return -10;
   if (act_bf16)
-    axb::launch_chained(axb::expert_combine_kernel<__nv_bfloat16>, static_cast<unsigned>(tokens), 128, 0, stream, static_cast<const __nv_bfloat16*>(y), place, static_cast<__nv_bfloat16*>(out), y_ld, out_ld, top, width);
+    axb::launch_chained(axb::expert_combine_kernel<__nv_bfloat16>, static_cast<unsigned>(tokens), 128, 0, stream,
+                        static_cast<const __nv_bfloat16*>(y), place, static_cast<__nv_bfloat16*>(out), y_ld, out_ld, top,
+                        width);
   else
-    axb::launch_chained(axb::expert_combine_kernel<float>, static_cast<unsigned>(tokens), 128, 0, stream, static_cast<const float*>(y), place, static_cast<float*>(out), y_ld, out_ld, top, width);
+    axb::launch_chained(axb::expert_combine_kernel<float>, static_cast<unsigned>(tokens), 128, 0, stream,
+                        static_cast<const float*>(y), place, static_cast<float*>(out), y_ld, out_ld, top, width);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

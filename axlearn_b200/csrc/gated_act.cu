@@ -51,15 +51,18 @@ static int launch_gated_act(const void* gu, void* out, int64_t rows, int F, int 
                             int act_bf16, float limit, float alpha, cudaStream_t stream) {
   if (act_bf16 && F % 8 == 0 && up_off % 8 == 0 && ld % 8 == 0 && out_ld == F) {
     const int64_t n8 = rows * (F / 8);
-    launch_chained(gated_act_vec_kernel<K>, static_cast<unsigned>((n8 + 255) / 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), n8, up_off, ld, out_ld, limit, alpha);
+    launch_chained(gated_act_vec_kernel<K>, static_cast<unsigned>((n8 + 255) / 256), 256, 0, stream,
+                   static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), n8, up_off, ld, out_ld, limit,
+                   alpha);
   } else {
     const int64_t n = rows * out_ld;
     const unsigned grid = static_cast<unsigned>((n + 255) / 256);
     if (act_bf16)
-      launch_chained(gated_act_kernel<__nv_bfloat16, K>, grid, 256, 0, stream, static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), n, F, up_off, ld, out_ld, limit, alpha);
+      launch_chained(gated_act_kernel<__nv_bfloat16, K>, grid, 256, 0, stream, static_cast<const __nv_bfloat16*>(gu),
+                     static_cast<__nv_bfloat16*>(out), n, F, up_off, ld, out_ld, limit, alpha);
     else
-      launch_chained(gated_act_kernel<float, K>, grid, 256, 0, stream, static_cast<const float*>(gu), static_cast<float*>(out), n, F,
-                                                           up_off, ld, out_ld, limit, alpha);
+      launch_chained(gated_act_kernel<float, K>, grid, 256, 0, stream, static_cast<const float*>(gu),
+                     static_cast<float*>(out), n, F, up_off, ld, out_ld, limit, alpha);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -432,8 +432,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
 template <int BN, int STAGES, bool A_MN, bool B_MN, typename OutT, bool FUSED = false>
 static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda,
                        int64_t ldb, int64_t ldc, int accumulate, int* status, int max_ctas,
-                       cudaStream_t stream, const FusedParams* fused = nullptr, int group_mode = 0, int num_groups = 1, const int* group_index = nullptr,
-                       int64_t c_group_stride = 0, int group_block_rows = kBlockM) {
+                       cudaStream_t stream, const FusedParams* fused = nullptr, int group_mode = 0,
+                       int num_groups = 1, const int* group_index = nullptr, int64_t c_group_stride = 0,
+                       int group_block_rows = kBlockM) {
   // Grouped mode 1 stacks the groups' B matrices along the outer dim of one tensor map.
   const uint64_t b_stack = group_mode == 1 ? static_cast<uint64_t>(num_groups) : 1;
   CUtensorMap ta, tb;
@@ -508,7 +509,8 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   // warp contributes to.
   if (grid > cap) grid = cap;
   if (grid < 1) return -12;
-  GemmParams p{M, N, K, C, ldc, status, accumulate, group_mode, num_groups, group_index, B_MN ? K : N, c_group_stride, group_block_rows};
+  GemmParams p{M, N, K, C, ldc, status, accumulate, group_mode, num_groups, group_index, B_MN ? K : N,
+               c_group_stride, group_block_rows};
   kernel<<<grid, FUSED ? kFusedThreads : kNumThreads, kSmem, stream>>>(ta, tb, tl, p, fp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -586,9 +588,11 @@ extern "C" int axb_gemm_bf16_grouped(const void* A, const void* B, void* C, int 
   if (a_mn_major == (AM ? 1 : 0) && b_mn_major == (BM ? 1 : 0) && out_fp32 == (sizeof(T) == 4)) { \
     if (N >= 256)                                                                                  \
       return launch_gemm<256, 4, AM, BM, T>(A, B, C, M, N, K, lda, ldb, ldc, 0, status, max_ctas,  \
-                                            stream, nullptr, mode, num_groups, group_index, c_group_stride, block_rows);  \
+                                            stream, nullptr, mode, num_groups, group_index,        \
+                                            c_group_stride, block_rows);                           \
     return launch_gemm<128, 6, AM, BM, T>(A, B, C, M, N, K, lda, ldb, ldc, 0, status, max_ctas,    \
-                                          stream, nullptr, mode, num_groups, group_index, c_group_stride, block_rows);                \
+                                          stream, nullptr, mode, num_groups, group_index,          \
+                                          c_group_stride, block_rows);                             \
   }
   AXB_GROUPED_CASE(false, false, __nv_bfloat16)
   AXB_GROUPED_CASE(false, true, __nv_bfloat16)

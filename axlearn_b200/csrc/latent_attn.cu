@@ -598,7 +598,8 @@ extern "C" int axb_latent_prep(const axb::LatentArgs* args, cudaStream_t stream)
   if (a.act_bf16 && a.qbuf == nullptr && a.lat != nullptr && !(aligned & 7)) {
     const int64_t ctas = (static_cast<int64_t>(a.B) * a.T + axb::kLvTokens - 1) / axb::kLvTokens;
     if (smem * axb::kLvTokens <= 48 * 1024) {
-      axb::launch_chained(axb::latent_prep_vec_kernel, static_cast<unsigned>(ctas), 64 * axb::kLvTokens, smem * axb::kLvTokens, stream, a);
+      axb::launch_chained(axb::latent_prep_vec_kernel, static_cast<unsigned>(ctas), 64 * axb::kLvTokens,
+                          smem * axb::kLvTokens, stream, a);
       return axb::latent_launched();
     }
   }
