@@ -109,8 +109,25 @@ class _Sigs:
     axb_sumsq = [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_float, c_int, c_void_p]
 
 
+# Names that torch does not promise, with the public or the safe way behind them.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # pylint: disable=protected-access
+_device_index = getattr(torch._C, "_cuda_getDevice", None)  # pylint: disable=protected-access
+
+
 def _stream() -> int:
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())  # pylint: disable=protected-access
+    if _raw_stream is None or _device_index is None:
+        return torch.cuda.current_stream().cuda_stream  # 2 us more
+    return _raw_stream(_device_index())
+
+
+def _transformed() -> bool:
+    """Whether forward-mode differentiation or a function transform is on, which know torch's operators but not a kernel
+    behind their back; unknown counts as on."""
+    try:
+        # pylint: disable-next=protected-access
+        return torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+    except AttributeError:
+        return True
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -679,8 +696,7 @@ def embedding(ids: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     if not (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.requires_grad and torch.is_grad_enabled()
             and w.shape[1] % 8 == 0 and w.numel() > 0 and ids.dtype == torch.int64 and ids.numel() < 1 << 30
             and type(w) in (torch.Tensor, torch.nn.Parameter)  # (not a traced or wrapped table)
-            and torch.autograd.forward_ad._current_level < 0  # pylint: disable=protected-access
-            and not torch._C._are_functorch_transforms_active()):  # pylint: disable=protected-access
+            and not _transformed()):
         return torch.nn.functional.embedding(ids, w)
     return _Embedding.apply(ids, w)
 
@@ -689,8 +705,7 @@ def scaled(x: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
     """``x * g.to(x.dtype)`` for a scalar ``g`` on the device."""
     dense = x if x.is_contiguous() else x.t() if x.dim() == 2 and x.t().is_contiguous() else None
     if (dense is None or not x.is_cuda or x.dtype != torch.bfloat16 or g.dtype != torch.float32 or g.numel() != 1
-            or x.numel() % 8 or x.data_ptr() % 16 or torch.is_grad_enabled()
-            or torch._C._are_functorch_transforms_active()):  # pylint: disable=protected-access
+            or x.numel() % 8 or torch.is_grad_enabled() or _transformed() or x.data_ptr() % 16):
         return x * g.to(x.dtype)
     out = torch.empty_like(dense)
     _check(lib().axb_scale_bf16(dense.data_ptr(), g.data_ptr(), out.data_ptr(), x.numel(), _stream()), "axb_scale_bf16")

@@ -275,6 +275,27 @@ def test_embedding_gradient_can_be_differentiated_again():
     assert torch.equal(back, torch.ones_like(back))
 
 
+def test_embedding_and_scaling_under_transforms(monkeypatch):
+    """Function transforms and forward mode go through torch's operators, as does everything where they cannot be told."""
+    from axlearn_b200.ops import cuda_ops
+
+    w, tangent = (torch.randn(6, 16, device="cuda").bfloat16() for _ in range(2))
+    ids = torch.tensor([1, 1, 4], device="cuda")
+    grad = torch.func.grad(lambda t: cuda_ops.embedding(ids, t).float().sum())(w)
+    assert torch.equal(grad.float().sum(1), 16.0 * torch.tensor([0, 2, 0, 0, 1, 0], device="cuda"))
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(w.clone().requires_grad_(), tangent)
+        out = torch.autograd.forward_ad.unpack_dual(cuda_ops.embedding(ids, dual))
+        assert torch.equal(out.tangent, tangent[ids])
+    g = torch.tensor(0.37, device="cuda")
+    with torch.no_grad():
+        rows = torch.func.vmap(lambda row: cuda_ops.scaled(row, g))(w)
+        assert torch.equal(rows, w * g.bfloat16())
+        monkeypatch.delattr(torch._C, "_are_functorch_transforms_active")  # another version of torch
+        assert cuda_ops._transformed()  # pylint: disable=protected-access
+        assert torch.equal(cuda_ops.scaled(w, g), rows)
+
+
 @pytest.mark.parametrize("shape", [(8,), (3, 2056), (70001, 8)])
 def test_scaled_equals_the_product(shape):
     from axlearn_b200.ops import cuda_ops
