@@ -42,3 +42,27 @@ def test_kernel_shape_follows_the_environment(monkeypatch):
     assert decode_ops._kernel_shape(64, 8, 4) == (512, 2)        # pylint: disable=protected-access
     monkeypatch.setenv("AXB_DECODE_ATTN", "head1")
     assert decode_ops._kernel_shape(64, 8, 4) == (2048, 8)       # pylint: disable=protected-access
+
+
+@pytest.mark.parametrize("batch,kv,group,tokens,want", [
+    (1, 16, 1, 320, 8),        # few CTAs: as many as a cluster merges
+    (1, 8, 4, 4000, 16),       # 8 would leave most SMs empty
+    (16, 8, 4, 2048, 3),       # 128 CTAs: one wave of three per SM
+    (64, 32, 1, 2000, 1),      # more than a wave of CTAs as it is
+    (1, 8, 4, 40, 1),          # half a tile for each of four warps
+    (1, 8, 4, 16, 1),
+    (4, 2, 9, 2048, 8),        # nine query heads are two CTAs
+])
+def test_tile_splits(batch, kv, group, tokens, want):
+    assert decode_ops.tile_splits(batch, kv, group, tokens) == want
+
+
+def test_tile_splits_stay_within_a_wave_and_a_cluster():
+    for batch in (1, 2, 7, 16, 64, 300):
+        for kv, group in ((32, 1), (8, 4), (2, 16), (1, 1)):
+            for tokens in (1, 31, 64, 1000, 100000):
+                s = decode_ops.tile_splits(batch, kv, group, tokens)
+                ctas = batch * kv * ((group + 7) // 8)
+                assert 1 <= s <= 16 and s * 32 <= max(tokens, 32)
+                assert s == 1 or s * ctas <= 3 * 148
+                assert s <= 8 or 16 * ctas <= 148
