@@ -412,8 +412,9 @@ rope_append_kernel(const __nv_bfloat16* qkv, __nv_bfloat16* q_out, __nv_bfloat16
 
 }  // namespace axb
 
-// Scratch needed by axb_decode_attn for `splits > 1`: floats.
+// Scratch needed by axb_decode_attn: floats.  Up to a cluster's splits meet without any.
 extern "C" int64_t axb_decode_attn_scratch_floats(int B, int num_q_heads, int splits) {
+  if (splits <= axb::kMaxClusterSplits) return 0;
   return static_cast<int64_t>(B) * num_q_heads * splits * (axb::kHeadDim + 2);
 }
 
@@ -436,7 +437,7 @@ extern "C" int axb_decode_attn(const void* q, const void* k_pool, const void* v_
   p.part_out = scratch;
   p.part_ml = scratch == nullptr ? nullptr
                                  : scratch + static_cast<int64_t>(B) * num_q_heads * splits * kHeadDim;
-  if (splits > 1 && scratch == nullptr) return -10;
+  if (splits > kMaxClusterSplits && scratch == nullptr) return -10;
   p.num_q_heads = num_q_heads;
   p.num_kv_heads = num_kv_heads;
   p.page_size = page_size;
@@ -464,9 +465,10 @@ extern "C" int axb_rope_append_paged(const void* qkv, void* q_out, void* k_pool,
   if (head_dim != kHeadDim) return -10;
   if (B <= 0) return 0;
   dim3 grid(num_q_heads + 2 * num_kv_heads, B);
-  launch_chained(rope_append_kernel, grid, kHeadDim / 2, 0, stream, static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out),
-      static_cast<__nv_bfloat16*>(k_pool), static_cast<__nv_bfloat16*>(v_pool), page_table, lengths,
-      num_q_heads, num_kv_heads, page_size, max_pages, log2f(theta), apply_rope);
+  launch_chained(rope_append_kernel, grid, kHeadDim / 2, 0, stream, static_cast<const __nv_bfloat16*>(qkv),
+                 static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_pool),
+                 static_cast<__nv_bfloat16*>(v_pool), page_table, lengths, num_q_heads, num_kv_heads, page_size,
+                 max_pages, log2f(theta), apply_rope);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

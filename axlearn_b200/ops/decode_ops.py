@@ -58,8 +58,9 @@ def _lib():
 
 
 def _kernel_shape(batch: int, num_kv_heads: int, group: int) -> tuple[int, int]:
-    """``(CTAs of one split, CTAs that fit one SM)`` that ``default_splits`` reckons with: 128 threads each, residency limited by registers -- 64 with the occupancy
-    bound / 125 / 193 for the per-head kernel with 1 / 2 / 4 query heads per CTA, 225 for the
+    """``(CTAs of one split, CTAs that fit one SM)`` that ``default_splits`` reckons with, those of two kernels of one to
+    four query heads a CTA that are no longer here: 128 threads each, residency limited by registers -- 64 with the
+    occupancy bound / 125 / 193 for the per-head kernel with 1 / 2 / 4 query heads per CTA, 225 for the
     row-contiguous kernel of four KV heads x four query heads."""
     mode = os.environ.get("AXB_DECODE_ATTN", "")
     natural = 4 if group % 4 == 0 else 2 if group % 2 == 0 else 1
@@ -73,8 +74,9 @@ def _kernel_shape(batch: int, num_kv_heads: int, group: int) -> tuple[int, int]:
 
 
 def default_splits(batch: int, num_kv_heads: int, group: int, max_len: int, page_size: int, sms: int = 148) -> int:
-    """KV splits for callers that fix them without ``tile_splits`` (which the engine uses): enough CTAs for up to four per SM without splitting below 8 pages; once that grid
-    is more than one wave of resident CTAs, the nearby split count whose last wave is fullest (the
+    """KV splits by CTAs of up to four query heads, for callers that have fixed theirs by it; ``tile_splits`` is the rule
+    for the kernel as it is, and the engine's.  Enough CTAs for up to four per SM without splitting below 8 pages; once
+    that grid is more than one wave of resident CTAs, the nearby split count whose last wave is fullest (the
     CTAs of a decode step all run about equally long, so a grid of 1.15 waves takes the time of 2)."""
     ctas, resident = _kernel_shape(batch, num_kv_heads, group)
     pages = max(1, max_len // page_size)
@@ -115,8 +117,9 @@ def paged_decode_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.
     assert page_table.dtype == torch.int32 and lengths.dtype == torch.int32 and page_table.is_contiguous()
     if out is None:
         out = torch.empty_like(q)
-    if splits > 1 and scratch is None:
-        scratch = torch.empty(_lib().axb_decode_attn_scratch_floats(b, nq, splits), dtype=torch.float32, device=q.device)
+    if scratch is None:
+        floats = _lib().axb_decode_attn_scratch_floats(b, nq, splits)
+        scratch = torch.empty(floats, dtype=torch.float32, device=q.device) if floats else None
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(h)
     rc = _lib().axb_decode_attn(q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), page_table.data_ptr(),
                                 lengths.data_ptr(), out.data_ptr(), None if scratch is None else scratch.data_ptr(),
