@@ -81,9 +81,8 @@ def test_gemm_deterministic():
                                    (8, 12288, 4096), (16, 22016, 4096), (48, 4096, 4096), (8, 32768, 4096), (5, 9504, 2112)])
 @pytest.mark.parametrize("b_t", [False, True])
 def test_skinny_gemm_split_k(m, n, k, b_t):
-    """Decode-shaped problems (one row block): 64-column tiles, split over K or cut into equal
-    runs of (tile, k-block) units per SM (stream-K) where the plan says so; bf16 and fp32 outputs,
-    with and without accumulation, repeated to exercise the counters."""
+    """Decode-shaped problems (at most 128 rows) as the kernel's own plan lays them out: K slices met in a cluster where
+    it splits; bf16 and fp32 outputs, with and without accumulation, repeated."""
     from axlearn_b200.ops import cuda_ops
 
     torch.manual_seed(2)
@@ -107,8 +106,8 @@ def test_skinny_gemm_split_k(m, n, k, b_t):
 @pytest.mark.parametrize("n,k", [(8, 64), (136, 72), (1000, 8), (4096, 640), (18952, 128), (37896, 64)])
 @pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, True)])
 def test_skinny_gemm_edges(m, n, k, a_t, b_t):
-    """Row counts at the edges of the tiles, feature and K remainders, one wave of wide CTAs and one more; every
-    split gives the same sums.  fp32 sums of K bf16 products: the error is a few K * 2^-24 of sum |a b|."""
+    """Row counts at the edges of the tiles, feature and K remainders, one wave of wide CTAs and one more, at the split
+    of the kernel's own plan.  fp32 sums of K bf16 products: the error is a few K * 2^-24 of sum |a b|."""
     from axlearn_b200.ops import cuda_ops
 
     torch.manual_seed(3)
@@ -123,6 +122,44 @@ def test_skinny_gemm_edges(m, n, k, a_t, b_t):
     acc = base.clone()
     cuda_ops.gemm(a, b, out=acc, accumulate=True)
     assert ((acc.double() - ref - base.double()).abs() <= bound + 2.0 ** -22 * (ref.abs() + base.abs())).all()
+    cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("m", [1, 13, 16, 50, 100, 128])
+@pytest.mark.parametrize("n,k", [(8, 64), (136, 72), (264, 520), (1000, 648)])
+@pytest.mark.parametrize("x_t", [False, True])
+@pytest.mark.parametrize("w_t", [False, True])
+def test_skinny_gemm_every_split(m, n, k, x_t, w_t):
+    """Each number of K slices up to the blocks of K (slices of unequal length, row counts that it does not divide), all
+    four layouts, both outputs, with and without accumulation; bounds as above, and a bf16 output half a unit more."""
+    from axlearn_b200.ops import cuda_ops
+
+    g = torch.Generator(device="cuda").manual_seed(k)
+    pad = (m + 7) // 8 * 8
+    x = torch.randn(k, pad, device="cuda", generator=g) if x_t else torch.randn(m, k, device="cuda", generator=g)
+    w = torch.randn(n, k, device="cuda", generator=g) if w_t else torch.randn(k, n, device="cuda", generator=g)
+    x, w = x.bfloat16(), w.bfloat16()
+    a, b = (x[:, :m].t() if x_t else x).double(), (w.t() if w_t else w).double()
+    ref, bound = a @ b, 4 * k * 2.0 ** -24 * (a.abs() @ b.abs()) + 1e-30
+    base = torch.randn(m, n, device="cuda", generator=g)
+    status = cuda_ops.status_word()
+    for split in range(1, 9):
+        for dtype in (torch.float32, torch.bfloat16):
+            for accumulate in (False, True):
+                start = base.to(dtype)
+                out = start.clone()
+                rc = cuda_ops.lib().axb_gemm_skinny(
+                    x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, x.shape[1], w.shape[1], n, int(x_t),
+                    int(not w_t), int(dtype == torch.float32), int(accumulate), split, 0, status.data_ptr(),
+                    cuda_ops._stream())  # pylint: disable=protected-access
+                if split > (k + 63) // 64:
+                    assert rc == -15 and torch.equal(out, start)
+                    continue
+                want = ref + start.double() if accumulate else ref
+                limit = bound + 2.0 ** -22 * (ref.abs() + start.double().abs())
+                if dtype == torch.bfloat16:
+                    limit = limit + 2.0 ** -8 * (want.abs() + limit)
+                assert rc == 0 and ((out.double() - want).abs() <= limit).all(), (split, dtype, accumulate)
     cuda_ops.check_status()
 
 
