@@ -163,6 +163,31 @@ def test_skinny_gemm_every_split(m, n, k, x_t, w_t):
     cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("m", [2, 15, 17, 31, 32, 33])
+@pytest.mark.parametrize("blocks", [1, 3, 22, 45])
+def test_skinny_gemm_stages_of_two_blocks(m, blocks):
+    """Slices of odd and even numbers of 64-deep blocks, shorter and longer than the ring of stages, with a K remainder,
+    at the row counts around which partial sums change hands in another way; every split, accumulating into bf16."""
+    from axlearn_b200.ops import cuda_ops
+
+    n, k = 392, 64 * blocks - 8
+    g = torch.Generator(device="cuda").manual_seed(m * 100 + blocks)
+    x = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    w = torch.randn(k, n, device="cuda", generator=g).bfloat16()
+    start = torch.randn(m, n, device="cuda", generator=g).bfloat16()
+    want = x.double() @ w.double() + start.double()
+    limit = 4 * k * 2.0 ** -24 * (x.double().abs() @ w.double().abs()) + 2.0 ** -22 * (want.abs() + start.double().abs())
+    limit = limit + 2.0 ** -8 * (want.abs() + limit)
+    status = cuda_ops.status_word()
+    for split in range(1, min(8, blocks) + 1):
+        out = start.clone()
+        assert cuda_ops.lib().axb_gemm_skinny(
+            x.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, k, n, n, 0, 1, 0, 1, split, 0, status.data_ptr(),
+            cuda_ops._stream()) == 0  # pylint: disable=protected-access
+        assert ((out.double() - want).abs() <= limit).all(), split
+    cuda_ops.check_status()
+
+
 def _close_elementwise(out, ref, atol, rtol):
     """Per-element ``|out - ref| <= atol + rtol * |ref|`` (an error confined to small outputs or one
     tile edge cannot hide behind the largest value)."""
