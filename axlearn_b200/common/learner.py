@@ -226,18 +226,9 @@ def _fused_update(fused: opt_lib.FusedSpec, *, grads, state, params, specs, shad
         gn = g_norm  # Stays on device: the kernel reads the scale from memory.
         grad_scale = torch.clamp(fused.clip_max_norm / (gn + fused.clip_eps), max=1.0)
         add_summary("gradient_scale", grad_scale)
-    count = (adam_state.count + 1).to(torch.int32)
-    t = int(count)
-    lr = fused.learning_rate(t)
-    s = fused.update_schedule(t)
-    add_summary("lr/schedule_step" if fused.decoupled else "schedule_step", count)
-    add_summary("lr/schedule_scale" if fused.decoupled else "schedule_scale", lr)
-    if fused.decoupled:
-        add_summary("update/schedule_step", count)
-        add_summary("update/schedule_scale", s)
-        step_lr, step_wd = s * lr, s * fused.weight_decay
-    else:
-        step_lr, step_wd = lr, lr * fused.weight_decay
+    count, step_scalars, host_summaries = fused_scalars(fused, state)
+    for name, value in host_summaries.items():
+        add_summary(name, value)
     optim.multi_tensor_adamw(
         params=[flat_p[p].value for p, _ in live],
         grads=[g for _, g in live],
@@ -245,16 +236,29 @@ def _fused_update(fused: opt_lib.FusedSpec, *, grads, state, params, specs, shad
         nus=[flat_v[p] for p, _ in live],
         shadows=[shadows.get(p) for p, _ in live],
         wd_scales=[float(scales[p]) for p, _ in live],
-        step=t, lr=step_lr, weight_decay=step_wd, b1=fused.b1, b2=fused.b2, eps=fused.eps,
-        grad_scale=grad_scale,
+        **step_scalars, b1=fused.b1, b2=fused.b2, eps=fused.eps, grad_scale=grad_scale,
     )
-    # Rebuild the state with incremented counters (same structure as the generic chain).
-    new_adam = opt_lib.ScaleByAdamState(count, adam_state.mu, adam_state.nu)
-    return _rebuild_fused_state(state, fused, new_adam, count)
+    return rebuild_fused_state(state, fused, count)
 
 
-def _rebuild_fused_state(state, fused: opt_lib.FusedSpec, new_adam, count):
+def fused_scalars(fused: opt_lib.FusedSpec, state) -> tuple:
+    """What the next step of the closed form takes from the host: ``(its counter, {step, lr, weight_decay}, summaries)``."""
+    count = (fused.locate(state)[0].count + 1).to(torch.int32)
+    t = int(count)
+    lr = fused.learning_rate(t)
+    s = fused.update_schedule(t)
+    if fused.decoupled:
+        summaries = {"lr/schedule_step": count, "lr/schedule_scale": lr,
+                     "update/schedule_step": count, "update/schedule_scale": s}
+        return count, dict(step=t, lr=s * lr, weight_decay=s * fused.weight_decay), summaries
+    summaries = {"schedule_step": count, "schedule_scale": lr}
+    return count, dict(step=t, lr=lr, weight_decay=lr * fused.weight_decay), summaries
+
+
+def rebuild_fused_state(state, fused: opt_lib.FusedSpec, count):
+    """``state`` with its counters at ``count`` (same structure as the generic chain's)."""
     adam_state, counters, chain_index = fused.locate(state)
+    new_adam = opt_lib.ScaleByAdamState(count, adam_state.mu, adam_state.nu)
 
     def rebuild_inner(inner_state):
         inner = list(inner_state)

@@ -54,6 +54,7 @@ from axlearn_b200.common.learner import Learner
 from axlearn_b200.common.metrics import MetricAccumulator
 from axlearn_b200.common.module import Module, OutputCollection, functional
 from axlearn_b200.common.optimizer_base import OptParam
+from axlearn_b200.common.step_graph import StepGraphs
 from axlearn_b200.common.summary_writer import BaseWriter, SummaryWriter
 from axlearn_b200.common.utils import (
     TensorSpec,
@@ -146,6 +147,7 @@ class SpmdTrainer(Module):
         self._trainer_state: Optional[dict] = None
         self._shadows: Optional[Any] = None
         self._has_param_noise = False
+        self._step_graphs = StepGraphs()
         self._device = torch.device(cfg.device) if cfg.device else _default_device()
         self._mesh = mesh or create_mesh(cfg.mesh_shape, cfg.mesh_axis_names)
         self._step_times = collections.deque(maxlen=100)
@@ -242,6 +244,7 @@ class SpmdTrainer(Module):
         """Low-precision copies of float parameters that the forward pass reads (identical to
         the masters when train_dtype is the parameter dtype)."""
         cfg = self._config
+        self._step_graphs.forget()
         types = dict(flatten_items(self.learner.update_types(self._model_param_specs)))
         from axlearn_b200.common.learner import should_update_with_optimizers, UpdateType
 
@@ -457,10 +460,21 @@ class SpmdTrainer(Module):
 
     def _train_step(self, batch: dict) -> dict:
         """Forward, backward and update on one per-process batch (already on device)."""
-        cfg = self._config
         state = self._trainer_state
-        new_key, _noise_key, fwd_key, _learner_key = prng.split(state["prng_key"], 4)
+        new_key, noise_key, fwd_key, _learner_key = prng.split(state["prng_key"], 4)
         batch = _shard_sequence(self.input.dispatch_global_batch(batch), self._mesh)
+        out = self._step_graphs.run(self, batch)
+        if out is None:
+            loss, aux, oc = self._forward_backward(batch, fwd_key, noise_key)
+            fsdp.wait_pending(self._device if self._device.type == "cuda" else None)
+            state["learner"], learner_summaries = self._apply_update(oc)
+            out = {"loss": loss, "aux": aux, "summaries": {"model": oc.summaries, "learner": learner_summaries}}
+        state["prng_key"] = new_key
+        return out
+
+    def _forward_backward(self, batch: dict, fwd_key: Optional[Tensor], noise_key: Optional[Tensor] = None) -> tuple:
+        """``(loss, aux, output collection)`` of one batch; gradients land on the shadows."""
+        cfg = self._config
         self._zero_grads()
         steps = max(1, cfg.grad_accumulation_steps)
         micro_batches = _split_batch(batch, steps)
@@ -478,7 +492,7 @@ class SpmdTrainer(Module):
             # still land on the clean shadows (reference: axlearn/common/trainer.py:1305-1307).
             step_params = self._shadows
             if self._has_param_noise:
-                step_params = self.model.apply_parameter_noise_recursively(_noise_key, self._shadows)
+                step_params = self.model.apply_parameter_noise_recursively(noise_key, self._shadows)
             (micro_loss, aux), oc = functional(
                 self.model, key, step_params, [micro], is_training=True, method="forward")
             # Micro-batch gradients are averaged (reference: gradient_accumulation.py:96-351).
@@ -490,7 +504,14 @@ class SpmdTrainer(Module):
         if acc is not None:
             oc.summaries.clear()
             oc.summaries.update(acc.summaries())
-        fsdp.wait_pending(self._device if self._device.type == "cuda" else None)
+        # Each rank's loss is its share of the global mean (normalised by the global number of
+        # live targets); the reported loss is the sum of the shares over the batch axes.
+        return coll.all_reduce_scalar(loss.detach().float(), ("data", "expert", "fsdp", "seq")), aux, oc
+
+    def _apply_update(self, oc: OutputCollection) -> tuple:
+        """Synchronises the shadows' gradients and updates parameters, moments and shadows in place; returns the new
+        learner state and the learner's summaries."""
+        state = self._trainer_state
         if self._mesh is not None and self._mesh.shape.get("pipeline", 1) > 1:
             # A stage that does not touch a replicated parameter still takes part in its reduction.
             for _, sh in flatten_items(self._shadows):
@@ -498,24 +519,20 @@ class SpmdTrainer(Module):
                     sh.grad = torch.zeros_like(sh)
         grads = tree_map(lambda s: s.grad if s.requires_grad else None, self._shadows)
         grad_sync.sync_grads(grads, specs=self._model_param_specs, mesh=self._mesh)
-        summaries = {"model": oc.summaries}
         learner_oc = OutputCollection({}, {}, {})
         from axlearn_b200.common.module import InvocationContext, set_current_context
 
         lctx = InvocationContext(name="learner", parent=None, module=self.learner, state=None,
                                  is_training=True, prng_key=None, output_collection=learner_oc)
         with set_current_context(lctx, require_parent=False):
-            state["learner"] = self.learner.update(
+            learner_state = self.learner.update(
                 model_params=state["model"], gradients=grads, state=state["learner"],
                 param_specs=self._model_param_specs, state_updates=oc.state_updates, shadows=self._shadows)
-        summaries["learner"] = learner_oc.summaries
         if self._device.type == "cuda":
+            from axlearn_b200.parallel import fsdp_fused
+
             fsdp_fused.invalidate_all()  # the shards changed: gather buffers are stale
-        state["prng_key"] = new_key
-        # Each rank's loss is its share of the global mean (normalised by the global number of
-        # live targets); the reported loss is the sum of the shares over the batch axes.
-        global_loss = coll.all_reduce_scalar(loss.detach().float(), ("data", "expert", "fsdp", "seq"))
-        return {"loss": global_loss, "aux": aux, "summaries": summaries}
+        return learner_state, learner_oc.summaries
 
     def _zero_grads(self) -> None:
         def visit(node, stacked):

@@ -786,12 +786,21 @@ ce_fwd_bwd_bf16_vec_kernel(bf16* __restrict__ logits, const int64_t* __restrict_
 // p (fp32 master), m, v fp32; g bf16 or fp32; optional bf16 shadow written with the new p.
 //   g' = g * grad_scale[0];  m = b1 m + (1-b1) g';  v = b2 v + (1-b2) g'^2
 //   p -= lr * (m / bc1) / (sqrt(v / bc2) + eps) + wd * p
+// `scalars` (null: the arguments count): lr, bc1, bc2 in device memory and the decay at `wd_at`, for launches in a graph that
+// is replayed with other ones each time.
 template <typename G>
 __global__ void adamw_kernel(float* __restrict__ p, const G* __restrict__ g, float* __restrict__ m,
                              float* __restrict__ v, bf16* __restrict__ shadow,
                              const float* __restrict__ grad_scale, int64_t n, float lr, float wd,
-                             float b1, float b2, float eps, float bc1, float bc2) {
+                             float b1, float b2, float eps, float bc1, float bc2, const float* __restrict__ scalars,
+                             int wd_at) {
   const float gs = grad_scale ? *grad_scale : 1.f;
+  if (scalars != nullptr) {
+    lr = scalars[0];
+    bc1 = scalars[1];
+    bc2 = scalars[2];
+    wd = scalars[wd_at];
+  }
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x * 4;
   for (int64_t i = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) * 4; i < n;
        i += stride) {
@@ -842,6 +851,15 @@ __global__ void adamw_kernel(float* __restrict__ p, const G* __restrict__ g, flo
       }
     }
   }
+}
+
+struct StoredFloats {
+  static constexpr int kMax = 32;
+  float v[kMax];
+};
+
+__global__ void store_floats_kernel(float* __restrict__ dst, const StoredFloats f, int n) {
+  if (static_cast<int>(threadIdx.x) < n) dst[threadIdx.x] = f.v[threadIdx.x];
 }
 
 // ------------------------------------------------------------------------------ sum of squares
@@ -1115,20 +1133,44 @@ extern "C" int axb_ce_fwd_bwd(void* logits, int is_fp32, const int64_t* targets,
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
-extern "C" int axb_adamw(float* p, const void* g, int g_is_bf16, float* m, float* v, void* shadow,
-                         const float* grad_scale, int64_t n, float lr, float wd, float b1, float b2,
-                         float eps, float bc1, float bc2, cudaStream_t stream) {
+static int launch_adamw(float* p, const void* g, int g_is_bf16, float* m, float* v, void* shadow,
+                        const float* grad_scale, int64_t n, float lr, float wd, float b1, float b2, float eps, float bc1,
+                        float bc2, const float* scalars, int wd_at, cudaStream_t stream) {
   // 134 M parameters, blocks per SM: 4 638 us, 8 640, 16 613 (574 at the copy rate); two vectors a thread or loads past
   // the caches gain nothing on top, 32 contiguous bytes a thread take twice as long.
   const int grid = grid_for((n + 3) / 4, 256, 148 * 16);
   if (g_is_bf16)
     adamw_kernel<bf16><<<grid, 256, 0, stream>>>(p, static_cast<const bf16*>(g), m, v,
                                                  static_cast<bf16*>(shadow), grad_scale, n, lr, wd,
-                                                 b1, b2, eps, bc1, bc2);
+                                                 b1, b2, eps, bc1, bc2, scalars, wd_at);
   else
     adamw_kernel<float><<<grid, 256, 0, stream>>>(p, static_cast<const float*>(g), m, v,
                                                   static_cast<bf16*>(shadow), grad_scale, n, lr, wd,
-                                                  b1, b2, eps, bc1, bc2);
+                                                  b1, b2, eps, bc1, bc2, scalars, wd_at);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+extern "C" int axb_adamw(float* p, const void* g, int g_is_bf16, float* m, float* v, void* shadow,
+                         const float* grad_scale, int64_t n, float lr, float wd, float b1, float b2,
+                         float eps, float bc1, float bc2, cudaStream_t stream) {
+  return launch_adamw(p, g, g_is_bf16, m, v, shadow, grad_scale, n, lr, wd, b1, b2, eps, bc1, bc2, nullptr, 0, stream);
+}
+
+// The same with lr, bc1, bc2 and the decay `scalars[wd_at]` in device memory, where axb_store_floats puts them.
+extern "C" int axb_adamw_scalars(float* p, const void* g, int g_is_bf16, float* m, float* v, void* shadow,
+                                 const float* grad_scale, int64_t n, const float* scalars, int wd_at, float b1, float b2,
+                                 float eps, cudaStream_t stream) {
+  return launch_adamw(p, g, g_is_bf16, m, v, shadow, grad_scale, n, 0.f, 0.f, b1, b2, eps, 1.f, 1.f, scalars, wd_at,
+                      stream);
+}
+
+// dst[0 .. n) = values (host memory, free again when the call returns: they travel as the kernel's arguments); n <= 32.
+extern "C" int axb_store_floats(float* dst, const float* values, int n, cudaStream_t stream) {
+  StoredFloats f;
+  if (n < 0 || n > StoredFloats::kMax) return -10;
+  for (int i = 0; i < n; ++i) f.v[i] = values[i];
+  for (int i = n; i < StoredFloats::kMax; ++i) f.v[i] = 0.f;
+  store_floats_kernel<<<1, StoredFloats::kMax, 0, stream>>>(dst, f, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -102,6 +102,9 @@ class _Sigs:
                       c_float, c_int64, c_int, c_int, c_void_p]
     axb_adamw = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_float,
                  c_float, c_float, c_float, c_float, c_float, c_float, c_void_p]
+    axb_adamw_scalars = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int,
+                         c_float, c_float, c_float, c_void_p]
+    axb_store_floats = [c_void_p, c_void_p, c_int, c_void_p]
     axb_embedding_bwd = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
     axb_embedding_bwd_bytes = [c_int, c_int, c_int]
     axb_scale_bf16 = [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]
@@ -716,7 +719,42 @@ def scaled(x: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
 # Optimizer.
 # ------------------------------------------------------------------------------------------
 
-_scale_one: dict[int, torch.Tensor] = {}
+_adamw = threading.local()
+
+
+class AdamwScalars:
+    """The scalars of AdamW steps in device memory: learning rate, bias corrections and one decay per weight of it."""
+
+    _FLOATS, _FIRST_DECAY = 32, 3
+
+    def __init__(self, device):
+        self.values = torch.zeros(self._FLOATS, dtype=torch.float32, device=device)
+        self._decays: list = []
+
+    def place(self, decay_scale: float) -> int:
+        """Where the decay of parameters with this weight of it is found."""
+        if decay_scale not in self._decays:
+            if self._FIRST_DECAY + len(self._decays) == self._FLOATS:
+                raise RuntimeError("too many different weight decays")
+            self._decays.append(decay_scale)
+        return self._FIRST_DECAY + self._decays.index(decay_scale)
+
+    def store(self, *, step: int, lr: float, weight_decay: float, b1: float, b2: float) -> None:
+        """In stream order; the numbers travel as a kernel's arguments, so there is no host buffer to guard."""
+        values = [lr, 1.0 - b1**step, 1.0 - b2**step, *(weight_decay * s for s in self._decays)]
+        _check(lib().axb_store_floats(self.values.data_ptr(), (c_float * len(values))(*values), len(values), _stream()),
+               "axb_store_floats")
+
+
+@contextlib.contextmanager
+def adamw_scalars(scalars: AdamwScalars):
+    """``multi_tensor_adamw`` of the calling thread reads its scalars from ``scalars`` inside (a step being captured)."""
+    before = getattr(_adamw, "scalars", None)
+    _adamw.scalars = scalars
+    try:
+        yield
+    finally:
+        _adamw.scalars = before
 
 
 def multi_tensor_adamw(params, grads, mus, nus, shadows, wd_scales, *, step: int, lr: float,
@@ -730,6 +768,7 @@ def multi_tensor_adamw(params, grads, mus, nus, shadows, wd_scales, *, step: int
     bc1, bc2 = 1.0 - b1**step, 1.0 - b2**step
     h = lib()
     stream = _stream()
+    stored = getattr(_adamw, "scalars", None)
     for p, g, m, v, sh, ws in zip(params, grads, mus, nus, shadows, wd_scales):
         assert p.is_contiguous() and m.is_contiguous() and v.is_contiguous()
         g = g.contiguous()
@@ -739,6 +778,11 @@ def multi_tensor_adamw(params, grads, mus, nus, shadows, wd_scales, *, step: int
         if sh is not None and sh is not p:
             assert sh.dtype == torch.bfloat16 and sh.is_contiguous()
             shadow_ptr = sh.data_ptr()
+        if stored is not None:
+            _check(h.axb_adamw_scalars(p.data_ptr(), g.data_ptr(), 1 if g.dtype == torch.bfloat16 else 0, m.data_ptr(),
+                                       v.data_ptr(), shadow_ptr, gs.data_ptr(), p.numel(), stored.values.data_ptr(),
+                                       stored.place(ws), b1, b2, eps, stream), "axb_adamw_scalars")
+            continue
         _check(h.axb_adamw(p.data_ptr(), g.data_ptr(), 1 if g.dtype == torch.bfloat16 else 0, m.data_ptr(),
                            v.data_ptr(), shadow_ptr, gs.data_ptr(), p.numel(), lr, weight_decay * ws, b1, b2,
                            eps, bc1, bc2, stream), "axb_adamw")

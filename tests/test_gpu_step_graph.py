@@ -1,0 +1,146 @@
+"""Captured training steps against steps run one launch after the other."""
+
+import pytest
+import torch
+
+from axlearn_b200.common import prng
+from axlearn_b200.common.base_layer import RematSpec, nothing_saveable
+from axlearn_b200.common.utils import flatten_items
+from axlearn_b200.experiments.text.gpt import fuji
+from axlearn_b200.experiments.text.gpt.common import (
+    adamw_decoupled_learner_config,
+    get_trainer_config_fn,
+    mesh_shape_from_axes,
+)
+
+pytestmark = pytest.mark.gpu
+_VOCAB = 512
+
+
+def _trainer(tmp_path, *, kv=None, remat=False, seed=0):
+    model = fuji.model_config(num_layers=2, hidden_dim=256, num_heads=4, num_kv_heads=kv, vocab_size=_VOCAB, rope_theta=1e4,
+                              shared_lm_head=True, ffn_dim=512, scan_chunk=1024, flash_attention=True)
+    if remat:
+        model.decoder.transformer.layer.remat_spec = RematSpec(prevent_cse=False, policy=nothing_saveable)
+    learner = adamw_decoupled_learner_config(peak_lr=1e-2, max_step=1000, weight_decay=0.1, lr_warmup_steps=4)
+    cfg = get_trainer_config_fn(
+        model_cfg=model, learner_cfg=learner, max_step=1000, train_batch_size=2, max_sequence_length=128,
+        vocab_size=_VOCAB, mesh_shape=mesh_shape_from_axes(), train_dtype=torch.bfloat16)()
+    cfg.dir, cfg.device = str(tmp_path), "cuda:0"
+    trainer = cfg.instantiate(parent=None)
+    trainer.init(prng.PRNGKey(seed))
+    return trainer
+
+
+def _batch(seed, rows=2, length=128):
+    tokens = torch.randint(0, _VOCAB, (rows, length + 1), dtype=torch.int32, generator=torch.Generator().manual_seed(seed))
+    return {"input_ids": tokens[:, :-1].contiguous(), "target_labels": tokens[:, 1:].contiguous(),
+            "target_num_bytes": torch.ones(rows, dtype=torch.int32)}
+
+
+def _captured(trainer) -> bool:
+    return trainer._step_graphs._captured is not None  # pylint: disable=protected-access
+
+
+def _eager(trainer):
+    trainer._step_graphs._capturable = False  # pylint: disable=protected-access
+    return trainer
+
+
+def _same(a, b, rel):
+    """Both trainers' parameters, moments and shadows: off by the order of sums in the gradients at most."""
+    for pick in (lambda t: t.trainer_state["model"], lambda t: t.trainer_state["learner"]["optimizer"][1][0].mu,
+                 lambda t: t.trainer_state["learner"]["optimizer"][1][0].nu, lambda t: t._shadows):
+        for (path, x), (_, y) in zip(flatten_items(pick(a)), flatten_items(pick(b))):
+            x, y = x.detach().double(), y.detach().double()
+            assert (x - y).norm() <= rel * y.norm() + 1e-12, path
+
+
+@pytest.mark.parametrize("kv,remat", [(None, True), (2, False)])
+def test_captured_steps_are_the_steps(tmp_path, kv, remat):
+    from axlearn_b200.ops import cuda_ops
+
+    a, b = _trainer(tmp_path, kv=kv, remat=remat), _eager(_trainer(tmp_path, kv=kv, remat=remat))
+    kept = []
+    for step in range(6):
+        before = cuda_ops.launch_count
+        x = a.train_step(_batch(step))
+        middle = cuda_ops.launch_count
+        y = b.train_step(_batch(step))
+        launches = cuda_ops.launch_count - middle
+        assert _captured(a) == (step >= 1) and not _captured(b)
+        # As many kernels, plus the one that stores the scalars in a replay.
+        assert middle - before == launches + (1 if step >= 1 else 0)
+        kept.append((x, y))
+    for x, y in kept:  # outputs of earlier steps are not those of later ones
+        torch.testing.assert_close(x["loss"], y["loss"], rtol=2e-3, atol=0)
+        assert list(x["summaries"]) == list(y["summaries"])
+        for part in x["summaries"]:
+            assert list(x["summaries"][part]) == list(y["summaries"][part])
+        for name in ("lr/schedule_scale", "lr/schedule_step", "update/schedule_scale", "update/schedule_step"):
+            assert x["summaries"]["learner"][name] == y["summaries"]["learner"][name]
+        torch.testing.assert_close(x["summaries"]["learner"]["gradient_norm"],
+                                   y["summaries"]["learner"]["gradient_norm"], rtol=2e-2, atol=0)
+    assert len({float(x["loss"]) for x, _ in kept}) == len(kept)
+    _same(a, b, 2e-2)
+    for (_, x), (_, y) in zip(flatten_items(a.trainer_state["learner"]), flatten_items(b.trainer_state["learner"])):
+        if isinstance(x, torch.Tensor) and x.dim() == 0:
+            assert torch.equal(x, y)
+    assert torch.equal(a.trainer_state["prng_key"], b.trainer_state["prng_key"])
+    cuda_ops.check_status()
+
+
+def test_other_shapes_hooks_and_states(tmp_path):
+    a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
+
+    def both(batch):
+        x, y = a.train_step(batch), b.train_step(batch)
+        torch.testing.assert_close(x["loss"], y["loss"], rtol=2e-3, atol=0)
+
+    for step in range(3):
+        both(_batch(step))
+    assert _captured(a)
+    graph = a._step_graphs._captured
+    for step, shape in enumerate([(1, 128), (2, 100), (2, 128), (2, 128)]):  # one of each: not captured
+        both(_batch(10 + step, *shape))
+        assert a._step_graphs._captured is graph
+    # A hook on a parameter runs, and the step with it.
+    seen = []
+    leaf = next(t for _, t in flatten_items(a._shadows) if t.requires_grad and t.dim() == 1)
+    handle = leaf.register_hook(lambda g: seen.append(g.shape))
+    both(_batch(20))
+    assert seen == [leaf.shape]
+    handle.remove()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(0), t)[1], lambda t: t):
+        both(_batch(21))
+    assert len(seen) > 2
+    both(_batch(22))
+    _same(a, b, 3e-2)
+    # New parameters in the trainer: not those of the graph.
+    for t in (a, b):
+        t.init(prng.PRNGKey(7))
+    assert not _captured(a)
+    for step in range(3):
+        both(_batch(30 + step))
+    assert _captured(a) and a._step_graphs._captured is not graph
+    _same(a, b, 2e-2)
+
+
+def test_not_captured(tmp_path, monkeypatch):
+    """Dropout, a subclass of a layer, too much memory."""
+    from axlearn_b200.common import layers, step_graph
+
+    a = _trainer(tmp_path)
+    assert step_graph.capturable(a)
+    a.model.decoder.output_dropout._config.rate = 0.1  # pylint: disable=protected-access
+    assert not step_graph.capturable(a)
+    b = _trainer(tmp_path)
+    b.model.decoder.output_norm.__class__ = type("Norm", (layers.RMSNorm,), {})
+    assert not step_graph.capturable(b)
+    monkeypatch.setattr(step_graph, "_MEMORY_SHARE", 1 << 40)
+    c = _trainer(tmp_path)
+    d = _eager(_trainer(tmp_path))
+    for step in range(3):
+        torch.testing.assert_close(c.train_step(_batch(step))["loss"], d.train_step(_batch(step))["loss"], rtol=2e-3, atol=0)
+        assert not _captured(c)
+    _same(c, d, 2e-2)
