@@ -188,6 +188,31 @@ def test_skinny_gemm_stages_of_two_blocks(m, blocks):
     cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("m", [129, 333, 666])
+@pytest.mark.parametrize("n", [8, 72, 128, 264, 520])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_accumulate_reads_c_by_vectors(m, n, dtype):
+    """Whole and cut 32-column pieces of C, rows beyond the last tile, a C whose rows lie apart; the rest of C stays."""
+    from axlearn_b200.ops import cuda_ops
+
+    k = 192
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    b = torch.randn(k, n, device="cuda", generator=g).bfloat16()
+    whole = torch.randn(m + 3, n + 16, device="cuda", generator=g).to(dtype)
+    before = whole.clone()
+    out = whole[:m, 8:n + 8]
+    cuda_ops.gemm(a, b, out=out, accumulate=True)
+    want = a.double() @ b.double() + before[:m, 8:n + 8].double()
+    limit = 4 * k * 2.0 ** -24 * (a.double().abs() @ b.double().abs()) + 2.0 ** -22 * want.abs()
+    if dtype == torch.bfloat16:
+        limit = limit + 2.0 ** -8 * (want.abs() + limit)
+    assert ((out.double() - want).abs() <= limit).all()
+    out.copy_(before[:m, 8:n + 8])
+    assert torch.equal(whole, before)
+    cuda_ops.check_status()
+
+
 def _close_elementwise(out, ref, atol, rtol):
     """Per-element ``|out - ref| <= atol + rtol * |ref|`` (an error confined to small outputs or one
     tile edge cannot hide behind the largest value)."""
