@@ -17,13 +17,14 @@ from typing import NamedTuple, Optional, Sequence
 import torch
 
 from axlearn_b200 import ops
+from axlearn_b200.common import sequence_mixer
 from axlearn_b200.common.attention import BaseStackedTransformerLayer, BaseTransformerLayer
 from axlearn_b200.common.base_layer import BaseLayer, ParameterSpec
 from axlearn_b200.common.config import REQUIRED, InstantiableConfig, Required, config_class
 from axlearn_b200.common.layers import Embedding
 from axlearn_b200.common.module import nowrap
 from axlearn_b200.common.sequence_mixer import PaddedLinear, vector_spec
-from axlearn_b200.ops import cuda_ops, hyper_ops, step_ops
+from axlearn_b200.ops import cuda_ops, hyper_ops, packed_ops, step_ops
 from axlearn_b200.ops.hyper_ops import padded
 
 Tensor = torch.Tensor
@@ -147,11 +148,11 @@ class HyperTransformerLayer(BaseTransformerLayer):
     def connections(self) -> dict:
         return {name: getattr(self, f"{name}_connection")() for name in self._names}
 
-    def run_sublayer(self, name: str, h: Tensor, *, start=None, live=None, state=None):
-        """``(branch, new state)`` of one sublayer on its normed input."""
+    def run_sublayer(self, name: str, h: Tensor, *, start=None, live=None, state=None, **packed):
+        """``(branch, new state)`` of one sublayer on its normed input; ``packed``: prompts without padding."""
         if name == "feed_forward":
             return self.feed_forward(h), state
-        branch, mixed = self.mixer(h, start=start, live=live, state=None if state is None else state["mixer"])
+        branch, mixed = self.mixer(h, start=start, live=live, state=None if state is None else state["mixer"], **packed)
         return branch, (None if state is None else {"mixer": mixed})
 
 
@@ -200,7 +201,7 @@ class HyperStackedTransformerLayer(BaseStackedTransformerLayer):
         """Index of the layer of every run, in order."""
         return list(self._order)
 
-    def _run(self, data: Tensor, *, start=None, live=None, states: Optional[dict] = None):
+    def _run(self, data: Tensor, *, start=None, live=None, states: Optional[dict] = None, **packed):
         cfg = self._config
         parts = [layer.connections() for layer in self._layers]
         step = dict(num_streams=cfg.num_streams, dtype=data.dtype)
@@ -213,7 +214,7 @@ class HyperStackedTransformerLayer(BaseStackedTransformerLayer):
                 streams, h = hyper_ops.hyper_step(
                     streams, branch, write=write, read=c.read, norm_scale=c.norm_scale, eps=c.norm_eps,
                     norm_offset=c.norm_offset, **step)
-                branch, state = layer.run_sublayer(name, h, start=start, live=live, state=state)
+                branch, state = layer.run_sublayer(name, h, start=start, live=live, state=state, **packed)
                 write = c.write
             new_states[f"run{run}"] = state
         _, h = hyper_ops.hyper_step(
@@ -246,9 +247,28 @@ class HyperStackedTransformerLayer(BaseStackedTransformerLayer):
         if time_step is None:
             return states, None
         live = time_step.to(torch.int32)
-        new, out = self._run(data, live=live, states=states)
+        packed = self._packing(data, live)
+        if packed is None:
+            new, out = self._run(data, live=live, states=states)
+        else:
+            new, out = self._run(packed.pack(data), live=live, states=states, packed=packed)
+            out = self.Output(data=packed.unpack(out.data))
         new["time_step"] = live.clone()
         return new, out
+
+    @nowrap
+    def _packing(self, data: Tensor, live: Tensor):
+        """How the prompts lie without their padding, None to run them padded."""
+        if not (data.is_cuda and data.dtype == torch.bfloat16 and live.is_cuda and live.dim() == 1) \
+                or torch.is_grad_enabled() or torch.cuda.is_current_stream_capturing():
+            return None
+        from axlearn_b200.common.routed_experts import RoutedFeedForward
+
+        rowwise = (GatedFeedForward, RoutedFeedForward, type(None))
+        if not all(type(layer) is HyperTransformerLayer and sequence_mixer.takes_packed(layer.children["mixer"])
+                   and type(layer.children.get("feed_forward")) in rowwise for layer in self._layers):
+            return None
+        return packed_ops.pack_prompts(live, data.shape[1])
 
     def extend_step(self, cached_states, data, *, live_step_len=None, page_pool=None, **kwargs):
         """``data [B, steps, D]`` after the tokens seen so far; ``live_step_len [B]``: valid new tokens per

@@ -93,12 +93,13 @@ class BaseSequenceMixer(BaseLayer):
     def init_states(self, *, batch_size: int, max_len: int, dtype: torch.dtype, device=None) -> dict:
         raise NotImplementedError(type(self))
 
-    def mix(self, proj: Tensor, columns: dict, *, start=None, live=None, state=None) -> tuple[Tensor, Any]:
-        """``(output projection of the mixed heads, new state)``."""
+    def mix(self, proj: Tensor, columns: dict, *, start=None, live=None, state=None, packed=None) -> tuple[Tensor, Any]:
+        """``(output projection of the mixed heads, new state)``; ``packed``: the rows are prompts without padding
+        (``ops/packed_ops.py``)."""
         raise NotImplementedError(type(self))
 
-    def forward(self, x: Tensor, *, start=None, live=None, state=None) -> tuple[Any, Any]:
-        return self.mix(self.i_proj(x), self._columns, start=start, live=live, state=state)
+    def forward(self, x: Tensor, *, start=None, live=None, state=None, **packed) -> tuple[Any, Any]:
+        return self.mix(self.i_proj(x), self._columns, start=start, live=live, state=state, **packed)
 
 
 def layout_sections(sections: Sequence[tuple]) -> tuple[dict, int]:
@@ -151,9 +152,9 @@ class GatedWindowAttention(BaseSequenceMixer):
         shape = RingKVCache.Shape(batch_size, max_len, s.kv_heads, s.dim, s.vdim)
         return self._children["kv_cache"].init_states(shape, dtype=dtype, device=device)
 
-    def mix(self, proj, columns, *, start=None, live=None, state=None):
+    def mix(self, proj, columns, *, start=None, live=None, state=None, packed=None):
         out, state = window_ops.window_attention(proj, self._spec, window_ops.WindowColumns(**columns),
-                                                 start=start, live=live, cache=state)
+                                                 start=start, live=live, cache=state, packed=packed)
         return self.o_proj(out), state
 
 
@@ -199,11 +200,11 @@ class GatedLinearAttention(BaseSequenceMixer):
         s = self._spec
         return torch.zeros((batch_size, s.heads, s.dim, s.vdim), dtype=torch.float32, device=device)
 
-    def mix(self, proj, columns, *, start=None, live=None, state=None):
+    def mix(self, proj, columns, *, start=None, live=None, state=None, packed=None):
         p = self.parameters
         out, state = gla_ops.gated_linear_attention(
             proj, p["gate_weight"].to(proj.dtype), p["gate_bias"], p["norm_scale"], self._spec,
-            gla_ops.GlaColumns(**columns), start=start, live=live, state=state)
+            gla_ops.GlaColumns(**columns), start=start, live=live, state=state, packed=packed)
         return self.o_proj(out), state
 
 
@@ -254,11 +255,15 @@ class LatentAttention(BaseSequenceMixer):
     def init_states(self, *, batch_size, max_len, dtype, device=None):
         return {"latent": torch.zeros((batch_size, max_len, self._spec.row_width), dtype=dtype, device=device)}
 
-    def mix(self, proj, columns, *, start=None, live=None, state=None):
+    def mix(self, proj, columns, *, start=None, live=None, state=None, packed=None):
         p = self.parameters
+        if packed is not None:  # expands keys and values of the cache's padded rows
+            proj = packed.unpack(proj)
         out, state = latent_ops.latent_attention(
             proj, p["latent_norm_scale"], p["key_weight"], p["value_weight"], self._spec,
             latent_ops.LatentColumns(**columns), start=start, live=live, cache=state)
+        if packed is not None:
+            out = packed.pack(out)
         return self.o_proj(out), state
 
 
@@ -310,12 +315,12 @@ class StateSpaceMixer(BaseSequenceMixer):
         return {"ssm": torch.zeros((batch_size, s.heads, s.state, s.vdim), dtype=torch.float32, device=device),
                 "conv": torch.zeros((batch_size, s.taps, s.channels), dtype=dtype, device=device)}
 
-    def mix(self, proj, columns, *, start=None, live=None, state=None):
+    def mix(self, proj, columns, *, start=None, live=None, state=None, packed=None):
         p = self.parameters
         weights = ssd_ops.SsdWeights(conv_w=p["conv_weight"], conv_b=p["conv_bias"], dt_bias=p["dt_bias"],
                                      a_log=p["a_log"], d=p["d"], norm_w=p["norm_scale"])
         out, state = ssd_ops.ssd_mix(proj, weights, self._spec, ssd_ops.SsdColumns(**columns), start=start, live=live,
-                                     state=state)
+                                     state=state, packed=packed)
         return self.o_proj(out), state
 
 
@@ -357,13 +362,14 @@ class ParallelMixer(BaseLayer):
     def init_states(self, **kwargs) -> dict:
         return {side: self._children[side].init_states(**kwargs) for side in ("left", "right")}
 
-    def forward(self, x: Tensor, *, start=None, live=None, state=None):
+    def forward(self, x: Tensor, *, start=None, live=None, state=None, **packed):
         proj = self.i_proj(x)
         outs, states = {}, {}
 
         def mix(side):
             outs[side], states[side] = getattr(self, side).mix(
-                proj, self._columns[side], start=start, live=live, state=None if state is None else state[side])
+                proj, self._columns[side], start=start, live=live, state=None if state is None else state[side],
+                **packed)
 
         if x.is_cuda and x.shape[1] == 1 and not torch.is_grad_enabled():
             # A decoding step's kernels are small: the two mixers run next to each other.  (The side stream's
@@ -381,3 +387,12 @@ class ParallelMixer(BaseLayer):
         pair = hyper_ops.NormedPair(outs["left"], outs["right"], p["left_norm_scale"], p["right_norm_scale"],
                                     self._config.norm_eps)
         return pair, states
+
+
+# Mixers whose sequences may lie one after the other without padding (exact types: a subclass may mix in another way).
+PACKED_MIXERS = frozenset({GatedWindowAttention, GatedLinearAttention, LatentAttention, StateSpaceMixer})
+
+
+def takes_packed(mixer) -> bool:
+    sides = [mixer.children["left"], mixer.children["right"]] if type(mixer) is ParallelMixer else [mixer]
+    return all(type(side) in PACKED_MIXERS for side in sides)

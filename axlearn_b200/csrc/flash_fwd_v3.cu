@@ -59,6 +59,8 @@ struct FlashFwd3Params {
   int64_t gate_ld, out_ld;
   int vdim, every, bias;
   int rot_dim;         // kLatent: size of the rotated part (H is the unrotated size)
+  const int* first;    // [B] packed prompts: the row at which a sequence's live tokens begin (q, k, v, gate and out), null: b T
+  const int* live;     // [B] their numbers
   float coef;          // query temperature 1 + coef * ln(floor((pos + 1) / every) + 1)
 };
 
@@ -168,6 +170,11 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int kv_head = head / (p.N / p.Nkv);
   const int t0 = pair * 256;
   const int n_qt = (p.T + 127) / 128;
+  // Packed prompts are one sequence to the tensor maps.  What lies behind a sequence's last key is the next one's, and the
+  // causal mask hides it.
+  const bool packed = kGated && p.first != nullptr;
+  const int seq_len = packed ? min(p.live[batch], p.T) : p.T;
+  const int seq_row = packed ? p.first[batch] : 0, map_batch = packed ? 0 : batch;
 
   // Key tiles [lo, hi) each query tile needs.
   int lo[2], hi[2];
@@ -175,9 +182,9 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   for (int x = 0; x < 2; ++x) {
     const int tx = t0 + x * 128;
     int l = 0, h = 0;
-    if (tx < p.T) {
-      int kv_len = p.S;
-      if (p.causal) kv_len = min(p.S, tx + 128 + p.q_offset);
+    if (tx < seq_len) {
+      int kv_len = packed ? seq_len : p.S;
+      if (p.causal) kv_len = min(kv_len, tx + 128 + p.q_offset);
       h = kv_len > 0 ? (kv_len + 127) / 128 : 0;
       if (kGeneral) {
         if (p.window >= 0) l = max(0, tx + p.q_offset - p.window) / 128;
@@ -236,7 +243,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
         for (int j = 0; j < H / 64; ++j)
           tma_load_4d(smem + L::kQ + x * L::kQTile + j * L::kSub, &tmap_q, q_full, j * 64, head,
-                      t0 + x * 128, batch);
+                      seq_row + t0 + x * 128, map_batch);
         if (kLatent)
           tma_load_4d(smem + L::kQ + x * L::kQTile + H / 64 * L::kSub, &tmap_qr, q_full, 0, head, t0 + x * 128, batch);
       }
@@ -256,7 +263,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
         for (int j = 0; j < H / 64; ++j)
           tma_load_4d(smem + L::kK + (st % KS) * L::kQTile + j * L::kSub, &tmap_k, &k_full[st], j * 64, kv_head,
-                      it * 128, batch);
+                      seq_row + it * 128, map_batch);
         if (kLatent)
           tma_load_4d(smem + L::kK + (st % KS) * L::kQTile + H / 64 * L::kSub, &tmap_kr, &k_full[st], 0, 0, it * 128, batch);
         if (g >= 2) {
@@ -267,7 +274,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
         for (int j = 0; j < H / 64; ++j)
           tma_load_4d(smem + L::kV + st * L::kTile + j * L::kSub, &tmap_v, &v_full[st], j * 64, kv_head,
-                      it * 128, batch);
+                      seq_row + it * 128, map_batch);
       }
     }
   } else if (warp == 1) {
@@ -564,7 +571,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
     if (kStrided && ok && nt > 0) {
       const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
-      const int64_t tok = static_cast<int64_t>(batch) * p.T + row;
+      const int64_t tok = (packed ? static_cast<int64_t>(seq_row) : static_cast<int64_t>(batch) * p.T) + row;
       __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + tok * p.out_ld + head * p.vdim;
       const __nv_bfloat16* grow = reinterpret_cast<const __nv_bfloat16*>(p.gate) + tok * p.gate_ld + head * p.vdim;
 #pragma unroll 1
@@ -575,7 +582,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         tmem_ld_wait();
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-          if (row < p.T && col + 8 * g < p.vdim) {  // vdim is a multiple of 8
+          if (row < seq_len && col + 8 * g < p.vdim) {  // vdim is a multiple of 8
             uint4 gate = make_uint4(0, 0, 0, 0);
             if (p.gate != nullptr) gate = *reinterpret_cast<const uint4*>(grow + col + 8 * g);
             const uint32_t gw[4] = {gate.x, gate.y, gate.z, gate.w};
@@ -720,12 +727,14 @@ static int run_flash_fwd3(const CUtensorMap& tq, const CUtensorMap& tk, const CU
 }
 
 template <int H, bool kGeneral, bool kGated = false>
-static int launch_flash_fwd3(const void* q, const void* k, const void* v, FlashFwd3Params p, cudaStream_t stream) {
+static int launch_flash_fwd3(const void* q, const void* k, const void* v, FlashFwd3Params p, cudaStream_t stream,
+                             int packed_rows = 0) {
   CUtensorMap tq, tk, tv;
   if (kGated) {
-    if (make_packed_map(&tq, q, p.B, p.T, p.N, p.H, p.gate_ld)) return -2;
-    if (make_packed_map(&tk, k, p.B, p.S, p.Nkv, p.H, p.gate_ld)) return -2;
-    if (make_packed_map(&tv, v, p.B, p.S, p.Nkv, p.vdim, p.gate_ld)) return -2;
+    const int seqs = p.first != nullptr ? 1 : p.B, length = p.first != nullptr ? packed_rows : p.T;
+    if (make_packed_map(&tq, q, seqs, length, p.N, p.H, p.gate_ld)) return -2;
+    if (make_packed_map(&tk, k, seqs, length, p.Nkv, p.H, p.gate_ld)) return -2;
+    if (make_packed_map(&tv, v, seqs, length, p.Nkv, p.vdim, p.gate_ld)) return -2;
   } else {
     if (make_bthd_map(&tq, q, p.B, p.T, p.N, H, 128)) return -2;
     if (make_bthd_map(&tk, k, p.B, p.S, p.Nkv, H, 128)) return -2;
@@ -772,6 +781,7 @@ extern "C" int axb_flash_fwd_v3(const void* q, const void* k, const void* v, voi
   p.window = window;
   p.status = status;
   p.gate = nullptr, p.gate_ld = 0, p.out_ld = 0, p.vdim = H, p.every = 1, p.bias = 0, p.rot_dim = 0, p.coef = 0.f;
+  p.first = nullptr, p.live = nullptr;
   const bool general = q_seg != nullptr || window >= 0 || logit_cap > 0.f;
   if (H == 128) {
     return general ? launch_flash_fwd3<128, true>(q, k, v, p, stream) : launch_flash_fwd3<128, false>(q, k, v, p, stream);
@@ -800,6 +810,7 @@ extern "C" int axb_flash_fwd_strided(const void* q, const void* k, const void* v
   p.sc = softmax_scale * 1.4426950408889634f, p.cap_in = 0.f, p.cap_out = 0.f;
   p.causal = 1, p.q_offset = 0, p.window = -1, p.status = status;
   p.gate = nullptr, p.gate_ld = 0, p.out_ld = 0, p.vdim = H, p.every = 1, p.bias = 0, p.rot_dim = 0, p.coef = 0.f;
+  p.first = nullptr, p.live = nullptr;
   CUtensorMap tq, tk, tv;
   if (make_strided_map(&tq, q, B, T, N, H, q_ld, q_batch) || make_strided_map(&tk, k, B, T, Nkv, H, kv_ld, kv_batch) ||
       make_strided_map(&tv, v, B, T, Nkv, H, kv_ld, kv_batch))
@@ -812,9 +823,10 @@ extern "C" int axb_flash_fwd_strided(const void* q, const void* k, const void* v
 // q / k / v / gate point at their first column in a packed projection [B, T, ld] (bf16); out [B, T, out_ld],
 // head h at column h * vdim.  Head sizes are multiples of 8 up to 128, as are ld, out_ld and the column
 // offsets (16-byte alignment).  gate may be null, coef 0 (no temperature), bias 0 (no distance bias).
-extern "C" int axb_flash_fwd_gated(const void* q, const void* k, const void* v, const void* gate, void* out, int B,
-                                   int T, int N, int Nkv, int dim, int vdim, int64_t ld, int64_t out_ld, float scale,
-                                   int window, float coef, int every, int bias, int* status, cudaStream_t stream) {
+static int flash_fwd_gated(const void* q, const void* k, const void* v, const void* gate, void* out, int B, int T, int N,
+                           int Nkv, int dim, int vdim, int64_t ld, int64_t out_ld, float scale, int window, float coef,
+                           int every, int bias, const int* first, const int* live, int rows, int* status,
+                           cudaStream_t stream) {
   using namespace axb;
   if (N % Nkv != 0 || dim > 128 || vdim > 128 || (dim % 8) || (vdim % 8) || (ld % 8) || (out_ld % 8) || window < 1 ||
       every < 1 || out_ld < static_cast<int64_t>(N) * vdim)
@@ -830,9 +842,27 @@ extern "C" int axb_flash_fwd_gated(const void* q, const void* k, const void* v, 
   p.sc = scale * 1.4426950408889634f, p.cap_in = 0.f, p.cap_out = 0.f;
   p.causal = 1, p.q_offset = 0, p.window = window - 1, p.status = status;
   p.gate = gate, p.gate_ld = ld, p.out_ld = out_ld, p.vdim = vdim, p.every = every, p.bias = bias, p.rot_dim = 0;
-  p.coef = coef;
-  if (dim <= 64 && vdim <= 64) return launch_flash_fwd3<64, true, true>(q, k, v, p, stream);
-  return launch_flash_fwd3<128, true, true>(q, k, v, p, stream);
+  p.coef = coef, p.first = first, p.live = live;
+  if (dim <= 64 && vdim <= 64) return launch_flash_fwd3<64, true, true>(q, k, v, p, stream, rows);
+  return launch_flash_fwd3<128, true, true>(q, k, v, p, stream, rows);
+}
+
+extern "C" int axb_flash_fwd_gated(const void* q, const void* k, const void* v, const void* gate, void* out, int B,
+                                   int T, int N, int Nkv, int dim, int vdim, int64_t ld, int64_t out_ld, float scale,
+                                   int window, float coef, int every, int bias, int* status, cudaStream_t stream) {
+  return flash_fwd_gated(q, k, v, gate, out, B, T, N, Nkv, dim, vdim, ld, out_ld, scale, window, coef, every, bias, nullptr,
+                         nullptr, 0, status, stream);
+}
+
+// The same for prompts without padding: rows first[b] .. first[b] + live[b] - 1 of the projection and of out (`rows` in all)
+// are sequence b's tokens, at most T of them.
+extern "C" int axb_flash_fwd_gated_packed(const void* q, const void* k, const void* v, const void* gate, void* out, int B,
+                                          int T, int N, int Nkv, int dim, int vdim, int64_t ld, int64_t out_ld,
+                                          float scale, int window, float coef, int every, int bias, const int* first,
+                                          const int* live, int rows, int* status, cudaStream_t stream) {
+  if (first == nullptr || live == nullptr || rows <= 0) return -10;
+  return flash_fwd_gated(q, k, v, gate, out, B, T, N, Nkv, dim, vdim, ld, out_ld, scale, window, coef, every, bias, first,
+                         live, rows, status, stream);
 }
 
 // Causal attention of whole prompts whose query rows are [dim | rot_dim] per head, whose unrotated keys are
@@ -860,7 +890,7 @@ extern "C" int axb_flash_fwd_latent(const void* q, const void* k, const void* kr
   p.sc = scale * 1.4426950408889634f, p.cap_in = 0.f, p.cap_out = 0.f;
   p.causal = 1, p.q_offset = 0, p.window = -1, p.status = status;
   p.gate = nullptr, p.gate_ld = 0, p.out_ld = out_ld, p.vdim = vdim, p.every = 1, p.bias = 0, p.coef = 0.f;
-  p.rot_dim = rot_dim;
+  p.rot_dim = rot_dim, p.first = nullptr, p.live = nullptr;
   auto map = [&](CUtensorMap* m, const void* base, int heads, int cols, int64_t head_ld, int64_t ld, int64_t batch_ld) {
     uint64_t dims[4] = {static_cast<uint64_t>(cols), static_cast<uint64_t>(heads), static_cast<uint64_t>(T),
                         static_cast<uint64_t>(B)};

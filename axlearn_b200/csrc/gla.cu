@@ -38,7 +38,10 @@ struct GlaArgs {
   float* seg_decay;      // [B, heads, segments, dim], log2
   const int* start;
   const int* live;
+  const int* first;      // [B] packed prompts: the row of proj and out at which a sequence's live tokens begin; null:
+                         // sequence b begins at row b T
   int64_t ld, out_ld;
+  int64_t rows;          // of proj and out: B T, or all live tokens
   int B, T, heads, dim, vdim, rank;
   int q_off, k_off, v_off, g_off, a1_off;
   int act_bf16, segments, seg_tokens;
@@ -58,6 +61,10 @@ __device__ __forceinline__ bool row_inactive(const GlaArgs& a, int b) {
 }
 __device__ __forceinline__ int live_tokens(const GlaArgs& a, int b) {
   return a.live != nullptr ? min(a.live[b], a.T) : a.T;
+}
+
+__device__ __forceinline__ int64_t first_row(const GlaArgs& a, int b) {
+  return a.first != nullptr ? a.first[b] : static_cast<int64_t>(b) * a.T;
 }
 
 constexpr int kGdThreads = 256;
@@ -361,9 +368,12 @@ __global__ void __launch_bounds__(kGcThreads, 2) gla_chunk_kernel(GlaArgs a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lc = (lane & 3) * 2;
   const bool inactive = row_inactive(a, b);
   const int live = inactive ? 0 : live_tokens(a, b);
-  const int t_lo = seg * a.seg_tokens, t_hi = a.segments > 1 ? min(a.T, t_lo + a.seg_tokens) : a.T;
+  // Tokens that have rows: the live ones of a packed prompt.
+  const int tokens = a.first != nullptr ? max(live, 0) : a.T;
+  const int64_t row0 = first_row(a, b);
+  const int t_lo = seg * a.seg_tokens, t_hi = a.segments > 1 ? min(tokens, t_lo + a.seg_tokens) : tokens;
   const int vcols = min(VS, a.vdim - d0);
-  const bf16* base = static_cast<const bf16*>(a.proj) + static_cast<int64_t>(b) * a.T * a.ld;
+  const bf16* base = static_cast<const bf16*>(a.proj) + row0 * a.ld;
   const bool vec = !((a.ld | a.q_off | a.k_off | a.v_off | a.g_off | a.dim | a.vdim) & 7);
   const bool vec_a1 = vec && !((a.a1_off | a.rank) & 7);
   const bool owner = warp < kWarpsV;
@@ -414,7 +424,7 @@ __global__ void __launch_bounds__(kGcThreads, 2) gla_chunk_kernel(GlaArgs a) {
       if (!kStateOnly) {
         const int n = min(kGcTok, t_hi - t0);
         for (int i = tid; i < n * vcols; i += kGcThreads) {
-          const int64_t tok = static_cast<int64_t>(b) * a.T + t0 + i / vcols;
+          const int64_t tok = row0 + t0 + i / vcols;
           if (slices == 1)
             static_cast<bf16*>(a.out)[tok * a.out_ld + h * a.vdim + i % vcols] = __float2bfloat16(0.f);
         }
@@ -816,7 +826,7 @@ __global__ void __launch_bounds__(kGcThreads, 2) gla_chunk_kernel(GlaArgs a) {
     }
     __syncthreads();
     const int n_out = min(kGcTok, t_hi - t0);
-    bf16* out = static_cast<bf16*>(a.out) + (static_cast<int64_t>(b) * a.T + t0) * a.out_ld + h * a.vdim;
+    bf16* out = static_cast<bf16*>(a.out) + (row0 + t0) * a.out_ld + h * a.vdim;
     if (vec) {
       const int c = (tid % (VS / 8)) * 8;
       bf16* p = out + (tid / (VS / 8)) * a.out_ld + c;
@@ -952,7 +962,9 @@ int launch_chunk(const GlaArgs& a, cudaStream_t stream) {
 
 bool gla_bad(const GlaArgs& a) {
   return a.B <= 0 || a.T <= 0 || a.heads <= 0 || a.dim <= 0 || a.dim > 512 || a.vdim <= 0 || a.rank <= 0 ||
-         a.rank > 512 || a.B > 65535 || a.heads > 65535 || a.out_ld < static_cast<int64_t>(a.heads) * a.vdim;
+         a.rank > 512 || a.B > 65535 || a.heads > 65535 || a.out_ld < static_cast<int64_t>(a.heads) * a.vdim ||
+         a.rows <= 0 ||
+         (a.first == nullptr ? a.rows != static_cast<int64_t>(a.B) * a.T : a.live == nullptr || a.start != nullptr);
 }
 
 template <typename T>
@@ -965,7 +977,7 @@ __global__ void gla_zero_tail_kernel(T* out, int64_t rows, int64_t ld, int first
 int gla_zero_tail(const GlaArgs& a, cudaStream_t stream) {
   const int used = a.heads * a.vdim;
   if (a.out_ld == used) return 0;
-  const int64_t rows = static_cast<int64_t>(a.B) * a.T, n = rows * (a.out_ld - used);
+  const int64_t rows = a.rows, n = rows * (a.out_ld - used);
   const unsigned grid = static_cast<unsigned>((n + 255) / 256);
   if (a.act_bf16)
     gla_zero_tail_kernel<<<grid, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(a.out), rows, a.out_ld, used);
@@ -979,7 +991,7 @@ int gla_zero_tail(const GlaArgs& a, cudaStream_t stream) {
 
 extern "C" int axb_gla_decode(const axb::GlaArgs* args, cudaStream_t stream) {
   const axb::GlaArgs& a = *args;
-  if (axb::gla_bad(a) || a.T != 1) return -10;
+  if (axb::gla_bad(a) || a.first != nullptr || a.T != 1) return -10;
   int rc;
   if (a.act_bf16)
     rc = a.vdim % 4 == 0 ? axb::launch_gla_decode<__nv_bfloat16, 4>(a, stream)
@@ -991,20 +1003,20 @@ extern "C" int axb_gla_decode(const axb::GlaArgs* args, cudaStream_t stream) {
 
 extern "C" int axb_gla_scan(const axb::GlaArgs* args, cudaStream_t stream) {
   const axb::GlaArgs& a = *args;
-  if (axb::gla_bad(a) || a.o_raw == nullptr) return -10;
+  if (axb::gla_bad(a) || a.first != nullptr || a.o_raw == nullptr) return -10;
   const int rc = a.act_bf16 ? axb::scan<__nv_bfloat16>(a, stream) : axb::scan<float>(a, stream);
   return rc ? rc : axb::gla_zero_tail(a, stream);
 }
 
 // bf16 only; dim <= 128, rank <= 128.  segments > 1 needs seg_state / seg_decay and seg_tokens a
-// multiple of 64 with segments * seg_tokens >= T; vdim > 128 needs o_raw.
+// multiple of 64 with segments * seg_tokens >= T; vdim > 128 needs o_raw and unpacked prompts.
 extern "C" int axb_gla_chunk(const axb::GlaArgs* args, cudaStream_t stream) {
   const axb::GlaArgs& a = *args;
   if (axb::gla_bad(a) || !a.act_bf16 || a.dim > 128 || a.rank > 128 || a.segments < 1) return -10;
   if (a.segments > 1 && (a.seg_state == nullptr || a.seg_decay == nullptr || a.seg_tokens % 64 ||
                          static_cast<int64_t>(a.segments) * a.seg_tokens < a.T))
     return -11;
-  if (a.vdim > 128 && a.o_raw == nullptr) return -11;
+  if (a.vdim > 128 && (a.o_raw == nullptr || a.first != nullptr)) return -11;
   int rc;
   if (a.dim <= 64)
     rc = a.vdim <= 64 ? axb::launch_chunk<64, 64>(a, stream) : axb::launch_chunk<64, 128>(a, stream);

@@ -47,7 +47,10 @@ struct SsdArgs {
   float* seg_decay;      // [B, H, segments], log2
   const int* start;
   const int* live;
+  const int* first;      // [B] packed prompts: the row of proj, xbc, y and out at which a sequence's live tokens begin; null:
+                         // sequence b begins at row b T
   int64_t ld, xbc_ld, out_ld;
+  int64_t rows;          // of proj and out: B T, or all live tokens
   int B, T, heads, vdim, state, groups, taps, norm_groups;
   int z_off, xbc_off, dt_off, act_bf16, segments, seg_tokens;
   float eps;
@@ -70,6 +73,11 @@ __device__ __forceinline__ bool ssd_inactive(const SsdArgs& a, int b) {
 __device__ __forceinline__ int ssd_live(const SsdArgs& a, int b) {
   return a.live != nullptr ? min(a.live[b], a.T) : a.T;
 }
+__device__ __forceinline__ int64_t ssd_row(const SsdArgs& a, int b) {
+  return a.first != nullptr ? a.first[b] : static_cast<int64_t>(b) * a.T;
+}
+// Tokens that have rows: the live ones of a packed prompt.
+__device__ __forceinline__ int ssd_tokens(const SsdArgs& a, int b) { return a.first != nullptr ? max(ssd_live(a, b), 0) : a.T; }
 __device__ __forceinline__ int ssd_channels(const SsdArgs& a) { return a.heads * a.vdim + 2 * a.groups * a.state; }
 
 template <int V>
@@ -122,12 +130,12 @@ template <typename T, int TAPS, int V>
 __global__ void __launch_bounds__(kConvThreads) ssd_conv_kernel(SsdArgs a) {
   const int channels = ssd_channels(a);
   const int c = (blockIdx.x * kConvThreads + threadIdx.x) * V, b = blockIdx.z, t0 = blockIdx.y * kConvTokens;
-  if (c >= channels || ssd_inactive(a, b)) return;
+  if (c >= channels || ssd_inactive(a, b) || t0 >= ssd_tokens(a, b)) return;
   const int taps = TAPS ? TAPS : a.taps;
   const int start = a.start != nullptr ? a.start[b] : 0;
-  const T* src = static_cast<const T*>(a.proj) + static_cast<int64_t>(b) * a.T * a.ld + a.xbc_off + c;
+  const T* src = static_cast<const T*>(a.proj) + ssd_row(a, b) * a.ld + a.xbc_off + c;
   const T* ring = static_cast<const T*>(a.ring) + static_cast<int64_t>(b) * taps * channels + c;
-  T* dst = static_cast<T*>(a.xbc) + static_cast<int64_t>(b) * a.T * a.xbc_ld + c;
+  T* dst = static_cast<T*>(a.xbc) + ssd_row(a, b) * a.xbc_ld + c;
   auto input = [&](int t, float (&f)[V]) {  // the input of token t, also of tokens before this block
     if (t >= 0) {
       load_v<V>(src + t * a.ld, f);
@@ -141,7 +149,7 @@ __global__ void __launch_bounds__(kConvThreads) ssd_conv_kernel(SsdArgs a) {
   float bias[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) bias[i] = a.conv_b[c + i];
-  const int t1 = min(a.T, t0 + kConvTokens);
+  const int t1 = min(ssd_tokens(a, b), t0 + kConvTokens);
   if (TAPS == 0) {
     for (int t = t0; t < t1; ++t) {
       float acc[V], x[V];
@@ -216,7 +224,7 @@ __global__ void ssd_ring_kernel(SsdArgs a) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
   if (c >= channels || ssd_inactive(a, b)) return;
   const int start = a.start != nullptr ? a.start[b] : 0, live = ssd_live(a, b);
-  const T* src = static_cast<const T*>(a.proj) + static_cast<int64_t>(b) * a.T * a.ld + a.xbc_off + c;
+  const T* src = static_cast<const T*>(a.proj) + ssd_row(a, b) * a.ld + a.xbc_off + c;
   T* ring = static_cast<T*>(a.ring) + static_cast<int64_t>(b) * a.taps * channels + c;
   for (int t = max(0, live - a.taps); t < live; ++t) ring[static_cast<int64_t>((start + t) % a.taps) * channels] = src[t * a.ld];
 }
@@ -576,11 +584,12 @@ __global__ void __launch_bounds__(kScThreads, 4) ssd_chunk_kernel(SsdArgs a) {
   const int group = h / (a.heads / a.groups);
   const bool inactive = ssd_inactive(a, b);
   const int live = inactive ? 0 : ssd_live(a, b);
-  const int t_lo = seg * a.seg_tokens, t_hi = a.segments > 1 ? min(a.T, t_lo + a.seg_tokens) : a.T;
+  const int tokens = ssd_tokens(a, b);
+  const int t_lo = seg * a.seg_tokens, t_hi = a.segments > 1 ? min(tokens, t_lo + a.seg_tokens) : tokens;
   const int t_live = min(live, t_hi);
-  const bf16* xbc = static_cast<const bf16*>(a.xbc) + static_cast<int64_t>(b) * a.T * a.xbc_ld;
-  const bf16* dt_col = static_cast<const bf16*>(a.proj) + static_cast<int64_t>(b) * a.T * a.ld + a.dt_off + h;
-  bf16* yout = static_cast<bf16*>(a.y) + static_cast<int64_t>(b) * a.T * inner + h * P + p0;
+  const bf16* xbc = static_cast<const bf16*>(a.xbc) + ssd_row(a, b) * a.xbc_ld;
+  const bf16* dt_col = static_cast<const bf16*>(a.proj) + ssd_row(a, b) * a.ld + a.dt_off + h;
+  bf16* yout = static_cast<bf16*>(a.y) + ssd_row(a, b) * inner + h * P + p0;
   const int x_off = h * P + p0, b_off = inner + group * N, c_off = b_off + a.groups * N;
   const bool vec_bc = !((a.xbc_ld | b_off | c_off | N) & 7), vec_x = !((a.xbc_ld | P | inner) & 7);
   const float rate = -expf(a.a_log[h]) * kL2e, dt_bias = a.dt_bias[h], skip = a.d[h];
@@ -872,7 +881,8 @@ int launched() { return cudaGetLastError() == cudaSuccess ? 0 : -4; }
 bool ssd_bad(const SsdArgs& a) {
   return a.B <= 0 || a.T <= 0 || a.heads <= 0 || a.vdim <= 0 || a.state <= 0 || a.groups <= 0 || a.heads % a.groups ||
          a.taps <= 0 || a.norm_groups <= 0 || (a.heads * a.vdim) % a.norm_groups || a.B > 65535 || a.heads > 65535 ||
-         a.out_ld < static_cast<int64_t>(a.heads) * a.vdim;
+         a.out_ld < static_cast<int64_t>(a.heads) * a.vdim || a.rows <= 0 ||
+         (a.first == nullptr ? a.rows != static_cast<int64_t>(a.B) * a.T : a.live == nullptr || a.start != nullptr);
 }
 
 template <typename T, int TAPS, int V>
@@ -965,7 +975,7 @@ int launch_chunk(const SsdArgs& a, cudaStream_t stream) {
 template <typename T>
 int norm(const SsdArgs& a, cudaStream_t stream) {
   const int inner = a.heads * a.vdim, width = inner / a.norm_groups;
-  const int64_t rows = static_cast<int64_t>(a.B) * a.T;
+  const int64_t rows = a.rows;
   const bool vec = !((width | inner | a.z_off | static_cast<int>(a.out_ld | a.ld)) & 7);
   const int want = ((vec ? width / 8 : width) + 31) / 32 * 32;
   const int threads = want < 32 ? 32 : (want > 256 ? 256 : want);
@@ -996,7 +1006,7 @@ extern "C" int axb_ssd_conv(const axb::SsdArgs* args, cudaStream_t stream) {
 // Outputs into a.y, token by token; needs a.xbc.  state <= 512.
 extern "C" int axb_ssd_scan(const axb::SsdArgs* args, cudaStream_t stream) {
   const axb::SsdArgs& a = *args;
-  if (axb::ssd_bad(a) || a.xbc == nullptr || a.state > 512) return -10;
+  if (axb::ssd_bad(a) || a.first != nullptr || a.xbc == nullptr || a.state > 512) return -10;
   return a.act_bf16 ? axb::scan<__nv_bfloat16>(a, stream) : axb::scan<float>(a, stream);
 }
 
@@ -1014,7 +1024,7 @@ extern "C" int axb_ssd_chunk(const axb::SsdArgs* args, cudaStream_t stream) {
 // One token per sequence; needs a.start.
 extern "C" int axb_ssd_decode(const axb::SsdArgs* args, cudaStream_t stream) {
   const axb::SsdArgs& a = *args;
-  if (axb::ssd_bad(a) || a.T != 1 || a.start == nullptr) return -10;
+  if (axb::ssd_bad(a) || a.first != nullptr || a.T != 1 || a.start == nullptr) return -10;
   if (a.act_bf16)
     return a.vdim % 4 == 0 ? axb::launch_decode<__nv_bfloat16, 4>(a, stream) : axb::launch_decode<__nv_bfloat16, 1>(a, stream);
   return a.vdim % 4 == 0 ? axb::launch_decode<float, 4>(a, stream) : axb::launch_decode<float, 1>(a, stream);

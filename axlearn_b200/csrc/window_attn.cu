@@ -36,6 +36,8 @@ struct WindowArgs {
   const int* live;
   float* part;           // decode splits: [B, H, splits, vdim + 2 rounded up to 4]
   int* tickets;          // [B * CTA groups], zero on entry and on exit
+  const int* first;      // [B] packed prompts (appending only): the row of proj at which a sequence's live tokens begin;
+                         // null: sequence b begins at row b T
   int64_t ld, out_ld;
   int B, T, heads, kv_heads, dim, vdim, slots, window;
   int q_off, k_off, v_off, g_off;  // g_off < 0: no gate
@@ -451,7 +453,7 @@ __global__ void __launch_bounds__(128) window_append_kernel(WindowArgs a) {
   for (int back = blockIdx.x; back < a.slots; back += gridDim.x) {
     const int t = live - 1 - back;
     if (t < 0 || start < 0) return;
-    const T* row = static_cast<const T*>(a.proj) + (static_cast<int64_t>(b) * a.T + t) * a.ld;
+    const T* row = static_cast<const T*>(a.proj) + ((a.first != nullptr ? a.first[b] : static_cast<int64_t>(b) * a.T) + t) * a.ld;
     const int64_t slot = static_cast<int64_t>(b) * a.slots + (start + t) % a.slots;
     const V* ks = reinterpret_cast<const V*>(row + a.k_off);
     const V* vs = reinterpret_cast<const V*>(row + a.v_off);

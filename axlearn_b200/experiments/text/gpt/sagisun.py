@@ -41,7 +41,7 @@ ARCHITECTURE = "Sagisun"
 Tensor = torch.Tensor
 # Kernels of an inference process (a first run without a built library compiles these).
 KERNEL_SOURCES = ("flash_fwd.cu", "flash_fwd_v3.cu", "gated_act.cu", "gemm.cu", "gemm_2cta.cu", "gemm_skinny.cu",
-                  "gla.cu", "hyper.cu", "step_frame.cu", "window_attn.cu")
+                  "gla.cu", "hyper.cu", "pack_rows.cu", "step_frame.cu", "window_attn.cu")
 # A window that never closes (a left mixer without a mask).
 _NO_WINDOW = 1 << 30
 

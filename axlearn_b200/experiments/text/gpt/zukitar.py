@@ -43,7 +43,7 @@ ARCHITECTURE = "Zukitar"
 Tensor = torch.Tensor
 # Kernels of an inference process (a first run without a built library compiles these).
 KERNEL_SOURCES = ("experts.cu", "flash_fwd.cu", "flash_fwd_v3.cu", "gated_act.cu", "gemm.cu", "gemm_2cta.cu",
-                  "gemm_skinny.cu", "hyper.cu", "latent_attn.cu", "skinny_group.cu", "ssd.cu", "step_frame.cu")
+                  "gemm_skinny.cu", "hyper.cu", "latent_attn.cu", "pack_rows.cu", "skinny_group.cu", "ssd.cu", "step_frame.cu")
 # The experts' gate: g sigmoid(alpha g).
 _EXPERT_ALPHA = 1.702
 

@@ -18,6 +18,7 @@ import torch.nn.functional as F
 
 from axlearn_b200.ops import dispatch
 from axlearn_b200.ops.hyper_ops import padded
+from axlearn_b200.ops.packed_ops import PackedRows
 
 Tensor = torch.Tensor
 
@@ -82,14 +83,20 @@ def reference_gated_linear_attention(proj, a2, a2_bias, norm_scale, spec: GlaSpe
 
 def gated_linear_attention(proj: Tensor, a2: Tensor, a2_bias: Tensor, norm_scale: Tensor, spec: GlaSpec,
                            cols: GlaColumns, *, start: Optional[Tensor] = None, live: Optional[Tensor] = None,
-                           state: Optional[Tensor] = None):
-    """``(out [B, T, out_width], state [B, H, dim, vdim])``.  start: int32 ``[B]``, only its sign matters
+                           state: Optional[Tensor] = None, packed: Optional[PackedRows] = None):
+    """``(out [B, T, out_width], state [B, H, dim, vdim])``; in- and output ``[1, rows, ...]`` for ``packed`` prompts.  start: int32 ``[B]``, only its sign matters
     here (negative: the row is not in this step).  live: int32 ``[B]`` valid tokens (None: T).  state: None
     starts from zero."""
     tensors = [proj, a2, a2_bias, norm_scale]
     grad = torch.is_grad_enabled() and any(x.requires_grad for x in tensors)
     if dispatch._cuda(*tensors) and not grad and proj.dtype in (torch.bfloat16, torch.float32):  # pylint: disable=protected-access
-        return _cuda_gla(proj, a2, a2_bias, norm_scale, spec, cols, start=start, live=live, state=state)
+        if packed is not None and not (
+                proj.dtype == torch.bfloat16 and spec.dim <= 128 and spec.rank <= 128 and spec.vdim <= 128):
+            out, state = _cuda_gla(packed.unpack(proj), a2, a2_bias, norm_scale, spec, cols, start=start, live=live,
+                                   state=state)
+            return packed.pack(out), state
+        return _cuda_gla(proj, a2, a2_bias, norm_scale, spec, cols, start=start, live=live, state=state, packed=packed)
+    assert packed is None
     b, t, _ = proj.shape
     if live is None:
         live = torch.full((b,), t, dtype=torch.int32, device=proj.device)
@@ -107,8 +114,8 @@ class _Args(ctypes.Structure):
     """Mirrors ``axb::GlaArgs``."""
 
     _fields_ = [(n, ctypes.c_void_p) for n in (
-        "proj", "a2", "a2_bias", "norm_w", "state", "out", "o_raw", "seg_state", "seg_decay", "start", "live")] + [
-        ("ld", ctypes.c_int64), ("out_ld", ctypes.c_int64)] + [(n, ctypes.c_int) for n in (
+        "proj", "a2", "a2_bias", "norm_w", "state", "out", "o_raw", "seg_state", "seg_decay", "start", "live",
+        "first")] + [("ld", ctypes.c_int64), ("out_ld", ctypes.c_int64), ("rows", ctypes.c_int64)] + [(n, ctypes.c_int) for n in (
             "B", "T", "heads", "dim", "vdim", "rank", "q_off", "k_off", "v_off", "g_off", "a1_off", "act_bf16",
             "segments", "seg_tokens")] + [(n, ctypes.c_float) for n in ("inv_tau", "q_scale", "eps")]
 
@@ -143,7 +150,7 @@ def prompt_segments(b: int, t: int, heads: int, vdim: int, sms: int = 148) -> tu
 
 
 def _cuda_gla(proj, a2, a2_bias, norm_scale, spec, cols, *, start, live, state, segments: Optional[tuple] = None,
-              kernel: Optional[str] = None):
+              kernel: Optional[str] = None, packed: Optional[PackedRows] = None):
     """``kernel``: "chunk" / "scan" overrides the choice for prompts; ``segments`` that of
     ``prompt_segments``."""
     from axlearn_b200.ops import cuda_ops
@@ -152,20 +159,22 @@ def _cuda_gla(proj, a2, a2_bias, norm_scale, spec, cols, *, start, live, state, 
     lib = _lib()
     proj, a2 = proj.contiguous(), a2.to(proj.dtype).contiguous()
     a2_bias, norm_scale = a2_bias.float().contiguous(), norm_scale.float().contiguous()
-    b, t, ld = proj.shape
-    start, live = _int32(start), _int32(live)
+    rows, ld = proj.shape[0] * proj.shape[1], proj.shape[2]
+    b, t = proj.shape[:2] if packed is None else (packed.live.shape[0], packed.max_len)
+    start, live = _int32(start), _int32(live if packed is None else packed.live)
     if state is None:
         state = torch.zeros((b, spec.heads, spec.dim, spec.vdim), dtype=torch.float32, device=proj.device)
     assert state.dtype == torch.float32 and state.is_contiguous()
     assert state.shape == (b, spec.heads, spec.dim, spec.vdim), (state.shape, spec)
     assert a2.shape == (spec.heads * spec.dim, spec.rank), (a2.shape, spec)
-    out = torch.empty((b, t, spec.out_width), dtype=proj.dtype, device=proj.device)
+    out = torch.empty((*proj.shape[:2], spec.out_width), dtype=proj.dtype, device=proj.device)
     a = _Args()
     a.proj, a.a2, a.a2_bias, a.norm_w = proj.data_ptr(), a2.data_ptr(), a2_bias.data_ptr(), norm_scale.data_ptr()
     a.state, a.out = state.data_ptr(), out.data_ptr()
     a.start = None if start is None else start.data_ptr()
     a.live = None if live is None else live.data_ptr()
-    a.ld, a.out_ld, a.B, a.T = ld, out.shape[-1], b, t
+    a.first = None if packed is None else packed.first.data_ptr()
+    a.ld, a.out_ld, a.rows, a.B, a.T = ld, out.shape[-1], rows, b, t
     a.heads, a.dim, a.vdim, a.rank = spec.heads, spec.dim, spec.vdim, spec.rank
     a.q_off, a.k_off, a.v_off, a.g_off, a.a1_off = cols.q, cols.k, cols.v, cols.g, cols.a1
     a.act_bf16 = int(proj.dtype == torch.bfloat16)

@@ -25,6 +25,7 @@ import torch.nn.functional as F
 
 from axlearn_b200.ops import dispatch
 from axlearn_b200.ops.hyper_ops import padded
+from axlearn_b200.ops.packed_ops import PackedRows
 
 Tensor = torch.Tensor
 
@@ -138,14 +139,18 @@ def reference_ssd_mix(proj, w: SsdWeights, spec: SsdSpec, cols: SsdColumns, *, s
 
 
 def ssd_mix(proj: Tensor, weights: SsdWeights, spec: SsdSpec, cols: SsdColumns, *, start: Optional[Tensor] = None,
-            live: Optional[Tensor] = None, state: Optional[dict] = None):
-    """``(out [B, T, out_width], state)``.  start: int32 ``[B]`` tokens the state has seen (None: zero);
+            live: Optional[Tensor] = None, state: Optional[dict] = None, packed: Optional[PackedRows] = None):
+    """``(out [B, T, out_width], state)``; both ``[1, rows, ...]`` for ``packed`` prompts.  start: int32 ``[B]`` tokens the state has seen (None: zero);
     negative takes the row out of the step.  live: int32 ``[B]`` valid new tokens (None: T).  state None
     starts from zero and keeps nothing."""
     tensors = [proj] + [getattr(weights, f.name) for f in dataclasses.fields(weights)]
     grad = torch.is_grad_enabled() and any(x.requires_grad for x in tensors)
     if dispatch._cuda(*tensors) and not grad and proj.dtype in (torch.bfloat16, torch.float32):  # pylint: disable=protected-access
-        return _cuda_ssd_mix(proj, weights, spec, cols, start=start, live=live, state=state)
+        if packed is not None and (proj.dtype != torch.bfloat16 or spec.state > 128):  # not the chunked kernel
+            out, state = _cuda_ssd_mix(packed.unpack(proj), weights, spec, cols, start=start, live=live, state=state)
+            return packed.pack(out), state
+        return _cuda_ssd_mix(proj, weights, spec, cols, start=start, live=live, state=state, packed=packed)
+    assert packed is None
     b, t, _ = proj.shape
     if live is None:
         live = torch.full((b,), t, dtype=torch.int32, device=proj.device)
@@ -165,8 +170,8 @@ class _Args(ctypes.Structure):
 
     _fields_ = [(n, ctypes.c_void_p) for n in (
         "proj", "conv_w", "conv_b", "dt_bias", "a_log", "d", "norm_w", "ssm", "ring", "xbc", "y", "out",
-        "seg_state", "seg_decay", "start", "live")] + [(n, ctypes.c_int64) for n in (
-            "ld", "xbc_ld", "out_ld")] + [(n, ctypes.c_int) for n in (
+        "seg_state", "seg_decay", "start", "live", "first")] + [(n, ctypes.c_int64) for n in (
+            "ld", "xbc_ld", "out_ld", "rows")] + [(n, ctypes.c_int) for n in (
                 "B", "T", "heads", "vdim", "state", "groups", "taps", "norm_groups", "z_off", "xbc_off", "dt_off",
                 "act_bf16", "segments", "seg_tokens")] + [("eps", ctypes.c_float)]
 
@@ -204,16 +209,18 @@ def chunk_ctas(spec: SsdSpec) -> int:
 
 
 def _cuda_ssd_mix(proj, w: SsdWeights, spec: SsdSpec, cols: SsdColumns, *, start, live, state,
-                  kernel: Optional[str] = None, segments: Optional[tuple] = None):
+                  kernel: Optional[str] = None, segments: Optional[tuple] = None,
+                  packed: Optional[PackedRows] = None):
     """``kernel``: "chunk" / "scan" overrides the choice for prompts; ``segments`` that of ``prompt_segments``."""
     from axlearn_b200.ops import cuda_ops
     from axlearn_b200.ops.window_ops import _int32
 
     lib = _lib()
     proj = proj.contiguous()
-    b, t, ld = proj.shape
-    start, live = _int32(start), _int32(live)
-    decode = t == 1 and start is not None and state is not None and kernel is None
+    rows, ld = proj.shape[0] * proj.shape[1], proj.shape[2]
+    b, t = proj.shape[:2] if packed is None else (packed.live.shape[0], packed.max_len)
+    start, live = _int32(start), _int32(live if packed is None else packed.live)
+    decode = packed is None and t == 1 and start is not None and state is not None and kernel is None
     if state is None:
         if start is not None:
             raise ValueError("a continued block needs its state")
@@ -227,19 +234,20 @@ def _cuda_ssd_mix(proj, w: SsdWeights, spec: SsdSpec, cols: SsdColumns, *, start
     assert ssm.shape == (b, spec.heads, spec.state, spec.vdim) and ring.shape == (b, spec.taps, spec.channels)
     vectors = {name: getattr(w, name).float().contiguous() for name in (
         "conv_w", "conv_b", "dt_bias", "a_log", "d", "norm_w")}
-    out = torch.empty((b, t, spec.out_width), dtype=proj.dtype, device=proj.device)
+    out = torch.empty((*proj.shape[:2], spec.out_width), dtype=proj.dtype, device=proj.device)
     a = _Args()
     for name, v in vectors.items():
         setattr(a, name, v.data_ptr())
     a.proj, a.ssm, a.ring, a.out = proj.data_ptr(), ssm.data_ptr(), ring.data_ptr(), out.data_ptr()
     a.start = None if start is None else start.data_ptr()
     a.live = None if live is None else live.data_ptr()
-    a.ld, a.out_ld, a.xbc_ld, a.B, a.T = ld, out.shape[-1], padded(spec.channels, 8), b, t
+    a.first = None if packed is None else packed.first.data_ptr()
+    a.ld, a.out_ld, a.xbc_ld, a.rows, a.B, a.T = ld, out.shape[-1], padded(spec.channels, 8), rows, b, t
     a.heads, a.vdim, a.state, a.groups, a.taps = spec.heads, spec.vdim, spec.state, spec.groups, spec.taps
     a.norm_groups, a.eps = spec.norm_groups, spec.eps
     a.z_off, a.xbc_off, a.dt_off = cols.z, cols.xbc, cols.dt
     a.act_bf16, a.segments, a.seg_tokens = int(proj.dtype == torch.bfloat16), 1, padded(t, CHUNK_TOKENS)
-    y = torch.empty((b, t, spec.inner), dtype=proj.dtype, device=proj.device)
+    y = torch.empty((rows, spec.inner), dtype=proj.dtype, device=proj.device)
     a.y = y.data_ptr()
     stream = cuda_ops._stream()  # pylint: disable=protected-access
     check = cuda_ops._check  # pylint: disable=protected-access
@@ -247,7 +255,7 @@ def _cuda_ssd_mix(proj, w: SsdWeights, spec: SsdSpec, cols: SsdColumns, *, start
         check(lib.axb_ssd_decode(ctypes.byref(a), stream), "axb_ssd_decode")
         check(lib.axb_ssd_norm(ctypes.byref(a), stream), "axb_ssd_norm")
         return out, keep
-    xbc = torch.empty((b, t, a.xbc_ld), dtype=proj.dtype, device=proj.device)
+    xbc = torch.empty((rows, a.xbc_ld), dtype=proj.dtype, device=proj.device)
     a.xbc = xbc.data_ptr()
     check(lib.axb_ssd_conv(ctypes.byref(a), stream), "axb_ssd_conv")
     if kernel is None:

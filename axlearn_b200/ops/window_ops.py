@@ -24,6 +24,7 @@ import torch.nn.functional as F
 
 from axlearn_b200.ops import dispatch
 from axlearn_b200.ops.hyper_ops import padded
+from axlearn_b200.ops.packed_ops import PackedRows
 
 Tensor = torch.Tensor
 
@@ -118,8 +119,8 @@ def reference_window_attention(proj, spec: WindowSpec, cols: WindowColumns, *, s
 
 
 def window_attention(proj: Tensor, spec: WindowSpec, cols: WindowColumns, *, start: Optional[Tensor] = None,
-                     live: Optional[Tensor] = None, cache: Optional[dict] = None):
-    """``(out [B, T, out_width], cache)``.
+                     live: Optional[Tensor] = None, cache: Optional[dict] = None, packed: Optional[PackedRows] = None):
+    """``(out [B, T, out_width], cache)``; in- and output ``[1, rows, ...]`` for ``packed`` prompts.
 
     start: int32 ``[B]`` tokens already stored (None: zero); a negative value takes the row out of the
     step (its output is zero, its cache untouched).  live: int32 ``[B]`` valid new tokens (None: T).
@@ -127,7 +128,11 @@ def window_attention(proj: Tensor, spec: WindowSpec, cols: WindowColumns, *, sta
     nothing before this block is seen)."""
     grad = torch.is_grad_enabled() and proj.requires_grad
     if dispatch._cuda(proj) and not grad and proj.dtype in (torch.bfloat16, torch.float32):  # pylint: disable=protected-access
-        return _cuda_window_attention(proj, spec, cols, start=start, live=live, cache=cache)
+        if packed is not None and not (packed.max_len >= FLASH_MIN_TOKENS and flash_supported(proj, spec, cols)):
+            out, cache = _cuda_window_attention(packed.unpack(proj), spec, cols, start=start, live=live, cache=cache)
+            return packed.pack(out), cache
+        return _cuda_window_attention(proj, spec, cols, start=start, live=live, cache=cache, packed=packed)
+    assert packed is None
     b, t, _ = proj.shape
     if start is None:
         start = torch.zeros(b, dtype=torch.int32, device=proj.device)
@@ -146,7 +151,7 @@ class _Args(ctypes.Structure):
     """Mirrors ``axb::WindowArgs``."""
 
     _fields_ = [(n, ctypes.c_void_p) for n in (
-        "proj", "k_ring", "v_ring", "out", "start", "live", "part", "tickets")] + [
+        "proj", "k_ring", "v_ring", "out", "start", "live", "part", "tickets", "first")] + [
         ("ld", ctypes.c_int64), ("out_ld", ctypes.c_int64)] + [(n, ctypes.c_int) for n in (
             "B", "T", "heads", "kv_heads", "dim", "vdim", "slots", "window", "q_off", "k_off", "v_off", "g_off",
             "splits", "every", "bias", "act_bf16")] + [("scale", ctypes.c_float), ("coef", ctypes.c_float)]
@@ -175,6 +180,10 @@ def _lib():
                                                                                ctypes.c_int, ctypes.c_void_p,
                                                                                ctypes.c_void_p])
         h.axb_flash_fwd_gated.restype = ctypes.c_int
+        gated = list(h.axb_flash_fwd_gated.argtypes)
+        h.axb_flash_fwd_gated_packed.argtypes = (
+            gated[:-2] + [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int] + gated[-2:])
+        h.axb_flash_fwd_gated_packed.restype = ctypes.c_int
         _signatures_set = True
     return h
 
@@ -209,19 +218,21 @@ def _int32(t: Optional[Tensor]) -> Optional[Tensor]:
     return t if t.dtype == torch.int32 and t.is_contiguous() else t.to(torch.int32).contiguous()
 
 
-def _cuda_window_attention(proj, spec, cols, *, start, live, cache):
+def _cuda_window_attention(proj, spec, cols, *, start, live, cache, packed: Optional[PackedRows] = None):
     from axlearn_b200.ops import cuda_ops
 
     lib = _lib()
     proj = proj.contiguous()
-    b, t, ld = proj.shape
-    start, live = _int32(start), _int32(live)
-    out = torch.empty((b, t, spec.out_width), dtype=proj.dtype, device=proj.device)
+    ld = proj.shape[2]
+    b, t = proj.shape[:2] if packed is None else (packed.live.shape[0], packed.max_len)
+    start, live = _int32(start), _int32(live if packed is None else packed.live)
+    out = torch.empty((*proj.shape[:2], spec.out_width), dtype=proj.dtype, device=proj.device)
     coef, every = spec.q_temp if spec.q_temp is not None else (0.0, 1)
     a = _Args()
     a.proj, a.out, a.ld, a.out_ld = proj.data_ptr(), out.data_ptr(), ld, out.shape[-1]
     a.start = None if start is None else start.data_ptr()
     a.live = None if live is None else live.data_ptr()
+    a.first = None if packed is None else packed.first.data_ptr()
     a.B, a.T, a.heads, a.kv_heads, a.dim, a.vdim = b, t, spec.heads, spec.kv_heads, spec.dim, spec.vdim
     a.window, a.slots = spec.window, 1
     if cache is not None:
@@ -234,7 +245,7 @@ def _cuda_window_attention(proj, spec, cols, *, start, live, cache):
     a.act_bf16, a.splits = int(proj.dtype == torch.bfloat16), 1
     stream = cuda_ops._stream()  # pylint: disable=protected-access
     check = cuda_ops._check  # pylint: disable=protected-access
-    if t == 1 and start is not None and cache is not None:
+    if packed is None and t == 1 and start is not None and cache is not None:
         ctas = lib.axb_window_decode_ctas(b, spec.heads, spec.kv_heads, spec.dim, spec.vdim)
         a.splits = decode_splits(ctas, min(spec.window, a.slots))
         part = None
@@ -247,11 +258,16 @@ def _cuda_window_attention(proj, spec, cols, *, start, live, cache):
         raise ValueError("a continued block needs its cache")
     if start is None and t >= FLASH_MIN_TOKENS and flash_supported(proj, spec, cols):
         base, e = proj.data_ptr(), proj.element_size()
-        check(lib.axb_flash_fwd_gated(
-            base + cols.q * e, base + cols.k * e, base + cols.v * e, base + cols.g * e if spec.gated else None,
-            out.data_ptr(), b, t, spec.heads, spec.kv_heads, spec.dim, spec.vdim, ld, out.shape[-1], spec.scale,
-            spec.window, float(coef), int(every), int(spec.distance_bias),
-            cuda_ops.status_word(proj.device).data_ptr(), stream), "axb_flash_fwd_gated")
+        sizes = (b, t, spec.heads, spec.kv_heads, spec.dim, spec.vdim, ld, out.shape[-1], spec.scale, spec.window,
+                 float(coef), int(every), int(spec.distance_bias))
+        where = (base + cols.q * e, base + cols.k * e, base + cols.v * e, base + cols.g * e if spec.gated else None,
+                 out.data_ptr())
+        status = cuda_ops.status_word(proj.device).data_ptr()
+        if packed is None:
+            check(lib.axb_flash_fwd_gated(*where, *sizes, status, stream), "axb_flash_fwd_gated")
+        else:
+            check(lib.axb_flash_fwd_gated_packed(*where, *sizes, packed.first.data_ptr(), live.data_ptr(), packed.rows,
+                                                 status, stream), "axb_flash_fwd_gated_packed")
     else:
         check(lib.axb_window_attn(ctypes.byref(a), stream), "axb_window_attn")
     if cache is not None:

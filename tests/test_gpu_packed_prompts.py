@@ -1,0 +1,126 @@
+"""Prompts without their padding against the padded ones: the mixers alone, and whole served models."""
+
+import pytest
+import torch
+
+from axlearn_b200.ops import gla_ops, packed_ops, ssd_ops, window_ops
+
+pytestmark = pytest.mark.gpu
+
+# Sequences of one token, of none, at the edges of the kernels' chunks and tiles, and of all of T.
+_LENGTHS = [[300, 1, 64, 65, 128, 255], [40, 40, 17], [1100, 700, 1], [129, 0, 256, 3]]
+
+
+def _packed(lengths, width, seed):
+    t = max(lengths)
+    live = torch.tensor(lengths, dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    proj = torch.randn(len(lengths), t, width, device="cuda", generator=g).bfloat16()
+    return packed_ops.PackedRows(live, t), live, proj
+
+
+def _alike(packed, out, padded):
+    """Bit by bit: a row's arithmetic does not know where the row lies."""
+    assert torch.equal(out, packed.pack(padded)) and out.shape[1] == packed.rows
+
+
+@pytest.mark.parametrize("lengths", _LENGTHS)
+@pytest.mark.parametrize("groups,segments", [(1, None), (2, 2)])
+def test_state_space(lengths, groups, segments):
+    spec = ssd_ops.SsdSpec(heads=4, vdim=64, state=64, groups=groups, taps=4, norm_groups=2, eps=1e-6)
+    cols = ssd_ops.SsdColumns(z=0, xbc=spec.inner, dt=spec.inner + spec.channels)
+    packed, live, proj = _packed(lengths, spec.inner + spec.channels + 8, 1)
+    w = ssd_ops.SsdWeights(*(torch.randn(n, device="cuda") * 0.3 for n in (
+        (4, spec.channels), (spec.channels,), (4,), (4,), (4,), (spec.inner,))))
+
+    def run(x, **more):
+        state = {"ssm": torch.zeros(len(lengths), 4, 64, 64, device="cuda"),
+                 "conv": torch.zeros(len(lengths), 4, spec.channels, device="cuda", dtype=torch.bfloat16)}
+        cut = segments and (segments, -(-max(lengths) // segments // 64) * 64 + 64)
+        return ssd_ops._cuda_ssd_mix(  # pylint: disable=protected-access
+            x, w, spec, cols, start=None, state=state, segments=cut or None, **more)
+
+    padded, want = run(proj, live=live)
+    out, state = run(packed.pack(proj), live=live, packed=packed)
+    _alike(packed, out, padded)
+    assert torch.equal(state["ssm"], want["ssm"]) and torch.equal(state["conv"], want["conv"])
+
+
+@pytest.mark.parametrize("lengths", _LENGTHS)
+@pytest.mark.parametrize("segments", [None, (3, 384)])
+def test_linear_attention(lengths, segments):
+    spec = gla_ops.GlaSpec(heads=4, dim=64, vdim=128, rank=16, tau=16.0, q_scale=0.125, eps=1e-6)
+    widths = [("q", 256), ("k", 256), ("v", 512), ("g", 512), ("a1", 16)]
+    cols, at = {}, 0
+    for name, n in widths:
+        cols[name], at = at, at + n
+    packed, live, proj = _packed(lengths, at, 2)
+    a2, bias, norm = (torch.randn(*n, device="cuda") * 0.2 for n in ((256, 16), (256,), (128,)))
+
+    def run(x, **more):
+        state = torch.zeros(len(lengths), 4, 64, 128, device="cuda")
+        return gla_ops._cuda_gla(x, a2.bfloat16(), bias, norm, spec, gla_ops.GlaColumns(**cols), start=None,  # pylint: disable=protected-access
+                                 state=state, segments=segments, **more)
+
+    padded, want = run(proj, live=live)
+    out, state = run(packed.pack(proj), live=live, packed=packed)
+    _alike(packed, out, padded)
+    assert torch.equal(state, want)
+
+
+@pytest.mark.parametrize("lengths", _LENGTHS)
+@pytest.mark.parametrize("dim,window", [(64, 100), (128, 33)])
+def test_window_attention(lengths, dim, window):
+    spec = window_ops.WindowSpec(heads=4, kv_heads=2, dim=dim, vdim=dim, window=window, scale=dim ** -0.5,
+                                 distance_bias=True, gated=True, q_temp=(0.1, 50))
+    cols = window_ops.WindowColumns(q=0, k=4 * dim, v=6 * dim, g=8 * dim)
+    packed, live, proj = _packed(lengths, 12 * dim, 3)
+
+    def run(x, **more):
+        cache = {n: torch.zeros(len(lengths), window, 2, dim, device="cuda", dtype=torch.bfloat16) for n in ("key", "value")}
+        return window_ops.window_attention(x, spec, cols, live=live, cache=cache, **more)
+
+    with torch.no_grad():
+        padded, want = run(proj)
+        out, cache = run(packed.pack(proj), packed=packed)
+    _alike(packed, out, padded)
+    assert torch.equal(cache["key"], want["key"]) and torch.equal(cache["value"], want["value"])
+
+
+@pytest.mark.parametrize("family", ["sagisun", "zukitar"])
+def test_served_prompts(family, monkeypatch):
+    """The engine's logits after ragged prompts and its steps behind them, packed and padded: the same up to products of
+    another number of rows, whose kernels sum in another order."""
+    from perf import cases
+    from axlearn_b200.ops import cuda_ops
+
+    case = dict(kind="serve", family=family, size="1B", layers=2 if family == "sagisun" else 3, batch=5, prompt=1011)
+    used = []
+    plain = packed_ops.pack_prompts
+
+    def pack(*args):
+        used.append(plain(*args))
+        return used[-1]
+
+    monkeypatch.setattr(packed_ops, "pack_prompts", pack)
+    got = cases.run(cases.prepare(case, 5))
+    assert used and all(p is not None and p.rows < 5 * 1011 for p in used)
+    monkeypatch.setattr(packed_ops, "pack_prompts", lambda *args: None)
+    want = cases.run(cases.prepare(case, 5))
+    for a, b in zip([got["prompt_logits"], *got["logits"]], [want["prompt_logits"], *want["logits"]]):
+        assert (a - b).norm() <= 2e-2 * b.norm()
+    cuda_ops.check_status()
+
+
+def test_where_packing_does_not_pay():
+    def pack(lengths, t):
+        return packed_ops.pack_prompts(torch.tensor(lengths, dtype=torch.int32, device="cuda"), t)
+
+    assert pack([4000], 8000) is None and pack([100, 40], 200) is None and pack([4000, 3990], 4000) is None
+    assert pack([4000, 8000], 4000) is None  # more tokens than rows: all of them
+    p = pack([0, 600, 700, -3], 2000)
+    assert p.rows == 1300 and p.first.tolist() == [0, 0, 600, 1300] and p.live.tolist() == [0, 600, 700, 0]
+    x = torch.arange(8000, device="cuda").reshape(4, 2000, 1)
+    y = p.pack(x)
+    assert y.flatten().tolist() == list(range(2000, 2600)) + list(range(4000, 4700))
+    assert torch.equal(p.pack(p.unpack(y)), y)
