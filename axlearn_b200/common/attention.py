@@ -318,8 +318,9 @@ class _FusedQKVProj(DenseGeneralBaseLayer):
             x = coll.tp_enter(x, "model")
         x = ops.share_input_grad(x)      # the three projections sum their input gradients in place
         outs = []
-        for p in range(3):
-            y = self._matmul(x, w[p].reshape(cshape[1], -1).to(x.dtype))
+        # (Unbound: the three gradients are stacked in one pass; of `w[p]` each is a zeroed tensor of all three, added up.)
+        for p, wp in enumerate(w.unbind(0)):
+            y = self._matmul(x, wp.reshape(cshape[1], -1).to(x.dtype))
             y = y.reshape(x.shape[:-1] + (cshape[2], cshape[3]))
             if cfg.bias:
                 y = y + self.parameters["bias"][p].to(y.dtype)
