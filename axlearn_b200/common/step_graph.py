@@ -158,7 +158,9 @@ class StepGraphs:
             return None
         signature = self._signature(trainer, batch)
         if signature is not None and (self._captured is None or self._captured.signature != signature):
-            if signature == self._last and self._captures < _MAX_CAPTURES:
+            device = trainer._device  # pylint: disable=protected-access
+            if signature == self._last and self._captures < _MAX_CAPTURES and (
+                    torch.cuda.mem_get_info(device)[0] > _most_memory(device)):
                 self._captures += 1
                 self._captured = None  # its memory is given back first
                 try:
@@ -201,6 +203,10 @@ def _copy(dst: list, src: list) -> None:
         torch._foreach_copy_(d, s)  # pylint: disable=protected-access
 
 
+def _most_memory(device: torch.device) -> int:
+    return torch.cuda.get_device_properties(device).total_memory // _MEMORY_SHARE
+
+
 def _capture(trainer, batch: Any, signature: tuple) -> _Captured:
     from axlearn_b200.ops import cuda_ops
     from axlearn_b200.parallel import fsdp
@@ -216,23 +222,27 @@ def _capture(trainer, batch: Any, signature: tuple) -> _Captured:
     leaves = tree_map(lambda t: t.detach().requires_grad_(t.requires_grad), shadows)
     reserved = torch.cuda.memory_reserved(device)
     before = cuda_ops.launch_count
-    graph = torch.cuda.CUDAGraph()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device)
+    stream.wait_stream(torch.cuda.current_stream(device))
     try:
         trainer._shadows = leaves  # pylint: disable=protected-access
-        with torch.cuda.graph(graph, capture_error_mode="thread_local"):
-            reserved = min(reserved, torch.cuda.memory_reserved(device))  # (the capture starts with an emptied cache)
-            loss, aux, collected = trainer._forward_backward(static, None)  # pylint: disable=protected-access
-            if any(True for _ in flatten_items(collected.state_updates)):
-                raise Refused("a layer updates its state")
-            with cuda_ops.adamw_scalars(scalars):
-                _, learner_summaries = trainer._apply_update(collected)  # pylint: disable=protected-access
+        # (Not `torch.cuda.graph`, which empties the allocator's cache: what runs next would pay for its memory again.)
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                loss, aux, collected = trainer._forward_backward(static, None)  # pylint: disable=protected-access
+                if any(True for _ in flatten_items(collected.state_updates)):
+                    raise Refused("a layer updates its state")
+                with cuda_ops.adamw_scalars(scalars):
+                    _, learner_summaries = trainer._apply_update(collected)  # pylint: disable=protected-access
+            finally:
+                graph.capture_end()
     finally:
         trainer._shadows = shadows  # pylint: disable=protected-access
         launches, cuda_ops.launch_count = cuda_ops.launch_count - before, before
         for _, leaf in flatten_items(leaves):
             fsdp.reset_grad_slices(leaf)
-    most = torch.cuda.get_device_properties(device).total_memory // _MEMORY_SHARE
-    if torch.cuda.memory_reserved(device) - reserved > most:
+    if torch.cuda.memory_reserved(device) - reserved > _most_memory(device):
         raise Refused("its activations would stay in too much memory")
     outputs = {"loss": loss, "aux": aux, "model": collected.summaries, "learner": learner_summaries}
     results: list = []
