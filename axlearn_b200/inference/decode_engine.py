@@ -327,7 +327,9 @@ class DecodeEngine(BaseDecodeEngine):
                     softmax_scale=self._softmax_scale)
                 branch = self._sum_ranks(self._product(attn.reshape(rows, self.nq_l * h), lw.wo))
                 x, hn = self._add_norm(x, branch, lw.ffn_norm)
-                act = decode_ops.swiglu_packed(self._product(hn, lw.wgu))
+                act = cuda_ops.gemm_swiglu(hn, lw.wgu)
+                if act is None:
+                    act = decode_ops.swiglu_packed(self._product(hn, lw.wgu))
                 branch = self._sum_ranks(self._product(act, lw.wdown))
             if lengths is None:
                 last = (slice(None), -1)

@@ -82,6 +82,8 @@ class _Sigs:
                      c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
     axb_gemm_bf16_2cta = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64,
                           c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
+    axb_gemm_swiglu_2cta = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64, c_void_p, c_int,
+                            c_void_p]
     axb_gemm_splitk_plan = [c_int, c_int, c_int]
     axb_multimem_allreduce = [ctypes.c_uint64, c_int64, c_int, c_int, c_void_p]
     axb_chain_launches = [c_int]
@@ -281,6 +283,25 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out: Optional[torch.Tensor] = None
                              a_mn, b_mn, 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0,
                              status_word(a.device).data_ptr(), max_ctas, _stream())
     _check(rc, "axb_gemm_bf16")
+    return out
+
+
+def gemm_swiglu(a: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """``silu(a @ w[:, :F]) * (a @ w[:, F:])`` of ``w [K, 2F]`` without writing the product, with the bits of ``gemm`` and a
+    pass over its result; None for what the kernel on CTA pairs does not take (few rows, other layouts)."""
+    m, k = a.shape
+    f = w.shape[1] // 2
+    if not (GEMM_VARIANT == "2cta" and m >= 512 and f % 8 == 0 and w.shape[1] == 2 * f >= 256 and w.shape[0] == k
+            and a.dtype == w.dtype == torch.bfloat16 and ((m + 255) // 256) * ((2 * f + 255) // 256) >= 64
+            and a.is_contiguous() and w.is_contiguous() and k % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0):
+        return None
+    out = torch.empty((m, f), dtype=torch.bfloat16, device=a.device)
+    rc = lib().axb_gemm_swiglu_2cta(
+        a.data_ptr(), w.data_ptr(), out.data_ptr(), m, f, k, k, 2 * f, f, status_word(a.device).data_ptr(),
+        max(8, _sm_count(a.device) - COMM_RESERVED_SMS) if COMM_RESERVED_SMS else 0, _stream())
+    if rc == -20:
+        return None
+    _check(rc, "axb_gemm_swiglu_2cta")
     return out
 
 

@@ -213,6 +213,26 @@ def test_accumulate_reads_c_by_vectors(m, n, dtype):
     cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("m,f,k", [(512, 4096, 64), (513, 4232, 136), (2304, 1096, 512), (4096, 504, 64), (8192, 136, 328),
+                                   (700, 11008, 1024)])
+def test_product_with_swiglu_epilogue(m, f, k):
+    """The bits of the product and the pass over it, at row, column and K remainders (columns of the other half read
+    beyond a tile's last one are not stored)."""
+    from axlearn_b200.ops import cuda_ops, decode_ops
+
+    g = torch.Generator(device="cuda").manual_seed(m + f)
+    a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(k, 2 * f, device="cuda", generator=g) * 2 * k ** -0.5).bfloat16()
+    out = cuda_ops.gemm_swiglu(a, w)
+    assert out is not None and torch.equal(out, decode_ops.swiglu_packed(cuda_ops.gemm(a, w)))
+    w[0, 3], w[0, f + 5] = float("inf"), float("nan")
+    a[:, 0] = a[:, 0].abs() + 0.5
+    want = decode_ops.swiglu_packed(cuda_ops.gemm(a, w))
+    torch.testing.assert_close(cuda_ops.gemm_swiglu(a, w), want, rtol=0, atol=0, equal_nan=True)
+    assert cuda_ops.gemm_swiglu(a[:100], w) is None and cuda_ops.gemm_swiglu(a.t().contiguous().t(), w) is None
+    cuda_ops.check_status()
+
+
 def _close_elementwise(out, ref, atol, rtol):
     """Per-element ``|out - ref| <= atol + rtol * |ref|`` (an error confined to small outputs or one
     tile edge cannot hide behind the largest value)."""
