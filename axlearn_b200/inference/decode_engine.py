@@ -9,7 +9,8 @@ persistent buffers, so the engine:
 * keeps per-layer K/V page pools ``[num_pages, page_size, Nkv_local, H]`` resident and appends in
   place (``rope_append_paged`` writes the rotated key / value of the new token straight into
   its page slot while producing the rotated query);
-* runs attention over the pages with the split-KV decode kernel (``paged_decode_attention``);
+* runs attention over the pages with the split-KV decode kernel, which does the append as well
+  (``rope_decode_attention``);
 * packs the projections so that a layer is four GEMMs on the tcgen05 kernel (QKV, output,
   gate|up, down); the residual adds are the GEMMs' accumulate epilogues on one GPU;
 * under tensor parallelism (heads and FFN columns split over the ``model`` group) fuses the two
@@ -368,12 +369,9 @@ class DecodeEngine(BaseDecodeEngine):
         for li, lw in enumerate(self.w["layers"]):
             hn = cuda_ops.rms_norm(x, lw.attn_norm, d.norm_eps)
             qkv = cuda_ops.gemm(hn, lw.wqkv, resident=True)
-            q = decode_ops.rope_append_paged(
-                qkv, self.k_pools[li], self.v_pools[li], self.page_table, self.lengths,
-                num_q_heads=self.nq_l, theta=d.rope_theta)
-            attn = decode_ops.paged_decode_attention(
-                q, self.k_pools[li], self.v_pools[li], self.page_table, self.lengths,
-                softmax_scale=self._softmax_scale, splits=self.splits, scratch=self._scratch)
+            attn = decode_ops.rope_decode_attention(
+                qkv, self.k_pools[li], self.v_pools[li], self.page_table, self.lengths, num_q_heads=self.nq_l,
+                theta=d.rope_theta, softmax_scale=self._softmax_scale, splits=self.splits, scratch=self._scratch)
             attn2 = attn.reshape(self.batch, self.nq_l * d.head_dim)
             if self.world > 1:
                 x = self._gemm_reduce(attn2, lw.wo, x, 2 * li)

@@ -34,6 +34,8 @@ def _lib():
         h.axb_decode_attn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                       c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]
         h.axb_decode_attn.restype = c_int
+        h.axb_rope_decode_attn.argtypes = [c_void_p] * 7 + [c_int] * 7 + [c_float, c_float, c_void_p]
+        h.axb_rope_decode_attn.restype = c_int
         h.axb_rope_append_paged.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                             c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p]
         h.axb_rope_append_paged.restype = c_int
@@ -161,6 +163,27 @@ def rope_append_paged(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Ten
                                       cuda_ops._stream())  # pylint: disable=protected-access
     cuda_ops._check(rc, "axb_rope_append_paged")  # pylint: disable=protected-access
     return q_out
+
+
+def rope_decode_attention(qkv: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, page_table: torch.Tensor,
+                          lengths: torch.Tensor, *, num_q_heads: int, theta: float, softmax_scale: float, splits: int,
+                          scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``rope_append_paged`` and ``paged_decode_attention`` of its queries in one launch: ``[B, Nq, H]``."""
+    b = qkv.shape[0]
+    _, page_size, nkv, h = k_pool.shape
+    assert qkv.is_contiguous() and qkv.shape[1] == (num_q_heads + 2 * nkv) * h and qkv.data_ptr() % 16 == 0
+    assert k_pool.is_contiguous() and v_pool.is_contiguous() and page_table.is_contiguous()
+    assert page_table.dtype == torch.int32 and lengths.dtype == torch.int32
+    out = torch.empty((b, num_q_heads, h), dtype=qkv.dtype, device=qkv.device)
+    if scratch is None:
+        floats = _lib().axb_decode_attn_scratch_floats(b, num_q_heads, splits)
+        scratch = torch.empty(floats, dtype=torch.float32, device=qkv.device) if floats else None
+    rc = _lib().axb_rope_decode_attn(qkv.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), page_table.data_ptr(),
+                                     lengths.data_ptr(), out.data_ptr(), None if scratch is None else scratch.data_ptr(),
+                                     b, num_q_heads, nkv, h, page_size, page_table.shape[1], splits, theta, softmax_scale,
+                                     cuda_ops._stream())  # pylint: disable=protected-access
+    cuda_ops._check(rc, "axb_rope_decode_attn")  # pylint: disable=protected-access
+    return out
 
 
 def rope_table(length: int, dim: int, theta: float, device) -> torch.Tensor:

@@ -324,6 +324,27 @@ def test_rope_append_writes_page_slot_and_rotates():
     assert torch.equal(k, k0) and torch.equal(v, v0)
 
 
+@pytest.mark.parametrize("nq,nkv", [(3, 3), (4, 2), (12, 4), (16, 2), (12, 1), (20, 2)])
+@pytest.mark.parametrize("page_size,splits", [(4, 1), (12, 2), (16, 5), (16, 8), (20, 9)])
+def test_rope_decode_attention_equals_append_and_attention(nq, nkv, page_size, splits):
+    """Bit for bit, attention and pools: new tokens at the edges of tiles, pages, warps' strides and splits, alone in their
+    tile or not, up to eight and more than eight query heads per KV head."""
+    from axlearn_b200.ops import decode_ops
+
+    lens = [1, 2, 15, 16, 17, 33, 63, 64, 65, 129, 224, 240]
+    b, max_pages, h = len(lens), 240 // page_size, 128
+    k, v, table = _pools(b, max_pages, page_size, nkv, h, seed=splits)
+    lengths = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(nq)
+    qkv = (2 * torch.randn(b, (nq + 2 * nkv) * h, device="cuda", generator=g)).bfloat16()
+    k1, v1 = k.clone(), v.clone()
+    q = decode_ops.rope_append_paged(qkv, k1, v1, table, lengths, num_q_heads=nq, theta=1e4)
+    want = decode_ops.paged_decode_attention(q, k1, v1, table, lengths, splits=splits)
+    out = decode_ops.rope_decode_attention(qkv, k, v, table, lengths, num_q_heads=nq, theta=1e4, softmax_scale=h ** -0.5,
+                                           splits=splits)
+    assert torch.equal(out, want) and torch.equal(k, k1) and torch.equal(v, v1)
+
+
 @pytest.mark.parametrize("b,t,nq,nkv", [(1, 1, 4, 4), (2, 127, 6, 2), (3, 129, 16, 1), (1, 300, 40, 8)])
 def test_prompt_attention_equals_rotation_copies_and_attention(b, t, nq, nkv):
     """Bit for bit what separate rotations, copies into the cache and attention on contiguous tensors give; rows of the
