@@ -29,6 +29,7 @@ from axlearn_b200.common.config import (
 from axlearn_b200.common.embedding import BaseEmbedding, TransformerTextEmbeddings
 from axlearn_b200.common.layers import Dropout, LayerNorm, set_dropout_rate_recursively
 from axlearn_b200.common.module import Module, child_context, nowrap
+from axlearn_b200.ops import step_ops
 from axlearn_b200.parallel import collectives as coll
 
 Tensor = torch.Tensor
@@ -189,6 +190,12 @@ class Decoder(BaseLayer):
         h = self.output_dropout(h)
         return states, {"hidden_states": h}
 
+    @nowrap
+    def _reads_positions(self) -> bool:
+        """Whether an ``extend_step`` looks at the tokens' positions outside the layers, which know their own."""
+        emb = self._children["emb"]
+        return "attention_mask" in self._children or type(emb) is not TransformerTextEmbeddings or "pos_emb" in emb.children
+
     def _attention_mask_biases(self, *, mode, input_ids, positions, segment_ids, cached_states, max_len):
         """Biases of the configured ``attention_mask`` layer (e.g. ALiBi).  Training and prefill see
         the ``[T, T]`` bias of the given tokens; a decoding step sees its rows of the bias over the
@@ -277,16 +284,18 @@ class Decoder(BaseLayer):
         (stacks that support it; None: all)."""
         time_step = cached_states["time_step"]
         steps = input_ids.shape[1]
-        # (One token, the decoding step: a launch less.)
-        positions = (time_step[:, None].long() if steps == 1
-                     else time_step[:, None] + torch.arange(steps, device=input_ids.device)[None])
+        input_batch = {"input_ids": input_ids}
+        if self._reads_positions():
+            # (One token, the decoding step: a launch less.)
+            input_batch["positions"] = (time_step[:, None].long() if steps == 1
+                                        else time_step[:, None] + torch.arange(steps, device=input_ids.device)[None])
         states, out = self._forward_for_mode(
             mode=ForwardMode.EXTEND_STEP,
-            input_batch={"input_ids": input_ids, "positions": positions},
+            input_batch=input_batch,
             cached_states=cached_states, cross_attention_data=cross_attention_data,
             cross_attention_logit_biases=cross_attention_logit_biases, page_pool=page_pool,
             live_step_len=live_step_len)
-        states["time_step"] = time_step + (steps if live_step_len is None else live_step_len)
+        states["time_step"] = step_ops.advance(time_step, steps if live_step_len is None else live_step_len)
         out["logits"] = self.compute_logits(out)
         return states, out
 

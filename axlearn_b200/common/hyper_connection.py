@@ -277,7 +277,7 @@ class HyperStackedTransformerLayer(BaseStackedTransformerLayer):
             raise NotImplementedError(f"unsupported arguments: page_pool, {sorted(kwargs)}")
         start = cached_states["time_step"]
         new, out = self._run(data, start=start, live=live_step_len, states=cached_states)
-        new["time_step"] = start + (data.shape[1] if live_step_len is None else live_step_len)
+        new["time_step"] = step_ops.advance(start, data.shape[1] if live_step_len is None else live_step_len)
         return new, out
 
 

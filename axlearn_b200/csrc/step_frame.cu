@@ -116,6 +116,13 @@ embed_rows_kernel(const uint4* __restrict__ table, const int64_t* ids, uint4* ou
   }
 }
 
+// out = counts + by.  A chained launch of its own only so that the chain does not end: the output product behind it starts its
+// weights while the last layer still runs.
+__global__ void __launch_bounds__(256) add_counts_kernel(const int* counts, const int* by, int* out, int n) {
+  chain_link();
+  for (int i = threadIdx.x; i < n; i += 256) out[i] = counts[i] + by[i];
+}
+
 // Tokens that a caller hands to a step, one CTA; ids outside [low, high) become 0, and `ok` tells whether there were none.
 __global__ void __launch_bounds__(256)
 take_tokens_kernel(const int64_t* ids, int64_t* tokens, int count, int64_t low, int64_t high, bool* ok) {
@@ -138,6 +145,14 @@ extern "C" int axb_take_tokens(const int64_t* ids, int64_t* tokens, int count, i
                                cudaStream_t stream) {
   if (count <= 0) return 0;
   axb::take_tokens_kernel<<<1, 256, 0, stream>>>(ids, tokens, count, low, high, ok);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+// out [n] = counts + by, a handful of numbers; chained like a step's other kernels.
+extern "C" int axb_add_counts(const int* counts, const int* by, int* out, int n, cudaStream_t stream) {
+  using namespace axb;
+  if (n <= 0) return 0;
+  launch_chained(add_counts_kernel, 1, 256, 0, stream, counts, by, out, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -284,6 +284,24 @@ def test_step_end_picks_as_torch_and_keeps(b, v, ld):
     assert torch.equal(lengths, want_lengths) and all(torch.equal(x, y) for x, y in kept)
 
 
+@pytest.mark.parametrize("b", [1, 3, 256, 300])
+def test_advance_in_a_captured_chain(b):
+    from axlearn_b200.ops import cuda_ops, step_ops
+
+    counts = torch.arange(b, dtype=torch.int32, device="cuda")
+    by = torch.arange(b, dtype=torch.int32, device="cuda") % 2
+    assert torch.equal(step_ops.advance(counts, by), counts + by) and torch.equal(step_ops.advance(counts, 2), counts + 2)
+    graph = torch.cuda.CUDAGraph()
+    before = cuda_ops.launch_count
+    with torch.cuda.graph(graph), cuda_ops.chained_launches():
+        out = step_ops.advance(step_ops.advance(counts, by), by)
+        plain = step_ops.advance(counts, 2)
+    assert cuda_ops.launch_count == before + 2
+    counts += 5
+    graph.replay()
+    assert torch.equal(out, counts + 2 * by) and torch.equal(plain, counts + 2)
+
+
 @pytest.mark.parametrize("width", [8, 264, 2048, 4104])
 def test_embed_rows_gathers_and_marks_bad_ids(width):
     from axlearn_b200.ops import cuda_ops, step_ops
