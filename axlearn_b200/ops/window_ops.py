@@ -159,6 +159,8 @@ class _Args(ctypes.Structure):
 
 _signatures_set = False
 _tickets: dict = {}
+# Up to this many splits of a decoding step meet in a thread-block cluster; more meet in memory, by tickets.
+CLUSTER_SPLITS = 8
 # Below this many new tokens per sequence the tensor-core kernel's 128-row tiles are mostly padding.
 FLASH_MIN_TOKENS = 32
 
@@ -201,8 +203,17 @@ def _ticket_buffer(device: torch.device, n: int) -> Tensor:
 
 
 def decode_splits(ctas: int, span: int, sms: int = 148) -> int:
-    """KV splits of a decoding step: one wave of two CTAs per SM, at least 64 keys each."""
+    """KV splits of a decoding step: one wave of two CTAs per SM at most.
+
+    Up to 1024 keys the splits of one cluster, of 24 keys or more: 32 keys take as long as the cluster's meeting (16 heads
+    on 4 of 128, us a launch, one split / 3 by tickets / 8 in a cluster: 210 keys 11.6 / 10.9 / 6.5, and 16 by tickets / 8 in
+    a cluster: 1024 keys 11.0 / 10.5).  Longer windows want more CTAs than a cluster has (32 heads on 8, 2048 keys: 32 splits
+    13.5, 8 in a cluster 18.7), of 64 keys or more."""
     want = max(1, (2 * sms) // max(1, ctas))
+    if span < 128:
+        return 1
+    if span <= 1024:
+        return min(want, CLUSTER_SPLITS, span // 24)
     return max(1, min(want, span // 64, 64))
 
 
@@ -249,7 +260,7 @@ def _cuda_window_attention(proj, spec, cols, *, start, live, cache, packed: Opti
         ctas = lib.axb_window_decode_ctas(b, spec.heads, spec.kv_heads, spec.dim, spec.vdim)
         a.splits = decode_splits(ctas, min(spec.window, a.slots))
         part = None
-        if a.splits > 1:
+        if a.splits > CLUSTER_SPLITS:
             part = torch.empty(b * spec.heads * a.splits * padded(spec.vdim + 2, 4), dtype=torch.float32, device=proj.device)
             a.part, a.tickets = part.data_ptr(), _ticket_buffer(proj.device, ctas).data_ptr()
         check(lib.axb_window_decode(ctypes.byref(a), stream), "axb_window_decode")

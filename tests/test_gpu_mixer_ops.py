@@ -199,6 +199,35 @@ def test_window_long_decode_splits(dtype):
     assert torch.equal(cache["key"].cpu(), ref["key"]) and torch.equal(cache["value"].cpu(), ref["value"])
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("sizes", [(4, 1, 128, 128), (3, 1, 40, 72), (4, 2, 300, 260), (2, 2, 16, 500)])
+@pytest.mark.parametrize("splits", [2, 3, 7, 8, 9])
+def test_window_decode_splits_meet(dtype, sizes, splits, monkeypatch):
+    """Splits that meet in a cluster (up to 8) or by tickets: sequences with fewer keys than splits, a wrapped ring, columns
+    that do not divide by the splits, a row out of the step.
+
+    In 32 bits a result is a mean of values of at most 5 with weights off by the roundings of scores below 64 (2^-18 each, the
+    last bits of 500 products) and of sums: 2e-4.  In 16 bits the output's rounding (2^-8 of it) comes on top."""
+    heads, kv, dim, vdim = sizes
+    monkeypatch.setattr(window_ops, "decode_splits", lambda *_: splits)
+    window, b = 100, 5
+    spec = window_ops.WindowSpec(heads, kv, dim, vdim, window, scale=dim ** -0.5, q_temp=(0.5, 10), distance_bias=True)
+    proj, cols = _window_case(dtype, heads, kv, dim, vdim, b, 1, seed=splits)
+    start = torch.tensor([0, 4, 99, 350, 1000], dtype=torch.int32)
+    live = torch.tensor([1, 1, 1, 1, 0], dtype=torch.int32)
+    g = torch.Generator().manual_seed(dim)
+    key, value = torch.randn(b, window, kv, dim, generator=g).to(dtype), torch.randn(b, window, kv, vdim, generator=g).to(dtype)
+    got, cache = window_ops.window_attention(
+        proj.cuda(), spec, cols, start=start.cuda(), live=live.cuda(), cache={"key": key.cuda(), "value": value.cuda()})
+    with dispatch.use_reference_ops():
+        want, ref = window_ops.window_attention(proj, spec, cols, start=start, live=live, cache={"key": key, "value": value})
+    want = want[:4].double()
+    err = (got[:4].cpu().double() - want).abs()
+    assert (err <= 2e-4 + (2 ** -7 if dtype == torch.bfloat16 else 0) * want.abs()).all(), err.max()
+    assert (got[4] == 0).all()
+    assert torch.equal(cache["key"].cpu(), ref["key"]) and torch.equal(cache["value"].cpu(), ref["value"])
+
+
 # ------------------------------------------------------------------------------ linear attention
 def _gla_case(dtype, heads, dim, vdim, rank, b, t, seed=0, z_scale=1.0, z_bias=1.5):
     g = torch.Generator().manual_seed(seed)
