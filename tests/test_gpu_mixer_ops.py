@@ -49,6 +49,33 @@ def test_hyper_step(dtype, rows, width, streams, pair):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [4, 60, 2044, 2048, 2052, 4096, 4100])
+@pytest.mark.parametrize("streams,pair", [(1, False), (4, True), (3, False)])
+def test_hyper_step_of_few_rows_equals_many(dtype, width, streams, pair):
+    """A decoding step's rows (one or two vectors a thread, or more) against the same rows among many.
+
+    Both kernels do the same sums of at most 10 terms per element, in one order, and differ in how the squares of a row are
+    added: n <= 4100 roundings of 2^-24 of sums of like sign, halved by the root: 2^-13 of an output is a bound many times
+    over; a 16-bit output may then round the other way (2^-8 of it)."""
+    g = torch.Generator().manual_seed(width)
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    ld, rows = hyper_ops.padded(width, 32), 600
+    x, a, b = rnd(1, rows, streams, width), rnd(1, rows, ld).to(dtype), rnd(1, rows, ld).to(dtype)
+    sa, sb, mix, out, read, norm = rnd(width), rnd(width), rnd(streams, streams), rnd(streams), rnd(streams), rnd(width)
+
+    def step(n):
+        branch = hyper_ops.NormedPair(a[:, :n], b[:, :n], sa, sb, 1e-5) if pair else a[:, :n]
+        return hyper_ops.hyper_step(x[:, :n], branch, write=hyper_ops.StreamWrite(mix, out, 0.7), read=read, norm_scale=norm,
+                                    eps=1e-5, norm_offset=1.0, num_streams=streams, dtype=dtype)
+
+    few, many = step(3), step(rows)
+    scale = x.abs().max().item() * mix.abs().sum(0).max().item() + 1.4 * a.float().abs().max().item() * (width ** 0.5 if pair else 1)
+    assert (few[0] - many[0][:, :3]).abs().max().item() <= 2 ** -13 * scale
+    got, want = few[1].float(), many[1][:, :3].float()
+    assert ((got - want).abs() <= (2 ** -13 + (2 ** -8 if dtype == torch.bfloat16 else 0)) * want.abs() + 2 ** -13 * scale).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_hyper_first_read_and_last_sum(dtype):
     x = torch.randn(2, 3, 40).to(dtype)
     read, norm = torch.randn(3), torch.randn(40)
