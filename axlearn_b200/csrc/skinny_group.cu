@@ -53,6 +53,25 @@ __device__ __forceinline__ uint4 ldg_stream(const __nv_bfloat16* p) {
 
 constexpr int kSkWarps = 4, kSkThreads = 32 * kSkWarps;
 
+// The group with rows that `want` groups with rows precede, and its rows: all lanes of a warp.  False: there is none.
+__device__ __forceinline__ bool group_with_rows(const SkinnyArgs& a, int want, int& g, int& lo, int& hi) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < a.groups; base += 32) {
+    const int i = min(base + lane, a.groups - 1);
+    const int from = a.offsets[i], to = a.offsets[i + 1];
+    const uint32_t full = __ballot_sync(0xffffffffu, base + lane < a.groups && to > from);
+    const uint32_t it = __ballot_sync(0xffffffffu, (full >> lane & 1) && __popc(full & ((1u << lane) - 1)) == want);
+    if (it != 0) {
+      const int at = __ffs(it) - 1;
+      g = base + at;
+      lo = __shfl_sync(0xffffffffu, from, at), hi = __shfl_sync(0xffffffffu, to, at);
+      return true;
+    }
+    want -= __popc(full);
+  }
+  return false;
+}
+
 }  // namespace
 
 // RT tiles of 8 rows per pass; kGate: two weight rows per result.
@@ -61,10 +80,15 @@ __global__ void __launch_bounds__(kSkThreads) skinny_mma_kernel(SkinnyArgs a) {
   using bf16 = __nv_bfloat16;
   constexpr int G = kGate ? 2 : 1;
   __shared__ float red[kSkWarps][G][16][RT * 8 + 1];
-  const int n0 = blockIdx.x * 16, g = blockIdx.y;
+  const int n0 = blockIdx.x * 16;
+  int g = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lq = lane & 3;
   int lo = 0, hi = a.rows;
-  if (a.offsets != nullptr) lo = a.offsets[g], hi = a.offsets[g + 1];
+  if (gridDim.y < a.groups) {
+    if (!group_with_rows(a, g, g, lo, hi)) return;
+  } else if (a.offsets != nullptr) {
+    lo = a.offsets[g], hi = a.offsets[g + 1];
+  }
   lo += blockIdx.z * RT * 8;
   if (lo >= hi) return;
   const bf16* w = static_cast<const bf16*>(a.w) + g * a.w_group;
@@ -174,7 +198,11 @@ __global__ void __launch_bounds__(256) skinny_plain_kernel(SkinnyArgs a) {
 
 template <int RT>
 static int launch_skinny(const SkinnyArgs& a, int passes, cudaStream_t stream) {
-  const dim3 grid((a.n + 15) / 16, a.groups, passes);
+  // Fewer rows than groups: as many groups as can have rows.  CTAs of empty groups cost the full ones their places on the
+  // SMs: a feed-forward of one token over 4 of
+  // 32 experts of 2048 x 1408 33.7 -> 32.3 us, over 8 of 128 52.5 -> 41.9.
+  const int groups = a.offsets != nullptr && a.rows < a.groups ? a.rows : a.groups;
+  const dim3 grid((a.n + 15) / 16, groups, passes);
   if (a.gate_kind >= 0)
     skinny_mma_kernel<RT, true><<<grid, kSkThreads, 0, stream>>>(a);
   else
