@@ -317,6 +317,13 @@ def test_gla_prompt_then_single_tokens(dtype, sizes, tau, z_bias):
             _close(state[r], states[r], 1e-4)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("sizes", [(1, 9, 258, 3), (1, 70, 1100, 16), (2, 300, 32, 17)])
+def test_gla_decode_beyond_what_it_asks_for_at_the_start(dtype, sizes):
+    """More value columns, key channels or gate inputs than a CTA has threads or registers for."""
+    test_gla_prompt_then_single_tokens(dtype, sizes, 16.0, 1.5)
+
+
 @pytest.mark.parametrize("sizes", [(2, 64, 64, 16), (2, 128, 128, 16), (2, 40, 256, 16)])
 @pytest.mark.parametrize("tau", [16.0, 0.5])
 def test_gla_segments_and_portions_agree(sizes, tau):
