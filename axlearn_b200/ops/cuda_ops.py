@@ -111,8 +111,8 @@ class _Sigs:
     axb_embedding_bwd = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
     axb_embedding_bwd_bytes = [c_int, c_int, c_int]
     axb_scale_bf16 = [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]
-    axb_sumsq_ctas = []
-    axb_sumsq = [c_void_p, c_int, c_int64, c_void_p, c_void_p, c_float, c_int, c_void_p]
+    axb_sumsq_ctas = [c_int]
+    axb_sumsq = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p]
 
 
 # Names that torch does not promise, with the public or the safe way behind them.
@@ -812,18 +812,16 @@ def multi_tensor_adamw(params, grads, mus, nus, shadows, wd_scales, *, step: int
 
 def sum_of_squares(tensors: Sequence[torch.Tensor], weights: Optional[Sequence[float]] = None) -> torch.Tensor:
     """Deterministic ``sum_i w_i * ||t_i||^2`` as a 0-d fp32 device tensor."""
-    dev = tensors[0].device
+    dev, count = tensors[0].device, len(tensors)
     h = lib()
-    out = torch.zeros(1, dtype=torch.float32, device=dev)
-    partial = torch.empty(h.axb_sumsq_ctas(), dtype=torch.float32, device=dev)
-    stream = _stream()
-    for i, t in enumerate(tensors):
-        if t.dtype not in (torch.bfloat16, torch.float32):
-            t = t.float()
-        t = t.contiguous()
-        w = 1.0 if weights is None else float(weights[i])
-        _check(h.axb_sumsq(t.data_ptr(), 1 if t.dtype == torch.bfloat16 else 0, t.numel(), partial.data_ptr(),
-                           out.data_ptr(), w, 1, stream), "axb_sumsq")
+    out = torch.empty(1, dtype=torch.float32, device=dev)
+    partial = torch.empty(h.axb_sumsq_ctas(count), dtype=torch.float32, device=dev)
+    flat = [(t if t.dtype in (torch.bfloat16, torch.float32) else t.float()).contiguous() for t in tensors]
+    _check(h.axb_sumsq((ctypes.c_void_p * count)(*(t.data_ptr() for t in flat)),
+                       (ctypes.c_int64 * count)(*(t.numel() for t in flat)),
+                       (c_int * count)(*(int(t.dtype == torch.bfloat16) for t in flat)),
+                       (ctypes.c_float * count)(*([1.0] * count if weights is None else map(float, weights))), count,
+                       partial.data_ptr(), out.data_ptr(), _stream()), "axb_sumsq")
     return out[0]
 
 

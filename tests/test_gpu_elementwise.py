@@ -182,6 +182,27 @@ def test_adamw_and_sumsq():
     assert ss.item() == cuda_ops.sum_of_squares([g, p], [1.0, 0.5]).item()
 
 
+@pytest.mark.parametrize("sizes", [[1], [0, 3], [4095, 4096, 4097], [7] * 65 + [0], [9_700_001, 5, 123], list(range(130))])
+def test_sum_of_squares_of_many_tensors(sizes):
+    """Chunks and their remainders, views off the 16-byte grid, empty tensors, more tensors than one launch takes.
+
+    A thread adds at most 442 squares in a row and a dozen sums follow: 2^-14 of a sum of positive terms is a bound."""
+    from axlearn_b200.ops import cuda_ops
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    tensors = [torch.randn(n + 1, device="cuda", generator=g).to([torch.float32, torch.bfloat16, torch.float16][i % 3])[i % 2:][:n]
+               for i, n in enumerate(sizes)]
+    weights = [1.0 + 0.25 * (i % 3) for i in range(len(sizes))]
+    want = sum(w * t.double().square().sum().item() for w, t in zip(weights, tensors))
+    got = cuda_ops.sum_of_squares(tensors, weights)
+    assert got.dtype == torch.float32 and got.shape == ()
+    assert abs(got.item() - want) <= 2 ** -14 * want
+    bad = [t.clone() for t in tensors]
+    if bad[-1].numel():
+        bad[-1][-1] = float("inf")
+        assert cuda_ops.sum_of_squares(bad, weights).item() == float("inf")
+
+
 @pytest.mark.parametrize("v,d,n", [(1, 8, 1), (7, 264, 5), (5000, 2056, 333), (4100, 512, 20000)])
 def test_embedding_gradient(v, d, n):
     """Rows nobody uses, short lists, rows above 32 tokens (walked in order), more columns than a block takes at once; the
