@@ -297,9 +297,14 @@ __global__ void __launch_bounds__(256) ssd_norm_kernel(SsdArgs a) {
   }
 }
 
-constexpr int kSdThreads = 256;
+constexpr int kSdThreads = 256, kSdTaps = 4;
 
 // V = 4: vdim is a multiple of 4; V = 1: any vdim.
+//
+// The state's first rows and the head's scalars are asked for ahead of everything else, and a channel's inputs and weights of
+// up to kSdTaps taps together: the trips to memory one after the other are what bounds a small batch.  With the norm behind
+// it, a chain of launches over different states, us, taps one by one / this: 64 heads of 64, state 128, batch 1 7.8 / 6.7,
+// 4 11.9 / 10.5, 16 25.1 / 21.9 (34 MB read and written: 10.2 at the copy rate), 64 76.9 / 68.8.
 template <typename T, int V>
 __global__ void __launch_bounds__(kSdThreads, 4) ssd_decode_kernel(SsdArgs a) {
   chain_link();
@@ -307,10 +312,7 @@ __global__ void __launch_bounds__(kSdThreads, 4) ssd_decode_kernel(SsdArgs a) {
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int P = a.vdim, N = a.state, inner = a.heads * P, channels = ssd_channels(a);
   T* yout = static_cast<T*>(a.y) + static_cast<int64_t>(b) * inner + h * P;
-  if (ssd_inactive(a, b)) {
-    for (int c = tid; c < P; c += kSdThreads) yout[c] = T(0.f);
-    return;
-  }
+  const int pos = a.start[b], alive = a.live != nullptr ? a.live[b] : 1;
   const int nc = (P + V - 1) / V;
   const int cols = min(nc, kSdThreads), groups = kSdThreads / cols, rg = tid / cols;
   float* S = a.ssm + (static_cast<int64_t>(b) * a.heads + h) * N * P;
@@ -331,18 +333,47 @@ __global__ void __launch_bounds__(kSdThreads, 4) ssd_decode_kernel(SsdArgs a) {
   float* s_c = s_b + N;   // [N]
   float* s_o = s_c + N;   // [row groups][P]
   const T* row = static_cast<const T*>(a.proj) + static_cast<int64_t>(b) * a.ld;
-  const int pos = a.start[b], here = pos % a.taps, group = h / (a.heads / a.groups);
+  const float dt_in = sf(row[a.dt_off + h]), dt_bias = a.dt_bias[h], a_log = a.a_log[h];
+  __shared__ float s_skip;
+  if (tid == kSdThreads - 1) s_skip = a.d[h];
+  const int group = h / (a.heads / a.groups);
+  auto channel = [&](int i) {
+    return i < P ? h * P + i : (i < P + N ? inner + group * N + i - P : inner + a.groups * N + group * N + i - P - N);
+  };
+  if (pos < 0 || alive <= 0) {  // row not in this step
+    for (int c = tid; c < P; c += kSdThreads) yout[c] = T(0.f);
+    return;
+  }
+  const int here = pos % a.taps;
   const bool owns_bc = h % (a.heads / a.groups) == 0;
   T* ring = static_cast<T*>(a.ring) + static_cast<int64_t>(b) * a.taps * channels;
-  const float dt = softplus_f(sf(row[a.dt_off + h]) + a.dt_bias[h]);
-  const float decay = expf(-expf(a.a_log[h]) * dt);
+  const float dt = softplus_f(dt_in + dt_bias);
+  const float decay = expf(-expf(a_log) * dt);
   for (int i = tid; i < P + 2 * N; i += kSdThreads) {
-    const int c = i < P ? h * P + i : (i < P + N ? inner + group * N + i - P : inner + a.groups * N + group * N + i - P - N);
+    const int c = channel(i);
     const T cur = row[a.xbc_off + c];
-    float acc = a.conv_b[c] + a.conv_w[static_cast<int64_t>(a.taps - 1) * channels + c] * sf(cur);
-    for (int j = 1, slot = here; j < a.taps && j <= pos; ++j) {
-      slot = slot == 0 ? a.taps - 1 : slot - 1;
-      acc += a.conv_w[static_cast<int64_t>(a.taps - 1 - j) * channels + c] * sf(ring[static_cast<int64_t>(slot) * channels + c]);
+    float acc = a.conv_b[c];
+    if (a.taps <= kSdTaps) {  // a channel's inputs and weights in one trip
+      float w[kSdTaps], x[kSdTaps];
+#pragma unroll
+      for (int j = 0, slot = here; j < kSdTaps; ++j) {
+        w[j] = x[j] = 0.f;
+        if (j < a.taps) w[j] = a.conv_w[static_cast<int64_t>(a.taps - 1 - j) * channels + c];
+        if (j > 0 && j < a.taps && j <= pos) {
+          slot = slot == 0 ? a.taps - 1 : slot - 1;
+          x[j] = sf(ring[static_cast<int64_t>(slot) * channels + c]);
+        }
+      }
+      acc += w[0] * sf(cur);
+#pragma unroll
+      for (int j = 1; j < kSdTaps; ++j)
+        if (j < a.taps && j <= pos) acc += w[j] * x[j];
+    } else {
+      acc += a.conv_w[static_cast<int64_t>(a.taps - 1) * channels + c] * sf(cur);
+      for (int j = 1, slot = here; j < a.taps && j <= pos; ++j) {
+        slot = slot == 0 ? a.taps - 1 : slot - 1;
+        acc += a.conv_w[static_cast<int64_t>(a.taps - 1 - j) * channels + c] * sf(ring[static_cast<int64_t>(slot) * channels + c]);
+      }
     }
     if (i < P || owns_bc) ring[static_cast<int64_t>(here) * channels + c] = cur;
     acc = silu_t(acc, T(0.f));
@@ -388,7 +419,7 @@ __global__ void __launch_bounds__(kSdThreads, 4) ssd_decode_kernel(SsdArgs a) {
   }
   __syncthreads();
   for (int p = tid; p < P; p += kSdThreads) {
-    float y = a.d[h] * s_x[p];
+    float y = s_skip * s_x[p];
     for (int g = 0; g < groups; ++g) y += s_o[g * P + p];
     yout[p] = T(y);
   }
