@@ -229,7 +229,6 @@ __global__ void __launch_bounds__(max_threads(S)) hyper_step_kernel(HyperArgs a)
 //   In a decoding step the weights come from HBM: Sagisun, 1B widths, batch 1, 16 steps and a prompt 3045 -> 2979.
 template <typename TS, typename T, int S, int V, int C>
 __global__ void __launch_bounds__(max_threads(S)) hyper_row_kernel(HyperArgs a) {
-  static_assert(S > 0, "");
   chain_link();
   __shared__ float2 scratch[32];
   __shared__ float s_mix[S * S], s_out[S], s_read[S];
@@ -355,8 +354,10 @@ static int launch_hyper(const HyperArgs& a, cudaStream_t stream) {
   if constexpr (S > 0) {
     const int per_thread = (a.width + threads * V - 1) / (threads * V);
     if (a.rows <= kRowCalls && per_thread <= 2) {
-      launch_chained(per_thread == 1 ? hyper_row_kernel<TS, T, S, V, 1> : hyper_row_kernel<TS, T, S, V, 2>,
-                     static_cast<unsigned>(a.rows), threads, 0, stream, a);
+      if (per_thread == 1)
+        launch_chained(hyper_row_kernel<TS, T, S, V, 1>, static_cast<unsigned>(a.rows), threads, 0, stream, a);
+      else
+        launch_chained(hyper_row_kernel<TS, T, S, V, 2>, static_cast<unsigned>(a.rows), threads, 0, stream, a);
       return cudaGetLastError() == cudaSuccess ? 0 : -4;
     }
   }

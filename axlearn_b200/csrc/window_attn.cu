@@ -548,9 +548,10 @@ static int launch_decode(const WindowArgs& a, bool aligned, cudaStream_t stream)
     cfg.numAttrs = static_cast<unsigned>(chain_attribute(attr, 1));
     cudaLaunchKernelEx(&cfg, aligned ? window_decode_kernel<T, GT, LPK, NC, U, true, true>
                                      : window_decode_kernel<T, GT, LPK, NC, U, false, true>, a);
+  } else if (aligned) {
+    launch_chained(window_decode_kernel<T, GT, LPK, NC, U, true, false>, grid, kWdThreads, 0, stream, a);
   } else {
-    launch_chained(aligned ? window_decode_kernel<T, GT, LPK, NC, U, true, false>
-                           : window_decode_kernel<T, GT, LPK, NC, U, false, false>, grid, kWdThreads, 0, stream, a);
+    launch_chained(window_decode_kernel<T, GT, LPK, NC, U, false, false>, grid, kWdThreads, 0, stream, a);
   }
   return cudaGetLastError() == cudaSuccess ? zero_tail<T>(a, stream) : -4;
 }
