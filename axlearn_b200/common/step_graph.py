@@ -5,7 +5,7 @@ eagerly, a step of a small decoder is some 240 launches behind 8 ms of Python, o
 layers of 512, 2 x 333 tokens: 8.7 ms; two layers of 2048, 2 x 2048 tokens: 8.8 ms, 6.5 ms of work on the GPU).  So a
 step that repeats is captured -- forward, backward, clipping, update -- and replayed; what changes from step to step
 on the host (schedules, bias corrections, counters, keys) is computed there each time and handed over in device
-memory.  The two steps take 1.2 and 6.9 ms then, 0.4 ms of it on the host.  Capturing takes some 15 ms once, in the
+memory.  The two steps take 0.8 and 7.1 ms then, 0.4 ms of it on the host.  Capturing takes some 15 ms once, in the
 second step.
 
 When a step is captured: one GPU, nothing in the model that draws random numbers, every layer of a type that is known

@@ -86,7 +86,7 @@ __device__ __forceinline__ void load_state(const float* p, float* v) {
 // Few CTAs (decoding at small batches) are bound by the row of trips to memory, so everything that no other load decides is
 // asked for at the start: the state's first rows, q, k, v, the gate, the decay's weights (of up to kGdRank) and the norm's.
 // A chain of launches over different states, us each, loads where they were used / this (16 heads): 64 x 128, batch 1 5.4 / 4.0,
-// 8 9.2 / 6.4, 64 21.9 / 19.1 (67 MB: 10.2 read and 10.2 written at the copy rate); 128 x 256, batch 1 17.1 / 8.4, 16 26.6 / 16.3.
+// 8 9.2 / 6.4, 64 21.9 / 19.1 (34 MB read and written: 10.2 at the copy rate); 128 x 256, batch 1 17.1 / 8.4, 16 26.6 / 16.3.
 template <typename T, int V>
 __global__ void __launch_bounds__(kGdThreads, 3) gla_decode_kernel(GlaArgs a) {
   chain_link();

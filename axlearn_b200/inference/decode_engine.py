@@ -7,9 +7,9 @@ cache that is rebuilt every step.  On a B200 the step is a fixed, short list of 
 persistent buffers, so the engine:
 
 * keeps per-layer K/V page pools ``[num_pages, page_size, Nkv_local, H]`` resident and appends in
-  place (``rope_append_paged`` writes the rotated key / value of the new token straight into
-  its page slot while producing the rotated query);
-* runs attention over the pages with the split-KV decode kernel, which does the append as well
+  place;
+* runs attention over the pages with the split-KV decode kernel, which also rotates the new
+  token's query and key and writes its key and value straight into their page slot
   (``rope_decode_attention``);
 * packs the projections so that a layer is four GEMMs on the tcgen05 kernel (QKV, output,
   gate|up, down); the residual adds are the GEMMs' accumulate epilogues on one GPU;

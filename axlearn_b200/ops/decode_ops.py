@@ -2,6 +2,7 @@
 
 * ``paged_decode_attention``: one query token per sequence over a paged KV cache.
 * ``rope_append_paged``: RoPE on q/k of the new token + store of k/v into its page slot.
+* ``rope_decode_attention``: both of them in one launch (what a decoding step runs).
 * ``swiglu_packed``: SwiGLU on a ``[rows, 2F]`` (gate | up) GEMM output.
 * ``OneShotAllReduce``: push-based all-reduce over peer memory for latency-bound messages.
 
