@@ -63,7 +63,7 @@ class _Transfers:
     def __init__(self, group, overlap: bool):
         self.group = group
         self.overlap = overlap
-        self._sends: list = []          # (work, tensor): tensors stay alive until the pass ends
+        self._sends: list = []          # (work, tensor): tensors stay alive until the transfer is over
         self._grad_recvs: dict = {}     # micro-batch -> (work, buffer)
 
     def send(self, x: Tensor, dst: int, *, deferred: bool = False) -> None:
@@ -95,6 +95,11 @@ class _Transfers:
             work.wait()
         self._sends.clear()
 
+    def drain_after_backward(self) -> None:
+        """From within a backward pass: ``drain`` when it ends, ahead of the return to who called it.  The graph, and
+        these operations with it, may be gone right after that, and a send that is dropped on its way never arrives."""
+        torch.autograd.Variable._execution_engine.queue_callback(self.drain)  # pylint: disable=protected-access
+
 
 class _Sent(torch.autograd.Function):
     """Sends ``x`` (micro-batch ``i``) to global rank ``dst``; returns a token that keeps the node
@@ -123,6 +128,7 @@ class _Received(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         ctx.transfers.send(g, ctx.src)
+        ctx.transfers.drain_after_backward()
         return None, None, None, None
 
 

@@ -83,6 +83,70 @@ def test_two_stage_pipeline_matches_single_process(tmp_path, schedule, microbatc
         assert torch.allclose(got[r][2], ref_emb, atol=3e-5, rtol=1e-3)
 
 
+def _drop_graph_worker(rank, world, port, q, schedule):
+    """Backward passes whose graph goes right behind them, on a first stage that is late with its receives."""
+    import datetime
+    import gc
+    import time
+
+    from axlearn_b200.common import pipeline
+    from axlearn_b200.common.layers import Linear
+    from axlearn_b200.common.module import functional
+    from axlearn_b200.common.utils import flatten_items
+    from axlearn_b200.parallel.mesh import create_mesh
+
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port), RANK=str(rank), WORLD_SIZE=str(world))
+    dist.init_process_group("gloo", rank=rank, world_size=world, timeout=datetime.timedelta(seconds=30))
+    try:
+        grad_from = pipeline._Transfers.grad_from  # pylint: disable=protected-access
+
+        def late(self, *args):
+            time.sleep(0.1)
+            return grad_from(self, *args)
+
+        pipeline._Transfers.grad_from = late  # pylint: disable=protected-access
+        schedule_cfg = (pipeline.StreamSchedule if schedule == "stream" else pipeline.GPipeSchedule).default_config()
+        layer = pipeline.Pipeline.default_config().set(
+            name="p", layer=Linear.default_config().set(input_dim=64, output_dim=64), num_layers=world,
+            num_microbatches=4, schedule=schedule_cfg)
+        with create_mesh((world,), ("pipeline",)):
+            module = layer.instantiate(parent=None)
+            params = module.initialize_parameters_recursively(torch.tensor([0, 0, 0, 0], dtype=torch.uint32))
+            for _, p in flatten_items(params):
+                p.requires_grad_()
+            x = torch.randn(4096, 64, generator=torch.Generator().manual_seed(0))
+            for _ in range(2):
+                out, _ = functional(module, None, params, [x], is_training=True)
+                (out.square().mean() / world).backward()
+                del out
+                gc.collect()
+                total = torch.ones(1)
+                dist.all_reduce(total)
+        q.put(to_plain((rank, params["layer"]["weight"].grad[0], params["layer"]["weight"].detach()[0])))
+    finally:
+        dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("schedule", ["gpipe", "stream"])
+def test_gradients_arrive_although_the_graph_is_dropped(schedule):
+    world = 2
+    ctx = mp.get_context("spawn")
+    q = ctx.Queue()
+    procs = [ctx.Process(target=_drop_graph_worker, args=(r, world, port, q, schedule))
+             for port in [_free_port()] for r in range(world)]
+    for p in procs:
+        p.start()
+    got = sorted((from_plain(q.get(timeout=60)) for _ in range(world)), key=lambda item: item[0])
+    for p in procs:
+        p.join(timeout=60)
+    assert [p.exitcode for p in procs] == [0] * world
+    weights = [w.clone().requires_grad_() for _, _, w in got]
+    x = torch.randn(4096, 64, generator=torch.Generator().manual_seed(0))
+    (2 * (x @ weights[0] @ weights[1]).square().mean()).backward()
+    for (_, grad, _), w in zip(got, weights):
+        torch.testing.assert_close(grad, w.grad, rtol=1e-4, atol=1e-6)
+
+
 def test_schedules_describe_the_pass():
     from axlearn_b200.common.pipeline import GPipeSchedule, StreamSchedule
 
