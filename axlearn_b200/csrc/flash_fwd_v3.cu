@@ -157,6 +157,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
                                   //      K stage (g + 1) & 1 with ONE commit on it_done[g & 1];
                                   //      the prologue counts as iteration -1
   uint64_t* v_full = bars + 5;    // [2]
+  uint64_t* v_last = bars + 7;    // packed prompts: the values of a sequence's last key tile, other rows among them
   uint64_t* s_full = bars + 9;    // [2] per query tile
   uint64_t* p_full = bars + 11;   // [2] per query tile, 8 arrivals
   uint64_t* pv_done = bars + 13;  // [2] per query tile, completes once
@@ -170,8 +171,9 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int kv_head = head / (p.N / p.Nkv);
   const int t0 = pair * 256;
   const int n_qt = (p.T + 127) / 128;
-  // Packed prompts are one sequence to the tensor maps.  What lies behind a sequence's last key is the next one's, and the
-  // causal mask hides it.
+  // Packed prompts are one sequence to the tensor maps.  What lies behind a sequence's last key is the next one's.  The causal
+  // mask hides its scores, whatever they are; its values would still be multiplied by the zero probabilities, and zero times
+  // an infinity or a NaN is not zero, so they are overwritten with zeros (`v_last`).
   const bool packed = kGated && p.first != nullptr;
   const int seq_len = packed ? min(p.live[batch], p.T) : p.T;
   const int seq_row = packed ? p.first[batch] : 0, map_batch = packed ? 0 : batch;
@@ -202,6 +204,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int g_lo = act0 ? (act1 ? min(lo[0], lo[1]) : lo[0]) : lo[1];
   const int g_hi = max(hi[0], hi[1]);
   const bool any = act0 || act1;
+  const bool foreign_values = packed && any && g_hi * 128 > seq_len;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
@@ -220,6 +223,7 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       mbar_init(&p_full[i], 8);
       mbar_init(&pv_done[i], 1);
     }
+    if (kGated) mbar_init(v_last, 1);
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -270,12 +274,27 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           const int v_need = (g & 1) ? (g - 1) / 2 : (g - 2) / 2;
           if (!mbar_wait(&it_done[g & 1], v_need & 1, p.status, kStatusWaitTimeoutProducer)) break;
         }
-        mbar_arrive_expect_tx(&v_full[st], L::kTile);
+        uint64_t* v_bar = foreign_values && it + 1 == g_hi ? v_last : &v_full[st];
+        mbar_arrive_expect_tx(v_bar, L::kTile);
 #pragma unroll
         for (int j = 0; j < H / 64; ++j)
-          tma_load_4d(smem + L::kV + st * L::kTile + j * L::kSub, &tmap_v, &v_full[st], j * 64, kv_head,
+          tma_load_4d(smem + L::kV + st * L::kTile + j * L::kSub, &tmap_v, v_bar, j * 64, kv_head,
                       seq_row + it * 128, map_batch);
       }
+    }
+  } else if (kGated && warp == 2) {
+    // ------------------------------------------------------------------ values of other sequences
+    // (A row of a tile is 128 contiguous bytes in each of its parts, whatever the swizzle.)
+    if (foreign_values && mbar_wait_warp_relaxed(v_last, 0, p.status, kStatusWaitTimeoutProducer)) {
+      const int st = (g_hi - 1 - g_lo) & 1;
+      uint8_t* tile = smem + L::kV + st * L::kTile;
+#pragma unroll
+      for (int j = 0; j < H / 64; ++j)
+        for (int at = (seq_len - (g_hi - 1) * 128) * 128 + lane * 16; at < L::kSub; at += 32 * 16)
+          *reinterpret_cast<uint4*>(tile + j * L::kSub + at) = make_uint4(0, 0, 0, 0);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&v_full[st]);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer

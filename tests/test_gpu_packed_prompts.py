@@ -87,6 +87,34 @@ def test_window_attention(lengths, dim, window):
     assert torch.equal(cache["key"], want["key"]) and torch.equal(cache["value"], want["value"])
 
 
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+def test_window_attention_keeps_sequences_apart(dim, bad):
+    """Last tiles of 1, 127 and 128 keys, neighbours shorter than a tile, more than one bad neighbour in a tile: nothing that
+    one sequence holds reaches another."""
+    lengths = [129, 300, 5, 3, 255, 128, 1, 40]
+    spec = window_ops.WindowSpec(heads=4, kv_heads=2, dim=dim, vdim=dim, window=100, scale=dim ** -0.5, distance_bias=True,
+                                 gated=True)
+    cols = window_ops.WindowColumns(q=0, k=4 * dim, v=6 * dim, g=8 * dim)
+    packed, live, proj = _packed(lengths, 12 * dim, 4)
+
+    def run(x):
+        cache = {n: torch.zeros(len(lengths), 100, 2, dim, device="cuda", dtype=torch.bfloat16) for n in ("key", "value")}
+        with torch.no_grad():
+            return window_ops.window_attention(packed.pack(x), spec, cols, live=live, cache=cache, packed=packed)
+
+    want, want_cache = run(proj)
+    for spoilt in ([1], [2, 3], [0, 5, 7], [6]):
+        x = proj.clone()
+        x[spoilt] = bad
+        got, cache = run(x)
+        kept = [i for i in range(len(lengths)) if i not in spoilt]
+        for i in kept:
+            rows = slice(packed.first[i].item(), packed.first[i].item() + lengths[i])
+            assert torch.equal(got[:, rows], want[:, rows]), (spoilt, i)
+        assert all(torch.equal(cache[n][kept], want_cache[n][kept]) for n in cache)
+
+
 @pytest.mark.parametrize("family", ["sagisun", "zukitar"])
 def test_served_prompts(family, monkeypatch):
     """The engine's logits after ragged prompts and its steps behind them, packed and padded: the same up to products of
