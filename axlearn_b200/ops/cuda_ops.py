@@ -107,6 +107,7 @@ class _Sigs:
     axb_adamw_scalars = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int,
                          c_float, c_float, c_float, c_void_p]
     axb_pack_rows = [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
+    axb_unpack_rows = [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p]
     axb_store_floats = [c_void_p, c_void_p, c_int, c_void_p]
     axb_embedding_bwd = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
     axb_embedding_bwd_bytes = [c_int, c_int, c_int]

@@ -43,8 +43,13 @@ class PackedRows:
         return x.reshape(-1, x.shape[-1]).index_select(0, self._rows_of[:self.rows])[None]
 
     def unpack(self, x: Tensor) -> Tensor:
-        """``[1, rows, D] -> [B, T, D]``; what padding holds means nothing (it reads the first row of all)."""
-        return x[0].index_select(0, self._row_of).reshape(-1, self.max_len, x.shape[-1])
+        """``[1, rows, D] -> [B, T, D]``, zeros for padding."""
+        x = x.contiguous()
+        out = torch.empty((self.live.shape[0], self.max_len, x.shape[-1]), dtype=x.dtype, device=x.device)
+        cuda_ops._check(cuda_ops.lib().axb_unpack_rows(  # pylint: disable=protected-access
+            x.data_ptr(), out.data_ptr(), self._row_of.data_ptr(), self._row_of.numel(), x.shape[-1] * x.element_size(),
+            cuda_ops._stream()), "axb_unpack_rows")  # pylint: disable=protected-access
+        return out
 
 
 def pack_prompts(live: Tensor, max_len: int) -> Optional[PackedRows]:

@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from axlearn_b200.ops import gla_ops, packed_ops, ssd_ops, window_ops
+from axlearn_b200.ops import gla_ops, latent_ops, packed_ops, ssd_ops, window_ops
 
 pytestmark = pytest.mark.gpu
 
@@ -113,6 +113,48 @@ def test_window_attention_keeps_sequences_apart(dim, bad):
             rows = slice(packed.first[i].item(), packed.first[i].item() + lengths[i])
             assert torch.equal(got[:, rows], want[:, rows]), (spoilt, i)
         assert all(torch.equal(cache[n][kept], want_cache[n][kept]) for n in cache)
+
+
+@pytest.mark.parametrize("width", [1, 7, 8, 264, 2048, 4104])
+def test_unpacked_padding_is_zero(width):
+    lengths = [3, 0, 300, 256, 1]
+    packed, _, x = _packed(lengths, width, 5)
+    got = packed.unpack(packed.pack(x))
+    want = x.clone()
+    for i, n in enumerate(lengths):
+        want[i, n:] = 0
+    assert torch.equal(got, want)
+    rows = packed.pack(x)
+    rows[:, 0] = float("nan")
+    assert not packed.unpack(rows)[1:].isnan().any()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_latent_attention_keeps_sequences_apart(bad):
+    """The first sequence as well, whose rows padding must not hold."""
+    lengths, heads, dim, rot, vdim, rank = [129, 300, 5, 255, 128, 40], 4, 64, 32, 64, 128
+    spec = latent_ops.LatentSpec(heads, dim, rot, vdim, rank, rot, 1000.0, 0.1, 1e-5)
+    cols = latent_ops.LatentColumns(q=0, c=heads * (dim + rot), r=heads * (dim + rot) + rank)
+    packed, live, proj = _packed(lengths, cols.r + rot, 6)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    norm = torch.ones(rank, device="cuda")
+    uk, uv = (0.1 * torch.randn(*n, device="cuda", generator=g).bfloat16() for n in ((rank, heads * dim), (heads * vdim, rank)))
+
+    def run(x):
+        cache = {"latent": torch.zeros(len(lengths), max(lengths), spec.row_width, device="cuda", dtype=torch.bfloat16)}
+        with torch.no_grad():
+            out, cache = latent_ops.latent_attention(packed.unpack(packed.pack(x)), norm, uk, uv, spec, cols, live=live, cache=cache)
+        return packed.pack(out), cache["latent"]
+
+    want, want_cache = run(proj)
+    for spoilt in (0, 2, 4):
+        x = proj.clone()
+        x[spoilt] = bad
+        got, cache = run(x)
+        for i, n in enumerate(lengths):
+            if i != spoilt:
+                rows = slice(packed.first[i].item(), packed.first[i].item() + n)
+                assert torch.equal(got[:, rows], want[:, rows]) and torch.equal(cache[i], want_cache[i]), (spoilt, i)
 
 
 @pytest.mark.parametrize("family", ["sagisun", "zukitar"])
