@@ -268,7 +268,9 @@ class HyperStackedTransformerLayer(BaseStackedTransformerLayer):
         if not all(type(layer) is HyperTransformerLayer and sequence_mixer.takes_packed(layer.children["mixer"])
                    and type(layer.children.get("feed_forward")) in rowwise for layer in self._layers):
             return None
-        return packed_ops.pack_prompts(live, data.shape[1])
+        packed = packed_ops.pack_prompts(live, data.shape[1])
+        # (Without tokens a sequence's output is that of the padding in its first place.)
+        return None if packed is None or packed.some_empty else packed
 
     def extend_step(self, cached_states, data, *, live_step_len=None, page_pool=None, **kwargs):
         """``data [B, steps, D]`` after the tokens seen so far; ``live_step_len [B]``: valid new tokens per

@@ -10,16 +10,17 @@ namespace axb {
 constexpr int kPackThreads = 256;
 
 // Block (tile of 256 positions, sequence).  first [B]: the packed row of a sequence's first token; live_out [B]: its live
-// tokens, clamped to [0, T]; total: of all.  rows_of: the padded row of each packed row; row_of: the packed row of each padded
+// tokens, clamped to [0, T]; total [2]: of all, and whether a sequence has none.  rows_of: the padded row of each packed row; row_of: the packed row of each padded
 // row, -1 for padding.
 __global__ void __launch_bounds__(kPackThreads)
 pack_rows_kernel(const int* __restrict__ live, int B, int T, int* __restrict__ first, int* __restrict__ live_out,
                  int* __restrict__ total, int* __restrict__ rows_of, int* __restrict__ row_of) {
   const int b = blockIdx.y, t = blockIdx.x * kPackThreads + threadIdx.x;
   __shared__ int partial[kPackThreads / 32];
-  int sum = 0;
-  for (int i = threadIdx.x; i < b; i += kPackThreads) sum += min(max(live[i], 0), T);
+  int sum = 0, none = 0;
+  for (int i = threadIdx.x; i < b; i += kPackThreads) sum += min(max(live[i], 0), T), none += live[i] <= 0;
   sum = __reduce_add_sync(0xffffffffu, sum);
+  none = __syncthreads_or(none != 0);
   if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = sum;
   __syncthreads();
   int begin = 0;
@@ -29,7 +30,7 @@ pack_rows_kernel(const int* __restrict__ live, int B, int T, int* __restrict__ f
   if (t == 0) {
     first[b] = begin;
     live_out[b] = n;
-    if (b == B - 1) *total = begin + n;
+    if (b == B - 1) total[0] = begin + n, total[1] = none || n == 0;
   }
   if (t >= T) return;
   const int padded = b * T + t;

@@ -26,17 +26,19 @@ MIN_PADDING = 0.1  # as a share of the rows
 
 class PackedRows:
     """Where the live tokens of a padded batch lie.  ``first``, ``live``: int32 ``[B]``, the first row of a sequence and how
-    many it has; ``rows`` of all; ``max_len``: T of the padded batch.  Waits for ``live`` (int32, on the GPU)."""
+    many it has; ``rows`` of all; ``max_len``: T of the padded batch; ``some_empty``: a sequence has no token, so no row that
+    could stand for it.  Waits for ``live`` (int32, on the GPU)."""
 
     def __init__(self, live: Tensor, max_len: int):
         b = live.shape[0]
         self.max_len = max_len
-        made = torch.empty(2 * b + 1 + 2 * b * max_len, dtype=torch.int32, device=live.device)
-        self.first, self.live, total, self._rows_of, self._row_of = made.split([b, b, 1, b * max_len, b * max_len])
+        made = torch.empty(2 * b + 2 + 2 * b * max_len, dtype=torch.int32, device=live.device)
+        self.first, self.live, total, self._rows_of, self._row_of = made.split([b, b, 2, b * max_len, b * max_len])
         cuda_ops._check(cuda_ops.lib().axb_pack_rows(  # pylint: disable=protected-access
             live.data_ptr(), b, max_len, self.first.data_ptr(), self.live.data_ptr(), total.data_ptr(),
             self._rows_of.data_ptr(), self._row_of.data_ptr(), cuda_ops._stream()), "axb_pack_rows")  # pylint: disable=protected-access
-        self.rows = int(total)
+        self.rows, some_empty = total.tolist()
+        self.some_empty = bool(some_empty)
 
     def pack(self, x: Tensor) -> Tensor:
         """``[B, T, D] -> [1, rows, D]``."""

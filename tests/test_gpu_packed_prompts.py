@@ -194,3 +194,21 @@ def test_where_packing_does_not_pay():
     y = p.pack(x)
     assert y.flatten().tolist() == list(range(2000, 2600)) + list(range(4000, 4700))
     assert torch.equal(p.pack(p.unpack(y)), y)
+
+
+@pytest.mark.parametrize("family", ["sagisun", "zukitar"])
+def test_served_prompt_without_tokens(family, monkeypatch):
+    """Among ragged prompts: its logits are still those of the padding in its first place, bit for bit."""
+    from perf import cases
+    from axlearn_b200.ops import cuda_ops
+
+    case = dict(kind="serve", family=family, size="1B", layers=2 if family == "sagisun" else 3, batch=5, prompt=1011)
+    state = cases.prepare(case, 5)
+    state["lengths"][1:3] = torch.tensor([0, 400])
+    engine = state["engine"]
+    engine.prefill(state["ids"], lengths=state["lengths"])
+    got = engine.logits.clone()
+    monkeypatch.setattr(packed_ops, "pack_prompts", lambda *args: None)
+    engine.prefill(state["ids"], lengths=state["lengths"])
+    assert torch.equal(got, engine.logits)
+    cuda_ops.check_status()
