@@ -37,7 +37,7 @@ from typing import Any, Optional
 import torch
 
 from axlearn_b200.common.utils import flatten_items
-from axlearn_b200.ops import cuda_ops, decode_ops, step_ops
+from axlearn_b200.ops import cuda_ops, decode_ops, packed_ops, step_ops
 
 Tensor = torch.Tensor
 
@@ -432,14 +432,17 @@ class ModuleDecodeEngine(BaseDecodeEngine):
         assert b == self.batch and t <= self.max_len, (prompt_ids.shape, self.batch, self.max_len)
         if lengths is None:
             lengths = torch.full((b,), t, dtype=torch.int32)
-        lengths = lengths.to(device=self.device, dtype=torch.int32)
+        lengths = lengths.to(dtype=torch.int32)
+        on_host = lengths if lengths.device.type == "cpu" else None
+        lengths = lengths.to(device=self.device)
         prompt_ids = prompt_ids.to(self.device)
         per_chunk = max(1, self._prefill_chunk_tokens // t)
         last, picked = [], []
         for b0 in range(0, b, per_chunk):
             b1 = min(b, b0 + per_chunk)
-            states, out = self._call("prefill_states", time_step=lengths[b0:b1],
-                                     input_batch={"input_ids": prompt_ids[b0:b1]}, max_sequence_length=self.max_len)
+            with packed_ops.lengths_known(None if on_host is None else on_host[b0:b1]):
+                states, out = self._call("prefill_states", time_step=lengths[b0:b1],
+                                         input_batch={"input_ids": prompt_ids[b0:b1]}, max_sequence_length=self.max_len)
             hidden = out["hidden_states"]
             for (_, mine), (_, new) in zip(flatten_items(self.states), flatten_items(states)):
                 mine[b0:b1].copy_(new)

@@ -9,6 +9,8 @@ tokens, 6873 / 6111 us; Zukitar, 16 of up to 1000, 11182 / 10013.
 
 from __future__ import annotations
 
+import contextlib
+import threading
 from typing import Optional
 
 import torch
@@ -24,12 +26,27 @@ MIN_TOKENS = 5000
 MIN_PADDING = 0.1  # as a share of the rows
 
 
+_known = threading.local()
+
+
+@contextlib.contextmanager
+def lengths_known(lengths: Optional[Tensor]):
+    """Prompts that the calling thread packs inside have these ``lengths [B]`` (a tensor in host memory; None: they are known
+    on the GPU alone), so that nobody waits for the GPU to tell them."""
+    before = getattr(_known, "lengths", None)
+    _known.lengths = lengths
+    try:
+        yield
+    finally:
+        _known.lengths = before
+
+
 class PackedRows:
     """Where the live tokens of a padded batch lie.  ``first``, ``live``: int32 ``[B]``, the first row of a sequence and how
     many it has; ``rows`` of all; ``max_len``: T of the padded batch; ``some_empty``: a sequence has no token, so no row that
-    could stand for it.  Waits for ``live`` (int32, on the GPU)."""
+    could stand for it.  Waits for ``live`` (int32, on the GPU) unless ``known``, the same in host memory, is given."""
 
-    def __init__(self, live: Tensor, max_len: int):
+    def __init__(self, live: Tensor, max_len: int, known: Optional[Tensor] = None):
         b = live.shape[0]
         self.max_len = max_len
         made = torch.empty(2 * b + 2 + 2 * b * max_len, dtype=torch.int32, device=live.device)
@@ -37,8 +54,11 @@ class PackedRows:
         cuda_ops._check(cuda_ops.lib().axb_pack_rows(  # pylint: disable=protected-access
             live.data_ptr(), b, max_len, self.first.data_ptr(), self.live.data_ptr(), total.data_ptr(),
             self._rows_of.data_ptr(), self._row_of.data_ptr(), cuda_ops._stream()), "axb_pack_rows")  # pylint: disable=protected-access
-        self.rows, some_empty = total.tolist()
-        self.some_empty = bool(some_empty)
+        if known is None:
+            self.rows, some_empty = total.tolist()
+            self.some_empty = bool(some_empty)
+        else:
+            self.rows, self.some_empty = _live_rows(known, max_len), int(known.min()) <= 0
 
     def pack(self, x: Tensor) -> Tensor:
         """``[B, T, D] -> [1, rows, D]``."""
@@ -54,10 +74,24 @@ class PackedRows:
         return out
 
 
+def _live_rows(lengths: Tensor, max_len: int) -> int:
+    return int(lengths.clamp(0, max_len).sum())
+
+
 def pack_prompts(live: Tensor, max_len: int) -> Optional[PackedRows]:
-    """The packing of right-padded prompts of ``live [B]`` tokens, None where it does not pay.  Waits for ``live``."""
+    """The packing of right-padded prompts of ``live [B]`` tokens, None where it does not pay.  Waits for ``live`` unless its
+    values are known (``lengths_known``)."""
     b = live.shape[0]
     if not 2 <= b <= 65535 or b * max_len < MIN_TOKENS or b * max_len >= 1 << 31:
         return None
-    packed = PackedRows(live.to(torch.int32).contiguous(), max_len)
-    return packed if 128 <= packed.rows <= (1 - MIN_PADDING) * b * max_len else None
+
+    def pays(rows):
+        return 128 <= rows <= (1 - MIN_PADDING) * b * max_len
+
+    known = getattr(_known, "lengths", None)
+    if known is not None and known.shape != live.shape:
+        known = None
+    if known is not None and not pays(_live_rows(known, max_len)):
+        return None
+    packed = PackedRows(live.to(torch.int32).contiguous(), max_len, known)
+    return packed if pays(packed.rows) else None

@@ -212,3 +212,48 @@ def test_served_prompt_without_tokens(family, monkeypatch):
     engine.prefill(state["ids"], lengths=state["lengths"])
     assert torch.equal(got, engine.logits)
     cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("lengths,t", [([4000, 4000], 4000), ([4000, 3990, 4000], 4000), ([4000, 8000], 4000), ([600, 700, 90], 2000),
+                                       ([0, 600, 700, -3], 2000), ([100, 2, 3], 2000), ([100, 40], 200)])
+def test_known_lengths_decide_without_a_wait(lengths, t):
+    known = torch.tensor(lengths, dtype=torch.int32)
+    live = known.cuda()
+    want = packed_ops.pack_prompts(live, t)
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        with packed_ops.lengths_known(known):
+            got = packed_ops.pack_prompts(live, t)
+        if want is not None:  # those of another batch are not this one's
+            with packed_ops.lengths_known(known[:1]), pytest.raises(RuntimeError, match="synchroniz"):
+                packed_ops.pack_prompts(live, t)
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
+    assert (got is None) == (want is None)
+    if got is not None:
+        assert (got.rows, got.some_empty) == (want.rows, want.some_empty)
+        assert torch.equal(got.first, want.first) and torch.equal(got.live, want.live)
+
+
+def test_engine_tells_the_lengths_it_knows(monkeypatch):
+    from perf import cases
+
+    case = dict(kind="serve", family="sagisun", size="1B", layers=2, batch=5, prompt=1011)
+    state = cases.prepare(case, 5)
+    engine, ids, lengths = state["engine"], state["ids"], state["lengths"]
+    used, plain = [], packed_ops.pack_prompts
+
+    def pack(*args):
+        used.append((plain(*args), getattr(packed_ops._known, "lengths", None)))  # pylint: disable=protected-access
+        return used[-1][0]
+
+    monkeypatch.setattr(packed_ops, "pack_prompts", pack)
+    logits = []
+    for given in (lengths, lengths.cpu(), lengths.cpu().long(), None):
+        engine.prefill(ids, lengths=given)
+        logits.append(engine.logits.clone())
+    assert torch.equal(logits[0], logits[1]) and torch.equal(logits[0], logits[2])
+    assert [p is not None for p, _ in used] == [True, True, True, False]
+    assert used[0][1] is None and all(torch.equal(k, lengths.cpu()) for _, k in used[1:3])
+    assert used[3][1].tolist() == [1011] * 5
+    assert getattr(packed_ops._known, "lengths", None) is None  # pylint: disable=protected-access
