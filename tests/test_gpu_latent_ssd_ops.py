@@ -285,6 +285,29 @@ def test_equal_logits_choose_the_lower_experts():
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("experts,top", [(4, 4), (12, 3), (32, 4), (65, 3), (300, 8)])
+@pytest.mark.parametrize("tokens,path", [(40, "skinny"), (200, "sorted")])
+def test_tokens_whose_logits_are_not_numbers(experts, top, tokens, path, dtype):
+    """They get some experts, each at most once, and the other tokens the bits that they have without them."""
+    d, f = 64, 64
+    h = _randn(tokens, d, seed=1, dtype=dtype)
+    logits = _randn(tokens, experts, seed=2)
+    gate_up, down = _randn(experts, 2 * f, d, seed=3, dtype=dtype, scale=0.2), _randn(experts, d, f, seed=4, dtype=dtype, scale=0.2)
+    kw = dict(top=top, width=d, hidden=f, gate=hyper_ops.Gate("clamped", limit=1.0), path=path)
+    want = expert_ops._cuda_expert_feed_forward(h, logits, gate_up, down, **kw)
+    bad = logits.clone()
+    bad[3], bad[17], bad[18], bad[36, experts // 2] = float("nan"), float("inf"), float("-inf"), float("nan")
+    bad[30, ::2] = float("nan")
+    x = h.clone()
+    x[3] = float("nan")
+    got = expert_ops._cuda_expert_feed_forward(x, bad, gate_up, down, **kw)
+    touched = [3, 17, 18, 30, 36]
+    others = [t for t in range(tokens) if t not in touched]
+    assert torch.equal(got[others], want[others])
+    assert got[17].isfinite().all() and (got[18] == 0).all()
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("rows", [1, 7, 8, 9, 40, 100])
 @pytest.mark.parametrize("heads,n,k", [(16, 512, 128), (5, 24, 40), (3, 7, 11), (2, 130, 72)])
 def test_head_products(heads, n, k, rows, dtype):
