@@ -15,6 +15,7 @@
 
 #include "chain.cuh"
 #include "mma_sync.cuh"
+#include "order.cuh"
 
 namespace axb {
 
@@ -40,37 +41,25 @@ constexpr int kRtThreads = 256, kRtWarps = kRtThreads / 32, kRtMaxExperts = 1024
 __device__ __forceinline__ float rf(float x) { return x; }
 __device__ __forceinline__ float rf(__nv_bfloat16 x) { return __bfloat162float(x); }
 
-// Torch's order of a maximum: NaN above everything, the lower expert of equals.  (Any total order does; without one the lanes
-// disagree on the winner of a row with NaN, and a later choice finds no expert left.)
-__device__ __forceinline__ bool is_nan(float x) { return (__float_as_uint(x) & 0x7fffffffu) > 0x7f800000u; }
-__device__ __forceinline__ bool beats(float a, int ia, float b, int ib) {
-  if (ia == 0x7fffffff || ib == 0x7fffffff) return ia < ib;  // no expert yet
-  const bool na = is_nan(a), nb = is_nan(b);
-  if (na || nb) return na && (!nb || ia < ib);
-  return a > b || (a == b && ia < ib);
-}
-
 // The warp's lanes hold the logits of experts lane + 32 i; calls put(choice, expert, score) on every lane.
+// Equal logits: the lower expert first; NaN counts as the largest.
 template <int EPL, typename F>
 __device__ __forceinline__ void warp_topk(const float* logits, int experts, int top, F put) {
   const int lane = threadIdx.x & 31;
-  float v[EPL];
+  uint32_t key[EPL];
 #pragma unroll
-  for (int i = 0; i < EPL; ++i) v[i] = lane + 32 * i < experts ? logits[lane + 32 * i] : -INFINITY;
-  uint32_t taken = 0;
+  for (int i = 0; i < EPL; ++i) key[i] = lane + 32 * i < experts ? order_key(logits[lane + 32 * i]) : kNoKey;
   for (int k = 0; k < top; ++k) {
-    float best = -INFINITY;
-    int at = 0x7fffffff;
+    uint32_t best = kNoKey;
+    int at = lane;
 #pragma unroll
     for (int i = 0; i < EPL; ++i)
-      if (!(taken >> i & 1) && lane + 32 * i < experts && beats(v[i], lane + 32 * i, best, at)) best = v[i], at = lane + 32 * i;
-    for (int off = 16; off > 0; off >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, off);
-      const int oa = __shfl_xor_sync(0xffffffffu, at, off);
-      if (beats(ov, oa, best, at)) best = ov, at = oa;
-    }
-    if ((at & 31) == lane) taken |= 1u << (at >> 5);
-    put(k, at, 1.f / (1.f + expf(-best)));
+      if (key[i] > best) best = key[i], at = lane + 32 * i;
+    warp_largest(best, at);
+#pragma unroll
+    for (int i = 0; i < EPL; ++i)
+      if (lane + 32 * i == at) key[i] = kNoKey;  // taken
+    put(k, at, 1.f / (1.f + expf(-key_value(best))));
   }
 }
 

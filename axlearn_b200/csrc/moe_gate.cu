@@ -22,6 +22,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "order.cuh"
+
 namespace axb {
 
 constexpr int kGateMaxPerLane = 8;    // experts per lane: E <= 256
@@ -85,36 +87,31 @@ gate_topk_kernel(GateParams p, int* __restrict__ index, float* __restrict__ gate
     const int64_t tok = static_cast<int64_t>(g) * p.S + s;
     float x[kGateMaxPerLane], mx, lse;
     load_token(p.logits + tok * p.E, p.E, p.cap, lane, x, mx, lse);
-    float score[kGateMaxPerLane];
+    uint32_t key[kGateMaxPerLane];
 #pragma unroll
     for (int i = 0; i < kGateMaxPerLane; ++i) {
       const bool on = lane + 32 * i < p.E;
-      score[i] = !on ? -INFINITY : (p.sigmoid ? 1.f / (1.f + expf(-x[i])) : expf(x[i] - lse));
-      acc[i] += on ? score[i] : 0.f;
+      const float score = p.sigmoid ? 1.f / (1.f + expf(-x[i])) : expf(x[i] - lse);
+      key[i] = on ? order_key(score) : kNoKey;
+      acc[i] += on ? score : 0.f;
     }
     if (lane == 0) lse_out[tok] = lse;
-    // k rounds of warp arg-max; ties go to the smaller expert id (as a stable top-k does).
+    // k rounds of warp arg-max; ties go to the smaller expert id (as a stable top-k does), NaN (of logits that are NaN or
+    // overflow) counts as the largest.
     for (int j = 0; j < p.K; ++j) {
-      float best = -INFINITY;
-      int best_e = 0x7fffffff;
+      uint32_t best = kNoKey;
+      int best_e = lane;
 #pragma unroll
-      for (int i = 0; i < kGateMaxPerLane; ++i) {
-        const int e = lane + 32 * i;
-        if (score[i] > best) best = score[i], best_e = e;  // ascending e within a lane: first wins
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-        if (ob > best || (ob == best && oe < best_e)) best = ob, best_e = oe;
-      }
+      for (int i = 0; i < kGateMaxPerLane; ++i)
+        if (key[i] > best) best = key[i], best_e = lane + 32 * i;  // ascending within a lane: first wins
+      warp_largest(best, best_e);
       if (lane == 0) {
         index[tok * p.K + j] = best_e;
-        gate[tok * p.K + j] = best;
+        gate[tok * p.K + j] = key_value(best);
       }
 #pragma unroll
       for (int i = 0; i < kGateMaxPerLane; ++i)
-        if (lane + 32 * i == best_e) score[i] = -INFINITY;  // taken
+        if (lane + 32 * i == best_e) key[i] = kNoKey;  // taken
     }
   }
   // Per-CTA partial sums of the scores, reduced over the warps in a fixed order.

@@ -1,0 +1,30 @@
+// Largest values among a warp's lanes, in torch's order: NaN above everything, the lower index of equals.  Floats are compared
+// as integers that sort alike: a total order, so that all lanes agree on the winner whatever the values, and one the warp's
+// integer reductions know (two of them instead of five pairs of shuffles).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace axb {
+
+constexpr uint32_t kNoKey = 0;  // below every value's
+
+__device__ __forceinline__ uint32_t order_key(float x) {
+  const uint32_t u = __float_as_uint(x);
+  if ((u & 0x7fffffffu) > 0x7f800000u) return 0xffffffffu;   // NaN
+  if ((u & 0x7fffffffu) == 0) return 0x80000000u;            // zeros are equal
+  return (u >> 31) ? ~u : u | 0x80000000u;
+}
+
+__device__ __forceinline__ float key_value(uint32_t key) {
+  return __uint_as_float((key >> 31) ? key & 0x7fffffffu : ~key);  // NaN for NaN's
+}
+
+// The largest key of the warp and the lowest index that has it.
+__device__ __forceinline__ void warp_largest(uint32_t& key, int& index) {
+  const uint32_t most = __reduce_max_sync(0xffffffffu, key);
+  index = static_cast<int>(__reduce_min_sync(0xffffffffu, key == most ? static_cast<uint32_t>(index) : 0x7fffffffu));
+  key = most;
+}
+
+}  // namespace axb

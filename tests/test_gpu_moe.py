@@ -159,6 +159,25 @@ def test_routing_kernel_matches_torch_statements(g, s, e, k, cap, logit_cap, sig
     assert torch.allclose(logits.grad, ref_logits.grad, atol=2e-5 if logit_cap == 0 else 5e-3, rtol=1e-4)
 
 
+@pytest.mark.parametrize("e,k", [(4, 4), (8, 2), (32, 3), (64, 8), (256, 8)])
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_routing_kernel_with_logits_that_are_not_numbers(e, k, sigmoid):
+    """Such tokens get k different experts; the others route as without them."""
+    from axlearn_b200.ops import moe_ops
+
+    g = torch.Generator(device="cuda").manual_seed(e)
+    logits = torch.randn(2, 150, e, device="cuda", generator=g)
+    bad = logits.clone()
+    bad[0, 3], bad[1, 40], bad[0, 149], bad[1, 0, e // 2] = float("nan"), float("inf"), float("-inf"), float("nan")
+    want = moe_ops.topk_gate(logits, k, 1000, sigmoid=sigmoid)
+    index, gate, slot, counts, _, _ = moe_ops.topk_gate(bad, k, 1000, sigmoid=sigmoid)
+    assert (index >= 0).all() and (index < e).all() and (slot >= 0).all() and counts.sum() == 2 * 150 * k
+    assert all(len(set(row)) == k for row in index.reshape(-1, k).tolist())
+    others = torch.ones(2, 150, dtype=torch.bool, device="cuda")
+    others[[0, 1, 0, 1], [3, 40, 149, 0]] = False
+    assert torch.equal(index[others], want[0][others]) and torch.equal(gate[others], want[1][others])
+
+
 def test_gating_layers_use_the_routing_kernel_and_match_the_step_by_step_path():
     from axlearn_b200.common import prng
     from axlearn_b200.common.mixture_of_experts import Top2Gating, TopKGating
