@@ -257,3 +257,37 @@ def test_engine_tells_the_lengths_it_knows(monkeypatch):
     assert used[0][1] is None and all(torch.equal(k, lengths.cpu()) for _, k in used[1:3])
     assert used[3][1].tolist() == [1011] * 5
     assert getattr(packed_ops._known, "lengths", None) is None  # pylint: disable=protected-access
+
+
+@pytest.mark.parametrize("family", ["sagisun", "zukitar"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_served_prompts_keep_sequences_apart(family, bad):
+    """A token whose embedding is spoilt, in one prompt of a packed batch: the others' logits and states keep their bits."""
+    from perf import cases
+    from axlearn_b200.common.utils import flatten_items
+    from axlearn_b200.ops import cuda_ops
+
+    case = dict(kind="serve", family=family, size="1B", layers=2 if family == "sagisun" else 3, batch=5, prompt=1011)
+    state = cases.prepare(case, 5)
+    engine, ids, lengths = state["engine"], state["ids"].clone(), state["lengths"]
+    table, token = engine.params["emb"]["token_emb"]["weight"], 77
+    row = table[token].clone()
+    ids[ids == token] = 78
+    for spoilt in (0, 2):
+        x = ids.clone()
+        x[spoilt, 5] = token
+
+        def run():
+            engine.prefill(x, lengths=lengths)
+            kept = [i for i in range(5) if i != spoilt]
+            columns = torch.arange(engine.logits.shape[1], device="cuda") != token  # the table is the output product's, too
+            states = [t[kept] for _, t in flatten_items(engine.states) if t.shape[0] == 5]
+            return [engine.logits[kept][:, columns].clone()] + states, engine.logits[spoilt].clone()
+
+        want, _ = run()
+        table[token] = bad
+        got, own = run()
+        table[token] = row
+        assert not own.isfinite().any()
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), spoilt
+    cuda_ops.check_status()
