@@ -595,7 +595,10 @@ _rope_tables: dict = {}
 
 def _rope_table(device: torch.device, floats: int) -> torch.Tensor:
     """Per-device scratch for the (sin, cos) table of one RoPE call (T * H floats).  Calls on
-    one stream run in order, so the table of a finished call may be overwritten by the next."""
+    one stream run in order, so the table of a finished call may be overwritten by the next.  A call that is captured gets
+    its own out of the graph's memory: replays run on other streams, and for as long as the graph lives."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(floats, dtype=torch.float32, device=device)
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
     t = _rope_tables.get(key)
     if t is None or t.numel() < floats:

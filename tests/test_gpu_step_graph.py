@@ -90,6 +90,39 @@ def test_captured_steps_are_the_steps(tmp_path, kv, remat):
     cuda_ops.check_status()
 
 
+def test_captured_steps_share_no_scratch(tmp_path):
+    """Tables of rotations are a graph's own: later, larger calls on the capture's stream and steps of another trainer whose
+    capture got the same stream do not touch them."""
+    from axlearn_b200.ops import cuda_ops
+
+    a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
+    a.train_step(_batch(0)), b.train_step(_batch(0))
+    tables = dict(cuda_ops._rope_tables)  # pylint: disable=protected-access
+    streams, plain = [], torch.cuda.Stream
+
+    def stream(*args, **kwargs):
+        streams.append(plain(*args, **kwargs))
+        return streams[-1]
+
+    torch.cuda.Stream = stream
+    try:
+        a.train_step(_batch(1))
+    finally:
+        torch.cuda.Stream = plain
+    b.train_step(_batch(1))
+    assert _captured(a) and streams
+    assert {k: t.data_ptr() for k, t in cuda_ops._rope_tables.items()} == {k: t.data_ptr() for k, t in tables.items()}  # pylint: disable=protected-access
+    positions = torch.arange(40_000, device="cuda")[None]
+    x = torch.randn(1, 40_000, 1, 64, device="cuda").bfloat16()
+    with torch.cuda.stream(streams[-1]):
+        cuda_ops.rope(x, positions, 1e4)
+    torch.cuda.synchronize()
+    for step in range(2, 5):
+        x, y = a.train_step(_batch(step)), b.train_step(_batch(step))
+        torch.testing.assert_close(x["loss"], y["loss"], rtol=2e-3, atol=0)
+    _same(a, b, 2e-2)
+
+
 def test_other_shapes_hooks_and_states(tmp_path):
     a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
 
