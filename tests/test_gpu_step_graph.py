@@ -177,3 +177,18 @@ def test_not_captured(tmp_path, monkeypatch):
         torch.testing.assert_close(c.train_step(_batch(step))["loss"], d.train_step(_batch(step))["loss"], rtol=2e-3, atol=0)
         assert not _captured(c)
     _same(c, d, 2e-2)
+
+
+def test_layers_are_looked_over_in_place(tmp_path, monkeypatch):
+    """What decides about a capture copies no configuration and asks for no field that is not there (either took longer than
+    half a small step)."""
+    from axlearn_b200.common import config, step_graph
+
+    a = _trainer(tmp_path)
+
+    def refuse(*args, **kwargs):
+        raise AssertionError(args)
+
+    monkeypatch.setattr(config.ConfigBase, "clone", refuse)
+    monkeypatch.setattr(config.ConfigBase, "_unknown", refuse)
+    assert step_graph.capturable(a)
