@@ -11,7 +11,7 @@ second step.
 When a step is captured: one GPU, nothing in the model that draws random numbers, every layer of a type that is known
 to put the same work on the GPU whatever the values (``_LAYERS``), the learner's closed-form AdamW, and a step of the
 same signature just before it: shapes of the batch, addresses of parameters, moments and shadows, and the switches
-that choose kernels. Everything else runs step by step as before, and so does a step under autograd hooks, function
+that choose kernels.  The configurations that a step reads are compared each time.  Everything else runs step by step as before, and so does a step under autograd hooks, function
 transforms, dispatch or function modes, anomaly detection, autocast, a running profiler trace or a caller's own
 capture.  A capture that fails, or that would keep more than a sixteenth of the GPU's memory, is given up for good.
 
@@ -88,6 +88,26 @@ def _layers_known(module) -> bool:
     return all(_layers_known(child) for child in module._children.values())  # pylint: disable=protected-access
 
 
+def _settings(trainer) -> tuple:
+    """What an eager step reads from configurations each time and a captured one does not."""
+
+    def values(cfg):
+        # (Lists by value: they may be changed in place.)
+        return [list(v) if type(v) is list else v for v in cfg._values.values()]  # pylint: disable=protected-access
+
+    def visit(module):
+        out.append((type(module), "forward" in vars(module), values(module._config)))  # pylint: disable=protected-access
+        for child in module._children.values():  # pylint: disable=protected-access
+            visit(child)
+
+    out: list = []
+    visit(trainer.model)
+    learner, cfg = trainer.learner, trainer._config  # pylint: disable=protected-access
+    out.append((type(trainer), cfg.grad_accumulation_steps, trainer._has_param_noise, type(learner),  # pylint: disable=protected-access
+                "update" in vars(learner), learner.ema, values(learner._config)))  # pylint: disable=protected-access
+    return tuple(out)
+
+
 def capturable(trainer) -> bool:
     """Whether the trainer's configuration allows a captured step (what a single call adds: ``_call_allows``)."""
     from axlearn_b200.common.learner import Learner
@@ -145,6 +165,7 @@ class StepGraphs:
 
     def __init__(self):
         self._capturable: Optional[bool] = None
+        self._settings: Optional[tuple] = None  # with which that was found
         self._captured: Optional[_Captured] = None
         self._last: Optional[tuple] = None
         self._captures = 0
@@ -155,8 +176,10 @@ class StepGraphs:
 
     def run(self, trainer, batch: Any) -> Optional[dict]:
         """The step's outputs, or None where the caller has to run it."""
-        if self._capturable is None:
-            self._capturable = capturable(trainer)
+        settings = _settings(trainer)
+        if self._capturable is None or (self._settings is not None and self._settings != settings):
+            self._capturable, self._settings = capturable(trainer), settings
+            self._captured = self._last = None
         if not self._capturable:
             return None
         signature = self._signature(trainer, batch)

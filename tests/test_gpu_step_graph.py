@@ -179,6 +179,42 @@ def test_not_captured(tmp_path, monkeypatch):
     _same(c, d, 2e-2)
 
 
+def test_settings_changed_after_the_capture(tmp_path):
+    """A rate, a constant of a norm, a weight of the loss, a list changed in place, a method of its own: as step by step."""
+    a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
+
+    def both(step, captured):
+        x, y = a.train_step(_batch(step)), b.train_step(_batch(step))
+        torch.testing.assert_close(x["loss"], y["loss"], rtol=2e-3, atol=0)
+        assert _captured(a) == captured
+        return float(x["loss"])
+
+    def change(fn):
+        fn(a), fn(b)
+
+    for step in range(3):
+        both(step, step >= 1)
+    change(lambda t: setattr(t.model.decoder.output_norm._config, "eps", 3.0))
+    before = both(3, False)
+    assert abs(both(4, True) - before) < 2
+    graph = a._step_graphs._captured
+    change(lambda t: t.learner._config.update_rules.append((".*never.*", None)))
+    both(5, False)
+    both(6, True)
+    assert a._step_graphs._captured is not graph
+    a.model.decoder.output_dropout._config.rate = 0.5
+    losses = [float(a.train_step(_batch(7))["loss"]) for _ in range(2)]
+    assert not _captured(a) and losses[0] != losses[1]
+    a.model.decoder.output_dropout._config.rate = 0.0
+    a.train_step(_batch(8)), a.train_step(_batch(8))
+    assert _captured(a)
+    calls = []
+    plain = a.model.forward
+    a.model.forward = lambda *args, **kwargs: (calls.append(0), plain(*args, **kwargs))[1]
+    a.train_step(_batch(9))
+    assert not _captured(a) and calls
+
+
 def test_layers_are_looked_over_in_place(tmp_path, monkeypatch):
     """What decides about a capture copies no configuration and asks for no field that is not there (either took longer than
     half a small step)."""
