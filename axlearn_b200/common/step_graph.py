@@ -8,7 +8,7 @@ on the host (schedules, bias corrections, counters, keys) is computed there each
 memory.  The two steps take 0.8 and 7.1 ms then, 0.4 ms of it on the host.  Capturing takes some 15 ms once, in the
 second step.
 
-When a step is captured: one GPU, nothing in the model that draws random numbers, every layer of a type that is known
+When a step is captured: one GPU, weights that the model reads in bf16, nothing in the model that draws random numbers, every layer of a type that is known
 to put the same work on the GPU whatever the values (``_LAYERS``), the learner's closed-form AdamW, and a step of the
 same signature just before it: shapes of the batch, addresses of parameters, moments and shadows, and the switches
 that choose kernels.  The configurations that a step reads are compared each time.  Everything else runs step by step as before, and so does a step under autograd hooks, function
@@ -207,6 +207,8 @@ class StepGraphs:
         shadows = flatten_items(trainer._shadows)  # pylint: disable=protected-access
         leaves = [t for _, t in shadows if isinstance(t, Tensor)]
         if not _call_allows(trainer, leaves) or not all(isinstance(t, Tensor) and t.is_cuda for _, t in inputs):
+            return None
+        if any(t.is_floating_point() and t.dtype != torch.bfloat16 for t in leaves):
             return None
         adam = trainer.learner.optimizer.fused.locate(state["learner"]["optimizer"])[0]
         held = leaves + [t for tree in (state["model"], adam.mu, adam.nu) for _, t in flatten_items(tree)]

@@ -801,7 +801,7 @@ def multi_tensor_adamw(params, grads, mus, nus, shadows, wd_scales, *, step: int
         if g.dtype not in (torch.bfloat16, torch.float32):
             g = g.float()
         shadow_ptr = None
-        if sh is not None and sh is not p:
+        if sh is not None and sh.data_ptr() != p.data_ptr():  # (32-bit training reads the masters themselves)
             assert sh.dtype == torch.bfloat16 and sh.is_contiguous()
             shadow_ptr = sh.data_ptr()
         if stored is not None:
