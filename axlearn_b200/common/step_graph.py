@@ -13,7 +13,8 @@ to put the same work on the GPU whatever the values (``_LAYERS``), the learner's
 same signature just before it: shapes of the batch, addresses of parameters, moments and shadows, and the switches
 that choose kernels.  The configurations that a step reads are compared each time.  Everything else runs step by step as before, and so does a step under autograd hooks, function
 transforms, dispatch or function modes, anomaly detection, autocast, a running profiler trace or a caller's own
-capture.  A capture that fails, or that would keep more than a sixteenth of the GPU's memory, is given up for good.
+capture.  A model whose gradients alone take more than a sixteenth of the GPU's memory is not tried; a capture that fails,
+or that would keep more than that, is given up for good.
 
 A graph keeps its activations' memory for as long as it lives; a trainer has one at a time and captures a few times at
 most.
@@ -185,8 +186,8 @@ class StepGraphs:
         signature = self._signature(trainer, batch)
         if signature is not None and (self._captured is None or self._captured.signature != signature):
             device = trainer._device  # pylint: disable=protected-access
-            if signature == self._last and self._captures < _MAX_CAPTURES and (
-                    torch.cuda.mem_get_info(device)[0] > _most_memory(device)):
+            if (signature == self._last and self._captures < _MAX_CAPTURES and _gradient_bytes(trainer) <= _most_memory(device)
+                    and torch.cuda.mem_get_info(device)[0] > _most_memory(device)):
                 self._captures += 1
                 self._captured = None  # its memory is given back first
                 try:
@@ -229,6 +230,12 @@ def _copy(dst: list, src: list) -> None:
         by_type[d.dtype][1].append(s)
     for d, s in by_type.values():
         torch._foreach_copy_(d, s)  # pylint: disable=protected-access
+
+
+def _gradient_bytes(trainer) -> int:
+    """What a captured step holds at least: gradients of its own."""
+    return sum(t.numel() * t.element_size() for _, t in flatten_items(trainer._shadows)  # pylint: disable=protected-access
+               if isinstance(t, Tensor) and t.requires_grad)
 
 
 def _most_memory(device: torch.device) -> int:

@@ -179,6 +179,25 @@ def test_not_captured(tmp_path, monkeypatch):
     _same(c, d, 2e-2)
 
 
+def test_gradients_beyond_the_bound_are_not_allocated_twice(tmp_path, monkeypatch):
+    """A model whose gradients do not fit the bound is not captured to find that out."""
+    from axlearn_b200.common import step_graph
+
+    tried = []
+    plain = step_graph._capture
+    monkeypatch.setattr(step_graph, "_capture", lambda *args: (tried.append(0), plain(*args))[1])
+    a = _trainer(tmp_path)
+    held = step_graph._gradient_bytes(a)
+    assert held == sum(2 * t.numel() for _, t in flatten_items(a._shadows))
+    monkeypatch.setattr(step_graph, "_most_memory", lambda device: held - 1)
+    for step in range(3):
+        a.train_step(_batch(step))
+    assert not tried and not _captured(a)
+    monkeypatch.setattr(step_graph, "_most_memory", lambda device: 1 << 30)
+    a.train_step(_batch(3))
+    assert tried and _captured(a)
+
+
 def test_settings_changed_after_the_capture(tmp_path):
     """A rate, a constant of a norm, a weight of the loss, a list changed in place, a method of its own: as step by step."""
     a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
