@@ -13,16 +13,17 @@ to put the same work on the GPU whatever the values (``_LAYERS``), the learner's
 same signature just before it: shapes of the batch, addresses of parameters, moments and shadows, and the switches
 that choose kernels.  The configurations that a step reads are compared each time.  Everything else runs step by step as before, and so does a step under autograd hooks, function
 transforms, dispatch or function modes, anomaly detection, autocast, a running profiler trace or a caller's own
-capture.  A model whose gradients alone take more than a sixteenth of the GPU's memory is not tried; a capture that fails,
-or that would keep more than that, is given up for good.
+capture.  A model whose gradients alone take more than a sixteenth of the GPU's memory is not tried, and a capture that would
+keep more than that is given up.  One that fails is tried again later, twice, and says so in the log.
 
 A graph keeps its activations' memory for as long as it lives; a trainer has one at a time and captures a few times at
-most.
+most for the same parameters.  Steps of two shapes in turn are not captured.
 """
 
 from __future__ import annotations
 
 import dataclasses
+import gc
 import logging
 from typing import Any, Callable, Optional
 
@@ -35,6 +36,9 @@ Tensor = torch.Tensor
 
 _MAX_CAPTURES = 4
 _MEMORY_SHARE = 16
+# Steps to wait after the first, the second, ... capture that failed for a reason that may pass (memory that somebody else
+# held); behind them no more is tried.
+_PAUSES = (100, 1000)
 
 _COMMON = "axlearn_b200.common."
 # Exact types: a subclass may do anything in its forward.
@@ -169,11 +173,12 @@ class StepGraphs:
         self._settings: Optional[tuple] = None  # with which that was found
         self._captured: Optional[_Captured] = None
         self._last: Optional[tuple] = None
-        self._captures = 0
+        self._captures = self._failures = self._pause = 0
 
     def forget(self) -> None:
         """Gives the captured step up, with what it holds: the trainer has got other parameters."""
         self._captured = self._last = None
+        self._captures = self._failures = self._pause = 0
 
     def run(self, trainer, batch: Any) -> Optional[dict]:
         """The step's outputs, or None where the caller has to run it."""
@@ -188,13 +193,23 @@ class StepGraphs:
             device = trainer._device  # pylint: disable=protected-access
             if (signature == self._last and self._captures < _MAX_CAPTURES and _gradient_bytes(trainer) <= _most_memory(device)
                     and torch.cuda.mem_get_info(device)[0] > _most_memory(device)):
-                self._captures += 1
                 self._captured = None  # its memory is given back first
+                if self._pause:
+                    self._pause -= 1
+                    return None
                 try:
                     self._captured = _capture(trainer, batch, signature)
-                except Exception as e:  # pylint: disable=broad-except
+                    self._captures += 1
+                except Refused as e:
                     logging.info("training step not captured: %s", e)
                     self._capturable = False
+                    return None
+                except Exception as e:  # pylint: disable=broad-except
+                    self._failures += 1
+                    self._capturable = self._failures <= len(_PAUSES)
+                    self._pause = _PAUSES[self._failures - 1] if self._capturable else 0
+                    logging.warning("training step not captured (attempt %d), %s: %s", self._failures,
+                                    f"tried again in {self._pause} steps" if self._capturable else "given up", e)
                     return None
         self._last = signature
         if signature is None or self._captured is None or self._captured.signature != signature:
@@ -259,6 +274,8 @@ def _capture(trainer, batch: Any, signature: tuple) -> _Captured:
     before = cuda_ops.launch_count
     graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream(device)
     stream.wait_stream(torch.cuda.current_stream(device))
+    collects = gc.isenabled()
+    gc.disable()  # garbage with CUDA objects in it would be destroyed in the middle, which ends a capture
     try:
         trainer._shadows = leaves  # pylint: disable=protected-access
         # (Not `torch.cuda.graph`, which empties the allocator's cache: what runs next would pay for its memory again.)
@@ -273,6 +290,8 @@ def _capture(trainer, batch: Any, signature: tuple) -> _Captured:
             finally:
                 graph.capture_end()
     finally:
+        if collects:
+            gc.enable()
         trainer._shadows = shadows  # pylint: disable=protected-access
         launches, cuda_ops.launch_count = cuda_ops.launch_count - before, before
         for _, leaf in flatten_items(leaves):

@@ -198,6 +198,48 @@ def test_gradients_beyond_the_bound_are_not_allocated_twice(tmp_path, monkeypatc
     assert tried and _captured(a)
 
 
+def test_a_capture_that_fails_is_tried_again(tmp_path, monkeypatch):
+    import gc
+
+    from axlearn_b200.common import step_graph
+
+    monkeypatch.setattr(step_graph, "_PAUSES", (2, 3))
+    a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
+    failures, collects = [], []
+    plain, update = step_graph._capture, a._apply_update
+
+    def capture(*args):
+        if len(failures) < 2:
+            failures.append(0)
+            raise RuntimeError("out of memory")
+        return plain(*args)
+
+    def apply_update(*args):
+        collects.append(gc.isenabled())
+        return update(*args)
+
+    monkeypatch.setattr(step_graph, "_capture", capture)
+    a._apply_update = apply_update
+    seen = []
+    for step in range(10):
+        x, y = a.train_step(_batch(step)), b.train_step(_batch(step))
+        torch.testing.assert_close(x["loss"], y["loss"], rtol=2e-3, atol=0)
+        seen.append((len(failures), _captured(a)))
+    # Steps 1 and 4 fail, 8 succeeds.
+    assert seen == [(0, False)] + [(1, False)] * 3 + [(2, False)] * 4 + [(2, True)] * 2
+    assert collects == [True] * 8 + [False] and gc.isenabled()
+    _same(a, b, 3e-2)
+    # What will not pass is not tried again, other parameters are.
+    c = _trainer(tmp_path)
+    monkeypatch.setattr(step_graph, "_capture", lambda *args: (failures.append(0), (_ for _ in ()).throw(step_graph.Refused("no")))[1])
+    for step in range(6):
+        c.train_step(_batch(step))
+    assert len(failures) == 3
+    for _ in range(6):
+        a.init(prng.PRNGKey(1))
+        assert a._step_graphs._captures == 0
+
+
 def test_settings_changed_after_the_capture(tmp_path):
     """A rate, a constant of a norm, a weight of the loss, a list changed in place, a method of its own: as step by step."""
     a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
