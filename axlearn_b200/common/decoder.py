@@ -192,9 +192,11 @@ class Decoder(BaseLayer):
 
     @nowrap
     def _reads_positions(self) -> bool:
-        """Whether an ``extend_step`` looks at the tokens' positions outside the layers, which know their own."""
+        """Whether an ``extend_step`` looks at the tokens' positions outside the layers, which know their own.  (A class of its
+        own may, in what it overrides.)"""
         emb = self._children["emb"]
-        return "attention_mask" in self._children or type(emb) is not TransformerTextEmbeddings or "pos_emb" in emb.children
+        return (type(self) is not Decoder or "_forward_for_mode" in vars(self) or "attention_mask" in self._children
+                or type(emb) is not TransformerTextEmbeddings or "pos_emb" in emb.children)
 
     def _attention_mask_biases(self, *, mode, input_ids, positions, segment_ids, cached_states, max_len):
         """Biases of the configured ``attention_mask`` layer (e.g. ALiBi).  Training and prefill see

@@ -55,3 +55,26 @@ def test_beam_search_top_beam_scores_are_consistent():
     lp = torch.log_softmax(logits.float(), dim=-1)
     score = sum(lp[0, t - 1, live[0, t]].item() for t in range(3, 8))
     assert abs(score - out.live_scores[0, 0].item()) < 1e-3 * max(1.0, abs(score))
+
+
+def test_steps_of_a_decoder_of_its_own_have_positions():
+    """A class that overrides the pass finds the tokens' positions in its batch, as in a prompt it may give them."""
+    from axlearn_b200.common.decoder import Decoder
+
+    seen = []
+
+    class Positioned(Decoder):
+        def _forward_for_mode(self, *, mode, input_batch, **kwargs):
+            seen.append(input_batch.get("positions"))
+            return super()._forward_for_mode(mode=mode, input_batch=input_batch, **kwargs)
+
+    model, params = _model()
+    decoder = model.decoder
+    decoder.__class__ = Positioned
+    ids = torch.tensor([[5, 6, 7, 8], [9, 10, 11, 12]])
+    run = lambda method, **kw: functional(decoder, None, params["decoder"], kw, method=method, is_training=False)[0]
+    states, _ = run("prefill_states", time_step=torch.tensor([3, 2], dtype=torch.int32), input_batch={"input_ids": ids},
+                    max_sequence_length=8)
+    states, _ = run("extend_step", cached_states=states, input_ids=ids[:, :1])
+    run("extend_step", cached_states=states, input_ids=ids[:, :2])
+    assert seen[1].tolist() == [[3], [2]] and seen[2].tolist() == [[4, 5], [3, 4]]
