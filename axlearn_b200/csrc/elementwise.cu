@@ -863,10 +863,9 @@ __global__ void store_floats_kernel(float* __restrict__ dst, const StoredFloats 
 }
 
 // ------------------------------------------------------------------------------ sum of squares
-// partial[blockIdx.x] = sum over this block's grid-stride share of x^2 (fixed assignment, so
-// the result is reproducible); the caller adds the partials in index order.
 // Squares of many tensors: a CTA takes one chunk of one of them (chunks of equal size over all tensors), so that a model's
-// gradients are one launch however many small ones there are.  Reading bounds it for large models and the launches for small
+// gradients are one launch however many small ones there are, and leaves its weighted sum in partial[its number]; which
+// elements a thread adds, and in which order, depends on the sizes alone.  Reading bounds it for large models and the launches for small
 // ones (a training step of two layers of 512, 9 gradients: 18 launches are 2 now, 763 -> 738 us).
 constexpr int kSumsqTensors = 64, kSumsqThreads = 512, kSumsqCtas = 148 * 16, kSumsqUnit = 8 * kSumsqThreads;
 
@@ -925,8 +924,9 @@ __global__ void __launch_bounds__(kSumsqThreads) sumsq_kernel(SumsqArgs a, float
   if (threadIdx.x == 0) partial[blockIdx.x] = s * a.weight[t];
 }
 
-// One CTA; a thread adds every blockDim-th partial in order, then the threads' sums meet in a fixed tree (592 partials: one
-// thread alone took 6 us, all of it waiting for one load and one addition after the other; now 1.6).
+// One CTA; a thread adds every blockDim-th partial in order, then the threads' sums meet in a fixed tree: up to 2368 partials
+// and one more per tensor.  (592 of them: one thread alone took 6 us, all of it waiting for one load and one addition after
+// the other; this way 1.6.)
 __global__ void sum_partials_kernel(const float* __restrict__ partial, int n, float* __restrict__ out) {
   __shared__ float red[32];
   float s = 0.f;
