@@ -29,7 +29,9 @@ the kernels depend on it.
 
 from __future__ import annotations
 
+import contextlib
 import dataclasses
+import gc
 import math
 import os
 from typing import Any, Optional
@@ -169,6 +171,30 @@ class BaseDecodeEngine:
         self._check_status()
         return out
 
+    @contextlib.contextmanager
+    def _capture(self):
+        """What is launched inside becomes ``self._graph``.  Unlike ``torch.cuda.graph`` this keeps the allocator's cache where
+        memory is not short: the next prompts take theirs from it again, and do not ask the driver for a dozen segments (0.3 to
+        5 ms each: 8 Sagisun prompts of up to 1500 tokens behind a capture 9.5 ms or, with bad luck, 50; 5.9 from the cache)."""
+        torch.cuda.synchronize(self.device)
+        free, total = torch.cuda.mem_get_info(self.device)
+        if free < total // 16:
+            torch.cuda.empty_cache()
+        graph = torch.cuda.CUDAGraph()
+        collects = gc.isenabled()
+        gc.disable()  # garbage with CUDA objects in it would be destroyed in the middle, which ends a capture
+        try:
+            with torch.cuda.stream(torch.cuda.Stream(device=self.device)):
+                graph.capture_begin()
+                try:
+                    yield
+                finally:
+                    graph.capture_end()
+        finally:
+            if collects:
+                gc.enable()
+        self._graph = graph
+
     def _ensure_graph(self) -> None:
         if self._use_graph and self._graph is None:
             # Warm up on a side stream (lazy module loading, tensor-map encoding), restoring
@@ -183,8 +209,7 @@ class BaseDecodeEngine:
             torch.cuda.current_stream(self.device).wait_stream(s)
             for t, old in zip(buffers, saved):
                 t.copy_(old)
-            self._graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self._graph), cuda_ops.chained_launches():
+            with self._capture(), cuda_ops.chained_launches():
                 # The assertion runs beside the step (behind it: 2.5 us more a step).
                 s.wait_stream(torch.cuda.current_stream(self.device))
                 with torch.cuda.stream(s):

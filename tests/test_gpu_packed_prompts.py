@@ -291,3 +291,27 @@ def test_served_prompts_keep_sequences_apart(family, bad):
         assert not own.isfinite().any()
         assert all(torch.equal(a, b) for a, b in zip(got, want)), spoilt
     cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("short", [False, True])
+def test_prompts_behind_a_capture_find_their_memory(short, monkeypatch):
+    """The capture of the step leaves the allocator's cache alone unless memory is short."""
+    from perf import cases
+
+    case = dict(kind="serve", family="sagisun", size="1B", layers=2, batch=5, prompt=1011)
+    state = cases.prepare(case, 5)
+    engine, want = state["engine"], cases.run(state)
+    engine._graph = None  # pylint: disable=protected-access
+    engine.prefill(state["ids"], lengths=state["lengths"])
+    if short:
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (1 << 20, 1 << 37))
+    torch.cuda.synchronize()
+    freed = torch.cuda.memory_stats()["segment.all.freed"]
+    engine.step_logits(state["continuation"][:, 0])
+    assert (torch.cuda.memory_stats()["segment.all.freed"] > freed) == short
+    made = torch.cuda.memory_stats()["segment.all.allocated"]
+    engine.prefill(state["ids"], lengths=state["lengths"])
+    assert (torch.cuda.memory_stats()["segment.all.allocated"] > made) == short
+    got = cases.run(state)
+    assert torch.equal(got["prompt_logits"], want["prompt_logits"])
+    assert all(torch.equal(a, b) for a, b in zip(got["logits"], want["logits"]))
