@@ -173,7 +173,8 @@ flash_fwd3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int n_qt = (p.T + 127) / 128;
   // Packed prompts are one sequence to the tensor maps.  What lies behind a sequence's last key is the next one's.  The causal
   // mask hides its scores, whatever they are; its values would still be multiplied by the zero probabilities, and zero times
-  // an infinity or a NaN is not zero, so they are overwritten with zeros (`v_last`).
+  // an infinity or a NaN is not zero, so they are overwritten with zeros (`v_last`) by a warp that is idle otherwise, while the
+  // tile's scores are computed.  (8 Sagisun prompts of up to 1500 tokens and 16 steps, us: 5688 without, 5669 with it.)
   const bool packed = kGated && p.first != nullptr;
   const int seq_len = packed ? min(p.live[batch], p.T) : p.T;
   const int seq_row = packed ? p.first[batch] : 0, map_batch = packed ? 0 : batch;

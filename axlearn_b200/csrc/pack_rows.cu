@@ -39,7 +39,9 @@ pack_rows_kernel(const int* __restrict__ live, int B, int T, int* __restrict__ f
 }
 
 // One CTA per padded row: its packed row, zeros for padding (what a kernel multiplies by the zero probabilities of padding
-// must be finite, whatever the sequences hold).
+// must be finite, whatever the sequences hold).  Reads and writes bound it.  16 Zukitar prompts of up to 1000 tokens and 16
+// steps, which unpack the latent layer's projection and the output: 9793 us with an index operator that fills padding with
+// a row, 9768 with this.
 template <typename V>
 __global__ void __launch_bounds__(kPackThreads)
 unpack_rows_kernel(const V* __restrict__ x, V* __restrict__ out, const int* __restrict__ row_of, int64_t width) {

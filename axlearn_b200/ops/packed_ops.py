@@ -3,8 +3,9 @@
 A batch of right-padded prompts ``[B, T]`` of which a third is padding pays a third of its products, norms and activations
 for rows that nobody reads.  Between the embedding and the output norm everything but the sequence mixers works row by row,
 so there the rows are the live tokens alone, ``[1, rows, D]``; the mixers' kernels take the row at which each sequence
-begins.  Served batches of prompts and 16 steps, one B200, padded / packed: Sagisun, 1B widths, 8 prompts of up to 1500
-tokens, 6873 / 6111 us; Zukitar, 16 of up to 1000, 11182 / 10013.
+begins and let nothing of a neighbour into a sequence, be it NaN.  Served batches of prompts and 16 steps, one B200, twenty
+sets of lengths in turn, median and largest us, padded / packed: Sagisun, 1B widths, 8 prompts of up to 1500 tokens, 6841 6868
+/ 5885 6185; Zukitar, 16 of up to 1000, 11325 11670 / 9794 10027.
 """
 
 from __future__ import annotations
@@ -19,8 +20,9 @@ from axlearn_b200.ops import cuda_ops
 
 Tensor = torch.Tensor
 
-# Rows padded / packed of a batch decide: the host has to wait for the lengths, which ends what it had launched ahead, about
-# 0.6 ms.  Batches with three eighths of padding and 16 steps, padded / packed us (Sagisun, Zukitar): 8 x 400 4197 / 4321, 6353
+# Rows padded / packed of a batch decide: where the lengths are known on the GPU alone, the host has to wait for them, which
+# ends what it had launched ahead (up to 0.6 ms; full prompts in four chunks of 16 x 400 with lengths from the host, waited for
+# or not, 9.05 / 8.81 ms).  Batches with three eighths of padding and 16 steps, padded / packed us (Sagisun, Zukitar): 8 x 400 4197 / 4321, 6353
 # / 6538; 32 x 128 4933 / 4882, 8590 / 8566; 16 x 400 5187 / 5048, 8169 / 7950; 8 x 1000 5700 / 5259, 7979 / 7516.
 MIN_TOKENS = 5000
 MIN_PADDING = 0.1  # as a share of the rows
