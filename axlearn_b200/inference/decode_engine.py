@@ -465,8 +465,9 @@ class ModuleDecodeEngine(BaseDecodeEngine):
         last, picked = [], []
         for b0 in range(0, b, per_chunk):
             b1 = min(b, b0 + per_chunk)
-            with packed_ops.lengths_known(None if on_host is None else on_host[b0:b1]):
-                states, out = self._call("prefill_states", time_step=lengths[b0:b1],
+            live = lengths[b0:b1]
+            with packed_ops.lengths_known(live, None if on_host is None else on_host[b0:b1]):
+                states, out = self._call("prefill_states", time_step=live,
                                          input_batch={"input_ids": prompt_ids[b0:b1]}, max_sequence_length=self.max_len)
             hidden = out["hidden_states"]
             for (_, mine), (_, new) in zip(flatten_items(self.states), flatten_items(states)):

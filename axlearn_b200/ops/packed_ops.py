@@ -32,15 +32,26 @@ _known = threading.local()
 
 
 @contextlib.contextmanager
-def lengths_known(lengths: Optional[Tensor]):
-    """Prompts that the calling thread packs inside have these ``lengths [B]`` (a tensor in host memory; None: they are known
-    on the GPU alone), so that nobody waits for the GPU to tell them."""
-    before = getattr(_known, "lengths", None)
-    _known.lengths = lengths
+def lengths_known(live: Tensor, lengths: Optional[Tensor]):
+    """Where the calling thread packs prompts of ``live [B]`` (int32, on the GPU) inside, they have these ``lengths [B]`` (the
+    same in host memory; None: nobody knows them there), so that it does not wait for the GPU to tell them.  Lengths that a
+    model has made of them are others, and are waited for."""
+    before = getattr(_known, "live", None), getattr(_known, "lengths", None)
+    _known.live, _known.lengths = live, lengths
     try:
         yield
     finally:
-        _known.lengths = before
+        _known.live, _known.lengths = before
+
+
+def _known_lengths(live: Tensor) -> Optional[Tensor]:
+    lengths = getattr(_known, "lengths", None)
+    if lengths is None:
+        return None
+    given = _known.live
+    same = (live.data_ptr(), live.shape, live.stride(), live.dtype) == (
+        given.data_ptr(), given.shape, given.stride(), given.dtype)
+    return lengths if same else None
 
 
 class PackedRows:
@@ -90,9 +101,7 @@ def pack_prompts(live: Tensor, max_len: int) -> Optional[PackedRows]:
     def pays(rows):
         return 128 <= rows <= (1 - MIN_PADDING) * b * max_len
 
-    known = getattr(_known, "lengths", None)
-    if known is not None and known.shape != live.shape:
-        known = None
+    known = _known_lengths(live)
     if known is not None and not pays(_live_rows(known, max_len)):
         return None
     packed = PackedRows(live.to(torch.int32).contiguous(), max_len, known)

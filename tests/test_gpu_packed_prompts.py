@@ -222,10 +222,10 @@ def test_known_lengths_decide_without_a_wait(lengths, t):
     want = packed_ops.pack_prompts(live, t)
     torch.cuda.set_sync_debug_mode("error")
     try:
-        with packed_ops.lengths_known(known):
+        with packed_ops.lengths_known(live, known):
             got = packed_ops.pack_prompts(live, t)
         if want is not None:  # those of another batch are not this one's
-            with packed_ops.lengths_known(known[:1]), pytest.raises(RuntimeError, match="synchroniz"):
+            with packed_ops.lengths_known(live[:1], known[:1]), pytest.raises(RuntimeError, match="synchroniz"):
                 packed_ops.pack_prompts(live, t)
     finally:
         torch.cuda.set_sync_debug_mode("default")
@@ -233,6 +233,18 @@ def test_known_lengths_decide_without_a_wait(lengths, t):
     if got is not None:
         assert (got.rows, got.some_empty) == (want.rows, want.some_empty)
         assert torch.equal(got.first, want.first) and torch.equal(got.live, want.live)
+
+
+@pytest.mark.parametrize("more", [1, -50, 400])
+def test_known_lengths_are_not_those_that_a_model_makes_of_them(more):
+    """A prefix that a model puts ahead of the prompts, say."""
+    known = torch.tensor([600, 700, 90], dtype=torch.int32)
+    live = known.cuda()
+    made = live + more
+    want = packed_ops.pack_prompts(made, 2000)
+    with packed_ops.lengths_known(live, known):
+        got = packed_ops.pack_prompts(made, 2000)
+    assert got.rows == want.rows == 1390 + 3 * more and torch.equal(got.live, made)
 
 
 def test_engine_tells_the_lengths_it_knows(monkeypatch):
