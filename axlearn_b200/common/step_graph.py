@@ -8,13 +8,14 @@ on the host (schedules, bias corrections, counters, keys) is computed there each
 memory.  The two steps take 0.8 and 7.1 ms then, 0.4 ms of it on the host.  Capturing takes some 15 ms once, in the
 second step.
 
-When a step is captured: one GPU, weights that the model reads in bf16, nothing in the model that draws random numbers, every layer of a type that is known
-to put the same work on the GPU whatever the values (``_LAYERS``), the learner's closed-form AdamW, and a step of the
-same signature just before it: shapes of the batch, addresses of parameters, moments and shadows, and the switches
-that choose kernels.  The configurations that a step reads are compared each time.  Everything else runs step by step as before, and so does a step under autograd hooks, function
-transforms, dispatch or function modes, anomaly detection, autocast, a running profiler trace or a caller's own
-capture.  A model whose gradients alone take more than a sixteenth of the GPU's memory is not tried, and a capture that would
-keep more than that is given up.  One that fails is tried again later, twice, and says so in the log.
+When a step is captured: one GPU, weights that the model reads in bf16, nothing in the model that draws random numbers,
+every layer of a type that is known to put the same work on the GPU whatever the values (``_LAYERS``), the learner's
+closed-form AdamW, and a step of the same signature just before it: shapes of the batch, addresses of parameters,
+moments and shadows, and the switches that choose kernels.  The configurations that a step reads are compared each time.
+Everything else runs step by step as before, and so does a step under autograd hooks, function transforms, dispatch or
+function modes, anomaly detection, autocast, a running profiler trace or a caller's own capture.  A model whose gradients
+alone take more than a sixteenth of the GPU's memory is not tried, and a capture that would keep more than that is given
+up.  One that fails is tried again later, twice, and says so in the log.
 
 A graph keeps its activations' memory for as long as it lives; a trainer has one at a time and captures a few times at
 most for the same parameters.  Steps of two shapes in turn are not captured.

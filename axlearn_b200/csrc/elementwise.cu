@@ -865,8 +865,8 @@ __global__ void store_floats_kernel(float* __restrict__ dst, const StoredFloats 
 // ------------------------------------------------------------------------------ sum of squares
 // Squares of many tensors: a CTA takes one chunk of one of them (chunks of equal size over all tensors), so that a model's
 // gradients are one launch however many small ones there are, and leaves its weighted sum in partial[its number]; which
-// elements a thread adds, and in which order, depends on the sizes alone.  Reading bounds it for large models and the launches for small
-// ones (a training step of two layers of 512, 9 gradients: 18 launches are 2 now, 763 -> 738 us).
+// elements a thread adds, and in which order, depends on sizes and alignment alone.  Reading bounds it for large models and
+// the launches for small ones (a training step of two layers of 512, 9 gradients: 18 launches are 2 now, 763 -> 738 us).
 constexpr int kSumsqTensors = 64, kSumsqThreads = 512, kSumsqCtas = 148 * 16, kSumsqUnit = 8 * kSumsqThreads;
 
 struct SumsqArgs {

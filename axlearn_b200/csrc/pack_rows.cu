@@ -10,8 +10,8 @@ namespace axb {
 constexpr int kPackThreads = 256;
 
 // Block (tile of 256 positions, sequence).  first [B]: the packed row of a sequence's first token; live_out [B]: its live
-// tokens, clamped to [0, T]; total [2]: of all, and whether a sequence has none.  rows_of: the padded row of each packed row; row_of: the packed row of each padded
-// row, -1 for padding.
+// tokens, clamped to [0, T]; total [2]: of all, and whether a sequence has none.  rows_of: the padded row of each packed
+// row; row_of: the packed row of each padded row, -1 for padding.
 __global__ void __launch_bounds__(kPackThreads)
 pack_rows_kernel(const int* __restrict__ live, int B, int T, int* __restrict__ first, int* __restrict__ live_out,
                  int* __restrict__ total, int* __restrict__ rows_of, int* __restrict__ row_of) {

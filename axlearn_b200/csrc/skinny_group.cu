@@ -199,8 +199,7 @@ __global__ void __launch_bounds__(256) skinny_plain_kernel(SkinnyArgs a) {
 template <int RT>
 static int launch_skinny(const SkinnyArgs& a, int passes, cudaStream_t stream) {
   // Fewer rows than groups: as many groups as can have rows.  CTAs of empty groups cost the full ones their places on the
-  // SMs: a feed-forward of one token over 4 of
-  // 32 experts of 2048 x 1408 33.7 -> 32.3 us, over 8 of 128 52.5 -> 41.9.
+  // SMs: a feed-forward of one token over 4 of 32 experts of 2048 x 1408 33.7 -> 32.3 us, over 8 of 128 52.5 -> 41.9.
   const int groups = a.offsets != nullptr && a.rows < a.groups ? a.rows : a.groups;
   const dim3 grid((a.n + 15) / 16, groups, passes);
   if (a.gate_kind >= 0)

@@ -84,9 +84,9 @@ def reference_gated_linear_attention(proj, a2, a2_bias, norm_scale, spec: GlaSpe
 def gated_linear_attention(proj: Tensor, a2: Tensor, a2_bias: Tensor, norm_scale: Tensor, spec: GlaSpec,
                            cols: GlaColumns, *, start: Optional[Tensor] = None, live: Optional[Tensor] = None,
                            state: Optional[Tensor] = None, packed: Optional[PackedRows] = None):
-    """``(out [B, T, out_width], state [B, H, dim, vdim])``; in- and output ``[1, rows, ...]`` for ``packed`` prompts.  start: int32 ``[B]``, only its sign matters
-    here (negative: the row is not in this step).  live: int32 ``[B]`` valid tokens (None: T).  state: None
-    starts from zero."""
+    """``(out [B, T, out_width], state [B, H, dim, vdim])``; in- and output ``[1, rows, ...]`` for ``packed`` prompts.
+    start: int32 ``[B]``, only its sign matters here (negative: the row is not in this step).  live: int32 ``[B]`` valid
+    tokens (None: T).  state: None starts from zero."""
     tensors = [proj, a2, a2_bias, norm_scale]
     grad = torch.is_grad_enabled() and any(x.requires_grad for x in tensors)
     if dispatch._cuda(*tensors) and not grad and proj.dtype in (torch.bfloat16, torch.float32):  # pylint: disable=protected-access

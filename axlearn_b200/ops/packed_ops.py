@@ -20,10 +20,11 @@ from axlearn_b200.ops import cuda_ops
 
 Tensor = torch.Tensor
 
-# Rows padded / packed of a batch decide: where the lengths are known on the GPU alone, the host has to wait for them, which
-# ends what it had launched ahead (up to 0.6 ms; full prompts in four chunks of 16 x 400 with lengths from the host, waited for
-# or not, 9.05 / 8.81 ms).  Batches with three eighths of padding and 16 steps, padded / packed us (Sagisun, Zukitar): 8 x 400 4197 / 4321, 6353
-# / 6538; 32 x 128 4933 / 4882, 8590 / 8566; 16 x 400 5187 / 5048, 8169 / 7950; 8 x 1000 5700 / 5259, 7979 / 7516.
+# Rows padded / packed of a batch decide: where the lengths are known on the GPU alone, the host has to wait for them,
+# which ends what it had launched ahead (up to 0.6 ms; full prompts in four chunks of 16 x 400 with lengths from the host,
+# waited for or not, 9.05 / 8.81 ms).  Batches with three eighths of padding and 16 steps, padded / packed us (Sagisun,
+# Zukitar): 8 x 400 4197 / 4321, 6353 / 6538; 32 x 128 4933 / 4882, 8590 / 8566; 16 x 400 5187 / 5048, 8169 / 7950;
+# 8 x 1000 5700 / 5259, 7979 / 7516.
 MIN_TOKENS = 5000
 MIN_PADDING = 0.1  # as a share of the rows
 
