@@ -141,8 +141,8 @@ def reference_ssd_mix(proj, w: SsdWeights, spec: SsdSpec, cols: SsdColumns, *, s
 def ssd_mix(proj: Tensor, weights: SsdWeights, spec: SsdSpec, cols: SsdColumns, *, start: Optional[Tensor] = None,
             live: Optional[Tensor] = None, state: Optional[dict] = None, packed: Optional[PackedRows] = None):
     """``(out [B, T, out_width], state)``; both ``[1, rows, ...]`` for ``packed`` prompts.
-    start: int32 ``[B]`` tokens the state has seen (None: zero); negative takes the row out of the step.  live: int32 ``[B]`` valid new tokens (None: T).  state None
-    starts from zero and keeps nothing."""
+    start: int32 ``[B]`` tokens the state has seen (None: zero); negative takes the row out of the step.  live: int32
+    ``[B]`` valid new tokens (None: T).  state None starts from zero and keeps nothing."""
     tensors = [proj] + [getattr(weights, f.name) for f in dataclasses.fields(weights)]
     grad = torch.is_grad_enabled() and any(x.requires_grad for x in tensors)
     if dispatch._cuda(*tensors) and not grad and proj.dtype in (torch.bfloat16, torch.float32):  # pylint: disable=protected-access
