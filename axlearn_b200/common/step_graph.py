@@ -15,7 +15,7 @@ moments and shadows, and the switches that choose kernels.  The configurations t
 Everything else runs step by step as before, and so does a step under autograd hooks, function transforms, dispatch or
 function modes, anomaly detection, autocast, a running profiler trace or a caller's own capture.  A model whose gradients
 alone take more than a sixteenth of the GPU's memory is not tried, and a capture that would keep more than that is given
-up.  One that fails is tried again later, twice, and says so in the log.
+up.  One that fails is tried again later, twice, and says so in the log.  With other parameters or settings all begins anew.
 
 A graph keeps its activations' memory for as long as it lives; a trainer has one at a time and captures a few times at
 most for the same parameters.  Steps of two shapes in turn are not captured.
@@ -174,11 +174,13 @@ class StepGraphs:
         self._settings: Optional[tuple] = None  # with which that was found
         self._captured: Optional[_Captured] = None
         self._last: Optional[tuple] = None
+        self._given_up = False
         self._captures = self._failures = self._pause = 0
 
     def forget(self) -> None:
         """Gives the captured step up, with what it holds: the trainer has got other parameters."""
         self._captured = self._last = None
+        self._given_up = False
         self._captures = self._failures = self._pause = 0
 
     def run(self, trainer, batch: Any) -> Optional[dict]:
@@ -187,7 +189,8 @@ class StepGraphs:
         if self._capturable is None or (self._settings is not None and self._settings != settings):
             self._capturable, self._settings = capturable(trainer), settings
             self._captured = self._last = None
-        if not self._capturable:
+            self._given_up = False
+        if not self._capturable or self._given_up:
             return None
         signature = self._signature(trainer, batch)
         if signature is not None and (self._captured is None or self._captured.signature != signature):
@@ -203,14 +206,14 @@ class StepGraphs:
                     self._captures += 1
                 except Refused as e:
                     logging.info("training step not captured: %s", e)
-                    self._capturable = False
+                    self._given_up = True
                     return None
                 except Exception as e:  # pylint: disable=broad-except
                     self._failures += 1
-                    self._capturable = self._failures <= len(_PAUSES)
-                    self._pause = _PAUSES[self._failures - 1] if self._capturable else 0
+                    self._given_up = self._failures > len(_PAUSES)
+                    self._pause = 0 if self._given_up else _PAUSES[self._failures - 1]
                     logging.warning("training step not captured (attempt %d), %s: %s", self._failures,
-                                    f"tried again in {self._pause} steps" if self._capturable else "given up", e)
+                                    "given up" if self._given_up else f"tried again in {self._pause} steps", e)
                     return None
         self._last = signature
         if signature is None or self._captured is None or self._captured.signature != signature:

@@ -240,6 +240,29 @@ def test_a_capture_that_fails_is_tried_again(tmp_path, monkeypatch):
         assert a._step_graphs._captures == 0
 
 
+@pytest.mark.parametrize("error", ["Refused", "RuntimeError"])
+def test_a_capture_given_up_is_tried_for_other_parameters(tmp_path, monkeypatch, error):
+    from axlearn_b200.common import step_graph
+
+    monkeypatch.setattr(step_graph, "_PAUSES", ())
+    a, plain = _trainer(tmp_path), step_graph._capture
+    kind = step_graph.Refused if error == "Refused" else RuntimeError
+
+    def fail(*args):
+        raise kind("no memory today")
+
+    monkeypatch.setattr(step_graph, "_capture", fail)
+    for step in range(3):
+        a.train_step(_batch(step))
+    monkeypatch.setattr(step_graph, "_capture", plain)
+    a.train_step(_batch(3))
+    assert not _captured(a)
+    a.init(prng.PRNGKey(1))
+    for step in range(2):
+        a.train_step(_batch(step))
+    assert _captured(a)
+
+
 def test_settings_changed_after_the_capture(tmp_path):
     """A rate, a constant of a norm, a weight of the loss, a list changed in place, a method of its own: as step by step."""
     a, b = _trainer(tmp_path), _eager(_trainer(tmp_path))
